@@ -7,6 +7,7 @@ are made in `prepare`.
 """
 import importlib
 import math
+import re
 
 import numpy as np
 import torch
@@ -158,11 +159,16 @@ def _slowest(expr):
     return tc.parse(expr)["out_idx"][-1]
 
 
-def prepare(case, seed):
+def _maker(case, seed):
+    """A function that makes the next input of so many elements, on the GPU."""
     dtype = torch.float64 if case["dtype"] == "f64" else torch.float32
-    code = tc.F64 if case["dtype"] == "f64" else tc.F32
     gen = torch.Generator(device="cuda").manual_seed(seed)
-    make = lambda n: torch.empty(n, dtype=dtype, device="cuda").uniform_(-1.0, 1.0, generator=gen)
+    return lambda n: torch.empty(n, dtype=dtype, device="cuda").uniform_(-1.0, 1.0, generator=gen)
+
+
+def prepare(case, seed):
+    code = tc.F64 if case["dtype"] == "f64" else tc.F32
+    make = _maker(case, seed)
     if case["call"] == "fused":
         lines = _fused_lines(case)
         counts = [_counts(line)[0] for line in lines]
@@ -219,3 +225,51 @@ def tolerance(case):
     p = tc.parse(case["expr"])
     chain = min(math.prod(p["sum_ext"]), 512)
     return {"rel": 7e-7 + 2.8e-8 * chain, "max": 6e-6 + 9e-8 * chain}
+
+
+def _taken_apart(expr):
+    """(indices of the output, of the left and of the right input; extents; operator) of an expression line."""
+    found = re.fullmatch(r"\s*\w+ \[(.*?)\] (\S+) sum\((.*?)\) \* \w+ \[(.*?)\] \* \w+ \[(.*?)\];", expr)
+    sized = lambda text: list(zip(text.split(",")[0::2], map(int, text.split(",")[1::2])))
+    out, summed = sized(found[1]), sized(found[3])
+    return [[i for i, _ in out], found[4].split(","), found[5].split(",")], dict(out + summed), found[2]
+
+
+def _added(expr, flat_c, flat_a, flat_b, only=None):
+    """C op A * B in 64 bits on flat tensors whose first index is the fastest; `only` = (index, first, last) keeps those values of an index."""
+    names, ext, op = _taken_apart(expr)
+    letter = {n: chr(97 + k) for k, n in enumerate(ext)}
+    a, b = (t.double().view([ext[i] for i in reversed(idx)]) for t, idx in ((flat_a, names[1]), (flat_b, names[2])))
+    if only:
+        index, first, last = only
+        a, b = (t.narrow(len(idx) - 1 - idx.index(index), first, last - first) if index in idx else t for t, idx in ((a, names[1]), (b, names[2])))
+    text = ["".join(letter[i] for i in reversed(idx)) for idx in names]
+    product = torch.einsum("%s,%s->%s" % (text[1], text[2], text[0]), a, b).reshape(-1)
+    if op == "=":
+        return product
+    return product.neg_().add_(flat_c) if op == "-=" else product.add_(flat_c)
+
+
+def exact(case, seed):
+    make = _maker(case, seed)
+    if case["call"] == "fused":
+        lines = _fused_lines(case)
+        taken = [_taken_apart(line) for line in lines]
+        counts = [[math.prod(ext[i] for i in idx) for idx in names] for names, ext, _ in taken]
+        c = make(counts[0][0])
+        lefts, rights = [make(n[1]) for n in counts], [make(n[2]) for n in counts]
+        for line, a, b in zip(lines, lefts, rights):
+            c = _added(line, c, a, b)
+        return c
+    names, ext, _ = _taken_apart(case["expr"])
+    counts, only = [math.prod(ext[i] for i in idx) for idx in names], None
+    if case["call"] == "shard":
+        # the first ranks get one value more where the extent does not divide
+        cut, (each, more) = names[0][-1], divmod(ext[names[0][-1]], case["world"])
+        first = case["rank"] * each + min(case["rank"], more)
+        only = (cut, first, first + each + (case["rank"] < more))
+        if only[1] == only[2]:
+            return None
+        counts[0] = counts[0] // ext[cut] * (only[2] - only[1])
+    result = _added(case["expr"], *(make(n) for n in counts), only=only)
+    return result.cpu().numpy() if case["call"] == "host" else result
