@@ -15,6 +15,7 @@
 // (DMMA m8n8k4, same fragment mapping as tc_contract_kernel) and the accumulators are scattered into the box with
 // the term's own (row, col) -> box-offset tables.  After the last term the box is added to C once.
 // fp64 only.  Operator per term: += or -=.
+#include <cuda.h>  // types of the tensor-map encoder only; the entry point is looked up at run time
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,6 +26,7 @@
 #include <string>
 #include <vector>
 
+#include "tc_fused_box.cuh"
 #include "tc_kernels.cuh"
 
 namespace {
@@ -77,7 +79,7 @@ __device__ __forceinline__ uint32_t box_pos(uint32_t e) { return e ^ (((e >> 4) 
 __global__ void __launch_bounds__(kThreads, 2) tc_fused_kernel(const __grid_constant__ FusedArgs p,
                                                                 const __grid_constant__ FusedPtrs ptrs,
                                                                 double* __restrict__ C) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
   double* box = reinterpret_cast<double*>(smem_raw);            // [box_elems], the output's order inside the box
   double* xs = box + kBoxElems;                                  // [kStages][IMG]
   double* ys = xs + kStages * IMG;                               // [kStages][IMG]
@@ -370,6 +372,14 @@ struct tc_fused_plan {
   FusedTerm* d_terms = nullptr;
   int64_t* d_box_off = nullptr;
   std::vector<int64_t*> d_koff;
+  // tc_fused_box_kernel (operands in tiled TMA boxes); box_kernel: the plan's inputs allow it
+  bool box_kernel = false;
+  tcbox::BoxArgs box{};
+  struct BoxDim { int out_pos; int64_t s_in; };
+  std::vector<BoxDim> box_x[kMaxTerms], box_y[kMaxTerms];  // dimensions 1.. of the inputs' maps
+  int32_t* d_pos = nullptr;
+  int* h_status = nullptr;  // host memory the kernel reports a wait that gave up in
+  int grid = 0;
   double flops = 0, bytes_fused = 0, bytes_separate = 0;
   std::string why;
 };
@@ -424,6 +434,91 @@ extern "C" int tc_fused_set_extents(tc_fused_plan* p, int n, const char* const* 
   }
   p->idx_extent = next;
   return TC_OK;
+}
+
+// Whether the plan runs on tc_fused_box_kernel, and what that kernel needs besides the pointers.  Its operands arrive as
+// tiled boxes of rank 5: the contraction must be one index, the fastest of both inputs and of even extent (rows then
+// start on 16 bytes), and an input may carry four output indices.
+static void box_build(tc_fused_plan* p) {
+  using namespace tcbox;
+  const FusedArgs& a = p->args;
+  BoxArgs& b = p->box;
+  b = BoxArgs{};
+  p->box_kernel = false;
+  b.n_terms = a.n_terms;
+  b.rank = a.rank;
+  int bits = 0;
+  for (int i = 0; i < a.rank; ++i) {
+    b.b[i] = a.b[i];
+    b.ext[i] = a.ext[i];
+    b.tiles[i] = a.tiles[i];
+    b.sc[i] = a.sc[i];
+    while ((1u << b.lg[i]) < a.b[i]) ++b.lg[i];
+    bits += (int)b.lg[i];
+  }
+  b.total_boxes = (uint32_t)a.total_boxes;
+  b.spin_limit = TC_SPIN_LIMIT;
+  if (bits > 12) return;
+  for (int k = 0; k < a.n_terms; ++k) {
+    const FusedTerm& T = p->h_terms[k];
+    if (p->terms[k].sum_idx.size() != 1 || T.kfast_x != 2 || T.kfast_y != 2) return;
+    if (p->box_x[k].size() > (size_t)kMapDims || p->box_y[k].size() > (size_t)kMapDims) return;
+    BoxTerm& t = b.term[k];
+    t.kflat = T.kflat;
+    t.bytes = (uint32_t)(T.rows + T.cols) * 128u;
+    t.alpha = T.alpha;
+    for (int d = 0; d < kMapDims; ++d) {
+      t.px[d] = d < (int)p->box_x[k].size() ? (int8_t)p->box_x[k][d].out_pos : (int8_t)-1;
+      t.py[d] = d < (int)p->box_y[k].size() ? (int8_t)p->box_y[k][d].out_pos : (int8_t)-1;
+    }
+  }
+  p->box_kernel = true;
+}
+
+// Hashed box positions of a term's rows (part 0) or columns (part 1).
+static void box_positions(const tc_fused_plan* p, int k, int part, int32_t* pos) {
+  const FusedTerm& T = p->h_terms[k];
+  const uint64_t* coord = part ? T.coord_n : T.coord_m;
+  for (int r = 0; r < kBox; ++r) {
+    if (r >= (part ? T.cols : T.rows)) { pos[r] = -1; continue; }
+    uint32_t e = 0;
+    int sh = 0;
+    for (int i = 0; i < p->args.rank; ++i) { e |= (uint32_t)((coord[r] >> (8 * i)) & 0xff) << sh; sh += (int)p->box.lg[i]; }
+    pos[r] = (int32_t)tcbox::box_hash(e);
+  }
+}
+
+// Rank-5 descriptor of one input: dimension 0 = contraction index, then the output indices it carries; box 16 x b_i.
+static bool encode_box_map(TcTensorMap* out, const void* base, const FusedArgs& a, uint32_t kflat,
+                           const std::vector<tc_fused_plan::BoxDim>& dims_in) {
+  typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static encode_fn fn = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<encode_fn>(f);
+  }();
+  if (!fn || (reinterpret_cast<uintptr_t>(base) & 15)) return false;
+  cuuint64_t dims[5] = {kflat, 1, 1, 1, 1}, strides[4];
+  cuuint32_t box[5] = {16, 1, 1, 1, 1};
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  int r = 1;
+  for (const tc_fused_plan::BoxDim& d : dims_in) {
+    dims[r] = a.ext[d.out_pos];
+    box[r] = a.b[d.out_pos];
+    strides[r - 1] = (cuuint64_t)d.s_in * 8;
+    ++r;
+  }
+  for (; r < 5; ++r) strides[r - 1] = (cuuint64_t)((kflat + 1) / 2 * 2) * 8;  // extent-1 padding: any aligned stride
+  for (int i = 0; i < 4; ++i)
+    if (strides[i] % 16 != 0 || strides[i] >= (cuuint64_t(1) << 40)) return false;
+  return fn(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, const_cast<void*>(base), dims,
+            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Host part of commit: box shape and per-term tables (needs no GPU).
@@ -539,11 +634,14 @@ static int fused_build(tc_fused_plan* p) {
     };
     T.kfast_x = mode_of(e.left_idx);
     T.kfast_y = mode_of(e.right_idx);
+    for (const Cls& c : cm) p->box_x[k].push_back({c.out_pos, c.s_in});
+    for (const Cls& c : cn) p->box_y[k].push_back({c.out_pos, c.s_in});
     double prod = out_elems * (double)kf;
     p->flops += 2.0 * prod;
     p->bytes_fused += 8.0 * (count_l + count_r);
     p->bytes_separate += 8.0 * (2.0 * out_elems + count_l + count_r);
   }
+  box_build(p);
   return TC_OK;
 }
 
@@ -610,6 +708,22 @@ extern "C" int tc_fused_commit(tc_fused_plan* p) {
     TC_CUDA_OK(cudaMemcpy(p->d_box_off, off.data(), off.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
     p->args.box_off = p->d_box_off;
   }
+  if (p->box_kernel) {
+    TC_CUDA_OK(cudaFuncSetAttribute(tcbox::tc_fused_box_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tcbox::box_smem_bytes()));
+    int per_sm = 0, sms = 0;
+    TC_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tcbox::tc_fused_box_kernel, tcbox::kBoxThreads, tcbox::box_smem_bytes()));
+    TC_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    p->grid = (int)std::min<int64_t>((int64_t)std::max(per_sm, 1) * sms, (int64_t)p->args.total_boxes);
+    std::vector<int32_t> pos(p->terms.size() * 2 * kBox);
+    for (size_t k = 0; k < p->terms.size(); ++k)
+      for (int part = 0; part < 2; ++part) box_positions(p, (int)k, part, &pos[(2 * k + part) * kBox]);
+    TC_CUDA_OK(cudaMalloc(&p->d_pos, pos.size() * sizeof(int32_t)));
+    TC_CUDA_OK(cudaMemcpy(p->d_pos, pos.data(), pos.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    TC_CUDA_OK(cudaHostAlloc(&p->h_status, sizeof(int), cudaHostAllocMapped));
+    *p->h_status = 0;
+    TC_CUDA_OK(cudaHostGetDevicePointer(&p->box.status, p->h_status, 0));
+    p->box.pos = p->d_pos;
+  }
   p->device = dev;
   p->committed = true;
   return TC_OK;
@@ -634,6 +748,20 @@ extern "C" int tc_execute_fused(tc_fused_plan* p, void* C, const void* const* A,
     ptrs.y[k] = static_cast<const double*>(B[k]);
   }
   if (reinterpret_cast<uintptr_t>(C) & 7) return TC_ERR_ALIGNMENT;
+  if (p->box_kernel) {
+    if (*static_cast<volatile int*>(p->h_status) != 0) return TC_ERR_DEVICE_WAIT;  // an earlier launch of this plan gave up
+    tcbox::BoxArgs b = p->box;
+    bool ok = true;
+    for (size_t k = 0; ok && k < p->terms.size(); ++k)
+      ok = encode_box_map(&b.x[k], A[k], p->args, b.term[k].kflat, p->box_x[k]) &&
+           encode_box_map(&b.y[k], B[k], p->args, b.term[k].kflat, p->box_y[k]);
+    if (ok) {
+      tcbox::tc_fused_box_kernel<<<(unsigned)p->grid, tcbox::kBoxThreads, tcbox::box_smem_bytes(), static_cast<cudaStream_t>(stream)>>>(
+          b, static_cast<double*>(C));
+      TC_CUDA_OK(cudaGetLastError());
+      return TC_OK;
+    }
+  }
   tc_fused_kernel<<<(unsigned)p->args.total_boxes, kThreads, fused_smem_bytes(p->args.n_terms), static_cast<cudaStream_t>(stream)>>>(
       p->args, ptrs, static_cast<double*>(C));
   TC_CUDA_OK(cudaGetLastError());
@@ -645,6 +773,8 @@ extern "C" void tc_fused_destroy(tc_fused_plan* p) {
   for (int64_t* d : p->d_koff) cudaFree(d);
   if (p->d_terms) cudaFree(p->d_terms);
   if (p->d_box_off) cudaFree(p->d_box_off);
+  if (p->d_pos) cudaFree(p->d_pos);
+  if (p->h_status) cudaFreeHost(p->h_status);
   delete p;
 }
 
@@ -670,7 +800,7 @@ extern "C" int tc_fused_describe(tc_fused_plan* p, char* buf, size_t cap) {
   o << "],\"boxes\":" << q->args.total_boxes << ",\"box_elems\":" << q->args.box_elems << ",\"rows_cols\":[";
   for (size_t k = 0; k < q->h_terms.size(); ++k) o << (k ? "," : "") << "[" << q->h_terms[k].rows << "," << q->h_terms[k].cols << "]";
   o << "],\"flops\":" << q->flops << ",\"bytes\":" << q->bytes_fused << ",\"bytes_term_by_term\":" << q->bytes_separate
-    << ",\"kernel\":\"tc_fused_kernel\",\"launches\":1}";
+    << ",\"kernel\":\"" << (q->box_kernel ? "tc_fused_box_kernel" : "tc_fused_kernel") << "\",\"launches\":1}";
   const std::string s = o.str();
   const size_t n = std::min(cap - 1, s.size());
   std::memcpy(buf, s.data(), n);
