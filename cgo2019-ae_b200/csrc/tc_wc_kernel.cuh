@@ -196,9 +196,12 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
         else decode(p.N, n0 + (i - BM), p.Nflat, &offy_n[i - BM], &unused);
       }
       group_bar_sync(1 + gi, CF::THREADS);
+      int64_t kx = ws_koff(p.koff_x, 0, kend, ptid), ky = ws_koff(p.koff_y, 0, kend, ptid);
       for (int ks = 0; ks < nk; ++ks, ++it) {
         const uint32_t s = it % STAGES;
-        if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.status, 2, p.spin_limit)) return;
+        const int64_t nx = ws_koff(p.koff_x, (uint32_t)(ks + 1) * BK, kend, ptid), ny = ws_koff(p.koff_y, (uint32_t)(ks + 1) * BK, kend, ptid);
+        // (one decision per warp: the loaders below shuffle)
+        if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.status, 2, p.spin_limit))) return;
         double* xs = gstage + s * CF::STAGE_ELEMS;
         double* ys = xs + CF::XIMG;
         const uint32_t k0 = (uint32_t)ks * BK;
@@ -209,8 +212,10 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
             if constexpr (CF::MODEY == LM_TMA_K) tma_load_2d(ys, &p.tmap_y, (int)k0, (int)n0, &full[s]);
           }
         }
-        ws_load<CF, BM, CF::MODEX>(xs, X, offx_m, p.koff_x, k0, kend, ptid, lgx);
-        ws_load<CF, BN, CF::MODEY>(ys, Y, offy_n, p.koff_y, k0, kend, ptid, lgy);
+        ws_load<CF, BM, CF::MODEX>(xs, X, offx_m, kx, ptid, lgx);
+        ws_load<CF, BN, CF::MODEY>(ys, Y, offy_n, ky, ptid, lgy);
+        kx = nx;
+        ky = ny;
         // tests only: one producer thread of CTA 0 never announces its copies of one stage
         if (p.test_fault == 1 && blockIdx.x == 0 && gi == 0 && it == 1 && ptid == 7) continue;
         mbar_arrive_on_copies(&full[s]);

@@ -128,14 +128,18 @@ struct WsCfg {
   static constexpr int CONSUMER_REGS = CONSUMER_REGS_RAW > 224 ? 224 : CONSUMER_REGS_RAW;
 };
 
-// Producer loaders.  A producer thread keeps what does not change inside a stage in
-// registers (its external offsets or its contraction offsets), so that one element
-// costs an add, a predicate and the copy.
+// Producer loaders.  A warp holds the contraction offsets of a stage in registers, one per lane (lane l: k0 + l % 16,
+// -1 beyond the contraction's end), read from the plan's table one stage ahead (ws_koff): a read per element put an L2
+// round trip -- shared memory leaves little L1 -- in front of every batch of copies.  Loaders take what they need by
+// shuffle; an element then costs an add, a sign test and the copy.
+__device__ __forceinline__ int64_t ws_koff(const int64_t* __restrict__ koff, uint32_t k0, uint32_t kend, int lane) {
+  const uint32_t k = k0 + (lane & 15);
+  return k < kend ? koff[k] : -1;
+}
 
 // 16 bytes along the external index, external-major image.
 template <class CF, int ROWS>
-__device__ __forceinline__ void ws_load_ext_vec(double* img, const double* __restrict__ g, const int64_t* s_off,
-                                                const int64_t* __restrict__ koff, uint32_t k0, uint32_t kend, int ptid) {
+__device__ __forceinline__ void ws_load_ext_vec(double* img, const double* __restrict__ g, const int64_t* s_off, int64_t kreg, int ptid) {
   constexpr int LD = ROWS + 4, VPR = ROWS / 2, T = CF::THREADS;
   const uint32_t sbase = smem_u32(img);
   if constexpr (VPR >= T && VPR % T == 0) {
@@ -145,106 +149,95 @@ __device__ __forceinline__ void ws_load_ext_vec(double* img, const double* __res
       const int64_t eo = s_off[ev * 2];
 #pragma unroll 8
       for (int kk = 0; kk < CF::BK; ++kk) {
-        const bool ok = eo >= 0 && k0 + kk < kend;
-        const double* src = ok ? g + eo + koff[k0 + kk] : g;
-        cp_async16(sbase + (uint32_t)(kk * LD + ev * 2) * 8u, src, ok);
+        const int64_t ko = __shfl_sync(0xffffffffu, kreg, kk);
+        const bool ok = (eo | ko) >= 0;
+        cp_async16(sbase + (uint32_t)(kk * LD + ev * 2) * 8u, ok ? g + eo + ko : g, ok);
       }
     }
   } else if constexpr (T % VPR == 0) {
     const int ev = ptid % VPR;
     const int64_t eo = s_off[ev * 2];
 #pragma unroll 8
-    for (int kk = ptid / VPR; kk < CF::BK; kk += T / VPR) {
-      const bool ok = eo >= 0 && k0 + kk < kend;
-      const double* src = ok ? g + eo + koff[k0 + kk] : g;
-      cp_async16(sbase + (uint32_t)(kk * LD + ev * 2) * 8u, src, ok);
+    for (int kb = 0; kb < CF::BK; kb += T / VPR) {
+      const int kk = kb + ptid / VPR;
+      const int64_t ko = __shfl_sync(0xffffffffu, kreg, kk);
+      const bool ok = (eo | ko) >= 0;
+      cp_async16(sbase + (uint32_t)(kk * LD + ev * 2) * 8u, ok ? g + eo + ko : g, ok);
     }
   } else {  // tile widths that neither divide nor are divided by the producer count
     static_assert(VPR * CF::BK % T == 0, "loader shape");
 #pragma unroll 4
-    for (int sl = ptid; sl < VPR * CF::BK; sl += T) {
-      const int ev = sl % VPR, kk = sl / VPR;
+    for (int sb = 0; sb < VPR * CF::BK; sb += T) {
+      const int sl = sb + ptid, ev = sl % VPR, kk = sl / VPR;
       const int64_t eo = s_off[ev * 2];
-      const bool ok = eo >= 0 && k0 + kk < kend;
-      const double* src = ok ? g + eo + koff[k0 + kk] : g;
-      cp_async16(sbase + (uint32_t)(kk * LD + ev * 2) * 8u, src, ok);
+      const int64_t ko = __shfl_sync(0xffffffffu, kreg, kk);
+      const bool ok = (eo | ko) >= 0;
+      cp_async16(sbase + (uint32_t)(kk * LD + ev * 2) * 8u, ok ? g + eo + ko : g, ok);
     }
   }
 }
 
 // 16 bytes along the contraction index, contraction-major image.
 template <class CF, int ROWS>
-__device__ __forceinline__ void ws_load_k_vec(double* img, const double* __restrict__ g, const int64_t* s_off,
-                                              const int64_t* __restrict__ koff, uint32_t k0, uint32_t kend, int ptid) {
+__device__ __forceinline__ void ws_load_k_vec(double* img, const double* __restrict__ g, const int64_t* s_off, int64_t kreg, int ptid) {
   constexpr int KV = CF::BK / 2, T = CF::THREADS;
   static_assert(T % KV == 0 && ROWS % (T / KV) == 0, "loader shape");
   const int kv = ptid % KV;
-  const uint32_t k = k0 + kv * 2;
-  const bool kok = k < kend;
-  const int64_t ko = kok ? koff[k] : 0;
+  const int64_t ko = __shfl_sync(0xffffffffu, kreg, kv * 2);
   const uint32_t sbase = smem_u32(img) + (uint32_t)(kv * 2) * 8u;
 #pragma unroll 8
   for (int r = ptid / KV; r < ROWS; r += T / KV) {
     const int64_t eo = s_off[r];
-    const bool ok = kok && eo >= 0;
-    const double* src = ok ? g + eo + ko : g;
-    cp_async16(sbase + (uint32_t)(r * CF::LDK) * 8u, src, ok);
+    const bool ok = (eo | ko) >= 0;
+    cp_async16(sbase + (uint32_t)(r * CF::LDK) * 8u, ok ? g + eo + ko : g, ok);
   }
 }
 
 // Element copies, external-major image.  lg = log2(lanes walking k): a warp covers 2^lg consecutive k
 // by 32 >> lg consecutive externals (whole 32-byte sectors along the operand's fastest index).
 template <class CF, int ROWS>
-__device__ __forceinline__ void ws_load_elem(double* img, const double* __restrict__ g, const int64_t* s_off,
-                                             const int64_t* __restrict__ koff, uint32_t k0, uint32_t kend, int ptid,
+__device__ __forceinline__ void ws_load_elem(double* img, const double* __restrict__ g, const int64_t* s_off, int64_t kreg, int ptid,
                                              int lg) {
   constexpr int LD = ROWS + 4, WARPS = CF::THREADS / 32;
   const int lane = ptid & 31, warp = ptid >> 5;
   const uint32_t sbase = smem_u32(img);
   if (lg == 0) {  // lanes walk the external index: few externals, all 16 k per thread
     constexpr int EG = ROWS / 32;  // groups of 32 externals
-#pragma unroll
     for (int eg = warp; eg < EG; eg += WARPS) {
       const int el = eg * 32 + lane;
       const int64_t eo = s_off[el];
 #pragma unroll 8
       for (int kk = 0; kk < CF::BK; ++kk) {
-        const bool ok = eo >= 0 && k0 + kk < kend;
-        const double* src = ok ? g + eo + koff[k0 + kk] : g;
-        cp_async8(sbase + (uint32_t)(kk * LD + el) * 8u, src, ok);
+        const int64_t ko = __shfl_sync(0xffffffffu, kreg, kk);
+        const bool ok = (eo | ko) >= 0;
+        cp_async8(sbase + (uint32_t)(kk * LD + el) * 8u, ok ? g + eo + ko : g, ok);
       }
     }
   } else {  // 4 lanes walk k, 8 lanes walk the external index: 4 contraction offsets live in registers
     const int lk = lane & 3, le = lane >> 2;
     int64_t ko[4];
-    bool kok[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t k = k0 + q * 4 + lk;
-      kok[q] = k < kend;
-      ko[q] = kok[q] ? koff[k] : 0;
-    }
+    for (int q = 0; q < 4; ++q) ko[q] = __shfl_sync(0xffffffffu, kreg, q * 4 + lk);
 #pragma unroll 4
     for (int eg = warp; eg < ROWS / 8; eg += WARPS) {
       const int el = eg * 8 + le;
       const int64_t eo = s_off[el];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const bool ok = kok[q] && eo >= 0;
-        const double* src = ok ? g + eo + ko[q] : g;
-        cp_async8(sbase + (uint32_t)((q * 4 + lk) * LD + el) * 8u, src, ok);
+        const bool ok = (eo | ko[q]) >= 0;
+        cp_async8(sbase + (uint32_t)((q * 4 + lk) * LD + el) * 8u, ok ? g + eo + ko[q] : g, ok);
       }
     }
   }
 }
 
+// kreg: this lane's contraction offset of the stage (ws_koff).
 template <class CF, int ROWS, int MODE>
-__device__ __forceinline__ void ws_load(double* img, const double* __restrict__ g, const int64_t* s_off,
-                                        const int64_t* __restrict__ koff, uint32_t k0, uint32_t kend, int ptid, int lg) {
-  if constexpr (MODE == LM_EXT_VEC) ws_load_ext_vec<CF, ROWS>(img, g, s_off, koff, k0, kend, ptid);
-  else if constexpr (MODE == LM_K_VEC) ws_load_k_vec<CF, ROWS>(img, g, s_off, koff, k0, kend, ptid);
+__device__ __forceinline__ void ws_load(double* img, const double* __restrict__ g, const int64_t* s_off, int64_t kreg, int ptid, int lg) {
+  if constexpr (MODE == LM_EXT_VEC) ws_load_ext_vec<CF, ROWS>(img, g, s_off, kreg, ptid);
+  else if constexpr (MODE == LM_K_VEC) ws_load_k_vec<CF, ROWS>(img, g, s_off, kreg, ptid);
   else if constexpr (MODE == LM_TMA_K) return;  // fetched by the producer's TMA copy
-  else ws_load_elem<CF, ROWS>(img, g, s_off, koff, k0, kend, ptid, lg);
+  else ws_load_elem<CF, ROWS>(img, g, s_off, kreg, ptid, lg);
 }
 
 // Fragment pair of the DMMA mapping: tile elements (e, e+1) at contraction index k.
@@ -395,9 +388,13 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
       };
       const bool pf = accumulate && p.prefetch_dist != 0 && !sliced;
       if (pf && !p.c_stream) prefetch_c();
+      int64_t kx = ws_koff(p.koff_x, kbeg, kend, ptid), ky = ws_koff(p.koff_y, kbeg, kend, ptid);
       for (int ks = 0; ks < nk; ++ks, ++it) {
         const uint32_t s = it % STAGES;
-        if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.status, 2, p.spin_limit)) return;
+        // offsets of the next stage: in flight while this one is copied
+        const int64_t nx = ws_koff(p.koff_x, kbeg + (uint32_t)(ks + 1) * BK, kend, ptid), ny = ws_koff(p.koff_y, kbeg + (uint32_t)(ks + 1) * BK, kend, ptid);
+        // (one decision per warp: the loaders below shuffle)
+        if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.status, 2, p.spin_limit))) return;
         double* xs = gstage + s * CF::STAGE_ELEMS;
         double* ys = xs + CF::XIMG;
         const uint32_t k0 = kbeg + (uint32_t)ks * BK;
@@ -408,8 +405,10 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
             if constexpr (CF::MODEY == LM_TMA_K) tma_load_2d(ys, &p.tmap_y, (int)k0, (int)n0, &full[s]);
           }
         }
-        ws_load<CF, BM, CF::MODEX>(xs, X, offx_m, p.koff_x, k0, kend, ptid, lgx);
-        ws_load<CF, BN, CF::MODEY>(ys, Y, offy_n, p.koff_y, k0, kend, ptid, lgy);
+        ws_load<CF, BM, CF::MODEX>(xs, X, offx_m, kx, ptid, lgx);
+        ws_load<CF, BN, CF::MODEY>(ys, Y, offy_n, ky, ptid, lgy);
+        kx = nx;
+        ky = ny;
         // tests only: one producer thread of CTA 0 never announces its copies of one stage, so that stage stays
         // "not full" and every thread that depends on it runs out of polls
         if (p.test_fault == 1 && blockIdx.x == 0 && gi == 0 && it == 1 && ptid == 7) continue;
