@@ -93,10 +93,11 @@ struct TcKernelArgs {
   uint32_t spin_limit;  // polls a bounded wait may take before it gives up
   int32_t test_fault;   // tests only: 1 = the persistent kernel's producers leave one stage unannounced
   int32_t out_bufs, img_sets, ring_stages;  // persistent tcgen05 kernel: how its shared memory is carved (set at launch)
-  const int64_t* koff_x;  // [Kflat] offset of flattened contraction index k inside X
+  const int64_t* koff_x;  // [Kflat] offset of flattened contraction index k inside X (-1: no such value, persistent fp64 kernels)
   const int64_t* koff_y;  // [Kflat] the same inside Y
   int32_t lanes_k_x;  // element-wise loader: consecutive lanes that walk k (1 = lanes walk the external index)
   int32_t lanes_k_y;
+  int32_t kstep_x, kstep_y;  // ... and the step between the positions that neighbouring lanes take (1 or 4; persistent fp64 kernels)
   int32_t vec_c;     // contiguous output elements a thread may touch with one access (1, 2 or 4)
   int32_t beta;      // 1: C is read and accumulated into; 0: C is overwritten
   double alpha;      // +1 or -1
@@ -155,6 +156,7 @@ struct tc_plan {
   struct TcHostPipe* host = nullptr;  // device buffers, streams and slab plans of the host-pointer path
   size_t ws_bytes = 0;
   int sm_count = TC_DEFAULT_SMS;  // multiprocessors of the device the plan is committed on
+  bool block_k = true;  // the planner may cut the contraction into 4 x 4 blocks (see tc_plan_build)
   int passes = 1;   // sequential launches over consecutive contraction ranges, each accumulating into C
   std::mutex* host_mu = nullptr;  // serialises tc_execute_host on this plan (its device buffers are shared)
   int64_t size_c = 0, size_a = 0, size_b = 0;  // elements spanned (max offset + 1)

@@ -266,6 +266,29 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     }
   }
 
+  // K, fp64: where each input's fastest index is a contraction index, but not the same one, either order of the
+  // flattened contraction walks one of the two in 8-byte pieces of different sectors.  Both digits are cut by four and
+  // the low parts put first -- (4 of X's, 4 of Y's, the rest): a K step of sixteen is then a 4 x 4 block of which both
+  // inputs read whole sectors.  Extents that four does not divide are rounded up; positions beyond them have offset -1
+  // in the tables, which the loaders of the persistent fp64 kernels (and only they) turn into zeros.
+  int64_t kcut_x = 0, kcut_y = 0;  // extents of the two digits that were cut (0: none)
+  if (p->dtype == TC_F64 && p->block_k && x_k_unit && y_k_unit && !dk.empty() && dk[0].s_in == 1 && dk[0].s_out != 1 &&
+      dk.size() + 2 <= (size_t)TC_MAX_DIMS) {
+    for (size_t j = 1; j < dk.size(); ++j) {
+      if (dk[j].s_out != 1) continue;
+      const Dim x = dk[0], y = dk[j];
+      kcut_x = x.extent;
+      kcut_y = y.extent;
+      std::vector<Dim> r = {{4, x.s_in, x.s_out}, {4, y.s_in, y.s_out}};
+      r.push_back({(x.extent + 3) / 4, x.s_in * 4, x.s_out * 4});
+      r.push_back({(y.extent + 3) / 4, y.s_in * 4, y.s_out * 4});
+      for (size_t i = 1; i < dk.size(); ++i)
+        if (i != j) r.push_back(dk[i]);
+      dk = r;
+      break;
+    }
+  }
+
   TcKernelArgs& a = p->args;
   std::memset(&a, 0, sizeof(a));
   int64_t mf = 1, nf = 1, kf = 1;
@@ -289,6 +312,10 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       r /= kd.extent[d];
       ox += c * kd.s_in[d];
       oy += c * kd.s_out[d];
+    }
+    if (kcut_x > 0) {
+      const int64_t vx = k % 4 + 4 * (k / 16 % kd.extent[2]), vy = k / 4 % 4 + 4 * (k / 16 / kd.extent[2] % kd.extent[3]);
+      if (vx >= kcut_x || vy >= kcut_y) ox = oy = -1;
     }
     p->h_koff_x[k] = ox;
     p->h_koff_y[k] = oy;
@@ -331,6 +358,13 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   };
   loader(a.M, true, &c.vec_x, &c.kvec_x, &a.lanes_k_x);
   loader(a.N, false, &c.vec_y, &c.kvec_y, &a.lanes_k_y);
+  a.kstep_x = a.kstep_y = 1;
+  if (kcut_x > 0) {
+    // Y's unit stride is the second digit: its lanes walk every fourth position; pairs of k along X must not straddle its end
+    a.lanes_k_y = 32 / es;
+    a.kstep_y = 4;
+    if (kcut_x % V != 0) c.kvec_x = false;
+  }
   // An operand is a plain 2-D matrix (k fastest, then the flattened external index at a constant pitch)
   // when it has one fused contraction dimension of stride 1 and its external dimensions are contiguous
   // among themselves: then a tile of the flattened class is a box, which TMA can fetch (rows 16 bytes apart or more).
@@ -509,9 +543,29 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   // Persistent kernels do not split K, except the fp64 reduce-add kernel: on request (forced tile and split_k), or
   // where the planner kept it for a problem of few tiles (about four work items per SM, slices of at least 16 steps).
   const bool ws_kernel = c.math == TC_MATH_DMMA && c.variant == 2;
+  if (kcut_x > 0 && !(c.math == TC_MATH_DMMA && persistent)) {  // kernels that know no holes in the contraction
+    p->block_k = false;
+    const int st = tc_plan_build(p, why);
+    p->block_k = true;
+    return st;
+  }
   if (persistent && ws_kernel && p->opt.split_k > 1) ksplit = std::min<int64_t>(p->opt.split_k, ksteps);
   else if (persistent && ws_kernel && slice_persistent)
-    ksplit = std::max<int64_t>(1, std::min<int64_t>((4 * sms + tiles - 1) / tiles, ksteps / 16));
+  {
+    // Work items (slice, tile) are dealt to two groups per SM: as many slices as fill whole rounds of them.  One item
+    // more than a round costs a round (312 x 296 outputs: 15 tiles in 40 slices are 600 items on 296 groups, 3 rounds for
+    // 2.03 rounds of work; 39 slices are 2 rounds).  The first number of rounds that leaves under 5 % of the groups
+    // idle, else the best of four.
+    const int64_t slots = 2 * sms;
+    double best_fill = 0;
+    for (int64_t rounds = 1; rounds <= 4 && best_fill < 0.95; ++rounds) {
+      const int64_t ks = std::min<int64_t>(rounds * slots / tiles, ksteps / 16);
+      if (ks < 1) continue;
+      const int64_t items = ks * tiles, used = (items + slots - 1) / slots;
+      const double fill = (double)items / (double)(used * slots);
+      if (fill > best_fill) { best_fill = fill; ksplit = ks; }
+    }
+  }
   else if (persistent) ksplit = 1;
   else if (p->opt.split_k > 1) ksplit = std::min<int64_t>(p->opt.split_k, ksteps);
   else if (p->opt.split_k == 0 && tiles * 2 <= sms && ksteps >= 16)

@@ -180,7 +180,8 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
     // ------------------------------------------------------------ producer ----
     reg_dec<CF::PRODUCER_REGS>();
     const int ptid = tid - (CWARPS + gi * PW) * 32;
-    const int lgx = p.lanes_k_x == 1 ? 0 : 2, lgy = p.lanes_k_y == 1 ? 0 : 2;
+    // element copies: 0 = lanes walk the external index, else the step between the positions of the 4 lanes that walk k
+    const int lgx = p.lanes_k_x == 1 ? 0 : p.kstep_x, lgy = p.lanes_k_y == 1 ? 0 : p.kstep_y;
     uint32_t it = 0, titer = 0;
     for (uint32_t tile = first; tile < total; tile += step, ++titer) {
       // Two table sets used alternately: the barrier below is passed only when every producer of the group has

@@ -193,15 +193,15 @@ __device__ __forceinline__ void ws_load_k_vec(double* img, const double* __restr
   }
 }
 
-// Element copies, external-major image.  lg = log2(lanes walking k): a warp covers 2^lg consecutive k
-// by 32 >> lg consecutive externals (whole 32-byte sectors along the operand's fastest index).
+// Element copies, external-major image.  kstep 0: lanes walk the external index.  kstep 1 or 4: four lanes walk k in
+// steps of kstep (where its 32-byte sectors lie) and eight the external index.
 template <class CF, int ROWS>
 __device__ __forceinline__ void ws_load_elem(double* img, const double* __restrict__ g, const int64_t* s_off, int64_t kreg, int ptid,
-                                             int lg) {
+                                             int kstep) {
   constexpr int LD = ROWS + 4, WARPS = CF::THREADS / 32;
   const int lane = ptid & 31, warp = ptid >> 5;
   const uint32_t sbase = smem_u32(img);
-  if (lg == 0) {  // lanes walk the external index: few externals, all 16 k per thread
+  if (kstep == 0) {  // lanes walk the external index: few externals, all 16 k per thread
     constexpr int EG = ROWS / 32;  // groups of 32 externals
     for (int eg = warp; eg < EG; eg += WARPS) {
       const int el = eg * 32 + lane;
@@ -214,10 +214,10 @@ __device__ __forceinline__ void ws_load_elem(double* img, const double* __restri
       }
     }
   } else {  // 4 lanes walk k, 8 lanes walk the external index: 4 contraction offsets live in registers
-    const int lk = lane & 3, le = lane >> 2;
+    const int kl = (lane & 3) * kstep, kq = kstep == 1 ? 4 : 1, le = lane >> 2;
     int64_t ko[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) ko[q] = __shfl_sync(0xffffffffu, kreg, q * 4 + lk);
+    for (int q = 0; q < 4; ++q) ko[q] = __shfl_sync(0xffffffffu, kreg, q * kq + kl);
 #pragma unroll 4
     for (int eg = warp; eg < ROWS / 8; eg += WARPS) {
       const int el = eg * 8 + le;
@@ -225,7 +225,7 @@ __device__ __forceinline__ void ws_load_elem(double* img, const double* __restri
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const bool ok = (eo | ko[q]) >= 0;
-        cp_async8(sbase + (uint32_t)((q * 4 + lk) * LD + el) * 8u, ok ? g + eo + ko[q] : g, ok);
+        cp_async8(sbase + (uint32_t)((q * kq + kl) * LD + el) * 8u, ok ? g + eo + ko[q] : g, ok);
       }
     }
   }
@@ -359,7 +359,8 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
     // ------------------------------------------------------------ producer ----
     reg_dec<CF::PRODUCER_REGS>();
     const int ptid = tid - 2 * CF::CONSUMER_THREADS - gi * CF::THREADS;
-    const int lgx = p.lanes_k_x == 1 ? 0 : 2, lgy = p.lanes_k_y == 1 ? 0 : 2;
+    // element copies: 0 = lanes walk the external index, else the step between the positions of the 4 lanes that walk k
+    const int lgx = p.lanes_k_x == 1 ? 0 : p.kstep_x, lgy = p.lanes_k_y == 1 ? 0 : p.kstep_y;
     uint32_t it = 0, titer = 0;
     for (uint32_t tile = first; tile < total; tile += step, ++titer) {
       const uint32_t par = titer & 1;

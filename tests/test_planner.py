@@ -266,3 +266,13 @@ def test_operands_that_are_matrices_are_marked_as_boxes(pkg):
     assert flags("C [a,64,b,8,c,512] += sum(d,64) * A [d,a,b] * B [d,c];", pkg.F32)[0]
     assert not flags("C [a,64,b,8,c,512] += sum(d,64) * A [d,b,a] * B [d,c];", pkg.F32)[0]
     assert flags("C [a,64,b,8,c,512] += sum(d,64) * A [a,b,d] * B [d,c];", pkg.F32)[2]
+
+
+def test_blocked_contractions_name_every_value_once(pkg):
+    """Two inputs that start with different contraction indices: 4 x 4 blocks of K, rounded up, with holes."""
+    for c, d in ((64, 64), (61, 66), (4, 130), (63, 5)):
+        p = _plan(pkg, "t3 [a,2048,b,2048] += sum(c,%d,d,%d) * t2 [c,a,d] * v2 [d,b,c];" % (c, d)).describe()
+        assert p["kernel"].startswith("dmma_w") and [k["extent"] for k in p["K"][:2]] == [4, 4]
+        assert p["Kflat"] == (c + 3) // 4 * 4 * ((d + 3) // 4 * 4)
+    small = _plan(pkg, "t3 [a,20,b,20] += sum(c,6,d,7) * t2 [c,a,d] * v2 [d,b,c];").describe()
+    assert small["Kflat"] == 42   # kernels that know no holes keep the plain order
