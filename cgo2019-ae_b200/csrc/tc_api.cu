@@ -203,6 +203,37 @@ static bool encode_output_map(TcTensorMap* out, const void* base, const TcOutMap
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same output as the boxes of the output-resident kernel's cut tiles (TcBoxMap).
+static bool encode_box_output_map(TcTensorMap* out, const void* base, const TcBoxMap& o) {
+  typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static encode_fn fn = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<encode_fn>(f);
+  }();
+  if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || o.rank < 1 || o.rank > 5) return false;
+  cuuint64_t dims[5] = {1, 1, 1, 1, 1}, strides[4];
+  cuuint32_t box[5] = {1, 1, 1, 1, 1};
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  for (int d = 0; d < o.rank; ++d) {
+    dims[d] = o.ext[d];
+    box[d] = o.box[d];
+    if (d > 0) strides[d - 1] = (cuuint64_t)o.stride[d] * 8;
+    if (box[d] > 256) return false;
+  }
+  for (int d = std::max(o.rank, 1); d < 5; ++d) strides[d - 1] = d > 1 ? strides[d - 2] * dims[d - 1] : (dims[0] + 1) / 2 * 16;  // extent-1 padding
+  for (int i = 0; i < 4; ++i)
+    if (strides[i] % 16 != 0 || strides[i] >= (cuuint64_t(1) << 40)) return false;
+  return fn(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, const_cast<void*>(base), dims,
+            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int tc_kernel_shape(const TcKernelChoice& c, int* threads, int* smem_bytes, int* bk) {
   if (bk) *bk = TC_BK;
   tc_inst_fn fn = pick_inst(c);
@@ -278,8 +309,8 @@ int tc_launch_contraction(const tc_plan& p, const TcKernelArgs& args, void* C, c
     // The C-resident kernel moves whole output tiles as boxes of the rank-5 view of C: the view must exist and the
     // base must be 16-byte aligned.  Otherwise the same tiles run on the persistent kernel that reaches C through
     // reduce-adds or plain read-modify-writes.
-    const bool ok = c.tma_ct && p.opt.tma != 1 && p.opt.tma != 2 &&
-                    encode_output_map(&a.tmap_ct, C, a.cmap, (uint32_t)a.bm, 2, (uint32_t)a.bn / 2);
+    const bool ok = c.box_c && p.opt.tma != 1 && p.opt.tma != 2 && encode_box_output_map(&a.tmap_ct, C, a.cbox);
+    if (ok) a.c_tensor = 0;
     if (!ok) {
       TcKernelChoice alt = c;
       alt.variant = 2;

@@ -74,6 +74,27 @@ struct TcOutMap {
   int64_t stride[2];   // element strides of ext[]
 };
 
+// How the tiles of the persistent fp64 kernels cut a class's flattened index.  The class is read as three digits: e0
+// values of the fastest, e1 of the next (1: none), and the rest; a tile holds b0 x b1 values of the first two (b0 * b1
+// rows at most, row r being value r % b0 of the first and r / b0 of the second) and one of the rest; t0 and t1 tiles lie
+// along them.  b1 = 1 with e0 the whole class is the plain range of the flattened index.
+struct TcCut {
+  uint32_t b0, b1, e0, e1, t0, t1;
+};
+
+// The output as a tensor of rank <= 5 in which a cut tile is one box (output-resident kernel).  Dimension 0 is the M
+// class's first digit; slot[] says at which dimension the others are (0: absent): N's first and second digit, M's
+// second, then up to two dimensions that the rest of M and of N consist of (mr / nr: extent of the first of them).  One
+// rest dimension of each class may share a dimension of the box map where the two are neighbours in C (mr0 == nr0): its
+// coordinate is m_step times the one plus n_step times the other.
+struct TcBoxMap {
+  int32_t rank;
+  uint32_t ext[5], box[5];
+  int64_t stride[5];   // elements
+  int8_t n0, n1, m1, mr0, mr1, nr0, nr1;
+  uint32_t mr, nr, m_step, n_step;
+};
+
 // Everything a kernel launch needs besides the three tensor pointers.
 // "M" is the external class of operand X (the one holding the output's fastest
 // index after the planner's optional operand swap), "N" the class of operand Y.
@@ -82,6 +103,9 @@ struct TcKernelArgs {
   uint32_t Mflat, Nflat, Kflat;
   uint32_t tiles_m, tiles_n;
   uint32_t mblock_w;  // persistent kernels walk the tiles in column blocks of this many M tiles (0: M fastest over all of M)
+  TcCut mcut, ncut;    // persistent fp64 kernels: the index ranges of a tile
+  TcBoxMap cbox;       // ... and, for the output-resident kernel, the tile as a box of C
+  int32_t rows_across_x, rows_across_y;  // element copies: lanes walk the second digit of the cut (where the operand's sectors lie)
   int32_t bm, bn;    // CTA tile of the chosen kernel
   int32_t c_mode;    // 0: read-modify-write epilogue, 1: accumulators start from C,
                      // 2: bulk asynchronous reduce-add from shared memory (persistent kernels)
@@ -110,7 +134,7 @@ struct TcKernelArgs {
                          // kernel has room to stage a whole tile, else as 1
   TcOutMap cmap;         // ... the view of C they are boxes of
   TcTensorMap tmap_c;    // its rank-5 descriptor with box (warp rows, 1, 8, 1, 1)
-  TcTensorMap tmap_ct;   // the same tensor with box (bm, 2, bn / 2, 1, 1)
+  TcTensorMap tmap_ct;   // the same tensor with box (bm, 2, bn / 2, 1, 1); output-resident kernel: cbox
   int* status;       // device word: 0, or the code of a wait that ran out of polls (persistent kernels)
 };
 
@@ -127,6 +151,7 @@ struct TcKernelChoice {
   bool tma_xe, tma_ye;  // ... with the flattened external index fastest and k at a constant pitch (fp32 persistent kernel)
   bool tma_c;           // a warp's 8-row output batch is a box of a rank-5 tensor over C
   bool tma_ct;          // ... and so is a whole bm x bn tile
+  bool box_c;           // a cut tile is a box of C (args.cbox)
 };
 
 struct TcHostPipe;
@@ -156,6 +181,7 @@ struct tc_plan {
   struct TcHostPipe* host = nullptr;  // device buffers, streams and slab plans of the host-pointer path
   size_t ws_bytes = 0;
   int sm_count = TC_DEFAULT_SMS;  // multiprocessors of the device the plan is committed on
+  int box_order = -1;    // the M class is ordered for the cut tiles of the output-resident kernel: its dimension that comes second (see tc_plan_build)
   bool block_k = true;  // the planner may cut the contraction into 4 x 4 blocks (see tc_plan_build)
   int passes = 1;   // sequential launches over consecutive contraction ranges, each accumulating into C
   std::mutex* host_mu = nullptr;  // serialises tc_execute_host on this plan (its device buffers are shared)

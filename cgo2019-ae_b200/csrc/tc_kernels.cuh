@@ -249,6 +249,20 @@ __device__ __forceinline__ void decode(const TcDims& d, uint32_t flat, uint32_t 
 // whole sweep over N, and a few tiles of Y -- instead of sweeping ALL of X once per row of tiles, which for large
 // outputs pushes the operands out of L2 behind the stream of C (measured: 26.6 -> 22.2 TFLOP/s as the output grew
 // from 4 to 33 GB).
+// Flattened index of row r of tile number t of a cut class (persistent fp64 kernels), or 0xffffffff beyond the tile or
+// the class.
+struct CutTile { uint32_t v0, v1, rest; };
+__device__ __forceinline__ CutTile cut_tile(const TcCut& c, uint32_t t) {
+  const uint32_t q0 = t / c.t0, q1 = q0 / c.t1;
+  return {(t - q0 * c.t0) * c.b0, (q0 - q1 * c.t1) * c.b1, q1};
+}
+__device__ __forceinline__ uint32_t cut_flat(const TcCut& c, const CutTile& t, uint32_t r) {
+  const uint32_t i1 = c.b1 == 1 ? 0u : r / c.b0, i0 = r - i1 * c.b0;
+  const uint32_t v0 = t.v0 + i0, v1 = t.v1 + i1;
+  if (i0 >= c.b0 || i1 >= c.b1 || v0 >= c.e0 || v1 >= c.e1) return 0xffffffffu;
+  return v0 + c.e0 * (v1 + c.e1 * t.rest);
+}
+
 __device__ __forceinline__ void tile_coords(const TcKernelArgs& p, uint32_t tile, uint32_t* tm, uint32_t* tn) {
   const uint32_t w = p.mblock_w;
   if (w == 0) { *tm = tile % p.tiles_m; *tn = tile / p.tiles_m; return; }

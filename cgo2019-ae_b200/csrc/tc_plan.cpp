@@ -129,6 +129,114 @@ void out_box_view(const TcKernelArgs& a, int es, int bm, int bn, TcOutMap* map, 
   *per_tile = ne.size() == 1 || ne[0] % bn == 0;
 }
 
+// Cut tiles of the output-resident kernel: how its bm x bn tile is laid over the output so that it is one box of a
+// rank-<=5 view of C.  Per class either the dimensions fused as far as they are contiguous in C, of which a tile takes a
+// range of the first, or the planner's own dimensions, of which it takes ranges of the first two -- what an output with
+// short runs needs (24-element runs: 5 of them make 120 of 128 rows).  Every even b0 and every c0 is tried; the score is
+// the number of tiles (rows that a tile leaves unused cost as much as used ones) times a penalty for short pieces: of C
+// (b0 elements, or b0 * c0 where the next index of C is N's first) and of an operand whose fastest index is external.
+struct BoxPlan {
+  bool ok = false;
+  double score = 0, tiles = 0;
+  TcCut m{}, n{};
+  TcBoxMap map{};
+  int across_x = 0, across_y = 0;
+};
+BoxPlan plan_boxes(const std::vector<Dim>& dm, const std::vector<Dim>& dn, uint32_t bm, uint32_t bn) {
+  BoxPlan best;
+  if (dm.empty() || dm[0].s_out != 1 || dm[0].extent % 2 != 0) return best;
+  for (const std::vector<Dim>* l : {&dm, &dn})
+    for (const Dim& d : *l)
+      if ((d.s_out != 1 && d.s_out % 2 != 0) || d.s_out <= 0 || d.s_out >= (int64_t(1) << 36) || d.extent >= (int64_t(1) << 31)) return best;
+  auto fuse_out = [](const std::vector<Dim>& l) {
+    std::vector<Dim> r;
+    for (const Dim& d : l) {
+      if (!r.empty() && d.s_out == r.back().s_out * r.back().extent) r.back().extent *= d.extent;
+      else r.push_back(d);
+    }
+    return r;
+  };
+  auto unit_at = [](const std::vector<Dim>& l) {
+    for (size_t i = 0; i < l.size(); ++i)
+      if (l[i].extent > 1 && l[i].s_in == 1) return (int)i;
+    return -1;
+  };
+  auto product = [](const std::vector<Dim>& l, size_t from) {
+    int64_t r = 1;
+    for (size_t i = from; i < l.size(); ++i) r *= l[i].extent;
+    return r;
+  };
+  auto piece = [](double bytes) { return bytes >= 256 ? 1.0 : bytes >= 128 ? 1.02 : bytes >= 64 ? 1.08 : bytes >= 32 ? 1.25 : 1.7; };
+  auto gather = [](int64_t run) { return run >= 4 ? 1.0 : run >= 2 ? 1.15 : 1.4; };
+  const int ux = unit_at(dm), uy = unit_at(dn);
+  const std::vector<Dim> fm = fuse_out(dm), fn = fuse_out(dn);
+  for (int two_m = 0; two_m < 2; ++two_m)
+    for (int two_n = 0; two_n < 2; ++two_n) {
+      const std::vector<Dim>&lm = two_m ? dm : fm, &ln = two_n ? dn : fn;
+      if ((two_m && dm.size() < 2) || (two_n && dn.size() < 2)) continue;
+      const size_t m_rest = two_m ? 2 : 1, n_rest = two_n ? 2 : 1;
+      if (lm.size() > m_rest + 2 || ln.size() > n_rest + 2) continue;
+      // six dimensions fit where the one left of each class are neighbours in C and share a dimension of the map
+      const bool shared = lm.size() + ln.size() == 6 && lm.size() == m_rest + 1 && ln.size() == n_rest + 1 &&
+                          lm.back().extent * ln.back().extent < (int64_t(1) << 31) &&
+                          (lm.back().s_out == ln.back().s_out * ln.back().extent || ln.back().s_out == lm.back().s_out * lm.back().extent);
+      if (lm.size() + ln.size() > 5 && !shared) continue;
+      const int64_t e0 = lm[0].extent, e1 = two_m ? lm[1].extent : 1, f0 = ln.empty() ? 1 : ln[0].extent, f1 = two_n ? ln[1].extent : 1;
+      const int64_t rest = product(lm, m_rest) * product(ln, ln.empty() ? 0 : n_rest);
+      for (uint32_t b0 = std::min<int64_t>(bm, e0); b0 >= 2; b0 -= 2) {
+        const int64_t t0 = (e0 + b0 - 1) / b0;
+        const int64_t t1 = two_m ? (e1 + bm / b0 - 1) / (bm / b0) : 1;
+        const uint32_t b1 = two_m ? (uint32_t)((e1 + t1 - 1) / t1) : 1;
+        for (uint32_t c0 = std::min<int64_t>(bn, f0); c0 >= 1; --c0) {
+          const int64_t s0 = (f0 + c0 - 1) / c0;
+          const int64_t s1 = two_n ? (f1 + bn / c0 - 1) / (bn / c0) : 1;
+          const uint32_t c1 = two_n ? (uint32_t)((f1 + s1 - 1) / s1) : 1;
+          const double tiles = (double)(t0 * t1) * (double)(s0 * s1) * (double)rest;
+          if (tiles >= 2.0e9) continue;
+          const bool adjacent = b0 == e0 && !ln.empty() && ln[0].s_out == e0;
+          double score = tiles * piece(8.0 * b0 * (adjacent ? c0 : 1));
+          if (ux >= 0) score *= gather(ux == 0 ? b0 : ux == 1 && two_m ? b1 : 1);
+          if (uy >= 0) score *= gather(uy == 0 ? c0 : uy == 1 && two_n ? c1 : 1);
+          if (best.ok && score >= best.score) continue;
+          best.ok = true;
+          best.score = score;
+          best.tiles = tiles;
+          best.m = {b0, b1, (uint32_t)e0, (uint32_t)e1, (uint32_t)t0, (uint32_t)t1};
+          best.n = {c0, c1, (uint32_t)f0, (uint32_t)f1, (uint32_t)s0, (uint32_t)s1};
+          best.across_x = ux == 1 && two_m && b1 > 1 ? (int)b1 : 0;
+          best.across_y = uy == 1 && two_n && c1 > 1 ? (int)c1 : 0;
+          TcBoxMap& o = best.map;
+          o = TcBoxMap{};
+          o.mr = o.nr = 1;
+          auto add = [&](const Dim& d, uint32_t box) {
+            o.ext[o.rank] = (uint32_t)d.extent;
+            o.stride[o.rank] = d.s_out;
+            o.box[o.rank] = box;
+            return (int8_t)o.rank++;
+          };
+          add(lm[0], b0);
+          if (!ln.empty()) o.n0 = add(ln[0], c0);
+          if (two_n) o.n1 = add(ln[1], c1);
+          if (two_m) o.m1 = add(lm[1], b1);
+          if (shared) {
+            const bool m_first = lm.back().s_out < ln.back().s_out;
+            Dim both = m_first ? lm.back() : ln.back();
+            o.m_step = m_first ? 1 : (uint32_t)both.extent;
+            o.n_step = m_first ? (uint32_t)both.extent : 1;
+            both.extent *= m_first ? ln.back().extent : lm.back().extent;
+            o.mr0 = o.nr0 = add(both, 1);
+            continue;
+          }
+          if (lm.size() > m_rest) { o.mr0 = add(lm[m_rest], 1); o.mr = (uint32_t)lm[m_rest].extent; }
+          if (lm.size() > m_rest + 1) o.mr1 = add(lm[m_rest + 1], 1);
+          if (ln.size() > n_rest) { o.nr0 = add(ln[n_rest], 1); o.nr = (uint32_t)ln[n_rest].extent; }
+          if (ln.size() > n_rest + 1) o.nr1 = add(ln[n_rest + 1], 1);
+        }
+      }
+    }
+  return best;
+}
+
 // The staged output layout of the fp32 kernels: a tile's rows split into runs of E0 elements that are contiguous in
 // the output (E0 a multiple of 4, tiles 16-byte aligned); `n_adjacent`: consecutive n are adjacent in the output
 // inside blocks of N's fastest extent, so a run and its n leave as one chunk.  Returns E0, or 0 where bulk copies do
@@ -243,7 +351,25 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       dn = fuse(dn);
     }
   }
-  if (p->dtype == TC_F64 && !x_k_unit && dm.size() > 1 && dm[0].s_in != 1 && dm[0].s_out == 1 && dm[0].extent % 4 == 0) {
+  // The output-resident kernel's tiles are cut over two of M's dimensions instead (plan_boxes): for it the dimensions stay
+  // whole, the one that comes second chosen by the cost model below.
+  const std::vector<Dim> dm_whole = dm;
+  auto box_dims = [&](int second) {
+    std::vector<Dim> r = dm_whole;
+    if (second > 1) std::rotate(r.begin() + 1, r.begin() + second, r.begin() + second + 1);
+    return r;
+  };
+  auto best_boxes = [&](uint32_t bm, uint32_t bn, int* order) {
+    BoxPlan best;
+    for (int second = 1; second < std::max<int>(2, (int)dm_whole.size()); ++second) {
+      if (p->box_order >= 0 && second != p->box_order) continue;
+      const BoxPlan q = plan_boxes(box_dims(second), dn, bm, bn);
+      if (q.ok && (!best.ok || q.score < best.score)) { best = q; *order = second; }
+    }
+    return best;
+  };
+  if (p->box_order >= 0) dm = box_dims(p->box_order);
+  else if (p->dtype == TC_F64 && !x_k_unit && dm.size() > 1 && dm[0].s_in != 1 && dm[0].s_out == 1 && dm[0].extent % 4 == 0) {
     for (size_t j = 1; j < dm.size(); ++j) {
       if (dm[j].s_in != 1 || dm[j].extent < 4 || dm[j].extent % 4 != 0) continue;
       if (dm.size() + 2 > (size_t)TC_MAX_DIMS) break;
@@ -435,23 +561,38 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       const double clk = 1.9e9, flop_per_clk = 37.0e12 / 148.0 / clk, byte_per_clk = 6.5e12 / 148.0 / clk;
       const double kpad = (double)((kf + 3) / 4 * 4);
       double best = 0;
+      // Outputs whose rows are shorter than a consumer warp's leave the reduce-add kernels element by element (their
+      // epilogue reads and writes C through registers, a round trip per batch); the resident tile takes them as boxes.
+      int64_t run_c = 0;
+      if (a.M.n > 0 && a.M.s_out[0] == 1) {
+        run_c = a.M.extent[0];
+        for (int d = 1; d < a.M.n && a.M.s_out[d] == run_c; ++d) run_c *= a.M.extent[d];
+      }
+      const bool short_runs = a.vec_c < 4 || run_c < 64;
       p->why.clear();
       for (const Cand& k : cands) {
         if (!tc_kernel_exists(TC_F64, TC_MATH_DMMA, k.bm, k.bn, k.variant)) continue;
-        if (k.variant == 3) {  // needs whole tiles to be boxes of a rank-5 view of C, and nothing that pins the epilogue
-          TcOutMap view;
-          bool per_warp = false, per_tile = false;
-          out_box_view(a, es, k.bm, k.bn, &view, &per_warp, &per_tile);
-          if (!per_tile || p->opt.tma == 1 || p->opt.tma == 2 || p->opt.c_path != 0) continue;
+        double tiles_c = (double)((mf + k.bm - 1) / k.bm) * (double)((nf + k.bn - 1) / k.bn);
+        if (p->box_order >= 0 && k.variant != 3) continue;  // the choice is made; M's dimensions are in its order
+        double out_elems = (double)k.bm * k.bn, idle = k.idle;
+        int order = -1;  // M's dimension that comes second
+        if (k.variant == 3) {  // needs tiles that are boxes of a rank-5 view of C, and nothing that pins the epilogue
+          if (p->opt.tma == 1 || p->opt.tma == 2 || p->opt.c_path != 0) continue;
           // ... and pays only where the output traffic is the longer side: per output element the memory system moves
           // 16 bytes while the pipe does 2 K flops, equal near K = 46.  On long contractions its single consumer group
           // and two producer warps measured a third slower than the two-group kernel (21 against 31 TFLOP/s).
-          if (2.0 * es / 6.5e12 < 0.85 * 2.0 * (double)kf / 37.0e12) continue;
+          const double limit = short_runs ? 3.0 : 1.0;
+          if (p->box_order < 0 && limit * 2.0 * es / 6.5e12 < 0.85 * 2.0 * (double)kf / 37.0e12) continue;
+          const BoxPlan bp = best_boxes(k.bm, k.bn, &order);
+          if (!bp.ok) continue;
+          tiles_c = bp.tiles;
+          out_elems = (double)mf * (double)nf / bp.tiles;
+        } else if (short_runs) {
+          idle += 9000.0;
         }
-        const double tiles_c = (double)((mf + k.bm - 1) / k.bm) * (double)((nf + k.bn - 1) / k.bn);
         const double products = 2.0 * k.bm * k.bn * kpad / (flop_per_clk * k.eff);
-        const double out_bytes = (e.op == 0 ? 1.0 : 2.0) * k.bm * k.bn * es;
-        const double per_tile = std::max(products + k.idle, out_bytes / (byte_per_clk * k.rate));
+        const double out_bytes = (e.op == 0 ? 1.0 : 2.0) * out_elems * es;
+        const double per_tile = std::max(products + idle, out_bytes / (byte_per_clk * k.rate));
         const double t = std::ceil(tiles_c / (double)sms) * per_tile / clk;
         // the first candidate (128 x 64, two groups) stays unless another is estimated a tenth faster: the model knows
         // tiles, waste and waves, not how well each loader shape feeds each tile
@@ -517,6 +658,13 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     }
     if (p->opt.variant > 0) variant = p->opt.variant - 1;
   }
+  int box_order = -1;
+  if (variant == 3 && c.math == TC_MATH_DMMA && p->box_order < 0 && best_boxes((uint32_t)bm, (uint32_t)bn, &box_order).ok) {
+    p->box_order = box_order;  // plan again with M's dimensions whole and in that order
+    const int st = tc_plan_build(p, why);
+    p->box_order = -1;
+    return st;
+  }
   c.bm = bm;
   c.bn = bn;
   c.variant = variant;
@@ -529,6 +677,31 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   a.bn = bn;
   a.tiles_m = (uint32_t)((mf + bm - 1) / bm);
   a.tiles_n = (uint32_t)((nf + bn - 1) / bn);
+  a.mcut = {(uint32_t)bm, 1, (uint32_t)mf, 1, a.tiles_m, 1};
+  a.ncut = {(uint32_t)bn, 1, (uint32_t)nf, 1, a.tiles_n, 1};
+  a.rows_across_x = a.rows_across_y = 0;
+  c.box_c = false;
+  bool plain_m = true, plain_n = true;  // tiles are plain ranges of the flattened index
+  if (tc_kernel_is_c_resident(c)) {
+    const BoxPlan bp = plan_boxes(dm, dn, (uint32_t)bm, (uint32_t)bn);
+    if (bp.ok) {
+      c.box_c = true;
+      a.mcut = bp.m;
+      a.ncut = bp.n;
+      a.cbox = bp.map;
+      a.rows_across_x = bp.across_x;
+      a.rows_across_y = bp.across_y;
+      const int64_t tm = mf / ((int64_t)bp.m.e0 * bp.m.e1) * bp.m.t0 * bp.m.t1, tn = nf / ((int64_t)bp.n.e0 * bp.n.e1) * bp.n.t0 * bp.n.t1;
+      auto plain = [](const TcCut& k, int64_t flat, int b) { return k.b0 == (uint32_t)b && k.b1 == 1 && (k.e0 == flat || k.e0 % b == 0); };
+      plain_m = plain(bp.m, mf, bm);
+      plain_n = plain(bp.n, nf, bn);
+      a.tiles_m = (uint32_t)tm;
+      a.tiles_n = (uint32_t)tn;
+      // a tiled TMA box of an operand takes consecutive values of the flattened index
+      if (bp.m.b1 > 1 && bp.m.b0 != bp.m.e0) c.tma_x = false;
+      if (bp.n.b1 > 1 && bp.n.b0 != bp.n.e0) c.tma_y = false;
+    }
+  }
   const int64_t tiles = (int64_t)a.tiles_m * a.tiles_n;
   const int bk = TC_BK;
   // Persistent kernels: walk the tiles in column blocks of 32 M tiles when one sweep over all of M would drag more
@@ -624,7 +797,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   c.tma_c = false;
   c.tma_ct = false;
   a.cmap = TcOutMap{};
-  if (persistent) out_box_view(a, es, bm, bn, &a.cmap, &c.tma_c, &c.tma_ct);
+  if (persistent && plain_m && plain_n) out_box_view(a, es, bm, bn, &a.cmap, &c.tma_c, &c.tma_ct);
 
   double prod = 1.0;
   for (int64_t x : p->idx_extent) prod *= (double)x;
@@ -668,9 +841,21 @@ std::string tc_plan_to_json(const tc_plan& p) {
       << ",\"tma_y\":" << (p.choice.tma_y ? "true" : "false") << ",\"tma_xe\":" << (p.choice.tma_xe ? "true" : "false")
       << ",\"tma_ye\":" << (p.choice.tma_ye ? "true" : "false") << ",\"tma_c\":" << (p.choice.tma_c ? "true" : "false") << ",\"tma_ct\":" << (p.choice.tma_ct ? "true" : "false")
       << ",\"lanes_k_x\":" << a.lanes_k_x
-      << ",\"lanes_k_y\":" << a.lanes_k_y << ",\"vec_c\":" << a.vec_c << ",\"epi_run\":" << a.epi_run << ",\"epi_n_span\":" << a.epi_n_span << ",\"beta\":" << a.beta
+      << ",\"lanes_k_y\":" << a.lanes_k_y << ",\"vec_c\":" << a.vec_c << ",\"box\":[" << a.mcut.b0 << "," << a.mcut.b1 << "," << a.ncut.b0 << "," << a.ncut.b1 << "]" << ",\"epi_run\":" << a.epi_run << ",\"epi_n_span\":" << a.epi_n_span << ",\"beta\":" << a.beta
       << ",\"alpha\":" << a.alpha << ",\"workspace_bytes\":" << p.ws_bytes << ",\"launches\":" << p.launches
       << ",\"flops\":" << p.flops << ",\"bytes\":" << p.bytes;
+    if (p.choice.box_c) {
+      const TcBoxMap& b = a.cbox;
+      auto cut = [&](const TcCut& c) { o << "[" << c.b0 << "," << c.b1 << "," << c.e0 << "," << c.e1 << "," << c.t0 << "," << c.t1 << "]"; };
+      o << ",\"cbox\":{\"m\":";
+      cut(a.mcut);
+      o << ",\"n\":";
+      cut(a.ncut);
+      o << ",\"dims\":[";
+      for (int d = 0; d < b.rank; ++d) o << (d ? "," : "") << "[" << b.ext[d] << "," << b.box[d] << "," << b.stride[d] << "]";
+      o << "],\"slots\":[" << (int)b.n0 << "," << (int)b.n1 << "," << (int)b.m1 << "," << (int)b.mr0 << "," << (int)b.mr1 << "," << (int)b.nr0 << "," << (int)b.nr1
+        << "],\"steps\":[" << b.m_step << "," << b.n_step << "],\"rest\":[" << b.mr << "," << b.nr << "],\"across\":[" << a.rows_across_x << "," << a.rows_across_y << "]}";
+    }
   }
   o << "}";
   return o.str();

@@ -45,11 +45,14 @@ struct WcCfg {
   static constexpr int GROUPS = GROUPS_, WGM = WGM_, WGN = WGN_, CW = WGM * WGN;  // consumer warps per group
   static constexpr int WM = BM / WGM, WN = BN / WGN;
   static constexpr int CONSUMER_THREADS = CW * 32;
-  static constexpr int PWARPS = GROUPS == 1 ? 2 : 1;  // producer warps per group
+  // producer warps per group: two where every operand arrives 16 bytes (or a tiled copy) at a time, four where one is
+  // gathered element by element
+  static constexpr bool ELEM = MODEX == LM_ELEM || MODEY == LM_ELEM;
+  static constexpr int PWARPS = ELEM ? 4 : 2;
   static constexpr int THREADS = 32 * PWARPS;    // producer threads per group
-  // last warpgroup: the producer warps, then one warp per group whose first lane is the group's C thread
-  static constexpr int CTA_THREADS = GROUPS * CONSUMER_THREADS + 128;
-  static_assert(GROUPS * (PWARPS + 1) <= 4 && (GROUPS * CW) % 4 == 0, "warp roles");
+  // last warpgroup(s): the producer warps, then a warp whose first lane is the C thread
+  static constexpr int CTA_THREADS = CONSUMER_THREADS + (ELEM ? 256 : 128);
+  static_assert(CW % 4 == 0, "warp roles");
   static constexpr int LDK = BK + 2;
   static constexpr int LDX = MODEX == LM_K_VEC ? LDK : MODEX == LM_TMA_K ? BK : BM + 4;
   static constexpr int LDY = MODEY == LM_K_VEC ? LDK : MODEY == LM_TMA_K ? BK : BN + 4;
@@ -70,21 +73,25 @@ struct WcCfg {
   static_assert(SMEM_BYTES <= 232448, "shared memory");
 };
 
-// Coordinates of the box of the rank-5 view of C (TcOutMap) that holds the tile starting at (m0, n0):
-// {run offset, 0, (n inside N's fastest dimension) / 2, slower dimension, slowest dimension}.
-__device__ __forceinline__ void tile_box_coords(const TcKernelArgs& p, uint32_t m0, uint32_t n0, int (&c)[4]) {
-  const uint32_t e0 = p.cmap.e0, f0 = p.cmap.f0;
-  const int ne = p.cmap.ne, me = p.cmap.me;
-  int x3 = 0, x4 = 0;
-  const uint32_t rm = m0 / e0, rn = n0 / f0;
-  if (me == 2) { x3 = (int)(rm % p.cmap.ext[0]); x4 = (int)(rm / p.cmap.ext[0]); }
-  else if (me == 1) { if (ne == 0) x3 = (int)rm; else x4 = (int)rm; }
-  if (ne == 2) { x3 = (int)(rn % p.cmap.ext[0]); x4 = (int)(rn / p.cmap.ext[0]); }
-  else if (ne == 1) x3 = (int)rn;
-  c[0] = (int)(m0 % e0);
-  c[1] = (int)((n0 % f0) >> 1);
-  c[2] = x3;
-  c[3] = x4;
+// Coordinates of the box of C (TcBoxMap) that tile (tm, tn) is.
+__device__ __forceinline__ void tile_box_coords(const TcKernelArgs& p, uint32_t tm, uint32_t tn, int (&c)[5]) {
+  const TcBoxMap& o = p.cbox;
+  const CutTile mt = cut_tile(p.mcut, tm), nt = cut_tile(p.ncut, tn);
+  // (slots as selects: a run-time index would put the array into local memory)
+#pragma unroll
+  for (int d = 0; d < 5; ++d) {
+    uint32_t v = 0;
+    if (d == 0) v = mt.v0;
+    else if (d == o.n0) v = nt.v0;
+    else if (d == o.n1) v = nt.v1;
+    else if (d == o.m1) v = mt.v1;
+    else if (d == o.mr0 && d == o.nr0) v = mt.rest * o.m_step + nt.rest * o.n_step;
+    else if (d == o.mr0) v = mt.rest % o.mr;
+    else if (d == o.mr1) v = mt.rest / o.mr;
+    else if (d == o.nr0) v = nt.rest % o.nr;
+    else if (d == o.nr1) v = nt.rest / o.nr;
+    c[d] = (int)v;
+  }
 }
 
 template <class CF>
@@ -141,36 +148,44 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
     if ((tid & 31) != 0 || warp >= CWARPS + CF::GROUPS * (PW + 1)) return;
     const uint64_t tmap = reinterpret_cast<uint64_t>(&p.tmap_ct);
     const uint32_t ntiles = first < total ? (total - first + step - 1) / step : 0u;
-    auto fetch = [&](uint32_t j) {  // tile j of this group into buffer j & 1 (or just: the buffer is free)
-      const uint32_t b = j & 1u;
-      if (!accumulate) { mbar_arrive(&c_ready[b]); return; }
+    struct Corner { int c[5]; };
+    auto corner = [&](uint32_t j) {
       uint32_t tm, tn;
       tile_coords(p, first + j * step, &tm, &tn);
-      int c[4];
-      tile_box_coords(p, tm * BM, tn * BN, c);
-      mbar_arrive_expect_tx(&c_ready[b], BM * BN * 8);
+      Corner r;
+      tile_box_coords(p, tm, tn, r.c);
+      return r;
+    };
+    auto fetch = [&](uint32_t j, const Corner& at) {  // tile j of this group into buffer j & 1 (or just: the buffer is free)
+      const uint32_t b = j & 1u;
+      const int(&c)[5] = at.c;
+      if (!accumulate) { mbar_arrive(&c_ready[b]); return; }
+      mbar_arrive_expect_tx(&c_ready[b], p.mcut.b0 * p.mcut.b1 * p.ncut.b0 * p.ncut.b1 * 8u);
       asm volatile(
           "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];\n" ::"r"(
               smem_u32(gcbuf + b * CF::CTILE_ELEMS)),
-          "l"(tmap), "r"(c[0]), "r"(0), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(smem_u32(&c_ready[b]))
+          "l"(tmap), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(smem_u32(&c_ready[b]))
           : "memory");
     };
-    for (uint32_t j = 0; j < ntiles && j < (uint32_t)CF::CBUFS; ++j) fetch(j);
+    // the corners of the tiles in the two buffers and of the next: their divisions are done while the consumers work
+    Corner here = corner(0), after = corner(1);
+    if (ntiles > 0) fetch(0, here);
+    if (ntiles > 1) fetch(1, after);
     for (uint32_t j = 0; j < ntiles; ++j) {
       const uint32_t b = j & 1u;
+      const Corner next = corner(j + CF::CBUFS);
+      const int(&c)[5] = here.c;
       if (!mbar_wait(&c_staged[b], (j >> 1) & 1u, p.status, 6, p.spin_limit)) return;
-      uint32_t tm, tn;
-      tile_coords(p, first + j * step, &tm, &tn);
-      int c[4];
-      tile_box_coords(p, tm * BM, tn * BN, c);
       asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4, %5}], [%6];\n" ::"l"(tmap),
-                   "r"(c[0]), "r"(0), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(smem_u32(gcbuf + b * CF::CTILE_ELEMS))
+                   "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(smem_u32(gcbuf + b * CF::CTILE_ELEMS))
                    : "memory");
       asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
       if (j + CF::CBUFS < ntiles) {
         asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");  // the store has read the buffer: it may be refilled
-        fetch(j + CF::CBUFS);
+        fetch(j + CF::CBUFS, next);
       }
+      here = after;
+      after = next;
     }
     asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
     return;
@@ -190,11 +205,12 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
       int64_t* offy_n = offx_m + BM;
       uint32_t tm, tn;
       tile_coords(p, tile, &tm, &tn);
-      const uint32_t m0 = tm * BM, n0 = tn * BN;
+      const CutTile mt = cut_tile(p.mcut, tm), nt = cut_tile(p.ncut, tn);
+      const uint32_t m0 = cut_flat(p.mcut, mt, 0), n0 = cut_flat(p.ncut, nt, 0);
       for (int i = ptid; i < BM + BN; i += CF::THREADS) {
         int64_t unused;
-        if (i < BM) decode(p.M, m0 + i, p.Mflat, &offx_m[i], &unused);
-        else decode(p.N, n0 + (i - BM), p.Nflat, &offy_n[i - BM], &unused);
+        if (i < BM) decode(p.M, cut_flat(p.mcut, mt, i), p.Mflat, &offx_m[i], &unused);
+        else decode(p.N, cut_flat(p.ncut, nt, i - BM), p.Nflat, &offy_n[i - BM], &unused);
       }
       group_bar_sync(1 + gi, CF::THREADS);
       int64_t kx = ws_koff(p.koff_x, 0, kend, ptid), ky = ws_koff(p.koff_y, 0, kend, ptid);
@@ -213,8 +229,8 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
             if constexpr (CF::MODEY == LM_TMA_K) tma_load_2d(ys, &p.tmap_y, (int)k0, (int)n0, &full[s]);
           }
         }
-        ws_load<CF, BM, CF::MODEX>(xs, X, offx_m, kx, ptid, lgx);
-        ws_load<CF, BN, CF::MODEY>(ys, Y, offy_n, ky, ptid, lgy);
+        ws_load<CF, BM, CF::MODEX>(xs, X, offx_m, kx, ptid, lgx, p.rows_across_x, (int)p.mcut.b0);
+        ws_load<CF, BN, CF::MODEY>(ys, Y, offy_n, ky, ptid, lgy, p.rows_across_y, (int)p.ncut.b0);
         kx = nx;
         ky = ny;
         // tests only: one producer thread of CTA 0 never announces its copies of one stage
@@ -233,6 +249,18 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
   const int wm0 = (cw % CF::WGM) * WM, wn0 = (cw / CF::WGM) * WN;
   const double alpha = p.alpha;
   const int h0 = g & 1;  // which 16-byte half of its 32 bytes a thread visits first (see the header)
+  // Where this thread's pairs of rows lie in a tile buffer, whose order is (first digit of M, the tile's n, second digit
+  // of M): runs of b0 (even) outputs, n at a pitch of b0, the second digit at b0 * tile_n.  -1: beyond the tile.
+  const int b0 = (int)p.mcut.b0, tile_n = (int)(p.ncut.b0 * p.ncut.b1), tile_m = (int)(p.mcut.b0 * p.mcut.b1);
+  const bool dense = b0 == BM && tile_n == BN;
+  int mo[MB2][2];
+#pragma unroll
+  for (int i = 0; i < MB2; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int m = wm0 + 16 * i + 4 * t + 2 * h;
+      mo[i][h] = m < tile_m ? m % b0 + m / b0 * (b0 * tile_n) : -1;
+    }
   uint32_t it = 0, titer = 0;
   for (uint32_t tile = first; tile < total; tile += step, ++titer) {
     // acc[nb][2i + e][h]: row n = wn0 + 16 (nb >> 1) + 2 g + (nb & 1), column m = wm0 + 16 i + 4 t + e + 2 h
@@ -277,23 +305,50 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
     const uint32_t b = titer & 1u;
     if (!mbar_wait(&c_ready[b], (titer >> 1) & 1u, p.status, 4, p.spin_limit)) return;
     double* tb = gcbuf + b * CF::CTILE_ELEMS;
+    // (tiles that are plain ranges keep addresses the compiler knows: the general form cost 2.5 % on the 40^6 slab)
+    if (dense) {
 #pragma unroll
-    for (int nb = 0; nb < 2 * NB2; ++nb) {
-      double* row = tb + (wn0 + 16 * (nb >> 1) + 2 * g + (nb & 1)) * BM + wm0 + 4 * t;
+      for (int nb = 0; nb < 2 * NB2; ++nb) {
+        double* row = tb + (wn0 + 16 * (nb >> 1) + 2 * g + (nb & 1)) * BM + wm0 + 4 * t;
 #pragma unroll
-      for (int i = 0; i < MB2; ++i) {
-        double2* q = reinterpret_cast<double2*>(row + 16 * i);
-        // the thread's four consecutive outputs: lo = (m, m+1), hi = (m+2, m+3)
-        const double2 lo = make_double2(alpha * acc[nb][2 * i][0], alpha * acc[nb][2 * i + 1][0]);
-        const double2 hi = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
-        double2 first_v = h0 ? hi : lo, second_v = h0 ? lo : hi;
-        if (accumulate) {
-          const double2 c0 = q[h0], c1 = q[h0 ^ 1];
-          first_v.x += c0.x; first_v.y += c0.y;
-          second_v.x += c1.x; second_v.y += c1.y;
+        for (int i = 0; i < MB2; ++i) {
+          double2* q = reinterpret_cast<double2*>(row + 16 * i);
+          // the thread's four consecutive outputs: lo = (m, m+1), hi = (m+2, m+3)
+          const double2 lo = make_double2(alpha * acc[nb][2 * i][0], alpha * acc[nb][2 * i + 1][0]);
+          const double2 hi = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
+          double2 first_v = h0 ? hi : lo, second_v = h0 ? lo : hi;
+          if (accumulate) {
+            const double2 c0 = q[h0], c1 = q[h0 ^ 1];
+            first_v.x += c0.x; first_v.y += c0.y;
+            second_v.x += c1.x; second_v.y += c1.y;
+          }
+          q[h0] = first_v;
+          q[h0 ^ 1] = second_v;
         }
-        q[h0] = first_v;
-        q[h0 ^ 1] = second_v;
+      }
+    } else {
+#pragma unroll
+      for (int nb = 0; nb < 2 * NB2; ++nb) {
+        const int n = wn0 + 16 * (nb >> 1) + 2 * g + (nb & 1);
+        if (n >= tile_n) continue;
+        double* row = tb + n * b0;
+#pragma unroll
+        for (int i = 0; i < MB2; ++i) {
+          // the thread's four outputs: lo = (m, m+1), hi = (m+2, m+3), each pair in one run
+          const double2 lo = make_double2(alpha * acc[nb][2 * i][0], alpha * acc[nb][2 * i + 1][0]);
+          const double2 hi = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
+          const int q0 = h0 ? mo[i][1] : mo[i][0], q1 = h0 ? mo[i][0] : mo[i][1];
+          double2 first_v = h0 ? hi : lo, second_v = h0 ? lo : hi;
+          double2* f = reinterpret_cast<double2*>(row + q0);
+          double2* l = reinterpret_cast<double2*>(row + q1);
+          if (accumulate) {
+            const double2 c0 = q0 >= 0 ? *f : make_double2(0.0, 0.0), c1 = q1 >= 0 ? *l : make_double2(0.0, 0.0);
+            first_v.x += c0.x; first_v.y += c0.y;
+            second_v.x += c1.x; second_v.y += c1.y;
+          }
+          if (q0 >= 0) *f = first_v;
+          if (q1 >= 0) *l = second_v;
+        }
       }
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");

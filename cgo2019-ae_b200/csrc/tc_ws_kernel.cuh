@@ -197,14 +197,17 @@ __device__ __forceinline__ void ws_load_k_vec(double* img, const double* __restr
 // steps of kstep (where its 32-byte sectors lie) and eight the external index.
 template <class CF, int ROWS>
 __device__ __forceinline__ void ws_load_elem(double* img, const double* __restrict__ g, const int64_t* s_off, int64_t kreg, int ptid,
-                                             int kstep) {
+// `across` > 0 (kstep 0): the first across * b0 rows are visited with the second digit of the cut fastest, `across` values
+// of it: lanes then read neighbours of an operand whose fastest index is that digit.
+                                             int kstep, int across = 0, int b0 = 0) {
   constexpr int LD = ROWS + 4, WARPS = CF::THREADS / 32;
   const int lane = ptid & 31, warp = ptid >> 5;
   const uint32_t sbase = smem_u32(img);
   if (kstep == 0) {  // lanes walk the external index: few externals, all 16 k per thread
     constexpr int EG = ROWS / 32;  // groups of 32 externals
     for (int eg = warp; eg < EG; eg += WARPS) {
-      const int el = eg * 32 + lane;
+      int el = eg * 32 + lane;
+      if (across > 0 && el < across * b0) el = el % across * b0 + el / across;
       const int64_t eo = s_off[el];
 #pragma unroll 8
       for (int kk = 0; kk < CF::BK; ++kk) {
@@ -233,11 +236,12 @@ __device__ __forceinline__ void ws_load_elem(double* img, const double* __restri
 
 // kreg: this lane's contraction offset of the stage (ws_koff).
 template <class CF, int ROWS, int MODE>
-__device__ __forceinline__ void ws_load(double* img, const double* __restrict__ g, const int64_t* s_off, int64_t kreg, int ptid, int lg) {
+__device__ __forceinline__ void ws_load(double* img, const double* __restrict__ g, const int64_t* s_off, int64_t kreg, int ptid, int lg,
+                                        int across, int b0) {
   if constexpr (MODE == LM_EXT_VEC) ws_load_ext_vec<CF, ROWS>(img, g, s_off, kreg, ptid);
   else if constexpr (MODE == LM_K_VEC) ws_load_k_vec<CF, ROWS>(img, g, s_off, kreg, ptid);
   else if constexpr (MODE == LM_TMA_K) return;  // fetched by the producer's TMA copy
-  else ws_load_elem<CF, ROWS>(img, g, s_off, kreg, ptid, lg);
+  else ws_load_elem<CF, ROWS>(img, g, s_off, kreg, ptid, lg, across, b0);
 }
 
 // Fragment pair of the DMMA mapping: tile elements (e, e+1) at contraction index k.
@@ -372,10 +376,11 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
       uint32_t tm, tn, kbeg, kend;
       tile_coords(p, tile % tiles, &tm, &tn);
       const int nk = k_range(tile, &kbeg, &kend);
-      const uint32_t m0 = tm * BM, n0 = tn * BN;
+      const CutTile mt = cut_tile(p.mcut, tm), nt = cut_tile(p.ncut, tn);
+      const uint32_t m0 = cut_flat(p.mcut, mt, 0), n0 = cut_flat(p.ncut, nt, 0);
       for (int i = ptid; i < BM + BN; i += CF::THREADS) {
-        if (i < BM) decode(p.M, m0 + i, p.Mflat, &offx_m[i], &offc_m[i]);
-        else decode(p.N, n0 + (i - BM), p.Nflat, &offy_n[i - BM], &offc_n[i - BM]);
+        if (i < BM) decode(p.M, cut_flat(p.mcut, mt, i), p.Mflat, &offx_m[i], &offc_m[i]);
+        else decode(p.N, cut_flat(p.ncut, nt, i - BM), p.Nflat, &offy_n[i - BM], &offc_n[i - BM]);
       }
       mbar_arrive(&tab_full[par]);            // consumers may read the tables once all 64 have arrived
       group_bar_sync(1 + gi, CF::THREADS);    // ... and so may this group's producers
@@ -406,8 +411,8 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
             if constexpr (CF::MODEY == LM_TMA_K) tma_load_2d(ys, &p.tmap_y, (int)k0, (int)n0, &full[s]);
           }
         }
-        ws_load<CF, BM, CF::MODEX>(xs, X, offx_m, kx, ptid, lgx);
-        ws_load<CF, BN, CF::MODEY>(ys, Y, offy_n, ky, ptid, lgy);
+        ws_load<CF, BM, CF::MODEX>(xs, X, offx_m, kx, ptid, lgx, p.rows_across_x, (int)p.mcut.b0);
+        ws_load<CF, BN, CF::MODEY>(ys, Y, offy_n, ky, ptid, lgy, p.rows_across_y, (int)p.ncut.b0);
         kx = nx;
         ky = ny;
         // tests only: one producer thread of CTA 0 never announces its copies of one stage, so that stage stays

@@ -268,6 +268,74 @@ def test_operands_that_are_matrices_are_marked_as_boxes(pkg):
     assert flags("C [a,64,b,8,c,512] += sum(d,64) * A [a,b,d] * B [d,c];", pkg.F32)[2]
 
 
+def _wc_layouts():
+    """(expression, what it is for): outputs whose cut tiles take every form."""
+    yield "C [a,24,b,16,c,16,d,24,e,16,f,16] -= sum(g,24) * A [d,e,g,a] * B [g,f,b,c];"
+    yield "C [a,24,b,16,c,16,d,24,e,16,f,16] -= sum(g,24) * A [d,e,g,b] * B [g,f,a,c];"
+    yield "C [a,20,b,11,c,13,d,17,e,10,f,9] += sum(g,15) * A [d,e,g,c] * B [g,f,a,b];"
+    yield "C [a,10,b,26,c,7,d,5,e,12,f,31] = sum(g,22) * A [d,f,g,a] * B [g,e,b,c];"
+    yield "C [a,24,b,16,c,16,d,24,e,16,f,6] -= sum(g,24) * A [d,f,g,b] * B [g,e,a,c];"
+    yield "C [a,2,b,40,c,30,d,50] += sum(e,8) * A [a,e,b,d] * B [e,c];"
+    yield "C [a,400,b,300] += sum(c,16) * A [c,a] * B [c,b];"
+    yield "C [a,50,b,64,c,70,d,3] += sum(e,20) * A [d,a,e] * B [c,e,b];"
+
+
+@pytest.mark.parametrize("expr", list(_wc_layouts()))
+def test_cut_tiles_cover_the_output_once_and_are_boxes_of_it(pkg, expr):
+    """Output-resident kernel: the rows and columns of a cut tile, decoded through the index classes as the loaders do,
+    lie at the places of C that the tile's box in the rank-5 view has at the same place of the buffer."""
+    import numpy as np
+    d = _plan(pkg, expr, tile=(128, 64), variant=4).describe()
+    if "cbox" not in d:
+        d = _plan(pkg, expr).describe()
+    assert "cbox" in d, d["kernel"]
+    box = d["cbox"]
+
+    def class_out(dims, cut, tiles):
+        """Per tile: offsets in C of its rows (-1: none), as cut_flat and decode compute them."""
+        off = np.zeros(1, dtype=np.int64)
+        for q in dims:
+            off = (np.arange(q["extent"], dtype=np.int64)[:, None] * q["s_out"] + off[None, :]).reshape(-1)
+        b0, b1, e0, e1, t0, t1 = cut
+        out = []
+        for t in range(tiles):
+            v0, v1, rest = t % t0 * b0, t // t0 % t1 * b1, t // t0 // t1
+            rows = [v0 + r % b0 + e0 * (v1 + r // b0 + e1 * rest) if v0 + r % b0 < e0 and v1 + r // b0 < e1 else -1
+                    for r in range(b0 * b1)]
+            assert all(r < off.size for r in rows)
+            out.append((np.array([off[r] if r >= 0 else -1 for r in rows]), (v0, v1, rest)))
+        return out
+
+    assert box["m"][0] % 2 == 0 and box["m"][0] * box["m"][1] <= 128 and box["n"][0] * box["n"][1] <= 64
+    ms, ns = class_out(d["M"], box["m"], d["tiles"][0]), class_out(d["N"], box["n"], d["tiles"][1])
+    n0, n1, m1, mr0, mr1, nr0, nr1 = box["slots"]
+    seen = np.zeros(int(np.prod([e for e in d["expr"]["out_ext"]])), dtype=np.int32)
+    b0, nb = box["m"][0], box["n"][0] * box["n"][1]
+    for om, (mv0, mv1, mrest) in ms:
+        for on, (nv0, nv1, nrest) in ns:
+            corner = [mv0, 0, 0, 0, 0]
+            for slot, v in ((n0, nv0), (n1, nv1), (m1, mv1), (mr0, mrest % box["rest"][0]), (mr1, mrest // box["rest"][0]),
+                            (nr0, nrest % box["rest"][1]), (nr1, nrest // box["rest"][1])):
+                if slot:
+                    corner[slot] = v
+            if mr0 and mr0 == nr0:
+                corner[mr0] = mrest * box["steps"][0] + nrest * box["steps"][1]
+            # the box as the copy engine lays it out: first dimension fastest, -1 outside the tensor
+            place = np.zeros(1, dtype=np.int64)
+            for k, (ext, size, stride) in enumerate(box["dims"]):
+                at = corner[k] + np.arange(size, dtype=np.int64)
+                step = np.where(at < ext, at * stride, np.int64(-1) << 50)
+                place = (step[:, None] + place[None, :]).reshape(-1)
+            m, n = np.arange(om.size), np.arange(on.size)
+            pos = (m % b0 + m // b0 * (b0 * nb))[:, None] + (n * b0)[None, :]
+            want = np.where((om[:, None] >= 0) & (on[None, :] >= 0), om[:, None] + on[None, :], -1)
+            got = place[pos]
+            assert pos.max() < place.size
+            assert np.array_equal(np.where(got < 0, -1, got), want)
+            np.add.at(seen, want[want >= 0], 1)
+    assert (seen == 1).all()
+
+
 def test_blocked_contractions_name_every_value_once(pkg):
     """Two inputs that start with different contraction indices: 4 x 4 blocks of K, rounded up, with holes."""
     for c, d in ((64, 64), (61, 66), (4, 130), (63, 5)):
