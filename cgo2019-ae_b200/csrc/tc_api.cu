@@ -67,7 +67,7 @@ TC_KERNEL_LIST(TC_DECLARE)
   extern "C" int tc_inst_##NAME(int, int, const TcKernelArgs*, void*, const void*, const void*, cudaStream_t, int, int*, int*);
 TC_WS_KERNEL_LIST(TC_DECLARE_WS)
 #undef TC_DECLARE_WS
-#define TC_DECLARE_WC(NAME, BM, GROUPS, WGM, WGN, STAGES, VARIANT) \
+#define TC_DECLARE_WC(NAME, BM, BN, WGM, WGN, STAGES, VARIANT) \
   extern "C" int tc_inst_##NAME(int, int, const TcKernelArgs*, void*, const void*, const void*, cudaStream_t, int, int*, int*);
 TC_WC_KERNEL_LIST(TC_DECLARE_WC)
 #undef TC_DECLARE_WC
@@ -85,7 +85,7 @@ struct KernelEntry {
 template <typename T> constexpr int dtype_of() { return sizeof(T) == 8 ? TC_F64 : TC_F32; }
 #define TC_ENTRY(NAME, T, MATH, BM, BN, WMN, WNN, STAGES, MINB, VARIANT) {#NAME, dtype_of<T>(), MATH, BM, BN, VARIANT, tc_inst_##NAME},
 #define TC_WS_ENTRY(NAME, BM, BN, STAGES, VARIANT) {#NAME, TC_F64, TC_MATH_DMMA, BM, BN, VARIANT, tc_inst_##NAME},
-#define TC_WC_ENTRY(NAME, BM, GROUPS, WGM, WGN, STAGES, VARIANT) {#NAME, TC_F64, TC_MATH_DMMA, BM, 64, VARIANT, tc_inst_##NAME},
+#define TC_WC_ENTRY(NAME, BM, BN, WGM, WGN, STAGES, VARIANT) {#NAME, TC_F64, TC_MATH_DMMA, BM, BN, VARIANT, tc_inst_##NAME},
 #define TC_WT_ENTRY(NAME, BM, VARIANT) {#NAME, TC_F32, TC_MATH_TF32TC, BM, 128, VARIANT, tc_inst_##NAME},
 const KernelEntry kKernels[] = {TC_KERNEL_LIST(TC_ENTRY) TC_WS_KERNEL_LIST(TC_WS_ENTRY) TC_WC_KERNEL_LIST(TC_WC_ENTRY)
                                 TC_WT_KERNEL_LIST(TC_WT_ENTRY)};

@@ -112,16 +112,16 @@ int run_wt_variant(const TcKernelArgs* a, void* C, const void* X, const void* Y,
     return TC_ERR_INVALID_ARG;                                                                              \
   }
 
-#define TC_WC_CASE(MX, MY, BM, GROUPS, WGM, WGN, STAGES) \
-  if (vx == MX && vy == MY) return tck::run_wc_variant<tck::WcCfg<BM, GROUPS, WGM, WGN, STAGES, MX, MY>>(a, C, X, Y, s, mode, threads, smem);
-#define TC_WC_ROW(MX, BM, GROUPS, WGM, WGN, STAGES) \
-  TC_WC_CASE(MX, 0, BM, GROUPS, WGM, WGN, STAGES) TC_WC_CASE(MX, 1, BM, GROUPS, WGM, WGN, STAGES) \
-  TC_WC_CASE(MX, 2, BM, GROUPS, WGM, WGN, STAGES) TC_WC_CASE(MX, 3, BM, GROUPS, WGM, WGN, STAGES)
-#define TC_DEFINE_WC_INST(NAME, BM, GROUPS, WGM, WGN, STAGES)                                               \
+#define TC_WC_CASE(MX, MY, BM, BN, WGM, WGN, STAGES) \
+  if (vx == MX && vy == MY) return tck::run_wc_variant<tck::WcCfg<BM, BN, WGM, WGN, STAGES, MX, MY>>(a, C, X, Y, s, mode, threads, smem);
+#define TC_WC_ROW(MX, BM, BN, WGM, WGN, STAGES) \
+  TC_WC_CASE(MX, 0, BM, BN, WGM, WGN, STAGES) TC_WC_CASE(MX, 1, BM, BN, WGM, WGN, STAGES) \
+  TC_WC_CASE(MX, 2, BM, BN, WGM, WGN, STAGES) TC_WC_CASE(MX, 3, BM, BN, WGM, WGN, STAGES)
+#define TC_DEFINE_WC_INST(NAME, BM, BN, WGM, WGN, STAGES)                                               \
   extern "C" int NAME(int vx, int vy, const TcKernelArgs* a, void* C, const void* X, const void* Y,         \
                       cudaStream_t s, int mode, int* threads, int* smem) {                                  \
-    TC_WC_ROW(0, BM, GROUPS, WGM, WGN, STAGES) TC_WC_ROW(1, BM, GROUPS, WGM, WGN, STAGES)                   \
-    TC_WC_ROW(2, BM, GROUPS, WGM, WGN, STAGES) TC_WC_ROW(3, BM, GROUPS, WGM, WGN, STAGES)                   \
+    TC_WC_ROW(0, BM, BN, WGM, WGN, STAGES) TC_WC_ROW(1, BM, BN, WGM, WGN, STAGES)                   \
+    TC_WC_ROW(2, BM, BN, WGM, WGN, STAGES) TC_WC_ROW(3, BM, BN, WGM, WGN, STAGES)                   \
     return TC_ERR_INVALID_ARG;                                                                              \
   }
 

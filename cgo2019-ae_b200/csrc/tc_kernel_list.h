@@ -40,11 +40,13 @@
   X(dmma_ws_128x32, 128, 32, 4, 2)     \
   X(dmma_ws_64x96, 64, 96, 3, 2)
 
-// Persistent fp64 kernels that keep the output tile resident in shared memory (tc_wc_kernel.cuh): GROUPS consumer
-// groups of WGM x WGN warps, each on its own BM x 64 tile.
-//   X(name, BM, GROUPS, WGM, WGN, STAGES, VARIANT)
-#define TC_WC_KERNEL_LIST(X)            \
-  X(dmma_wc_128x64, 128, 1, 4, 2, 3, 3)
+// Persistent fp64 kernels that keep the output tile resident in shared memory (tc_wc_kernel.cuh): one consumer group of
+// WGM x WGN warps on a BM x BN tile.  The narrow one serves the short new index of integral transformations (8 to 48
+// values), on which a 64-wide tile computes up to three times what is asked for.
+//   X(name, BM, BN, WGM, WGN, STAGES, VARIANT)
+#define TC_WC_KERNEL_LIST(X)             \
+  X(dmma_wc_128x64, 128, 64, 4, 2, 3, 3) \
+  X(dmma_wc_128x32, 128, 32, 4, 2, 5, 3)
 
 // Persistent fp32 kernels on tcgen05 (tc_wt_kernel.cuh): BM x 128 tiles, two accumulators in tensor memory, the
 // output tile resident in shared memory.

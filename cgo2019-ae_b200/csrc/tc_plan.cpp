@@ -557,7 +557,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       // Constants come from the B200 measurements recorded beside the kernels; the device's SM count is the plan's.
       struct Cand { int bm, bn, variant; double idle, rate, eff; };  // eff: share of the DMMA rate its main loop reaches
       const Cand cands[] = {{128, 64, 2, 2100.0, 0.76, 0.90}, {64, 96, 2, 800.0, 0.76, 0.86}, {128, 32, 2, 1500.0, 0.76, 0.84},
-                            {128, 64, 3, 1450.0, 0.92, 0.92}};
+                            {128, 64, 3, 1450.0, 0.92, 0.92}, {128, 32, 3, 1200.0, 0.92, 0.84}};
       const double clk = 1.9e9, flop_per_clk = 37.0e12 / 148.0 / clk, byte_per_clk = 6.5e12 / 148.0 / clk;
       const double kpad = (double)((kf + 3) / 4 * 4);
       double best = 0;

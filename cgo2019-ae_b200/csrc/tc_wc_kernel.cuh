@@ -36,13 +36,13 @@
 
 namespace tck {
 
-// GROUPS consumer groups, each with its own tile, operand ring and output buffers, of WGM x WGN warps.
-template <int BM_, int GROUPS_, int WGM_, int WGN_, int STAGES_, int MODEX_, int MODEY_>
+// One consumer group of WGM x WGN warps with its operand ring and output buffers.
+template <int BM_, int BN_, int WGM_, int WGN_, int STAGES_, int MODEX_, int MODEY_>
 struct WcCfg {
   using T = double;
-  static constexpr int BM = BM_, BN = 64, BK = 16, STAGES = STAGES_;
+  static constexpr int BM = BM_, BN = BN_, BK = 16, STAGES = STAGES_;
   static constexpr int MODEX = MODEX_, MODEY = MODEY_;
-  static constexpr int GROUPS = GROUPS_, WGM = WGM_, WGN = WGN_, CW = WGM * WGN;  // consumer warps per group
+  static constexpr int GROUPS = 1, WGM = WGM_, WGN = WGN_, CW = WGM * WGN;  // consumer warps per group
   static constexpr int WM = BM / WGM, WN = BN / WGN;
   static constexpr int CONSUMER_THREADS = CW * 32;
   // producer warps per group: two where every operand arrives 16 bytes (or a tiled copy) at a time, four where one is
