@@ -712,16 +712,10 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
         }
         __syncwarp();
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const int64_t cn = offc_n[wn0 + 16 * (nb >> 1) + 2 * r + (nb & 1)];
-          if (cn < 0) continue;  // uniform across the warp
+          for (int r = 0; r < 4; ++r) {
+            cn[r] = offc_n[wn0 + 16 * (nb >> 1) + 2 * (r0 + r) + (nb & 1)];
 #pragma unroll
-          for (int m = lane; m < WM; m += 32) {
-            const int64_t co = offc_m[wm0 + m];
-            if (co < 0) continue;
-            double* q = C + cn + co;
-            const double v = cst[r * CF::CPITCH + m];
-            *q = accumulate ? v + *q : v;
+            for (int q = 0; q < MQ; ++q) old[r][q] = accumulate && (cn[r] | co[q]) >= 0 ? C[cn[r] + co[q]] : 0.0;
           }
         }
         __syncwarp();
@@ -730,7 +724,22 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
     __syncwarp();
     if (lane == 0) mbar_arrive(&tab_empty[par]);  // the producers may overwrite this table set
   }
+        // four rows at a time: their old values are all on the way before the first sum is stored (a row at a time,
+        // which is what the compiler must do where rows could overlap, every row waits for memory by itself)
+        constexpr int MQ = (WM + 31) / 32;
+        int64_t co[MQ];
+#pragma unroll
+        for (int q = 0; q < MQ; ++q) co[q] = lane + 32 * q < WM ? offc_m[wm0 + lane + 32 * q] : -1;
+#pragma unroll
+        for (int r0 = 0; r0 < 8; r0 += 4) {
+          int64_t cn[4];
+          double old[4][MQ];
   asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");  // outstanding bulk copies of this thread
 }
 
 }  // namespace tck
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int q = 0; q < MQ; ++q)
+              if ((cn[r] | co[q]) >= 0) C[cn[r] + co[q]] = cst[(r0 + r) * CF::CPITCH + lane + 32 * q] + old[r][q];
