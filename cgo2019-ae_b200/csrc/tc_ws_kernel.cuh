@@ -29,6 +29,8 @@
 // the kernel; its partners then run out of polls the same way, so the kernel
 // always terminates.  The host reads the status word after synchronising.
 #pragma once
+#include <type_traits>
+
 #include "tc_kernels.cuh"
 
 namespace tck {
@@ -195,10 +197,10 @@ __device__ __forceinline__ void ws_load_k_vec(double* img, const double* __restr
 
 // Element copies, external-major image.  kstep 0: lanes walk the external index.  kstep 1 or 4: four lanes walk k in
 // steps of kstep (where its 32-byte sectors lie) and eight the external index.
-template <class CF, int ROWS>
-__device__ __forceinline__ void ws_load_elem(double* img, const double* __restrict__ g, const int64_t* s_off, int64_t kreg, int ptid,
 // `across` > 0 (kstep 0): the first across * b0 rows are visited with the second digit of the cut fastest, `across` values
 // of it: lanes then read neighbours of an operand whose fastest index is that digit.
+template <class CF, int ROWS>
+__device__ __forceinline__ void ws_load_elem(double* img, const double* __restrict__ g, const int64_t* s_off, int64_t kreg, int ptid,
                                              int kstep, int across = 0, int b0 = 0) {
   constexpr int LD = ROWS + 4, WARPS = CF::THREADS / 32;
   const int lane = ptid & 31, warp = ptid >> 5;
@@ -468,36 +470,53 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
       }
     }
 
-    for (int ks = 0; ks < nk; ++ks, ++it) {
-      const uint32_t s = it % STAGES;
-      if (!mbar_wait(&full[s], (it / STAGES) & 1, p.status, 3, p.spin_limit)) return;
-      const double* xs = gstage + s * CF::STAGE_ELEMS;
-      const double* ys = xs + CF::XIMG;
-      const int kleft = (int)(kend - kbeg) - ks * BK;
-      const int nks = kleft >= BK ? BK / 4 : (kleft + 3) / 4;
+    // Products of the warp's first NBV groups of sixteen columns: at the ragged edge of N (67 columns on a 96-wide tile)
+    // groups that lie wholly outside the tensor cost the pipe as much as any other; so do a warp's rows that all do.
+    auto products = [&](auto nbv) {
+      constexpr int NBV = decltype(nbv)::value;
+      for (int ks = 0; ks < nk; ++ks, ++it) {
+        const uint32_t s = it % STAGES;
+        if (!mbar_wait(&full[s], (it / STAGES) & 1, p.status, 3, p.spin_limit)) return false;
+        const double* xs = gstage + s * CF::STAGE_ELEMS;
+        const double* ys = xs + CF::XIMG;
+        const int kleft = (int)(kend - kbeg) - ks * BK;
+        const int nks = kleft >= BK ? BK / 4 : (kleft + 3) / 4;
 #pragma unroll
-      for (int kq = 0; kq < BK / 4; ++kq) {
-        if (kq < nks) {
-          const int k = kq * 4 + t;
-          double2 xf[MB2], yf[NB2];
+        for (int kq = 0; kq < BK / 4; ++kq) {
+          if (kq < nks) {
+            const int k = kq * 4 + t;
+            double2 xf[MB2], yf[NB2];
 #pragma unroll
-          for (int i = 0; i < MB2; ++i) xf[i] = ws_frag<CF::MODEX, LDX>(xs, wm0 + 2 * g + i * 16, k);
+            for (int i = 0; i < MB2; ++i) xf[i] = ws_frag<CF::MODEX, LDX>(xs, wm0 + 2 * g + i * 16, k);
 #pragma unroll
-          for (int j = 0; j < NB2; ++j) yf[j] = ws_frag<CF::MODEY, LDY>(ys, wn0 + 2 * g + j * 16, k);
+            for (int j = 0; j < NBV; ++j) yf[j] = ws_frag<CF::MODEY, LDY>(ys, wn0 + 2 * g + j * 16, k);
 #pragma unroll
-          for (int j = 0; j < NB2; ++j)
+            for (int j = 0; j < NBV; ++j)
 #pragma unroll
-            for (int i = 0; i < MB2; ++i) {
-              dmma884(acc[2 * j][2 * i][0], acc[2 * j][2 * i][1], yf[j].x, xf[i].x);
-              dmma884(acc[2 * j][2 * i + 1][0], acc[2 * j][2 * i + 1][1], yf[j].x, xf[i].y);
-              dmma884(acc[2 * j + 1][2 * i][0], acc[2 * j + 1][2 * i][1], yf[j].y, xf[i].x);
-              dmma884(acc[2 * j + 1][2 * i + 1][0], acc[2 * j + 1][2 * i + 1][1], yf[j].y, xf[i].y);
-            }
+              for (int i = 0; i < MB2; ++i) {
+                dmma884(acc[2 * j][2 * i][0], acc[2 * j][2 * i][1], yf[j].x, xf[i].x);
+                dmma884(acc[2 * j][2 * i + 1][0], acc[2 * j][2 * i + 1][1], yf[j].x, xf[i].y);
+                dmma884(acc[2 * j + 1][2 * i][0], acc[2 * j + 1][2 * i][1], yf[j].y, xf[i].x);
+                dmma884(acc[2 * j + 1][2 * i + 1][0], acc[2 * j + 1][2 * i + 1][1], yf[j].y, xf[i].y);
+              }
+          }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);  // this warp no longer reads the stage
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);  // this warp no longer reads the stage
-    }
+      return true;
+    };
+    uint32_t tm, tn;
+    tile_coords(p, tile % tiles, &tm, &tn);
+    static_assert(NB2 <= 2, "groups of columns");
+    const bool plain_n = p.ncut.b0 == BN && p.ncut.e0 == p.Nflat, plain_m = p.mcut.b0 == BM && p.mcut.e0 == p.Mflat;
+    int cols = plain_n ? (int)p.Nflat - (int)(tn * BN) - wn0 : WN;  // of this warp's WN columns inside the tensor
+    if (plain_m && tm * BM + wm0 >= p.Mflat) cols = 0;
+    bool ok;
+    if (cols > WN - 16) ok = products(std::integral_constant<int, NB2>{});
+    else if (NB2 > 1 && cols > 0) ok = products(std::integral_constant<int, 1>{});
+    else ok = products(std::integral_constant<int, 0>{});
+    if (!ok) return;
 
     // ---- epilogue: read-modify-write of C (the tile was prefetched into L2 by the producers) ----
     if (!from_c && !mbar_wait(&tab_full[par], (titer >> 1) & 1, p.status, 4, p.spin_limit)) return;
@@ -513,8 +532,6 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
     // Tensor form of the same idea: a batch of 8 rows is one box of the rank-5 descriptor of C, so one tiled
     // TMA reduce-add (or store) per batch replaces eight per-row copies.  Rows and columns beyond the tensor are
     // clipped by the copy engine; boxes that lie outside altogether are not issued.
-    uint32_t tm, tn;
-    tile_coords(p, tile % tiles, &tm, &tn);
     const uint32_t m_idx = tm * BM + wm0, n_base = tn * BN + wn0;
     if (sliced) {
       // partial tile of this slice, [n][m] as tc_combine_kernel reads it (every element, padding included)
@@ -711,19 +728,6 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
           dst[1] = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
         }
         __syncwarp();
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            cn[r] = offc_n[wn0 + 16 * (nb >> 1) + 2 * (r0 + r) + (nb & 1)];
-#pragma unroll
-            for (int q = 0; q < MQ; ++q) old[r][q] = accumulate && (cn[r] | co[q]) >= 0 ? C[cn[r] + co[q]] : 0.0;
-          }
-        }
-        __syncwarp();
-      }
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&tab_empty[par]);  // the producers may overwrite this table set
-  }
         // four rows at a time: their old values are all on the way before the first sum is stored (a row at a time,
         // which is what the compiler must do where rows could overlap, every row waits for memory by itself)
         constexpr int MQ = (WM + 31) / 32;
@@ -734,12 +738,25 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
         for (int r0 = 0; r0 < 8; r0 += 4) {
           int64_t cn[4];
           double old[4][MQ];
-  asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");  // outstanding bulk copies of this thread
-}
-
-}  // namespace tck
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            cn[r] = offc_n[wn0 + 16 * (nb >> 1) + 2 * (r0 + r) + (nb & 1)];
+#pragma unroll
+            for (int q = 0; q < MQ; ++q) old[r][q] = accumulate && (cn[r] | co[q]) >= 0 ? C[cn[r] + co[q]] : 0.0;
+          }
 #pragma unroll
           for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int q = 0; q < MQ; ++q)
               if ((cn[r] | co[q]) >= 0) C[cn[r] + co[q]] = cst[(r0 + r) * CF::CPITCH + lane + 32 * q] + old[r][q];
+        }
+        __syncwarp();
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&tab_empty[par]);  // the producers may overwrite this table set
+  }
+  asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");  // outstanding bulk copies of this thread
+}
+
+}  // namespace tck
