@@ -312,7 +312,9 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
   const uint32_t tiles = p.tiles_m * p.tiles_n;
   const uint32_t total = tiles * p.ksplit;
   const bool sliced = p.ksplit > 1;
-  const uint32_t first = 2u * blockIdx.x + gi, step = 2u * gridDim.x;
+  // Items are dealt to all CTAs' first groups, then to all second groups, and so on: what is left for the last round
+  // then goes to as many SMs as there are items (dealt in pairs, 722 tiles put six on 65 SMs and four on 83).
+  const uint32_t first = blockIdx.x + gi * gridDim.x, step = 2u * gridDim.x;
   const bool accumulate = p.beta != 0;
   // contraction range [kb, ke) and number of K steps of work item `item`
   auto k_range = [&](uint32_t item, uint32_t* kb, uint32_t* ke) {
@@ -337,7 +339,7 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
     for (uint32_t t = 0;; ++t) {
       bool any = false;
       for (int g = 0; g < 2; ++g) {
-        if (2u * blockIdx.x + g + t * step >= total) continue;
+        if (blockIdx.x + g * gridDim.x + t * step >= total) continue;
         any = true;
         if (!mbar_wait(&staged[g], t & 1, p.status, 6, p.spin_limit)) return;
         const int* mb = mailbox + g * 8;
