@@ -1199,9 +1199,11 @@ __global__ void __launch_bounds__(CF::THREADS, CF::MIN_CTAS) tc_contract_kernel(
   }
 }
 
-// K-slice combine: C (op)= sum over slices of the partial tiles, slices in
-// ascending order (deterministic).  One CTA per output tile; the tile shape is
-// the producing kernel's (args.bm x args.bn).
+// K-slice combine: C (op)= sum over slices of the partial tiles, slices in ascending order (deterministic).  The tile
+// shape is the producing kernel's (args.bm x args.bn); blockIdx.x is the tile, blockIdx.y one of gridDim.y parts of it.
+// Latency-bound where the tiles are few: with one CTA per tile a 312 x 296 output left 133 SMs idle and each thread
+// summing 32 elements one after another; the launch therefore cuts tiles into parts until the GPU is covered several
+// times, and a thread has eight slices' values on the way.
 template <typename T>
 __global__ void __launch_bounds__(256) tc_combine_kernel(const __grid_constant__ TcKernelArgs p, T* __restrict__ C) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1217,19 +1219,21 @@ __global__ void __launch_bounds__(256) tc_combine_kernel(const __grid_constant__
     else decode(p.N, tile_n * BN + (i - BM), p.Nflat, &dummy, &offc_n[i - BM]);
   }
   __syncthreads();
-  const size_t tile_elems = (size_t)BM * BN;
+  const size_t tile_elems = (size_t)BM * BN, pitch = tiles * tile_elems;
   const T* ws = reinterpret_cast<const T*>(p.ws) + (size_t)bid * tile_elems;
   const T alpha = (T)p.alpha;
-  for (int e = threadIdx.x; e < BM * BN; e += 256) {
+  for (int e = threadIdx.x + 256 * blockIdx.y; e < BM * BN; e += 256 * gridDim.y) {
     const int ml = e % BM, nl = e / BM;
     const int64_t cm = offc_m[ml], cn = offc_n[nl];
     if (cm < 0 || cn < 0) continue;
     T s = T(0);
-    for (uint32_t sl = 0; sl < p.ksplit; ++sl) s += ws[sl * tiles * tile_elems + e];
+#pragma unroll 8
+    for (uint32_t sl = 0; sl < p.ksplit; ++sl) s += ws[sl * pitch + e];
     T r = alpha * s;
-    if (p.beta) r += C[cn + cm];
+    if (p.beta) r += old;
     C[cn + cm] = r;
   }
 }
 
 }  // namespace tck
+    const T old = p.beta ? C[cn + cm] : T(0);
