@@ -20,6 +20,22 @@ typedef int (*tc_inst_fn)(int mode_x, int mode_y, const TcKernelArgs* args, void
 
 namespace tck {
 
+// Launch that may overlap the end of the kernel before it in the stream (see chain_wait).
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 template <class CF>
 int run_variant(const TcKernelArgs* a, void* C, const void* X, const void* Y, cudaStream_t stream, int mode,
                 int* threads, int* smem_bytes) {
@@ -43,9 +59,8 @@ int run_variant(const TcKernelArgs* a, void* C, const void* X, const void* Y, cu
     return TC_OK;
   }
   const unsigned grid = a->tiles_m * a->tiles_n * a->ksplit;
-  kern<<<grid, CF::THREADS, CF::SMEM_BYTES, stream>>>(*a, static_cast<T*>(C), static_cast<const T*>(X),
-                                                       static_cast<const T*>(Y));
-  TC_CUDA_OK(cudaGetLastError());
+  TC_CUDA_OK(launch_chained(kern, dim3(grid), CF::THREADS, CF::SMEM_BYTES, stream, *a, static_cast<T*>(C), static_cast<const T*>(X),
+                            static_cast<const T*>(Y)));
   return TC_OK;
 }
 
