@@ -141,29 +141,39 @@ def parse(expr):
     return json.loads(buf.value.decode())
 
 
+_raw_stream = None
+
+
+def _current_stream(device_index):
+    """Address of torch's current stream on a device (0: the legacy default stream)."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        # the number itself where torch offers it: building a Stream object takes as long as the launch of a small kernel
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda index: torch.cuda.current_stream(index).cuda_stream)
+    return _raw_stream(device_index)
+
+
 def _stream(stream, *tensors):
     """cudaStream_t for a call: the caller's, else torch's current stream when the arguments are torch CUDA tensors
     (so that the launch is ordered with the surrounding torch work), else the legacy default stream."""
     if stream:
-        return ctypes.c_void_p(stream)
+        return stream
     for t in tensors:
-        if hasattr(t, "is_cuda") and t.is_cuda:
-            import torch
-            s = torch.cuda.current_stream(t.device).cuda_stream
-            return ctypes.c_void_p(s) if s else None
+        if getattr(t, "is_cuda", False):
+            return _current_stream(t.get_device()) or None
     return None
 
 
 def _ptr(x):
-    """Device/host address of a torch tensor, numpy array or raw int."""
-    if x is None:
-        return None
-    if isinstance(x, int):
-        return ctypes.c_void_p(x)
+    """Device/host address of a torch tensor, numpy array or raw int (ctypes converts it at the call)."""
     if hasattr(x, "data_ptr"):
-        return ctypes.c_void_p(x.data_ptr())
+        return x.data_ptr()
+    if x is None or isinstance(x, int):
+        return x
     if hasattr(x, "ctypes"):
-        return ctypes.c_void_p(x.ctypes.data)
+        return x.ctypes.data
     raise TypeError("expected a tensor, array or address, got %r" % type(x))
 
 
@@ -239,7 +249,9 @@ class Plan:
         """Enqueue C (op)= sum A*B on device tensors (torch CUDA tensors or raw device addresses)."""
         s = _stream(stream, C)
         if workspace is None:
-            _check(lib().tc_execute(self._h, _ptr(C), _ptr(A), _ptr(B), s), "tc_execute")
+            st = _lib.tc_execute(self._h, _ptr(C), _ptr(A), _ptr(B), s)
+            if st:
+                _check(st, "tc_execute")
         else:
             nbytes = workspace.numel() * workspace.element_size()
             _check(lib().tc_execute_ws(self._h, _ptr(C), _ptr(A), _ptr(B), _ptr(workspace), nbytes, s), "tc_execute_ws")
