@@ -249,13 +249,6 @@ __device__ __forceinline__ void decode(const TcDims& d, uint32_t flat, uint32_t 
   *off_out = oo;
 }
 
-// Tile number -> tile coordinates for the persistent kernels.  Plain order: M fastest over all of M.  With
-// mblock_w = w > 0 the tiles are walked in column blocks of w M tiles: inside a block M is fastest, then N, and a
-// block is finished over all of N before the next begins.  The tiles in flight at any time (one per consumer group
-// and SM, consecutive numbers) then share a handful of operand tiles -- w tiles of X that stay hot in L2 for the
-// whole sweep over N, and a few tiles of Y -- instead of sweeping ALL of X once per row of tiles, which for large
-// outputs pushes the operands out of L2 behind the stream of C (measured: 26.6 -> 22.2 TFLOP/s as the output grew
-// from 4 to 33 GB).
 // Flattened index of row r of tile number t of a cut class (persistent fp64 kernels), or 0xffffffff beyond the tile or
 // the class.
 struct CutTile { uint32_t v0, v1, rest; };
@@ -270,6 +263,13 @@ __device__ __forceinline__ uint32_t cut_flat(const TcCut& c, const CutTile& t, u
   return v0 + c.e0 * (v1 + c.e1 * t.rest);
 }
 
+// Tile number -> tile coordinates for the persistent kernels.  Plain order: M fastest over all of M.  With
+// mblock_w = w > 0 the tiles are walked in column blocks of w M tiles: inside a block M is fastest, then N, and a
+// block is finished over all of N before the next begins.  The tiles in flight at any time (one per consumer group
+// and SM, consecutive numbers) then share a handful of operand tiles -- w tiles of X that stay hot in L2 for the
+// whole sweep over N, and a few tiles of Y -- instead of sweeping ALL of X once per row of tiles, which for large
+// outputs pushes the operands out of L2 behind the stream of C (measured: 26.6 -> 22.2 TFLOP/s as the output grew
+// from 4 to 33 GB).
 __device__ __forceinline__ void tile_coords(const TcKernelArgs& p, uint32_t tile, uint32_t* tm, uint32_t* tn) {
   const uint32_t w = p.mblock_w;
   if (w == 0) { *tm = tile % p.tiles_m; *tn = tile / p.tiles_m; return; }
@@ -1238,6 +1238,7 @@ __global__ void __launch_bounds__(256) tc_combine_kernel(const __grid_constant__
     const int ml = e % BM, nl = e / BM;
     const int64_t cm = offc_m[ml], cn = offc_n[nl];
     if (cm < 0 || cn < 0) continue;
+    const T old = p.beta ? C[cn + cm] : T(0);
     T s = T(0);
 #pragma unroll 8
     for (uint32_t sl = 0; sl < p.ksplit; ++sl) s += ws[sl * pitch + e];
@@ -1248,4 +1249,3 @@ __global__ void __launch_bounds__(256) tc_combine_kernel(const __grid_constant__
 }
 
 }  // namespace tck
-    const T old = p.beta ? C[cn + cm] : T(0);
