@@ -467,6 +467,7 @@ static void box_build(tc_fused_plan* p) {
     t.kflat = T.kflat;
     t.bytes = (uint32_t)(T.rows + T.cols) * 128u;
     t.alpha = T.alpha;
+    t.full = T.rows == tcbox::kBox && T.cols == tcbox::kBox;
     for (int d = 0; d < kMapDims; ++d) {
       t.px[d] = d < (int)p->box_x[k].size() ? (int8_t)p->box_x[k][d].out_pos : (int8_t)-1;
       t.py[d] = d < (int)p->box_y[k].size() ? (int8_t)p->box_y[k][d].out_pos : (int8_t)-1;
@@ -484,7 +485,7 @@ static void box_positions(const tc_fused_plan* p, int k, int part, int32_t* pos)
     uint32_t e = 0;
     int sh = 0;
     for (int i = 0; i < p->args.rank; ++i) { e |= (uint32_t)((coord[r] >> (8 * i)) & 0xff) << sh; sh += (int)p->box.lg[i]; }
-    pos[r] = (int32_t)tcbox::box_hash(e);
+    pos[r] = (int32_t)tcbox::box_hash(e) * 8;
   }
 }
 

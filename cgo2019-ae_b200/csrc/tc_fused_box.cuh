@@ -8,8 +8,8 @@
 //   * CTAs are persistent, two per SM, and walk the boxes; tables are read once;
 //   * one PRODUCER thread issues two tiled copies per stage (16 k x 64 rows of each input, rank 5, 128-byte swizzle,
 //     zeros outside the tensor), up to kBoxStages stages ahead and across terms and boxes;
-//   * eight CONSUMER warps (32 x 16 products each) wait per stage on mbarriers and meet only once per term, before
-//     the term's products are added to the box;
+//   * eight CONSUMER warps (32 x 16 products each) wait per stage on mbarriers and once per term, before they
+//     add the term's products to the box, for the other warps' additions of the term before;
 //   * the box starts from C (asynchronous copies issued when the previous box has left, hidden behind the first
 //     term's products) and leaves as plain stores.
 //
@@ -17,12 +17,17 @@
 // A thread reads two consecutive k at once; MMA number 2 h + e of a stage takes k = 8 h + 2 t + e in slot t, for both
 // operands, so the sums are over the same k.  Block row g of an MMA stands for row perm(g) = (g & 1) * 4 + g / 2:
 // the two rows a quarter warp reads then differ in bit 2 and their chunks fall into different halves of the banks.
-// Box element e sits at position box_hash(e): its low four bits are XORed with a 4-bit code per higher bit.  The codes
-// of two bits of one index span a plane of GF(2)^4, planes of different indices (but the last and the second) meet in
-// zero only, so the accumulators of a warp, which vary over two or three indices, hit all banks evenly.
+// Box element e sits at position box_hash(e): its low four bits are XORed with a 4-bit code per higher bit.  Half a warp's
+// accumulators vary over both bits of one input's first index and over one bit each of the other input's first two; the
+// codes (found by search) make these four independent, so without bank conflicts, for every term of the CCSD(T) doubles
+// and for four in five of all assignments of six indices (two-way at most in the rest).
 //
-// Measured (nine doubles terms of CCSD(T), all extents 24, one B200): 9.78 ms on tc_fused_kernel, 4.76 ms here (17.3
-// TFLOP/s, 47 % of the DMMA rate; floor 2.23 ms of products).
+// Measured (nine doubles terms of CCSD(T), all extents 24, one B200): 9.78 ms on tc_fused_kernel, 3.95 ms here (20.9
+// TFLOP/s, 56 % of the DMMA rate; floor 2.23 ms of products).  On the way: one block barrier per term 4.76 ms; a barrier
+// that warps only arrive at when their additions are done, 104 registers a thread, eight old values read together 4.49;
+// positions as byte offsets, no tests in whole terms 4.14; conflict-free codes and both halves' reads first 3.95.  Without
+// any loads 4.43 of the 4.49 remained, the loads alone take 2.07, without the additions 3.68: what is left is the chain
+// of a term (wait, fragments, products, additions) with two CTAs of eight warps to cover it.
 #pragma once
 #include "tc_ws_kernel.cuh"
 
@@ -34,13 +39,17 @@ constexpr int kBox = 64;           // rows / columns of a term inside a box, at 
 constexpr int kBoxElems = 4096;
 constexpr int kBoxStages = 4;
 constexpr int kConsumers = 256;    // eight warps
-constexpr int kBoxThreads = kConsumers + 32;
+constexpr int kBoxThreads = kConsumers + 128;  // + a warpgroup whose first lane is the producer
+// registers: launched with 80 a thread (two CTAs of 384); what the consumers take is less than the producer's warpgroup gives
+constexpr int kProducerRegs = 24, kConsumerRegs = 104;
+static_assert(128 * kProducerRegs + 256 * kConsumerRegs <= 384 * 80, "register shares");
 constexpr int kImgBytes = kBox * 128;
 constexpr int kMapDims = 4;        // output indices an input may carry
 
 struct BoxTerm {
   uint32_t kflat, bytes;             // contraction length; bytes of one stage's two boxes
   int8_t px[kMapDims], py[kMapDims];  // output index of dimension 1 + d of the left / right input's map (-1: padding)
+  int32_t full;                       // 64 rows and 64 columns
   double alpha;
 };
 
@@ -53,13 +62,14 @@ struct BoxArgs {
   int64_t sc[kMaxRank];
   uint32_t total_boxes;
   uint32_t spin_limit;
-  const int32_t* pos;        // [terms][2][64] hashed box position of row r / column c, -1 beyond the term's rows
+  const int32_t* pos;        // [terms][2][64] hashed box position, in bytes, of row r / column c, -1 beyond the term's rows
   int* status;               // host-visible word: code of a wait that gave up
 };
 
 // 4-bit code XORed into the low bits of a box position for each of its bits 4..11.
 __host__ __device__ constexpr uint32_t box_code(int bit) {
-  return bit == 4 ? 5u : bit == 5 ? 10u : bit == 6 ? 9u : bit == 7 ? 14u : bit == 8 ? 13u : bit == 9 ? 6u : bit == 10 ? 4u : bit == 11 ? 8u : 0u;
+  constexpr uint32_t code[12] = {0, 0, 0, 0, 15, 12, 5, 2, 11, 8, 14, 12};
+  return code[bit];
 }
 __host__ __device__ constexpr uint32_t box_hash(uint32_t e) {
   uint32_t r = e;
@@ -89,19 +99,25 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
   int32_t* s_pos = reinterpret_cast<int32_t*>(box + kBoxElems);               // [terms][2][64]
   uint64_t* full = reinterpret_cast<uint64_t*>(s_pos + kMaxTerms * 2 * kBox);  // [stages]
   uint64_t* empty = full + kBoxStages;
+  uint64_t* added = empty + kBoxStages;  // every warp has added its products of a term to the box
+  uint64_t* c_ready = added + 1;         // the box holds C
+  unsigned char* box_b = reinterpret_cast<unsigned char*>(box);
   const uint32_t stage0 = tck::smem_u32(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
     for (int s = 0; s < kBoxStages; ++s) { tck::mbar_init(full + s, 1); tck::mbar_init(empty + s, kConsumers / 32); }
+    tck::mbar_init(added, kConsumers / 32);
+    tck::mbar_init(c_ready, kConsumers);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   for (int i = tid; i < p.n_terms * 2 * kBox; i += kBoxThreads) s_pos[i] = p.pos[i];
   __syncthreads();
 
-  if (warp == kConsumers / 32) {
+  if (warp >= kConsumers / 32) {
     // ------------------------------------------------------------ producer ----
-    if (lane != 0) return;
+    tck::reg_dec<kProducerRegs>();
+    if (tid != kConsumers) return;
     uint32_t it = 0;
     for (uint32_t bx = blockIdx.x; bx < p.total_boxes; bx += gridDim.x) {
       for (int k = 0; k < p.n_terms; ++k) {
@@ -131,12 +147,13 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
   }
 
   // -------------------------------------------------------------- consumer ----
+  tck::reg_inc<kConsumerRegs>();
   const int g = lane >> 2, t = lane & 3;
   const int pg = ((g & 1) << 2) | (g >> 1);
   const int wm0 = (warp & 1) * 32, wn0 = (warp >> 1) * 16;
   const uint32_t chunk = (uint32_t)((t ^ pg) << 4);
   const uint32_t fx = (uint32_t)(wm0 + pg) * 128u + chunk, fy = (uint32_t)(kImgBytes + (wn0 + pg) * 128) + chunk;
-  bool dead = false;  // a wait gave up: the barriers below are still met, so that every warp leaves
+  bool dead = false;  // a wait gave up: none is waited for any more, so that every warp leaves
 
   // this thread's box elements e = tid + 256 i: offset in C and coordinates are those of tid plus those of 256 i
   int64_t off_lo = 0;
@@ -156,7 +173,7 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
     *crd = c;
   };
   split((uint32_t)tid, &off_lo, &crd_lo);
-  int64_t* s_off_hi = reinterpret_cast<int64_t*>(empty + kBoxStages);   // [16]
+  int64_t* s_off_hi = reinterpret_cast<int64_t*>(c_ready + 1);            // [16]
   uint64_t* s_crd_hi = reinterpret_cast<uint64_t*>(s_off_hi + 16);      // [16]
   if (tid < 16) split((uint32_t)tid << 8, &s_off_hi[tid], &s_crd_hi[tid]);
   const uint32_t pos_lo = box_hash((uint32_t)tid);
@@ -186,15 +203,15 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
       const double* src = C + base + (ok ? off_lo + s_off_hi[i] : 0);
       tck::cp_async8(box_u32 + (pos_lo ^ box_hash((uint32_t)i << 8)) * 8u, src, ok);
     }
-    tck::cp_async_commit();
+    tck::mbar_arrive_on_copies(c_ready);
   };
 
   int64_t base = 0;
   uint64_t last = 0;
   corner_of(blockIdx.x, &base, &last);
   fetch_c(base, last);
-  uint32_t it = 0;
-  for (uint32_t bx = blockIdx.x; bx < p.total_boxes; bx += gridDim.x) {
+  uint32_t it = 0, terms = 0, boxes = 0;  // stages, terms and boxes so far
+  for (uint32_t bx = blockIdx.x; bx < p.total_boxes; bx += gridDim.x, ++boxes) {
     for (int k = 0; k < p.n_terms; ++k) {
       double acc[2][4][2];
 #pragma unroll
@@ -206,29 +223,39 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
         const uint32_t s = it % kBoxStages;
         if (!dead && !box_wait(&full[s], (it / kBoxStages) & 1, p.status, 3, p.spin_limit)) dead = true;
         const unsigned char* img = smem_raw + s * 2 * kImgBytes;
+        // (both halves of a whole stage are read before the first product: behind a branch the second half's reads would
+        // wait for the first half's products)
+        auto halves = [&](auto count) {
+          constexpr int H = decltype(count)::value;
+          double2 xf[H][4], yf[H][2];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (h == 0 || kfl - k0 > 8) {
-            double2 xf[4], yf[2];
+          for (int h = 0; h < H; ++h) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) xf[i] = *reinterpret_cast<const double2*>(img + (fx ^ (h * 64u)) + i * 1024);
+            for (int i = 0; i < 4; ++i) xf[h][i] = *reinterpret_cast<const double2*>(img + (fx ^ (h * 64u)) + i * 1024);
 #pragma unroll
-            for (int j = 0; j < 2; ++j) yf[j] = *reinterpret_cast<const double2*>(img + (fy ^ (h * 64u)) + j * 1024);
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-              for (int i = 0; i < 4; ++i) tck::dmma884(acc[j][i][0], acc[j][i][1], yf[j].x, xf[i].x);
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-              for (int i = 0; i < 4; ++i) tck::dmma884(acc[j][i][0], acc[j][i][1], yf[j].y, xf[i].y);
+            for (int j = 0; j < 2; ++j) yf[h][j] = *reinterpret_cast<const double2*>(img + (fy ^ (h * 64u)) + j * 1024);
           }
-        }
+#pragma unroll
+          for (int h = 0; h < H; ++h) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) tck::dmma884(acc[j][i][0], acc[j][i][1], yf[h][j].x, xf[h][i].x);
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) tck::dmma884(acc[j][i][0], acc[j][i][1], yf[h][j].y, xf[h][i].y);
+          }
+        };
+        if (kfl - k0 > 8) halves(std::integral_constant<int, 2>{});
+        else halves(std::integral_constant<int, 1>{});
         __syncwarp();
         if (lane == 0) tck::mbar_arrive(&empty[s]);
       }
-      // The products of this term go into the box: every (row, column) is one distinct element.  The barrier stands
-      // between this term's additions and those of the term before (and, for the first term, the box's values from C).
+      // The products of this term go into the box: every (row, column) is one distinct element.  Another warp may hold
+      // the same element in the term before (or, for the first term, its value of C may be on its way): a warp waits
+      // for all warps' additions of that term, and has its own term's products meanwhile.  Eight elements are read before
+      // any is written: one by one, which is what the compiler must do where they could meet, costs sixteen round trips.
       const int32_t* pm = s_pos + k * 2 * kBox + wm0 + t;
       const int32_t* pn = s_pos + k * 2 * kBox + kBox + wn0 + pg;
       const double alpha = p.term[k].alpha;
@@ -239,18 +266,35 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
         for (int h = 0; h < 2; ++h) qm[2 * i + h] = pm[8 * i + 4 * h];
 #pragma unroll
       for (int j = 0; j < 2; ++j) qn[j] = pn[8 * j];
-      if (k == 0) tck::cp_async_wait<0>();
-      asm volatile("bar.sync 1, %0;\n" ::"n"(kConsumers) : "memory");
+      if (!dead && !(k == 0 ? box_wait(c_ready, boxes & 1, p.status, 4, p.spin_limit) : box_wait(added, (terms - 1) & 1, p.status, 5, p.spin_limit)))
+        dead = true;
+      if (p.term[k].full) {  // 64 rows and columns: nothing to test
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < 2; ++j) {
+          double old[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+          for (int i = 0; i < 8; ++i) old[i] = *reinterpret_cast<const double*>(box_b + (qm[i] ^ qn[j]));
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
-            if ((qm[2 * i + h] | qn[j]) >= 0) box[qm[2 * i + h] ^ qn[j]] += alpha * acc[j][i][h];
+          for (int i = 0; i < 8; ++i) *reinterpret_cast<double*>(box_b + (qm[i] ^ qn[j])) = fma(alpha, acc[j][i >> 1][i & 1], old[i]);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          double old[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if ((qm[i] | qn[j]) >= 0) old[i] = *reinterpret_cast<const double*>(box_b + (qm[i] ^ qn[j]));
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if ((qm[i] | qn[j]) >= 0) *reinterpret_cast<double*>(box_b + (qm[i] ^ qn[j])) = fma(alpha, acc[j][i >> 1][i & 1], old[i]);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) tck::mbar_arrive(added);
+      ++terms;
     }
     // ---- the box leaves; the next one's values of C take its place ----
-    asm volatile("bar.sync 1, %0;\n" ::"n"(kConsumers) : "memory");
+    if (!dead && !box_wait(added, (terms - 1) & 1, p.status, 6, p.spin_limit)) dead = true;
 #pragma unroll
     for (int i = 0; i < 16; ++i)
       if (valid(crd_lo + s_crd_hi[i], last)) C[base + off_lo + s_off_hi[i]] = box[pos_lo ^ box_hash((uint32_t)i << 8)];
@@ -261,6 +305,6 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
   }
 }
 
-constexpr int box_smem_bytes() { return kBoxStages * 2 * kImgBytes + kBoxElems * 8 + kMaxTerms * 2 * kBox * 4 + 2 * kBoxStages * 8 + 32 * 8; }
+constexpr int box_smem_bytes() { return kBoxStages * 2 * kImgBytes + kBoxElems * 8 + kMaxTerms * 2 * kBox * 4 + (2 * kBoxStages + 2) * 8 + 32 * 8; }
 
 }  // namespace tcbox
