@@ -1,0 +1,148 @@
+"""Kernels and dispatch rules at the sizes where they can go wrong, against the CPU loop nest: cut tiles of the
+output-resident fp64 kernels, blocked contractions with holes, element epilogues, K slices combined in parts, kernels
+chained in a stream, the fused kernel's boxes.  fp64 tolerance as everywhere: 1e-12 of the largest value."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(pkg, orc, expr, seed=3, dtype="float64", **kw):
+    import torch
+    torch.cuda.set_device(0)
+    c0, a, b = orc.make_inputs(expr, seed, dtype)
+    ref = orc.contract(expr, c0.copy(), a, b)
+    plan = pkg.Plan(expr, pkg.F64 if dtype == "float64" else pkg.F32, **kw)
+    d = plan.describe()
+    dc, da, db = (torch.from_numpy(x).cuda() for x in (c0, a, b))
+    plan.execute(dc, da, db)
+    torch.cuda.synchronize()
+    err = orc.rel_error(dc.cpu().numpy(), ref)
+    assert plan.status() == 0
+    plan.close()
+    return d, err
+
+
+CUT = [
+    "C [a,24,b,8,c,7,d,10,e,6,f,5] -= sum(g,24) * A [d,e,g,a] * B [g,f,b,c];",     # runs of 24, five per tile, gathered across
+    "C [a,22,b,9,c,11,d,6,e,4,f,5] += sum(g,15) * A [d,e,g,b] * B [g,f,a,c];",     # 22-element runs: pairs straddle no quad
+    "C [a,10,b,26,c,7,d,5,e,4,f,3] = sum(g,22) * A [d,f,g,a] * B [g,e,b,c];",
+    "C [a,24,b,6,c,10,d,8,e,6,f,5] -= sum(g,24) * A [d,f,g,b] * B [g,e,a,c];",     # six dimensions, two sharing one of the map
+    "C [a,2,b,40,c,30,d,9] += sum(e,8) * A [a,e,b,d] * B [e,c];",                  # shortest runs
+    "C [a,30,b,7,c,26,d,10] += sum(e,33) * A [d,c,e,a] * B [e,b];",                # narrow tile's shape, ragged both ways
+]
+
+
+@pytest.mark.parametrize("tile", [(128, 64), (128, 32)])
+@pytest.mark.parametrize("expr", CUT)
+def test_cut_tiles_against_the_loop_nest(pkg, orc, expr, tile):
+    d, err = _run(pkg, orc, expr, tile=tile, variant=4)
+    assert d["kernel"] == "dmma_wc_%dx%d" % tile and "cbox" in d
+    assert err <= 1e-12, (d["cbox"], err)
+
+
+def test_cut_tiles_of_a_misaligned_output_run_without_boxes(pkg, orc):
+    import torch
+    expr = CUT[0]
+    c0, a, b = orc.make_inputs(expr, 5, "float64")
+    ref = orc.contract(expr, c0.copy(), a, b)
+    plan = pkg.Plan(expr, tile=(128, 64), variant=4)
+    buf = torch.zeros(c0.size + 1, dtype=torch.float64, device="cuda")
+    buf[1:].copy_(torch.from_numpy(c0))                                            # 8 bytes past an aligned address
+    plan.execute(buf[1:], torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda())
+    torch.cuda.synchronize()
+    assert plan.status() == 0 and orc.rel_error(buf[1:].cpu().numpy(), ref) <= 1e-12
+    plan.close()
+
+
+@pytest.mark.parametrize("c,d", [(61, 66), (64, 64), (4, 150), (63, 5), (3, 3)])
+@pytest.mark.parametrize("split", [0, 3])
+def test_blocked_contractions_against_the_loop_nest(pkg, orc, c, d, split):
+    expr = "t3 [a,150,b,70] += sum(c,%d,d,%d) * t2 [c,a,d] * v2 [d,b,c];" % (c, d)
+    desc, err = _run(pkg, orc, expr, tile=(128, 64), variant=3, split_k=split)
+    assert desc["Kflat"] == (c + 3) // 4 * 4 * ((d + 3) // 4 * 4) and err <= 1e-12
+
+
+@pytest.mark.parametrize("tile,variant", [((128, 64), 3), ((64, 96), 3), ((128, 32), 3)])
+@pytest.mark.parametrize("op", ["+=", "=", "-="])
+def test_odd_outputs_and_ragged_edges(pkg, orc, tile, variant, op):
+    # 67 columns: groups of columns outside the tensor; 61 x 13 rows: a warp's rows outside it; every row at odd offsets
+    _, err = _run(pkg, orc, "C [a,61,b,13,c,67,d,3] %s sum(e,21) * A [a,e,b,d] * B [e,c];" % op, tile=tile, variant=variant)
+    assert err <= 1e-12
+
+
+@pytest.mark.parametrize("dtype,tol", [("float64", 1e-12), ("float32", 1e-5)])
+@pytest.mark.parametrize("split", [2, 7, 19])
+def test_slices_combined_in_parts(pkg, orc, dtype, tol, split):
+    _, err = _run(pkg, orc, "C [a,70,b,45] -= sum(c,700) * A [c,a] * B [c,b];", dtype=dtype, split_k=split)
+    assert err <= tol
+
+
+@pytest.mark.parametrize("expr,kw", [
+    ("C [i,64,j,48,k,32] += sum(l,40) * A [l,k,i] * B [j,l];", {}),
+    ("C [a,70,b,45] += sum(c,700) * A [c,a] * B [c,b];", {"split_k": 5}),
+])
+def test_kernels_chained_in_a_stream_see_their_predecessors(pkg, orc, expr, kw):
+    """Each pass adds to what the pass before wrote, and reads an input that a kernel just before it wrote."""
+    import torch
+    c0, a, b = orc.make_inputs(expr, 6, "float64")
+    ref = c0.copy()
+    plan = pkg.Plan(expr, **kw)
+    dc, da, db = (torch.from_numpy(x).cuda() for x in (c0, a, b))
+    scaled = torch.empty_like(da)
+    for n in range(40):
+        torch.mul(da, float(n % 5 + 1), out=scaled)
+        plan.execute(dc, scaled, db)
+    for n in range(5):  # the loop nest once per factor: 40 passes are 8 of each
+        one = orc.contract(expr, c0 * 0, a * (n + 1), b)
+        ref = ref + 8 * one
+    torch.cuda.synchronize()
+    assert orc.rel_error(dc.cpu().numpy(), ref) <= 1e-12
+    plan.close()
+
+
+@pytest.mark.parametrize("k", [2, 8, 10, 16, 22, 34])
+@pytest.mark.parametrize("ext", [(4, 4, 4, 4, 4, 4), (5, 3, 9, 1, 6, 7), (10, 11, 4, 8, 2, 13)])
+def test_fused_boxes_against_the_loop_nest(pkg, orc, k, ext):
+    import torch
+    torch.cuda.set_device(0)
+    out = "t3 [h3,%d,h2,%d,h1,%d,p6,%d,p5,%d,p4,%d]" % ext
+    lines = ["%s %s sum(p7,%d) * x%d [%s] * y%d [%s];" % (out, op, k, n, l, n, r) for n, (op, l, r) in enumerate([
+        ("-=", "p7,p4,h1,h2", "p7,h3,p6,p5"), ("+=", "p7,p5,h2,h3", "p7,h1,p6,p4")])]
+    if ext[0] == 5:  # four indices in one input: two values each in a box
+        lines.append("%s -= sum(p7,%d) * x2 [p7,h3,p6] * y2 [p7,h1,h2,p5,p4];" % (out, k))
+    plan = pkg.FusedPlan(lines)
+    assert plan.describe()["kernel"] == "tc_fused_box_kernel"
+    c0 = orc.uniform(60, 0, orc.sizes(lines[0])[0])
+    ref, ins = c0.copy(), []
+    for n, line in enumerate(lines):
+        _, na, nb = orc.sizes(line)
+        a, b = orc.uniform(61 + n, 1, na), orc.uniform(61 + n, 2, nb)
+        ins.append((a, b))
+        orc.contract(line, ref, a, b)
+    dc = torch.from_numpy(c0).cuda()
+    plan.execute(dc, [torch.from_numpy(a).cuda() for a, _ in ins], [torch.from_numpy(b).cuda() for _, b in ins])
+    torch.cuda.synchronize()
+    assert orc.rel_error(dc.cpu().numpy(), ref) <= 1e-12
+    plan.close()
+
+
+@pytest.mark.parametrize("k", [160, 264, 520, 1032])
+def test_split_groups_of_the_persistent_fp32_kernel(pkg, orc, k):
+    """Odd and even numbers of K steps, a last step of eight, more than one tile per CTA: the two groups' turns."""
+    expr = "C [a,3072,b,2048] += sum(c,%d) * A [c,a] * B [c,b];" % k
+    import numpy as np
+    import torch
+    torch.cuda.set_device(0)
+    a = torch.rand(3072, k, device="cuda") - 0.5
+    b = torch.rand(2048, k, device="cuda") - 0.5
+    c = torch.rand(2048, 3072, device="cuda")
+    want = (c.double() + b.double() @ a.double().T).cpu().numpy()
+    plan = pkg.Plan(expr, pkg.F32)
+    assert plan.describe()["kernel"].startswith("tf32wt")
+    for n in range(3):
+        got = c.clone()
+        plan.execute(got, a, b)
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        assert np.abs(got.cpu().numpy() - want).max() / np.abs(want).max() <= 1e-5
+    plan.close()
