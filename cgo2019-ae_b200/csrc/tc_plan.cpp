@@ -132,7 +132,8 @@ void out_box_view(const TcKernelArgs& a, int es, int bm, int bn, TcOutMap* map, 
 // Cut tiles of the output-resident kernel: how its bm x bn tile is laid over the output so that it is one box of a
 // rank-<=5 view of C.  Per class either the dimensions fused as far as they are contiguous in C, of which a tile takes a
 // range of the first, or the planner's own dimensions, of which it takes ranges of the first two -- what an output with
-// short runs needs (24-element runs: 5 of them make 120 of 128 rows).  Every even b0 and every c0 is tried; the score is
+// short runs needs (24-element runs: 5 of them make 120 of 128 rows: triples term 24/16, K = 24, 155 us on one B200, 211
+// on the best flat tile of the other kernels, 261 on the 128 x 64 one).  Every even b0 and every c0 is tried; the score is
 // the number of tiles (rows that a tile leaves unused cost as much as used ones) times a penalty for short pieces: of C
 // (b0 elements, or b0 * c0 where the next index of C is N's first) and of an operand whose fastest index is external.
 struct BoxPlan {
@@ -188,6 +189,8 @@ BoxPlan plan_boxes(const std::vector<Dim>& dm, const std::vector<Dim>& dn, uint3
         const int64_t t1 = two_m ? (e1 + bm / b0 - 1) / (bm / b0) : 1;
         const uint32_t b1 = two_m ? (uint32_t)((e1 + t1 - 1) / t1) : 1;
         for (uint32_t c0 = std::min<int64_t>(bn, f0); c0 >= 1; --c0) {
+          // (an input read in pairs along N's first index: pairs lie in one run and tiles start on 16 bytes)
+          if (uy == 0 && dn[0].extent % 2 == 0 && c0 % 2 != 0) continue;
           const int64_t s0 = (f0 + c0 - 1) / c0;
           const int64_t s1 = two_n ? (f1 + bn / c0 - 1) / (bn / c0) : 1;
           const uint32_t c1 = two_n ? (uint32_t)((f1 + s1 - 1) / s1) : 1;

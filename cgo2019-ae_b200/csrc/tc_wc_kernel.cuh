@@ -28,7 +28,12 @@
 // letting the groups take turns on the tensor pipe made that worse.  What is left exposed is the epilogue itself:
 // 128 KB of shared-memory traffic per tile, about 1000 cycles beside 5600 of products at K = 40.
 //
-// Needs the output to be a rank-<=5 tensor in which a BM x 64 tile is one box (the planner's tma_ct test) and
+// Tiles: BM x 64, or BM x 32 where N is a short index (K = 64, 24 columns: 82 against 124 us), laid over one or two
+// dimensions of each class (TcCut).  A tile that takes b0 < BM values of the output's fastest index is a box too -- runs
+// of b0, the tile's n, then M's second dimension -- and the buffer has that order; operand rows are decoded digit by
+// digit.  Gathered operands get four producer warps (two: the gather set the pace).
+//
+// Needs the output to be a rank-<=5 tensor in which a cut tile is one box (plan_boxes in tc_plan.cpp) and
 // 16-byte aligned; rows and columns beyond the tensor are filled with zeros on load and clipped on store by
 // the copy engine.  Every mbarrier wait is bounded (args.spin_limit) and reports through args.status.
 #pragma once

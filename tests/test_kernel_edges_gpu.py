@@ -28,6 +28,7 @@ CUT = [
     "C [a,10,b,26,c,7,d,5,e,4,f,3] = sum(g,22) * A [d,f,g,a] * B [g,e,b,c];",
     "C [a,24,b,6,c,10,d,8,e,6,f,5] -= sum(g,24) * A [d,f,g,b] * B [g,e,a,c];",     # six dimensions, two sharing one of the map
     "C [a,2,b,40,c,30,d,9] += sum(e,8) * A [a,e,b,d] * B [e,c];",                  # shortest runs
+    "C [a,24,b,42,c,20,d,9] += sum(e,24) * A [e,a,c] * B [b,e,d];",                # an input read in pairs along N's first index
     "C [a,30,b,7,c,26,d,10] += sum(e,33) * A [d,c,e,a] * B [e,b];",                # narrow tile's shape, ragged both ways
 ]
 

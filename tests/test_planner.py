@@ -336,6 +336,15 @@ def test_cut_tiles_cover_the_output_once_and_are_boxes_of_it(pkg, expr):
     assert (seen == 1).all()
 
 
+def test_cut_tiles_keep_pairs_of_an_input_together(pkg):
+    """An input read 16 bytes at a time along N's first index: a tile starts at an even value of it and holds an even
+    number (21 of 42 would save a third of the tiles)."""
+    d = _plan(pkg, "C [a,24,b,42,c,200,d,9] += sum(e,24) * A [e,a,c] * B [b,e,d];", tile=(128, 64), variant=4).describe()
+    assert d["vec_y"] and d["cbox"]["n"][0] % 2 == 0 and d["cbox"]["n"][2] == 42
+    odd = _plan(pkg, "C [a,24,b,43,c,200,d,9] += sum(e,24) * A [e,a,c] * B [b,e,d];", tile=(128, 64), variant=4).describe()
+    assert not odd["vec_y"] and "cbox" in odd
+
+
 def test_blocked_contractions_name_every_value_once(pkg):
     """Two inputs that start with different contraction indices: 4 x 4 blocks of K, rounded up, with holes."""
     for c, d in ((64, 64), (61, 66), (4, 130), (63, 5)):
