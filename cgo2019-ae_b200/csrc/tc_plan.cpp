@@ -745,7 +745,18 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   else if (persistent) ksplit = 1;
   else if (p->opt.split_k > 1) ksplit = std::min<int64_t>(p->opt.split_k, ksteps);
   else if (p->opt.split_k == 0 && tiles * 2 <= sms && ksteps >= 16)
+  {
     ksplit = std::max<int64_t>(1, std::min<int64_t>((2 * sms) / tiles, ksteps / 8));
+    // fp64, 64 x 64: four CTAs fit an SM, and two of them leave its pipe half fed; slices of at least 16 steps fill all
+    // four (312 x 296 summed over 312 x 312, an operand loaded by vector: 25 tiles in 11 slices 1080 us, in 23 858 us).
+    // Plans whose scratch fits the allocation-free entry's array keep doing so.
+    if (c.math == TC_MATH_DMMA && bm == 64 && bn == 64) {
+      int64_t wide = std::min<int64_t>((4 * sms) / tiles, ksteps / 16);
+      const int64_t fits = (int64_t)TC_NOALLOC_MAX_WORKSPACE_BYTES / (tiles * bm * bn * es);
+      if (ksplit <= fits) wide = std::min(wide, fits);
+      ksplit = std::max(ksplit, wide);
+    }
+  }
   // The tensor cores accumulate fp32 with truncation: measured against exact sums on B200 the relative error of
   // one accumulation chain grows linearly with its length (2e-6 at K = 256, 7e-6 at 1024, 3e-5 at 4096), for
   // mma.sync and tcgen05 alike, while FFMA stays at 1e-6.  No tensor-core plan therefore runs a chain longer
