@@ -70,7 +70,8 @@ struct WtCfg {
   static constexpr int YIMG = ANY_TMA ? (YIMG_RAW + 255) / 256 * 256 : YIMG_RAW;
   static constexpr int STAGE_ELEMS = XIMG + YIMG;
   static constexpr uint32_t TMA_BYTES = (TMAX || TMAXE ? BM * BK * 4 : 0) + (TMAY || TMAYE ? BN * BK * 4 : 0);
-  static constexpr int FULL_ARRIVALS = THREADS + (ANY_TMA ? 1 : 0);  // the loaders' copies, and the announcement of the boxes
+  static constexpr bool BOXES = (TMAX || TMAXE) && (TMAY || TMAYE);  // both operands: one thread is the whole loader role
+  static constexpr int FULL_ARRIVALS = BOXES ? 1 : THREADS + (ANY_TMA ? 1 : 0);  // the loaders' copies, and the announcement of the boxes
   static constexpr int UMMA_ELEMS = 2 * BK * BM;         // hi and lo images of X for one K step (those of Y live in tensor memory)
   static constexpr int GROUPS = 1;                       // tiles a CTA works on at a time (launch arithmetic)
   // Six warpgroups: epilogue, epilogue, split, split, loaders, {MMA, fetch, store, a warp without work}.
@@ -438,6 +439,33 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wt_tf32_kernel(const __
     // -------------------------------------------------------------- loaders ----
     reg_inc<CF::LOADER_REGS>();
     const int ptid = tid - 512;
+    if constexpr (CF::BOXES) {
+      // Nothing but boxes: no offsets to look up and no other thread to meet (as one of 128 loaders that passed the
+      // contraction offsets from step to step -- a global load, a shared store, a barrier -- 562 instead of 555 us on
+      // 4096 x 4096 x 2048).
+      if (ptid != 0) return;
+      uint32_t g = 0;
+      for (uint32_t tile = first; tile < total; tile += step) {
+        uint32_t tm, tn;
+        tile_coords(p, tile, &tm, &tn);
+        const int m0 = (int)(tm * BM), n0 = (int)(tn * BN);
+        for (int it = 0; it < nk; ++it, ++g) {
+          const uint32_t s = g % STAGES;
+          if (g >= (uint32_t)STAGES && !mbar_wait(empty + s, ((g / STAGES) - 1) & 1u, p.status, 14, limit)) return;
+          // tests only: one stage is left unannounced, so that the waits on it run out
+          if (p.test_fault == 1 && blockIdx.x == 0 && g == 1) continue;
+          const int k0 = (int)(kbeg + it * BK);
+          float* xs = stages + s * CF::STAGE_ELEMS;
+          float* ys = xs + CF::XIMG;
+          mbar_arrive_expect_tx(full + s, CF::TMA_BYTES);
+          if constexpr (CF::TMAX) tma_load_2d(xs, &p.tmap_x, k0, m0, full + s);
+          else tma_load_2d(xs, &p.tmap_x, m0, k0, full + s);
+          if constexpr (CF::TMAY) tma_load_2d(ys, &p.tmap_y, k0, n0, full + s);
+          else tma_load_2d(ys, &p.tmap_y, n0, k0, full + s);
+        }
+      }
+      return;
+    }
     WtSlots<CF, BM, CF::MODEX, CF::LDX> slots_x;
     WtSlots<CF, BN, CF::MODEY, CF::LDY> slots_y;
     slots_x.init(ptid, p.lanes_k_x == 1 ? 0 : 3, p.M.extent[0]);
