@@ -184,22 +184,32 @@ BoxPlan plan_boxes(const std::vector<Dim>& dm, const std::vector<Dim>& dn, uint3
       if (lm.size() + ln.size() > 5 && !shared) continue;
       const int64_t e0 = lm[0].extent, e1 = two_m ? lm[1].extent : 1, f0 = ln.empty() ? 1 : ln[0].extent, f1 = two_n ? ln[1].extent : 1;
       const int64_t rest = product(lm, m_rest) * product(ln, ln.empty() ? 0 : n_rest);
+      // N's cuts, the one of fewest tiles first in line (its choice depends on M's only where a run and its n are one piece)
+      struct NCut { uint32_t c0, c1; int64_t s0, s1; double cost; };
+      std::vector<NCut> ncuts;
+      size_t fewest = 0;
+      for (uint32_t c0 = std::min<int64_t>(bn, f0); c0 >= 1; --c0) {
+        // (an input read in pairs along N's first index: pairs lie in one run and tiles start on 16 bytes)
+        if (uy == 0 && dn[0].extent % 2 == 0 && c0 % 2 != 0) continue;
+        const int64_t s0 = (f0 + c0 - 1) / c0;
+        const int64_t s1 = two_n ? (f1 + bn / c0 - 1) / (bn / c0) : 1;
+        const uint32_t c1 = two_n ? (uint32_t)((f1 + s1 - 1) / s1) : 1;
+        const double cost = (double)(s0 * s1) * (uy >= 0 ? gather(uy == 0 ? c0 : uy == 1 && two_n ? c1 : 1) : 1.0);
+        if (!ncuts.empty() && cost < ncuts[fewest].cost) fewest = ncuts.size();
+        ncuts.push_back({c0, c1, s0, s1, cost});
+      }
       for (uint32_t b0 = std::min<int64_t>(bm, e0); b0 >= 2; b0 -= 2) {
         const int64_t t0 = (e0 + b0 - 1) / b0;
         const int64_t t1 = two_m ? (e1 + bm / b0 - 1) / (bm / b0) : 1;
         const uint32_t b1 = two_m ? (uint32_t)((e1 + t1 - 1) / t1) : 1;
-        for (uint32_t c0 = std::min<int64_t>(bn, f0); c0 >= 1; --c0) {
-          // (an input read in pairs along N's first index: pairs lie in one run and tiles start on 16 bytes)
-          if (uy == 0 && dn[0].extent % 2 == 0 && c0 % 2 != 0) continue;
-          const int64_t s0 = (f0 + c0 - 1) / c0;
-          const int64_t s1 = two_n ? (f1 + bn / c0 - 1) / (bn / c0) : 1;
-          const uint32_t c1 = two_n ? (uint32_t)((f1 + s1 - 1) / s1) : 1;
+        const bool adjacent = b0 == e0 && !ln.empty() && ln[0].s_out == e0;
+        for (size_t nc = adjacent ? 0 : fewest; nc < (adjacent ? ncuts.size() : std::min(fewest + 1, ncuts.size())); ++nc) {
+          const uint32_t c0 = ncuts[nc].c0, c1 = ncuts[nc].c1;
+          const int64_t s0 = ncuts[nc].s0, s1 = ncuts[nc].s1;
           const double tiles = (double)(t0 * t1) * (double)(s0 * s1) * (double)rest;
           if (tiles >= 2.0e9) continue;
-          const bool adjacent = b0 == e0 && !ln.empty() && ln[0].s_out == e0;
-          double score = tiles * piece(8.0 * b0 * (adjacent ? c0 : 1));
+          double score = (double)(t0 * t1) * ncuts[nc].cost * (double)rest * piece(8.0 * b0 * (adjacent ? c0 : 1));
           if (ux >= 0) score *= gather(ux == 0 ? b0 : ux == 1 && two_m ? b1 : 1);
-          if (uy >= 0) score *= gather(uy == 0 ? c0 : uy == 1 && two_n ? c1 : 1);
           if (best.ok && score >= best.score) continue;
           best.ok = true;
           best.score = score;
@@ -431,23 +441,24 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   a.Kflat = (uint32_t)kf;
   p->kdims = kd;
 
-  // Contraction offset tables (one entry per flattened k).
+  // Contraction offset tables (one entry per flattened k), digits carried along as on an odometer.
   p->h_koff_x.assign(kf, 0);
   p->h_koff_y.assign(kf, 0);
-  for (int64_t k = 0; k < kf; ++k) {
-    int64_t r = k, ox = 0, oy = 0;
-    for (int d = 0; d < kd.n; ++d) {
-      const int64_t c = r % kd.extent[d];
-      r /= kd.extent[d];
-      ox += c * kd.s_in[d];
-      oy += c * kd.s_out[d];
+  {
+    int64_t digit[TC_MAX_DIMS] = {}, ox = 0, oy = 0;
+    for (int64_t k = 0; k < kf; ++k) {
+      const bool hole = kcut_x > 0 && (digit[0] + 4 * digit[2] >= kcut_x || digit[1] + 4 * digit[3] >= kcut_y);
+      p->h_koff_x[k] = hole ? -1 : ox;
+      p->h_koff_y[k] = hole ? -1 : oy;
+      for (int d = 0; d < kd.n; ++d) {
+        ox += kd.s_in[d];
+        oy += kd.s_out[d];
+        if (++digit[d] < (int64_t)kd.extent[d]) break;
+        ox -= (int64_t)kd.extent[d] * kd.s_in[d];
+        oy -= (int64_t)kd.extent[d] * kd.s_out[d];
+        digit[d] = 0;
+      }
     }
-    if (kcut_x > 0) {
-      const int64_t vx = k % 4 + 4 * (k / 16 % kd.extent[2]), vy = k / 4 % 4 + 4 * (k / 16 / kd.extent[2] % kd.extent[3]);
-      if (vx >= kcut_x || vy >= kcut_y) ox = oy = -1;
-    }
-    p->h_koff_x[k] = ox;
-    p->h_koff_y[k] = oy;
   }
 
   // Kernel family.
