@@ -189,6 +189,7 @@ int tc_fused_set_extents(tc_fused_plan* plan, int n, const char* const* index_na
 int tc_fused_commit(tc_fused_plan* plan);
 /* JSON: box shape, boxes, rows x cols per term, flops, bytes moved fused and term by term. */
 int tc_fused_describe(tc_fused_plan* plan, char* buf, size_t cap);
+/* TC_ERR_DEVICE_WAIT: a bounded wait in an earlier launch of this plan gave up, its output is invalid. */
 int tc_execute_fused(tc_fused_plan* plan, void* C, const void* const* A, const void* const* B, void* stream);
 void tc_fused_destroy(tc_fused_plan* plan);
 
