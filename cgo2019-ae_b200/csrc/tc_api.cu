@@ -371,8 +371,8 @@ int tc_launch_contraction(const tc_plan& p, const TcKernelArgs& args, void* C, c
     const unsigned want = (8u * (unsigned)p.sm_count + tiles - 1) / tiles;  // eight CTAs of 256 threads fill an SM
     const dim3 grid(tiles, std::max(1u, std::min(want, most)));
     const size_t smem = (size_t)(a.bm + a.bn) * sizeof(int64_t);
-    if (p.dtype == TC_F64) TC_CUDA_OK(tck::launch_chained(tck::tc_combine_kernel<double>, grid, 256, smem, stream, a, static_cast<double*>(C)));
-    else TC_CUDA_OK(tck::launch_chained(tck::tc_combine_kernel<float>, grid, 256, smem, stream, a, static_cast<float*>(C)));
+    if (p.dtype == TC_F64) TC_CUDA_OK(tck::launch_chained(true, tck::tc_combine_kernel<double>, grid, 256, smem, stream, a, static_cast<double*>(C)));
+    else TC_CUDA_OK(tck::launch_chained(true, tck::tc_combine_kernel<float>, grid, 256, smem, stream, a, static_cast<float*>(C)));
   }
   return TC_OK;
 }
