@@ -309,9 +309,10 @@ int tc_launch_contraction(const tc_plan& p, const TcKernelArgs& args, void* C, c
     // The C-resident kernel moves whole output tiles as boxes of the rank-5 view of C: the view must exist and the
     // base must be 16-byte aligned.  Otherwise the same tiles run on the persistent kernel that reaches C through
     // reduce-adds or plain read-modify-writes.
-    const bool ok = c.box_c && p.opt.tma != 1 && p.opt.tma != 2 && encode_box_output_map(&a.tmap_ct, C, a.cbox);
+    const bool ok = c.box_c && encode_box_output_map(&a.tmap_ct, C, a.cbox);
     if (ok) a.c_tensor = 0;
     if (!ok) {
+      a.vec_c = std::min(a.vec_c, a.standin_vec_c);
       TcKernelChoice alt = c;
       alt.variant = 2;
       fn = pick_inst(alt);

@@ -123,6 +123,7 @@ struct TcKernelArgs {
   int32_t lanes_k_y;
   int32_t kstep_x, kstep_y;  // ... and the step between the positions that neighbouring lanes take (1 or 4; persistent fp64 kernels)
   int32_t vec_c;     // contiguous output elements a thread may touch with one access (1, 2 or 4)
+  int32_t standin_vec_c;  // ... on the kernel that runs an output-resident plan's cut tiles where C cannot be boxes
   int32_t beta;      // 1: C is read and accumulated into; 0: C is overwritten
   double alpha;      // +1 or -1
   void* ws;          // K-slice partials: [ksplit][tiles][BN][BM]

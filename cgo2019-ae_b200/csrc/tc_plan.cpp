@@ -672,8 +672,10 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     }
     if (p->opt.variant > 0) variant = p->opt.variant - 1;
   }
+  // (tma 1 and 2 keep the copy engine away from C: such a plan runs on the stand-in and keeps its plain tiles)
   int box_order = -1;
-  if (variant == 3 && c.math == TC_MATH_DMMA && p->box_order < 0 && best_boxes((uint32_t)bm, (uint32_t)bn, &box_order).ok) {
+  const bool boxes_allowed = p->opt.tma != 1 && p->opt.tma != 2;
+  if (variant == 3 && c.math == TC_MATH_DMMA && boxes_allowed && p->box_order < 0 && best_boxes((uint32_t)bm, (uint32_t)bn, &box_order).ok) {
     p->box_order = box_order;  // plan again with M's dimensions whole and in that order
     const int st = tc_plan_build(p, why);
     p->box_order = -1;
@@ -696,13 +698,17 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   a.rows_across_x = a.rows_across_y = 0;
   c.box_c = false;
   bool plain_m = true, plain_n = true;  // tiles are plain ranges of the flattened index
-  if (tc_kernel_is_c_resident(c)) {
+  a.standin_vec_c = a.vec_c;
+  if (tc_kernel_is_c_resident(c) && boxes_allowed) {
     const BoxPlan bp = plan_boxes(dm, dn, (uint32_t)bm, (uint32_t)bn);
     if (bp.ok) {
       c.box_c = true;
       a.mcut = bp.m;
       a.ncut = bp.n;
       a.cbox = bp.map;
+      // The stand-in's epilogue takes four consecutive rows as four neighbours in C: true inside a cut tile only where
+      // its runs are whole fours.  Else it goes element by element.
+      if (bp.m.b0 % 4 != 0) a.standin_vec_c = std::min(a.vec_c, 2);
       a.rows_across_x = bp.across_x;
       a.rows_across_y = bp.across_y;
       const int64_t tm = mf / ((int64_t)bp.m.e0 * bp.m.e1) * bp.m.t0 * bp.m.t1, tn = nf / ((int64_t)bp.n.e0 * bp.n.e1) * bp.n.t0 * bp.n.t1;
@@ -866,7 +872,7 @@ std::string tc_plan_to_json(const tc_plan& p) {
       << ",\"tma_y\":" << (p.choice.tma_y ? "true" : "false") << ",\"tma_xe\":" << (p.choice.tma_xe ? "true" : "false")
       << ",\"tma_ye\":" << (p.choice.tma_ye ? "true" : "false") << ",\"tma_c\":" << (p.choice.tma_c ? "true" : "false") << ",\"tma_ct\":" << (p.choice.tma_ct ? "true" : "false")
       << ",\"lanes_k_x\":" << a.lanes_k_x
-      << ",\"lanes_k_y\":" << a.lanes_k_y << ",\"vec_c\":" << a.vec_c << ",\"box\":[" << a.mcut.b0 << "," << a.mcut.b1 << "," << a.ncut.b0 << "," << a.ncut.b1 << "]" << ",\"epi_run\":" << a.epi_run << ",\"epi_n_span\":" << a.epi_n_span << ",\"beta\":" << a.beta
+      << ",\"lanes_k_y\":" << a.lanes_k_y << ",\"vec_c\":" << a.vec_c << ",\"standin_vec_c\":" << a.standin_vec_c << ",\"box\":[" << a.mcut.b0 << "," << a.mcut.b1 << "," << a.ncut.b0 << "," << a.ncut.b1 << "]" << ",\"epi_run\":" << a.epi_run << ",\"epi_n_span\":" << a.epi_n_span << ",\"beta\":" << a.beta
       << ",\"alpha\":" << a.alpha << ",\"workspace_bytes\":" << p.ws_bytes << ",\"launches\":" << p.launches
       << ",\"flops\":" << p.flops << ",\"bytes\":" << p.bytes;
     if (p.choice.box_c) {

@@ -55,6 +55,17 @@ def test_cut_tiles_of_a_misaligned_output_run_without_boxes(pkg, orc):
     plan.close()
 
 
+@pytest.mark.parametrize("c_path", [0, 2])
+@pytest.mark.parametrize("tma", [1, 2])
+@pytest.mark.parametrize("expr", [
+    "C [a,28,b,60,c,20,d,60] += sum(g,200) * A [d,a,g,b] * B [g,c];",               # the boxes would hold runs of 14
+    "C [a,36,b,40,c,7,d,12] += sum(e,16) * A [e,a,c] * B [e,b,d];",                 # ... of 18
+])
+def test_output_resident_plans_kept_from_the_copy_engine(pkg, orc, expr, tma, c_path):
+    d, err = _run(pkg, orc, expr, tile=(128, 64), variant=4, tma=tma, c_path=c_path)
+    assert "cbox" not in d and err <= 1e-12
+
+
 @pytest.mark.parametrize("c,d", [(61, 66), (64, 64), (4, 150), (63, 5), (3, 3)])
 @pytest.mark.parametrize("split", [0, 3])
 def test_blocked_contractions_against_the_loop_nest(pkg, orc, c, d, split):

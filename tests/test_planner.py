@@ -353,3 +353,38 @@ def test_blocked_contractions_name_every_value_once(pkg):
         assert p["Kflat"] == (c + 3) // 4 * 4 * ((d + 3) // 4 * 4)
     small = _plan(pkg, "t3 [a,20,b,20] += sum(c,6,d,7) * t2 [c,a,d] * v2 [d,b,c];").describe()
     assert small["Kflat"] == 42   # kernels that know no holes keep the plain order
+
+
+def _short_run_cuts():
+    """Output-resident plans whose cuts hold runs that are not whole fours (14 of 28, 18 of 36, ...)."""
+    yield "C [a,28,b,60,c,20,d,60] += sum(g,200) * A [d,a,g,b] * B [g,c];"
+    yield "C [a,36,b,40,c,7,d,12] += sum(e,16) * A [e,a,c] * B [e,b,d];"
+    yield "C [a,52,b,44,c,9,d,52] -= sum(e,24) * A [d,a,e,b] * B [e,c];"
+
+
+@pytest.mark.parametrize("expr", list(_short_run_cuts()) + list(_wc_layouts()))
+def test_rows_the_stand_in_takes_together_are_neighbours_in_the_output(pkg, expr):
+    """Where an output cannot be addressed as boxes, the cut tiles run on a kernel that moves standin_vec_c consecutive
+    rows of a tile as neighbours in C."""
+    import numpy as np
+    d = _plan(pkg, expr, tile=(128, 64), variant=4).describe()
+    b0, b1, e0, e1, t0, t1 = d["cbox"]["m"] if "cbox" in d else (128, 1, d["Mflat"], 1, d["tiles"][0], 1)
+    off = np.zeros(1, dtype=np.int64)
+    for q in d["M"]:
+        off = (np.arange(q["extent"], dtype=np.int64)[:, None] * q["s_out"] + off[None, :]).reshape(-1)
+    for t in range(d["tiles"][0]):
+        v0, v1, rest = t % t0 * b0, t // t0 % t1 * b1, t // t0 // t1
+        rows = [v0 + r % b0 + e0 * (v1 + r // b0 + e1 * rest) if r < b0 * b1 and v0 + r % b0 < e0 and v1 + r // b0 < e1 else -1
+                for r in range(128)]
+        for r in range(0, 128, 4) if d["standin_vec_c"] == 4 else ():
+            four = [off[q] if q >= 0 else -1 for q in rows[r:r + 4]]
+            assert four == [-1] * 4 or four == [four[0] + i for i in range(4)], (d["cbox"]["m"], t, r)
+
+
+@pytest.mark.parametrize("tma", [1, 2])
+@pytest.mark.parametrize("expr", list(_short_run_cuts()))
+def test_outputs_kept_from_the_copy_engine_have_plain_tiles(pkg, expr, tma):
+    boxes = _plan(pkg, expr, tile=(128, 64), variant=4).describe()
+    assert boxes["cbox"]["m"][0] % 4 == 2 and boxes["vec_c"] == 4 and boxes["standin_vec_c"] == 2
+    plain = _plan(pkg, expr, tile=(128, 64), variant=4, tma=tma).describe()
+    assert "cbox" not in plain and plain["tiles"] == [(plain["Mflat"] + 127) // 128, (plain["Nflat"] + 63) // 64]
