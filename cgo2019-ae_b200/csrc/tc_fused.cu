@@ -523,7 +523,8 @@ static bool encode_box_map(TcTensorMap* out, const void* base, const FusedArgs& 
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Host part of commit: box shape and per-term tables (needs no GPU).
+// Host part of commit: box shape and per-term tables (needs no GPU).  Whatever an earlier commit that failed has left in
+// the plan is built anew.
 static int fused_build(tc_fused_plan* p) {
   const TcExpr& e0 = p->terms[0];
   const int rank = (int)e0.out_idx.size();
@@ -636,6 +637,8 @@ static int fused_build(tc_fused_plan* p) {
     };
     T.kfast_x = mode_of(e.left_idx);
     T.kfast_y = mode_of(e.right_idx);
+    p->box_x[k].clear();
+    p->box_y[k].clear();
     for (const Cls& c : cm) p->box_x[k].push_back({c.out_pos, c.s_in});
     for (const Cls& c : cn) p->box_y[k].push_back({c.out_pos, c.s_in});
     double prod = out_elems * (double)kf;
@@ -676,9 +679,24 @@ static void fused_koff(const tc_fused_plan* p, size_t k, std::vector<int64_t>* k
 
 static int fused_smem_bytes(int n_terms) { return (kBoxElems + 2 * kStages * IMG) * 8 + n_terms * (2 * kBox * 8 + 2 * kTabK * 8 + 2 * kBox * 4); }
 
+// Gives back what a commit has allocated.
+static void fused_release(tc_fused_plan* p) {
+  for (int64_t* d : p->d_koff) cudaFree(d);
+  p->d_koff.clear();
+  if (p->d_terms) cudaFree(p->d_terms);
+  if (p->d_box_off) cudaFree(p->d_box_off);
+  if (p->d_pos) cudaFree(p->d_pos);
+  if (p->h_status) cudaFreeHost(p->h_status);
+  p->d_terms = nullptr;
+  p->d_box_off = nullptr;
+  p->d_pos = nullptr;
+  p->h_status = nullptr;
+}
+
 extern "C" int tc_fused_commit(tc_fused_plan* p) {
   if (!p) return TC_ERR_INVALID_ARG;
   if (p->committed) return TC_OK;
+  fused_release(p);  // a commit that failed half-way
   int st = fused_build(p);
   if (st != TC_OK) return st;
   int dev = 0;
@@ -772,11 +790,7 @@ extern "C" int tc_execute_fused(tc_fused_plan* p, void* C, const void* const* A,
 
 extern "C" void tc_fused_destroy(tc_fused_plan* p) {
   if (!p) return;
-  for (int64_t* d : p->d_koff) cudaFree(d);
-  if (p->d_terms) cudaFree(p->d_terms);
-  if (p->d_box_off) cudaFree(p->d_box_off);
-  if (p->d_pos) cudaFree(p->d_pos);
-  if (p->h_status) cudaFreeHost(p->h_status);
+  fused_release(p);
   delete p;
 }
 
@@ -785,9 +799,7 @@ extern "C" int tc_fused_describe(tc_fused_plan* p, char* buf, size_t cap) {
   tc_fused_plan tmp;
   const tc_fused_plan* q = p;
   if (!p->committed) {  // run the host part on a copy (needs no GPU)
-    tmp.terms = p->terms;
-    tmp.idx_names = p->idx_names;
-    tmp.idx_extent = p->idx_extent;
+    tmp = *p;
     const int st = fused_build(&tmp);
     if (st != TC_OK) {
       std::snprintf(buf, cap, "{\"error\":\"%s\"}", tmp.why.c_str());
@@ -801,6 +813,19 @@ extern "C" int tc_fused_describe(tc_fused_plan* p, char* buf, size_t cap) {
   for (int i = 0; i < q->args.rank; ++i) o << (i ? "," : "") << q->args.b[i];
   o << "],\"boxes\":" << q->args.total_boxes << ",\"box_elems\":" << q->args.box_elems << ",\"rows_cols\":[";
   for (size_t k = 0; k < q->h_terms.size(); ++k) o << (k ? "," : "") << "[" << q->h_terms[k].rows << "," << q->h_terms[k].cols << "]";
+  o << "],\"maps\":[";  // per term: the output indices that its left and its right input's map carry
+  for (size_t k = 0; k < q->h_terms.size(); ++k) {
+    auto carried = [&](const std::vector<tc_fused_plan::BoxDim>& dims) {
+      o << "[";
+      for (size_t d = 0; d < dims.size(); ++d) o << (d ? "," : "") << dims[d].out_pos;
+      o << "]";
+    };
+    o << (k ? ",[" : "[");
+    carried(q->box_x[k]);
+    o << ",";
+    carried(q->box_y[k]);
+    o << "]";
+  }
   o << "],\"flops\":" << q->flops << ",\"bytes\":" << q->bytes_fused << ",\"bytes_term_by_term\":" << q->bytes_separate
     << ",\"kernel\":\"" << (q->box_kernel ? "tc_fused_box_kernel" : "tc_fused_kernel") << "\",\"launches\":1}";
   const std::string s = o.str();

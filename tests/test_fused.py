@@ -44,6 +44,55 @@ def test_fused_plan_shape_without_a_gpu(pkg):
     assert one["box"] == [40, 40] and one["rows_cols"] == [[40, 40]]
 
 
+def _retried(pkg, lines):
+    """A plan whose first commit met a limit in its last term, given extents that fit."""
+    plan = pkg.FusedPlan(lines, extents={"q7": 1 << 31})
+    with pytest.raises(pkg.TcError) as e:
+        plan.commit()
+    assert e.value.status == 3
+    names = (pkg.ctypes.c_char_p * 1)(b"q7")
+    assert pkg.lib().tc_fused_set_extents(plan._h, 1, names, (pkg.ctypes.c_int64 * 1)(16)) == 0
+    return plan
+
+
+RETRIED = [
+    ["t3 [a,33,b,20] += sum(p7,16) * x1 [p7,a] * y1 [p7,b];", "t3 [a,33,b,20] -= sum(q7,16) * x2 [q7,a] * y2 [q7,b];"],
+    ["t3 [a,8,b,9,c,5,d,7] += sum(p7,16) * x1 [p7,c,a] * y1 [p7,b,d];", "t3 [a,8,b,9,c,5,d,7] -= sum(q7,16) * x2 [q7,b,a] * y2 [q7,d,c];"],
+    ["t3 [h3,8,h2,8,h1,4,p6,5,p5,4,p4,9] += sum(p7,10) * x1 [p7,p4,h1,h2] * y1 [p7,h3,p6,p5];",
+     "t3 [h3,8,h2,8,h1,4,p6,5,p5,4,p4,9] += sum(q7,10) * x2 [q7,p5,h1,h2] * y2 [q7,h3,p6,p4];"],
+]
+
+
+@pytest.mark.parametrize("lines", RETRIED)
+def test_a_commit_after_one_that_failed_builds_the_plan_anew(pkg, lines):
+    got = _retried(pkg, lines).describe()
+    fresh = pkg.FusedPlan(lines, extents={"q7": 16}).describe()
+    assert got == fresh and got["kernel"] == "tc_fused_box_kernel"
+    for left, right in got["maps"]:
+        assert sorted(left + right) == list(range(got["rank"]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lines", RETRIED)
+def test_a_plan_committed_on_a_second_try_against_the_loop_nests(pkg, orc, lines):
+    import torch
+    torch.cuda.set_device(0)
+    sized = [lines[0], lines[1].replace("q7,10)", "q7,16)")]
+    plan = _retried(pkg, lines)
+    c0 = orc.uniform(62, 0, orc.sizes(lines[0])[0])
+    ref, ins = c0.copy(), []
+    for n, line in enumerate(sized):
+        _, na, nb = orc.sizes(line)
+        a, b = orc.uniform(63 + n, 1, na), orc.uniform(63 + n, 2, nb)
+        orc.contract(line, ref, a, b)
+        ins.append((torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()))
+    dc = torch.from_numpy(c0).cuda()
+    plan.execute(dc, [a for a, _ in ins], [b for _, b in ins])
+    torch.cuda.synchronize()
+    assert orc.rel_error(dc.cpu().numpy(), ref) <= 1e-12
+    plan.close()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("name,terms,sum_name,ext", [
     ("sd2", SD2, "p7", dict(h3=16, h2=16, h1=16, p6=16, p5=16, p4=16, p7=16)),
