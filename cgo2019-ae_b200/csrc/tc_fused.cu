@@ -15,7 +15,7 @@
 // (DMMA m8n8k4, same fragment mapping as tc_contract_kernel) and the accumulators are scattered into the box with
 // the term's own (row, col) -> box-offset tables.  After the last term the box is added to C once.
 // fp64 only.  Operator per term: += or -=.  Plans whose inputs can arrive as tiled boxes run on tc_fused_box_kernel
-// (tc_fused_box.cuh) instead: 3.95 against 9.78 ms on the nine doubles terms of CCSD(T), extents 24.
+// (tc_fused_box.cuh) instead: 3.93 against 9.78 ms on the nine doubles terms of CCSD(T), extents 24.
 #include <cuda.h>  // types of the tensor-map encoder only; the entry point is looked up at run time
 #include <cuda_runtime.h>
 

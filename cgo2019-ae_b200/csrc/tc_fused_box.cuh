@@ -10,8 +10,9 @@
 //     zeros outside the tensor), up to kBoxStages stages ahead and across terms and boxes;
 //   * eight CONSUMER warps (32 x 16 products each) wait per stage on mbarriers and once per term, before they
 //     add the term's products to the box, for the other warps' additions of the term before;
-//   * the box starts from C (asynchronous copies issued when the previous box has left, hidden behind the first
-//     term's products) and leaves as plain stores.
+//   * the first term's products are stored, the others' added; C's old values are read and the box added to them
+//     once, at the end, as in tc_fused_kernel: one rounding against C's magnitude however many terms there are (a box
+//     that starts from C has every term rounded against it; no faster either, 3.94 against 3.93 ms).
 //
 // Shared-memory layouts.  Operand images are [row][16 k], the 16-byte chunk c of row r at chunk position c ^ (r & 7).
 // A thread reads two consecutive k at once; MMA number 2 h + e of a stage takes k = 8 h + 2 t + e in slot t, for both
@@ -22,12 +23,13 @@
 // codes (found by search) make these four independent, so without bank conflicts, for every term of the CCSD(T) doubles
 // and for four in five of all assignments of six indices (two-way at most in the rest).
 //
-// Measured (nine doubles terms of CCSD(T), all extents 24, one B200): 9.78 ms on tc_fused_kernel, 3.95 ms here (20.9
-// TFLOP/s, 56 % of the DMMA rate; floor 2.23 ms of products).  On the way: one block barrier per term 4.76 ms; a barrier
+// Measured (nine doubles terms of CCSD(T), all extents 24, one B200): 9.78 ms on tc_fused_kernel, 3.93 ms here (21.1
+// TFLOP/s, 57 % of the DMMA rate; floor 2.23 ms of products).  On the way: one block barrier per term 4.76 ms; a barrier
 // that warps only arrive at when their additions are done, 104 registers a thread, eight old values read together 4.49;
-// positions as byte offsets, no tests in whole terms 4.14; conflict-free codes and both halves' reads first 3.95.  Without
-// any loads 4.43 of the 4.49 remained, the loads alone take 2.07, without the additions 3.68: what is left is the chain
-// of a term (wait, fragments, products, additions) with two CTAs of eight warps to cover it.
+// positions as byte offsets, no tests in whole terms 4.14; conflict-free codes and both halves' reads first 3.95; the
+// first term stored, C added at the end 3.93.  Without any loads 4.43 of the 4.49 remained, the loads alone take 2.07,
+// without the additions 3.68: what is left is the chain of a term (wait, fragments, products, additions) with two CTAs
+// of eight warps to cover it.
 #pragma once
 #include "tc_ws_kernel.cuh"
 
@@ -100,7 +102,7 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
   uint64_t* full = reinterpret_cast<uint64_t*>(s_pos + kMaxTerms * 2 * kBox);  // [stages]
   uint64_t* empty = full + kBoxStages;
   uint64_t* added = empty + kBoxStages;  // every warp has added its products of a term to the box
-  uint64_t* c_ready = added + 1;         // the box holds C
+  uint64_t* left = added + 1;            // every warp has read its part of the finished box
   unsigned char* box_b = reinterpret_cast<unsigned char*>(box);
   const uint32_t stage0 = tck::smem_u32(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -108,7 +110,7 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
   if (tid == 0) {
     for (int s = 0; s < kBoxStages; ++s) { tck::mbar_init(full + s, 1); tck::mbar_init(empty + s, kConsumers / 32); }
     tck::mbar_init(added, kConsumers / 32);
-    tck::mbar_init(c_ready, kConsumers);
+    tck::mbar_init(left, kConsumers / 32);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   for (int i = tid; i < p.n_terms * 2 * kBox; i += kBoxThreads) s_pos[i] = p.pos[i];
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
     *crd = c;
   };
   split((uint32_t)tid, &off_lo, &crd_lo);
-  int64_t* s_off_hi = reinterpret_cast<int64_t*>(c_ready + 1);            // [16]
+  int64_t* s_off_hi = reinterpret_cast<int64_t*>(left + 1);              // [16]
   uint64_t* s_crd_hi = reinterpret_cast<uint64_t*>(s_off_hi + 16);      // [16]
   if (tid < 16) split((uint32_t)tid << 8, &s_off_hi[tid], &s_crd_hi[tid]);
   const uint32_t pos_lo = box_hash((uint32_t)tid);
@@ -195,23 +197,12 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
     *last = l;
   };
   auto valid = [&](uint64_t crd, uint64_t last) { return ((last - crd) & 0x8080808080808080ull) == 0x8080808080808080ull; };
-  const uint32_t box_u32 = tck::smem_u32(box);
-  auto fetch_c = [&](int64_t base, uint64_t last) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const bool ok = valid(crd_lo + s_crd_hi[i], last);
-      const double* src = C + base + (ok ? off_lo + s_off_hi[i] : 0);
-      tck::cp_async8(box_u32 + (pos_lo ^ box_hash((uint32_t)i << 8)) * 8u, src, ok);
-    }
-    tck::mbar_arrive_on_copies(c_ready);
-  };
 
   int64_t base = 0;
   uint64_t last = 0;
-  corner_of(blockIdx.x, &base, &last);
-  fetch_c(base, last);
   uint32_t it = 0, terms = 0, boxes = 0;  // stages, terms and boxes so far
   for (uint32_t bx = blockIdx.x; bx < p.total_boxes; bx += gridDim.x, ++boxes) {
+    corner_of(bx, &base, &last);
     for (int k = 0; k < p.n_terms; ++k) {
       double acc[2][4][2];
 #pragma unroll
@@ -252,10 +243,11 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
         __syncwarp();
         if (lane == 0) tck::mbar_arrive(&empty[s]);
       }
-      // The products of this term go into the box: every (row, column) is one distinct element.  Another warp may hold
-      // the same element in the term before (or, for the first term, its value of C may be on its way): a warp waits
-      // for all warps' additions of that term, and has its own term's products meanwhile.  Eight elements are read before
-      // any is written: one by one, which is what the compiler must do where they could meet, costs sixteen round trips.
+      // The products of this term go into the box: every (row, column) is one distinct element, and a term's rows and
+      // columns are the whole box.  Another warp may hold the same element in the term before (or, for the first term,
+      // still read it out): a warp waits for all warps' additions of that term (for the box before to have left), and
+      // has its own term's products meanwhile.  Eight elements are read before any is written: one by one, which is
+      // what the compiler must do where they could meet, costs sixteen round trips.
       const int32_t* pm = s_pos + k * 2 * kBox + wm0 + t;
       const int32_t* pn = s_pos + k * 2 * kBox + kBox + wn0 + pg;
       const double alpha = p.term[k].alpha;
@@ -266,9 +258,15 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
         for (int h = 0; h < 2; ++h) qm[2 * i + h] = pm[8 * i + 4 * h];
 #pragma unroll
       for (int j = 0; j < 2; ++j) qn[j] = pn[8 * j];
-      if (!dead && !(k == 0 ? box_wait(c_ready, boxes & 1, p.status, 4, p.spin_limit) : box_wait(added, (terms - 1) & 1, p.status, 5, p.spin_limit)))
+      if (!dead && !(k == 0 ? boxes == 0 || box_wait(left, (boxes - 1) & 1, p.status, 4, p.spin_limit) : box_wait(added, (terms - 1) & 1, p.status, 5, p.spin_limit)))
         dead = true;
-      if (p.term[k].full) {  // 64 rows and columns: nothing to test
+      if (k == 0) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if ((qm[i] | qn[j]) >= 0) *reinterpret_cast<double*>(box_b + (qm[i] ^ qn[j])) = alpha * acc[j][i >> 1][i & 1];
+      } else if (p.term[k].full) {  // 64 rows and columns: nothing to test
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           double old[8];
@@ -293,15 +291,16 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
       if (lane == 0) tck::mbar_arrive(added);
       ++terms;
     }
-    // ---- the box leaves; the next one's values of C take its place ----
+    // ---- the box is added to C: the old values are on their way before the last term's additions are waited for ----
+    double old[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) old[i] = valid(crd_lo + s_crd_hi[i], last) ? C[base + off_lo + s_off_hi[i]] : 0.0;
     if (!dead && !box_wait(added, (terms - 1) & 1, p.status, 6, p.spin_limit)) dead = true;
 #pragma unroll
     for (int i = 0; i < 16; ++i)
-      if (valid(crd_lo + s_crd_hi[i], last)) C[base + off_lo + s_off_hi[i]] = box[pos_lo ^ box_hash((uint32_t)i << 8)];
-    if (bx + gridDim.x < p.total_boxes) {
-      corner_of(bx + gridDim.x, &base, &last);
-      fetch_c(base, last);
-    }
+      if (valid(crd_lo + s_crd_hi[i], last)) C[base + off_lo + s_off_hi[i]] = old[i] + box[pos_lo ^ box_hash((uint32_t)i << 8)];
+    __syncwarp();
+    if (lane == 0) tck::mbar_arrive(left);
   }
 }
 

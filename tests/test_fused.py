@@ -159,3 +159,30 @@ def test_fused_terms_with_other_shapes(pkg, orc):
         torch.cuda.synchronize()
         assert orc.rel_error(dc.cpu().numpy(), ref) <= 1e-12, lines[0]
         plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p7,kernel", [(16, "tc_fused_box_kernel"), (15, "tc_fused_kernel")])
+def test_terms_are_summed_before_they_meet_the_output(pkg, orc, p7, kernel):
+    """One rounding against C's magnitude however many terms there are: with values of C around 1e6 and terms around 1,
+    the result is within half a unit in the last place of C plus the exact sum of the terms (whose own error, 1e-12 of
+    their largest value as everywhere, is a thousandth of that unit)."""
+    import torch
+    torch.cuda.set_device(0)
+    lines = _lines(SD2, dict(h3=5, h2=8, h1=6, p6=4, p5=9, p4=7, p7=p7), "p7")
+    plan = pkg.FusedPlan(lines)
+    assert plan.describe()["kernel"] == kernel
+    c0 = orc.uniform(70, 0, orc.sizes(lines[0])[0]) * 1e6
+    total, ins = np.zeros_like(c0), []
+    for n, line in enumerate(lines):
+        _, na, nb = orc.sizes(line)
+        a, b = orc.uniform(71 + n, 1, na), orc.uniform(71 + n, 2, nb)
+        orc.contract(line, total, a, b)
+        ins.append((torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()))
+    dc = torch.from_numpy(c0).cuda()
+    plan.execute(dc, [a for a, _ in ins], [b for _, b in ins])
+    torch.cuda.synchronize()
+    got = dc.cpu().numpy()
+    off = np.abs(got.astype(np.longdouble) - (c0.astype(np.longdouble) + total.astype(np.longdouble)))
+    assert (off <= 0.5 * np.spacing(np.abs(got)) + 1e-12 * np.abs(total).max()).all()
+    plan.close()
