@@ -85,6 +85,9 @@ _SIGNATURES = {
                                             ctypes.POINTER(ctypes.c_int64)]),
     "tc_fused_commit": (ctypes.c_int, [ctypes.c_void_p]),
     "tc_fused_describe": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_size_t]),
+    "tc_fused_set_test_fault": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
+    "tc_fused_status": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)]),
+    "tc_fused_status_reset": (ctypes.c_int, [ctypes.c_void_p]),
     "tc_execute_fused": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p),
                                         ctypes.POINTER(ctypes.c_void_p), ctypes.c_void_p]),
     "tc_fused_destroy": (None, [ctypes.c_void_p]),
@@ -335,7 +338,7 @@ class FusedPlan:
     """Several contractions accumulated into one output in a single pass over it (e.g. the nine CCSD(T) terms
     of cogent/input_strings/ccsd_t/original-expressions/sd_t_d2.in); fp64."""
 
-    def __init__(self, exprs, dtype=F64, extents=None):
+    def __init__(self, exprs, dtype=F64, extents=None, test_fault=0):
         self._h = ctypes.c_void_p()
         self.exprs = list(exprs)
         arr = (ctypes.c_char_p * len(self.exprs))(*[e.encode() for e in self.exprs])
@@ -345,6 +348,17 @@ class FusedPlan:
             an = (ctypes.c_char_p * len(names))(*[n.encode() for n in names])
             ae = (ctypes.c_int64 * len(names))(*[int(extents[n]) for n in names])
             _check(lib().tc_fused_set_extents(self._h, len(names), an, ae), "tc_fused_set_extents")
+        if test_fault:
+            _check(lib().tc_fused_set_test_fault(self._h, test_fault), "tc_fused_set_test_fault")
+
+    def status(self):
+        """Status word (synchronises): 0 unless a bounded wait in one of this plan's launches gave up."""
+        v = ctypes.c_int()
+        _check(lib().tc_fused_status(self._h, ctypes.byref(v)), "tc_fused_status")
+        return v.value
+
+    def status_reset(self):
+        _check(lib().tc_fused_status_reset(self._h), "tc_fused_status_reset")
 
     def commit(self):
         _check(lib().tc_fused_commit(self._h), "tc_fused_commit")

@@ -15,7 +15,7 @@
 // (DMMA m8n8k4, same fragment mapping as tc_contract_kernel) and the accumulators are scattered into the box with
 // the term's own (row, col) -> box-offset tables.  After the last term the box is added to C once.
 // fp64 only.  Operator per term: += or -=.  Plans whose inputs can arrive as tiled boxes run on tc_fused_box_kernel
-// (tc_fused_box.cuh) instead: 3.93 against 9.78 ms on the nine doubles terms of CCSD(T), extents 24.
+// (tc_fused_box.cuh) instead: 3.94 against 9.78 ms on the nine doubles terms of CCSD(T), extents 24.
 #include <cuda.h>  // types of the tensor-map encoder only; the entry point is looked up at run time
 #include <cuda_runtime.h>
 
@@ -381,6 +381,7 @@ struct tc_fused_plan {
   int32_t* d_pos = nullptr;
   int* h_status = nullptr;  // host memory the kernel reports a wait that gave up in
   int grid = 0;
+  int test_fault = 0;
   double flops = 0, bytes_fused = 0, bytes_separate = 0;
   std::string why;
 };
@@ -458,7 +459,8 @@ static void box_build(tc_fused_plan* p) {
     bits += (int)b.lg[i];
   }
   b.total_boxes = (uint32_t)a.total_boxes;
-  b.spin_limit = TC_SPIN_LIMIT;
+  b.spin_limit = p->test_fault ? (1u << 14) : TC_SPIN_LIMIT;
+  b.test_fault = p->test_fault;
   if (bits > 12) return;
   for (int k = 0; k < a.n_terms; ++k) {
     const FusedTerm& T = p->h_terms[k];
@@ -746,6 +748,29 @@ extern "C" int tc_fused_commit(tc_fused_plan* p) {
   }
   p->device = dev;
   p->committed = true;
+  return TC_OK;
+}
+
+extern "C" int tc_fused_set_test_fault(tc_fused_plan* p, int fault) {
+  if (!p || fault < 0 || fault > 1) return TC_ERR_INVALID_ARG;
+  if (p->committed) return TC_ERR_STATE;
+  p->test_fault = fault;
+  return TC_OK;
+}
+
+extern "C" int tc_fused_status(tc_fused_plan* p, int* device_status) {
+  if (!p || !device_status) return TC_ERR_INVALID_ARG;
+  if (!p->committed) return TC_ERR_STATE;
+  TC_CUDA_OK(cudaDeviceSynchronize());
+  *device_status = p->h_status ? *static_cast<volatile int*>(p->h_status) : 0;
+  return TC_OK;
+}
+
+extern "C" int tc_fused_status_reset(tc_fused_plan* p) {
+  if (!p) return TC_ERR_INVALID_ARG;
+  if (!p->committed) return TC_ERR_STATE;
+  TC_CUDA_OK(cudaDeviceSynchronize());
+  if (p->h_status) *static_cast<volatile int*>(p->h_status) = 0;
   return TC_OK;
 }
 

@@ -12,7 +12,7 @@
 //     add the term's products to the box, for the other warps' additions of the term before;
 //   * the first term's products are stored, the others' added; C's old values are read and the box added to them
 //     once, at the end, as in tc_fused_kernel: one rounding against C's magnitude however many terms there are (a box
-//     that starts from C has every term rounded against it; no faster either, 3.94 against 3.93 ms).
+//     that starts from C has every term rounded against it; no faster either, 3.94 ms).
 //
 // Shared-memory layouts.  Operand images are [row][16 k], the 16-byte chunk c of row r at chunk position c ^ (r & 7).
 // A thread reads two consecutive k at once; MMA number 2 h + e of a stage takes k = 8 h + 2 t + e in slot t, for both
@@ -23,11 +23,11 @@
 // codes (found by search) make these four independent, so without bank conflicts, for every term of the CCSD(T) doubles
 // and for four in five of all assignments of six indices (two-way at most in the rest).
 //
-// Measured (nine doubles terms of CCSD(T), all extents 24, one B200): 9.78 ms on tc_fused_kernel, 3.93 ms here (21.1
+// Measured (nine doubles terms of CCSD(T), all extents 24, one B200): 9.78 ms on tc_fused_kernel, 3.94 ms here (20.9
 // TFLOP/s, 57 % of the DMMA rate; floor 2.23 ms of products).  On the way: one block barrier per term 4.76 ms; a barrier
 // that warps only arrive at when their additions are done, 104 registers a thread, eight old values read together 4.49;
 // positions as byte offsets, no tests in whole terms 4.14; conflict-free codes and both halves' reads first 3.95; the
-// first term stored, C added at the end 3.93.  Without any loads 4.43 of the 4.49 remained, the loads alone take 2.07,
+// first term stored, C added at the end 3.94.  Without any loads 4.43 of the 4.49 remained, the loads alone take 2.07,
 // without the additions 3.68: what is left is the chain of a term (wait, fragments, products, additions) with two CTAs
 // of eight warps to cover it.
 #pragma once
@@ -64,6 +64,7 @@ struct BoxArgs {
   int64_t sc[kMaxRank];
   uint32_t total_boxes;
   uint32_t spin_limit;
+  int32_t test_fault;        // tests only: 1 = the first CTA's producer leaves its second stage out
   const int32_t* pos;        // [terms][2][64] hashed box position, in bytes, of row r / column c, -1 beyond the term's rows
   int* status;               // host-visible word: code of a wait that gave up
 };
@@ -121,6 +122,10 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
     tck::reg_dec<kProducerRegs>();
     if (tid != kConsumers) return;
     uint32_t it = 0;
+    auto drain = [&]() {  // copies land while this CTA has its shared memory, also where the consumers have given up
+      for (uint32_t j = it > kBoxStages ? it - kBoxStages : 0u; j < it; ++j)
+        box_wait(&full[j % kBoxStages], (j / kBoxStages) & 1, p.status, 7, p.spin_limit);
+    };
     for (uint32_t bx = blockIdx.x; bx < p.total_boxes; bx += gridDim.x) {
       for (int k = 0; k < p.n_terms; ++k) {
         int cx[4] = {0, 0, 0, 0}, cy[4] = {0, 0, 0, 0};
@@ -138,13 +143,15 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
         const uint32_t kfl = p.term[k].kflat, bytes = p.term[k].bytes;
         for (uint32_t k0 = 0; k0 < kfl; k0 += 16, ++it) {
           const uint32_t s = it % kBoxStages;
-          if (!box_wait(&empty[s], ((it / kBoxStages) & 1) ^ 1, p.status, 2, p.spin_limit)) return;
+          if (!box_wait(&empty[s], ((it / kBoxStages) & 1) ^ 1, p.status, 2, p.spin_limit)) { drain(); return; }
+          if (p.test_fault == 1 && blockIdx.x == 0 && it == 1) continue;
           tck::mbar_arrive_expect_tx(&full[s], bytes);
           box_load(stage0 + s * 2 * kImgBytes, &p.x[k], (int)k0, cx, &full[s]);
           box_load(stage0 + s * 2 * kImgBytes + kImgBytes, &p.y[k], (int)k0, cy, &full[s]);
         }
       }
     }
+    drain();
     return;
   }
 
@@ -155,7 +162,10 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
   const int wm0 = (warp & 1) * 32, wn0 = (warp >> 1) * 16;
   const uint32_t chunk = (uint32_t)((t ^ pg) << 4);
   const uint32_t fx = (uint32_t)(wm0 + pg) * 128u + chunk, fy = (uint32_t)(kImgBytes + (wn0 + pg) * 128) + chunk;
-  bool dead = false;  // a wait gave up: none is waited for any more, so that every warp leaves
+  // A wait gave up: the warp goes on to the end of its box without waiting or announcing anything and leaves there.  The
+  // other warps' waits on it run out too, so none of this box reaches C.  (Leaving at the next term takes a vote
+  // between every wait and its additions: 3.94 -> 3.96 ms on the nine terms.)
+  bool dead = false;
 
   // this thread's box elements e = tid + 256 i: offset in C and coordinates are those of tid plus those of 256 i
   int64_t off_lo = 0;
@@ -241,7 +251,7 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
         if (kfl - k0 > 8) halves(std::integral_constant<int, 2>{});
         else halves(std::integral_constant<int, 1>{});
         __syncwarp();
-        if (lane == 0) tck::mbar_arrive(&empty[s]);
+        if (lane == 0 && !dead) tck::mbar_arrive(&empty[s]);
       }
       // The products of this term go into the box: every (row, column) is one distinct element, and a term's rows and
       // columns are the whole box.  Another warp may hold the same element in the term before (or, for the first term,
@@ -288,14 +298,14 @@ __global__ void __launch_bounds__(kBoxThreads, 2) tc_fused_box_kernel(const __gr
         }
       }
       __syncwarp();
-      if (lane == 0) tck::mbar_arrive(added);
+      if (lane == 0 && !dead) tck::mbar_arrive(added);
       ++terms;
     }
     // ---- the box is added to C: the old values are on their way before the last term's additions are waited for ----
     double old[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) old[i] = valid(crd_lo + s_crd_hi[i], last) ? C[base + off_lo + s_off_hi[i]] : 0.0;
-    if (!dead && !box_wait(added, (terms - 1) & 1, p.status, 6, p.spin_limit)) dead = true;
+    if (!__all_sync(0xffffffffu, !dead && box_wait(added, (terms - 1) & 1, p.status, 6, p.spin_limit))) return;
 #pragma unroll
     for (int i = 0; i < 16; ++i)
       if (valid(crd_lo + s_crd_hi[i], last)) C[base + off_lo + s_off_hi[i]] = old[i] + box[pos_lo ^ box_hash((uint32_t)i << 8)];

@@ -189,7 +189,12 @@ int tc_fused_set_extents(tc_fused_plan* plan, int n, const char* const* index_na
 int tc_fused_commit(tc_fused_plan* plan);
 /* JSON: box shape, boxes, rows x cols per term, flops, bytes moved fused and term by term. */
 int tc_fused_describe(tc_fused_plan* plan, char* buf, size_t cap);
-/* TC_ERR_DEVICE_WAIT: a bounded wait in an earlier launch of this plan gave up, its output is invalid. */
+/* Tests only, before commit; 1: one stage of the kernel's operands never arrives, so that its bounded waits run out. */
+int tc_fused_set_test_fault(tc_fused_plan* plan, int fault);
+/* Status word of the plan's launches so far (synchronises the device): 0, or the code of a bounded wait that gave up --
+ * the output of that launch is invalid.  tc_execute_fused answers TC_ERR_DEVICE_WAIT until the word is reset. */
+int tc_fused_status(tc_fused_plan* plan, int* device_status);
+int tc_fused_status_reset(tc_fused_plan* plan);
 int tc_execute_fused(tc_fused_plan* plan, void* C, const void* const* A, const void* const* B, void* stream);
 void tc_fused_destroy(tc_fused_plan* plan);
 

@@ -186,3 +186,49 @@ def test_terms_are_summed_before_they_meet_the_output(pkg, orc, p7, kernel):
     off = np.abs(got.astype(np.longdouble) - (c0.astype(np.longdouble) + total.astype(np.longdouble)))
     assert (off <= 0.5 * np.spacing(np.abs(got)) + 1e-12 * np.abs(total).max()).all()
     plan.close()
+
+
+def test_fused_status_calls_check_their_arguments(pkg):
+    plan = pkg.FusedPlan(RETRIED[0], extents={"q7": 16})
+    lib = pkg.lib()
+    word = pkg.ctypes.c_int()
+    assert lib.tc_fused_status(plan._h, pkg.ctypes.byref(word)) == 7 and lib.tc_fused_status_reset(plan._h) == 7
+    assert lib.tc_fused_status(None, pkg.ctypes.byref(word)) == 2 and lib.tc_fused_status(plan._h, None) == 2
+    assert lib.tc_fused_status_reset(None) == 2
+    assert lib.tc_fused_set_test_fault(plan._h, 2) == 2 and lib.tc_fused_set_test_fault(None, 1) == 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p7", [10, 40])  # the stage left out is the second term's, or the first term's second
+def test_a_fused_wait_that_gives_up_reports_and_leaves_the_output(pkg, orc, p7):
+    """One CTA never gets one stage: its waits run out, the kernel ends, the status word says so, that CTA's boxes of C
+    are as they were, and the context goes on working."""
+    import torch
+    torch.cuda.set_device(0)
+    lines = _lines(SD2, dict(h3=4, h2=4, h1=4, p6=4, p5=4, p4=4, p7=p7), "p7")  # one box
+    c0, total, ins = orc.uniform(80, 0, orc.sizes(lines[0])[0]), None, []
+    total = c0.copy()
+    for n, line in enumerate(lines):
+        _, na, nb = orc.sizes(line)
+        a, b = orc.uniform(81 + n, 1, na), orc.uniform(81 + n, 2, nb)
+        orc.contract(line, total, a, b)
+        ins.append((torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()))
+    lefts, rights = [a for a, _ in ins], [b for _, b in ins]
+    bad = pkg.FusedPlan(lines, test_fault=1)
+    assert bad.describe()["kernel"] == "tc_fused_box_kernel"
+    dc = torch.from_numpy(c0).cuda()
+    bad.execute(dc, lefts, rights)
+    assert bad.status() != 0
+    assert np.array_equal(dc.cpu().numpy(), c0)
+    with pytest.raises(pkg.TcError) as e:
+        bad.execute(dc, lefts, rights)
+    assert e.value.status == 9
+    bad.status_reset()
+    assert bad.status() == 0
+    bad.execute(dc, lefts, rights)
+    assert bad.status() != 0
+    bad.close()
+    good = pkg.FusedPlan(lines)
+    good.execute(dc, lefts, rights)
+    assert good.status() == 0 and orc.rel_error(dc.cpu().numpy(), total) <= 1e-12
+    good.close()
