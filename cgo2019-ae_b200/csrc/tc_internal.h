@@ -183,6 +183,7 @@ struct tc_plan {
   size_t ws_bytes = 0;
   int sm_count = TC_DEFAULT_SMS;  // multiprocessors of the device the plan is committed on
   int box_order = -1;    // the M class is ordered for the cut tiles of the output-resident kernel: its dimension that comes second (see tc_plan_build)
+  int box_bm = 0, box_bn = 0;  // ... and the tile
   bool block_k = true;  // the planner may cut the contraction into 4 x 4 blocks (see tc_plan_build)
   int passes = 1;   // sequential launches over consecutive contraction ranges, each accumulating into C
   std::mutex* host_mu = nullptr;  // serialises tc_execute_host on this plan (its device buffers are shared)

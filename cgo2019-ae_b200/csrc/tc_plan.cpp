@@ -554,7 +554,11 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   const int64_t sms = p->sm_count > 0 ? p->sm_count : TC_DEFAULT_SMS;
   int bm = 128, bn = 128, variant = 0;
   bool slice_persistent = false;  // the persistent reduce-add kernel with K slices (few tiles, long contraction)
-  if (p->opt.tile_m > 0 || p->opt.tile_n > 0) {
+  if (p->box_order >= 0) {  // second pass: the tile is the first pass's
+    bm = p->box_bm;
+    bn = p->box_bn;
+    variant = 3;
+  } else if (p->opt.tile_m > 0 || p->opt.tile_n > 0) {
     bm = p->opt.tile_m;
     bn = p->opt.tile_n;
     variant = p->opt.variant > 0 ? p->opt.variant - 1 : 0;
@@ -582,12 +586,15 @@ int tc_plan_build(tc_plan* p, std::string* why) {
         run_c = a.M.extent[0];
         for (int d = 1; d < a.M.n && a.M.s_out[d] == run_c; ++d) run_c *= a.M.extent[d];
       }
-      const bool short_runs = a.vec_c < 4 || run_c < 64;
+      // Where the caller names the variant and leaves the tile to the planner, the model knows no cut tiles: they would
+      // draw the choice to tiles that the named variant is not compiled for.
+      const bool named = p->opt.variant > 0;
+      const bool short_runs = !named && (a.vec_c < 4 || run_c < 64);
       p->why.clear();
       for (const Cand& k : cands) {
         if (!tc_kernel_exists(TC_F64, TC_MATH_DMMA, k.bm, k.bn, k.variant)) continue;
         double tiles_c = (double)((mf + k.bm - 1) / k.bm) * (double)((nf + k.bn - 1) / k.bn);
-        if (p->box_order >= 0 && k.variant != 3) continue;  // the choice is made; M's dimensions are in its order
+        if (named && k.variant == 3 && k.bn == 32) continue;
         double out_elems = (double)k.bm * k.bn, idle = k.idle;
         int order = -1;  // M's dimension that comes second
         if (k.variant == 3) {  // needs tiles that are boxes of a rank-5 view of C, and nothing that pins the epilogue
@@ -596,11 +603,18 @@ int tc_plan_build(tc_plan* p, std::string* why) {
           // 16 bytes while the pipe does 2 K flops, equal near K = 46.  On long contractions its single consumer group
           // and two producer warps measured a third slower than the two-group kernel (21 against 31 TFLOP/s).
           const double limit = short_runs ? 3.0 : 1.0;
-          if (p->box_order < 0 && limit * 2.0 * es / 6.5e12 < 0.85 * 2.0 * (double)kf / 37.0e12) continue;
-          const BoxPlan bp = best_boxes(k.bm, k.bn, &order);
-          if (!bp.ok) continue;
-          tiles_c = bp.tiles;
-          out_elems = (double)mf * (double)nf / bp.tiles;
+          if (limit * 2.0 * es / 6.5e12 < 0.85 * 2.0 * (double)kf / 37.0e12) continue;
+          if (named) {
+            TcOutMap view;
+            bool per_warp = false, per_tile = false;
+            out_box_view(a, es, k.bm, k.bn, &view, &per_warp, &per_tile);
+            if (!per_tile) continue;
+          } else {
+            const BoxPlan bp = best_boxes(k.bm, k.bn, &order);
+            if (!bp.ok) continue;
+            tiles_c = bp.tiles;
+            out_elems = (double)mf * (double)nf / bp.tiles;
+          }
         } else if (short_runs) {
           idle += 9000.0;
         }
@@ -677,6 +691,8 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   const bool boxes_allowed = p->opt.tma != 1 && p->opt.tma != 2;
   if (variant == 3 && c.math == TC_MATH_DMMA && boxes_allowed && p->box_order < 0 && best_boxes((uint32_t)bm, (uint32_t)bn, &box_order).ok) {
     p->box_order = box_order;  // plan again with M's dimensions whole and in that order
+    p->box_bm = bm;
+    p->box_bn = bn;
     const int st = tc_plan_build(p, why);
     p->box_order = -1;
     return st;

@@ -388,3 +388,18 @@ def test_outputs_kept_from_the_copy_engine_have_plain_tiles(pkg, expr, tma):
     assert boxes["cbox"]["m"][0] % 4 == 2 and boxes["vec_c"] == 4 and boxes["standin_vec_c"] == 2
     plain = _plan(pkg, expr, tile=(128, 64), variant=4, tma=tma).describe()
     assert "cbox" not in plain and plain["tiles"] == [(plain["Mflat"] + 127) // 128, (plain["Nflat"] + 63) // 64]
+
+
+@pytest.mark.parametrize("expr,options,kernel", [
+    ("C [a,18,b,76,c,8,d,221,e,2,f,2] = sum(k,8) * A [k,d] * B [k,e,f,b,c,a];", dict(variant=4, tma=1), "dmma_wc_128x64"),
+    ("C [a,16,b,268,c,4,d,48,e,9] -= sum(k,215) * A [b,c,k] * B [e,d,k,a];", dict(variant=4, tma=2), "dmma_wc_128x64"),
+    ("C [a,4,b,16,c,32,d,16,e,140,f,8] = sum(k,4) * A [e,a,d,c,k] * B [k,f,b];", dict(variant=4, tma=3, c_path=1), "dmma_wc_128x64"),
+    ("C [a,70,b,13,c,20,d,270] += sum(k,4,l,26,m,19) * A [k,m,a,d,l] * B [c,m,l,b,k];", dict(variant=4, tma=4, c_path=3), "dmma_wc_128x64"),
+    ("C [a,8,b,64,c,275,d,22] -= sum(k,8,l,39,m,1) * A [m,d,l,k,c] * B [m,l,k,a,b];", dict(variant=4, c_path=1), "dmma_wc_128x64"),
+    ("C [a,48,b,48,c,18,d,9,e,25] += sum(k,9) * A [c,b,k,a] * B [d,k,e];", dict(variant=2), "dmma_128x64_w8"),
+    ("C [a,8,b,96,c,236,d,48] = sum(k,4,l,7) * A [l,k,b] * B [k,l,d,c,a];", dict(variant=1, tma=3), "dmma_64x96_w4"),
+])
+def test_a_named_variant_gets_a_tile_it_has(pkg, expr, options, kernel):
+    """Variant named, tile left to the planner: the choice does not follow the rules for cut tiles to one that the
+    variant is not compiled for."""
+    assert _plan(pkg, expr, **options).describe()["kernel"] == kernel
