@@ -440,6 +440,9 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   a.Nflat = (uint32_t)nf;
   a.Kflat = (uint32_t)kf;
   p->kdims = kd;
+  // Rules on the length of the contraction go by its true length: a sum is not long enough to be sliced, and does not
+  // need scratch, because its positions were rounded up.
+  const int64_t k_true = kcut_x > 0 ? kf / (16 * ((kcut_x + 3) / 4) * ((kcut_y + 3) / 4)) * kcut_x * kcut_y : kf;
 
   // Contraction offset tables (one entry per flattened k), digits carried along as on an odometer.
   p->h_koff_x.assign(kf, 0);
@@ -577,7 +580,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       const Cand cands[] = {{128, 64, 2, 2100.0, 0.76, 0.90}, {64, 96, 2, 800.0, 0.76, 0.86}, {128, 32, 2, 1500.0, 0.76, 0.84},
                             {128, 64, 3, 1450.0, 0.92, 0.92}, {128, 32, 3, 1200.0, 0.92, 0.84}};
       const double clk = 1.9e9, flop_per_clk = 37.0e12 / 148.0 / clk, byte_per_clk = 6.5e12 / 148.0 / clk;
-      const double kpad = (double)((kf + 3) / 4 * 4);
+      const double kpad = (double)((k_true + 3) / 4 * 4);
       double best = 0;
       // Outputs whose rows are shorter than a consumer warp's leave the reduce-add kernels element by element (their
       // epilogue reads and writes C through registers, a round trip per batch); the resident tile takes them as boxes.
@@ -603,7 +606,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
           // 16 bytes while the pipe does 2 K flops, equal near K = 46.  On long contractions its single consumer group
           // and two producer warps measured a third slower than the two-group kernel (21 against 31 TFLOP/s).
           const double limit = short_runs ? 3.0 : 1.0;
-          if (limit * 2.0 * es / 6.5e12 < 0.85 * 2.0 * (double)kf / 37.0e12) continue;
+          if (limit * 2.0 * es / 6.5e12 < 0.85 * 2.0 * (double)k_true / 37.0e12) continue;
           if (named) {
             TcOutMap view;
             bool per_warp = false, per_tile = false;
@@ -675,8 +678,8 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       // ... unless its 128-row tiles pad the problem much more than 64-row ones would while the small kernel can
       // at least load one operand by vector (measured on 312 x 296 outputs: 20 % more padded work cost 20 %)
       const bool padding_ok = 2 * t128 * 100 <= t64 * 112 || (!c.vec_x && !c.vec_y);
-      if (c.math == TC_MATH_DMMA && p->opt.split_k == 0 && (kf + TC_BK - 1) / TC_BK >= 64 && t128 * ((kf + TC_BK - 1) / TC_BK / 16) >= 2 * sms &&
-          padding_ok && tc_kernel_exists(TC_F64, TC_MATH_DMMA, 128, 64, 2)) {
+      const int64_t steps = (k_true + TC_BK - 1) / TC_BK;
+      if (c.math == TC_MATH_DMMA && p->opt.split_k == 0 && steps >= 64 && t128 * (steps / 16) >= 2 * sms && padding_ok && tc_kernel_exists(TC_F64, TC_MATH_DMMA, 128, 64, 2)) {
         bm = 128; bn = 64; variant = 2;
         slice_persistent = true;
       } else {
@@ -747,7 +750,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
 
   // K split: only when the tile count cannot fill the GPU and K is long.
   int64_t ksplit = 1;
-  const int64_t ksteps = (kf + bk - 1) / bk;
+  const int64_t ksteps = (k_true + bk - 1) / bk;
   const bool persistent = tc_kernel_is_persistent(c);
   // Persistent kernels do not split K, except the fp64 reduce-add kernel: on request (forced tile and split_k), or
   // where the planner kept it for a problem of few tiles (about four work items per SM, slices of at least 16 steps).
@@ -816,8 +819,9 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     a.ksplit = 1;
   }
   if (p->passes == 1) {
-    int64_t chunk_steps = (ksteps + ksplit - 1) / ksplit;
-    ksplit = (ksteps + chunk_steps - 1) / chunk_steps;
+    const int64_t steps = (kf + bk - 1) / bk;  // positions, rounded-up ones among them
+    int64_t chunk_steps = (steps + ksplit - 1) / ksplit;
+    ksplit = (steps + chunk_steps - 1) / chunk_steps;
     a.ksplit = (uint32_t)ksplit;
     a.k_chunk = (uint32_t)(chunk_steps * bk);
   }

@@ -74,6 +74,19 @@ def test_blocked_contractions_against_the_loop_nest(pkg, orc, c, d, split):
     assert desc["Kflat"] == (c + 3) // 4 * 4 * ((d + 3) // 4 * 4) and err <= 1e-12
 
 
+def test_contractions_that_were_rounded_up_run_without_scratch(pkg, orc):
+    import torch
+    expr = "t3 [a,1200,b,512] += sum(c,30,d,30) * t2 [c,a,d] * v2 [d,b,c];"
+    c0, a, b = orc.make_inputs(expr, 8, "float64")
+    ref = orc.contract(expr, c0.copy(), a, b)
+    plan = pkg.Plan(expr).commit()
+    dc, da, db = (torch.from_numpy(x).cuda() for x in (c0, a, b))
+    plan.execute_noalloc(dc, da, db)
+    torch.cuda.synchronize()
+    assert plan.workspace_bytes() == 0 and plan.status() == 0 and orc.rel_error(dc.cpu().numpy(), ref) <= 1e-12
+    plan.close()
+
+
 @pytest.mark.parametrize("tile,variant", [((128, 64), 3), ((64, 96), 3), ((128, 32), 3)])
 @pytest.mark.parametrize("op", ["+=", "=", "-="])
 def test_odd_outputs_and_ragged_edges(pkg, orc, tile, variant, op):

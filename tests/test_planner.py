@@ -403,3 +403,20 @@ def test_a_named_variant_gets_a_tile_it_has(pkg, expr, options, kernel):
     """Variant named, tile left to the planner: the choice does not follow the rules for cut tiles to one that the
     variant is not compiled for."""
     assert _plan(pkg, expr, **options).describe()["kernel"] == kernel
+
+
+@pytest.mark.parametrize("expr", [
+    "t3 [a,1200,b,512] += sum(c,30,d,30) * t2 [c,a,d] * v2 [d,b,c];",                         # 900 values, 1024 positions
+    "C [a,24,b,64,c,33,d,8] = sum(k,5,l,1,m,292) * A [m,b,l,d,k] * B [k,l,a,m,c];",           # 1460 and 2336
+    "C [a,16,b,8,c,6,d,5,e,31] += sum(k,12,l,34,m,2) * A [l,e,b,d,k,m,c] * B [m,k,l,a];",     # 816 and 1728
+    "C [a,67,b,14,c,6,d,48] += sum(k,344,l,2) * A [l,k,a] * B [k,d,b,l,c];",                  # 688 and 1376
+])
+def test_rounding_a_contraction_up_asks_for_no_scratch(pkg, expr):
+    """... so that such a plan runs without a workspace, through the entry that never allocates and on several streams."""
+    assert _plan(pkg, expr).describe()["workspace_bytes"] == 0
+
+
+def test_rounding_a_contraction_up_makes_no_further_slices(pkg):
+    """split_k is bounded by the steps of the true length: 2 x 7 values are one step, not the two of 4 x 8 positions."""
+    d = _plan(pkg, "C [a,38,b,282,c,8,d,163] += sum(k,2,l,7) * A [k,d,a,l,c] * B [l,b,k];", split_k=2, tile=(128, 64), variant=3).describe()
+    assert d["ksplit"] == 1 and d["workspace_bytes"] == 0
