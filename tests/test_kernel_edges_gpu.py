@@ -66,12 +66,13 @@ def test_output_resident_plans_kept_from_the_copy_engine(pkg, orc, expr, tma, c_
     assert "cbox" not in d and err <= 1e-12
 
 
-@pytest.mark.parametrize("c,d", [(61, 66), (64, 64), (4, 150), (63, 5), (3, 3)])
+@pytest.mark.parametrize("c,d", [(61, 66), (64, 64), (4, 150), (7, 41), (63, 50), (5, 10), (3, 3)])
 @pytest.mark.parametrize("split", [0, 3])
 def test_blocked_contractions_against_the_loop_nest(pkg, orc, c, d, split):
     expr = "t3 [a,150,b,70] += sum(c,%d,d,%d) * t2 [c,a,d] * v2 [d,b,c];" % (c, d)
     desc, err = _run(pkg, orc, expr, tile=(128, 64), variant=3, split_k=split)
-    assert desc["Kflat"] == (c + 3) // 4 * 4 * ((d + 3) // 4 * 4) and err <= 1e-12
+    rounded = (c + 3) // 4 * 4 * ((d + 3) // 4 * 4)
+    assert desc["Kflat"] == (c * d if (c, d) in ((3, 3), (5, 10)) else rounded) and err <= 1e-12  # 78 and 92 % more: plain order
 
 
 def test_contractions_that_were_rounded_up_run_without_scratch(pkg, orc):

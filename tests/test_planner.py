@@ -347,7 +347,7 @@ def test_cut_tiles_keep_pairs_of_an_input_together(pkg):
 
 def test_blocked_contractions_name_every_value_once(pkg):
     """Two inputs that start with different contraction indices: 4 x 4 blocks of K, rounded up, with holes."""
-    for c, d in ((64, 64), (61, 66), (4, 130), (63, 5)):
+    for c, d in ((64, 64), (61, 66), (4, 130), (63, 50), (7, 41), (62, 62)):
         p = _plan(pkg, "t3 [a,2048,b,2048] += sum(c,%d,d,%d) * t2 [c,a,d] * v2 [d,b,c];" % (c, d)).describe()
         assert p["kernel"].startswith("dmma_w") and [k["extent"] for k in p["K"][:2]] == [4, 4]
         assert p["Kflat"] == (c + 3) // 4 * 4 * ((d + 3) // 4 * 4)
@@ -420,3 +420,10 @@ def test_rounding_a_contraction_up_makes_no_further_slices(pkg):
     """split_k is bounded by the steps of the true length: 2 x 7 values are one step, not the two of 4 x 8 positions."""
     d = _plan(pkg, "C [a,38,b,282,c,8,d,163] += sum(k,2,l,7) * A [k,d,a,l,c] * B [l,b,k];", split_k=2, tile=(128, 64), variant=3).describe()
     assert d["ksplit"] == 1 and d["workspace_bytes"] == 0
+
+
+@pytest.mark.parametrize("c,d", [(30, 30), (22, 22), (2, 200), (200, 2), (100, 3), (6, 50), (5, 5), (17, 17), (63, 5), (5, 8000)])
+def test_contractions_that_blocks_would_pad_keep_the_plain_order(pkg, c, d):
+    """More than a tenth of added products where X can be read by vector, more than a third where it cannot."""
+    p = _plan(pkg, "t3 [a,2048,b,2048] += sum(c,%d,d,%d) * t2 [c,a,d] * v2 [d,b,c];" % (c, d)).describe()
+    assert p["Kflat"] == c * d
