@@ -112,6 +112,7 @@ struct TcKernelArgs {
   int32_t c_stream;  // cache-streaming hints on accesses to C
   uint32_t prefetch_dist;  // blocks ahead whose output tile is prefetched into L2 (0 = off)
   uint32_t k_chunk;  // flattened contraction range per K slice (multiple of the K step)
+  uint32_t k_seg, k_segs;  // K steps that are added up in one chain and how many such segments a slice has (persistent fp64 reduce-add kernel)
   uint32_t ksplit;   // number of K slices (1 = the kernel applies the result to C itself)
   uint32_t k_first;  // first flattened contraction index of this launch (plans that run K in sequential passes)
   uint32_t spin_limit;  // polls a bounded wait may take before it gives up

@@ -758,11 +758,11 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   if (tc_kernel_is_persistent(c) && a.tiles_m > 64 && a.tiles_n > 1 && (double)mf * (double)kf * es > 4.0e6) a.mblock_w = 32;
 
   // K split: only when the tile count cannot fill the GPU and K is long.
-  int64_t ksplit = 1;
+  int64_t ksplit = 1, seg_steps = int64_t(1) << 27;  // seg_steps: the longest chain of additions inside a slice
   const int64_t ksteps = (k_true + bk - 1) / bk;
   const bool persistent = tc_kernel_is_persistent(c);
   // Persistent kernels do not split K, except the fp64 reduce-add kernel: on request (forced tile and split_k), or
-  // where the planner kept it for a problem of few tiles (about four work items per SM, slices of at least 16 steps).
+  // where the planner kept it for a problem of few tiles.
   const bool ws_kernel = c.math == TC_MATH_DMMA && c.variant == 2;
   if (kcut_x > 0 && !(c.math == TC_MATH_DMMA && persistent)) {  // kernels that know no holes in the contraction
     p->block_k = false;
@@ -771,12 +771,11 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     return st;
   }
   if (persistent && ws_kernel && p->opt.split_k > 1) ksplit = std::min<int64_t>(p->opt.split_k, ksteps);
-  else if (persistent && ws_kernel && slice_persistent)
-  {
-    // Work items (slice, tile) are dealt to two groups per SM: as many slices as fill whole rounds of them.  One item
-    // more than a round costs a round (312 x 296 outputs: 15 tiles in 40 slices are 600 items on 296 groups, 3 rounds for
-    // 2.03 rounds of work; 39 slices are 2 rounds).  The first number of rounds that leaves under 5 % of the groups
-    // idle, else the best of four.
+  else if (persistent && ws_kernel && slice_persistent) {
+    // Work items (slice, tile) are dealt to two groups per SM: as many slices (of at least 16 steps) as fill whole rounds
+    // of the groups.  One item more than a round costs a round (312 x 296 outputs summed over 312 x 312, 15 tiles: 40
+    // slices are 600 items on 296 groups, three rounds for 2.03 rounds of work, 975 us; 39 are two, 789 us; 19 are one,
+    // 806 us).  The first number of rounds that leaves under 5 % of the groups idle, else the best of four.
     const int64_t slots = 2 * sms;
     double best_fill = 0;
     for (int64_t rounds = 1; rounds <= 4 && best_fill < 0.95; ++rounds) {
@@ -786,6 +785,11 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       const double fill = (double)items / (double)(used * slots);
       if (fill > best_fill) { best_fill = fill; ksplit = ks; }
     }
+    // ... each added up in segments no longer than four items per SM (of at least 16 steps) would make slices, so that
+    // few slices do not lengthen the chains of additions: in one chain, 19 slices of that sum are 2.5e-15 from a sum by
+    // pairs, 40 slices 1.8e-15.
+    const int64_t most = std::max<int64_t>(1, std::min<int64_t>((4 * sms + tiles - 1) / tiles, ksteps / 16));
+    seg_steps = (ksteps + most - 1) / most;
   }
   else if (persistent) ksplit = 1;
   else if (p->opt.split_k > 1) ksplit = std::min<int64_t>(p->opt.split_k, ksteps);
@@ -833,6 +837,9 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     ksplit = (steps + chunk_steps - 1) / chunk_steps;
     a.ksplit = (uint32_t)ksplit;
     a.k_chunk = (uint32_t)(chunk_steps * bk);
+    const int64_t segs = (chunk_steps + seg_steps - 1) / seg_steps;
+    a.k_seg = (uint32_t)((chunk_steps + segs - 1) / segs);
+    a.k_segs = (uint32_t)((chunk_steps + a.k_seg - 1) / a.k_seg);
   }
   if (tiles * ksplit >= (int64_t(1) << 31)) { *why = "too many tiles"; return TC_ERR_UNSUPPORTED; }
   p->ws_bytes = ksplit > 1 ? (size_t)(ksplit * tiles * bm * bn) * es : 0;
@@ -895,7 +902,7 @@ std::string tc_plan_to_json(const tc_plan& p) {
       << ",\"math\":\"" << (p.choice.math == TC_MATH_DMMA ? "dmma" : p.choice.math == TC_MATH_TF32X3 ? "tf32x3" : p.choice.math == TC_MATH_TF32TC ? "tf32x3_tcgen05" : (p.dtype == TC_F64 ? "dfma" : "ffma"))
       << "\",\"kernel\":\"" << tc_kernel_name(p.choice) << "\",\"tile\":[" << p.choice.bm << "," << p.choice.bn << "," << TC_BK
       << "],\"variant\":" << p.choice.variant << ",\"tiles\":[" << a.tiles_m << "," << a.tiles_n << "],\"estimate_us\":" << p.estimate_s * 1e6 << ",\"mblock_w\":" << a.mblock_w << ",\"ksplit\":" << a.ksplit
-      << ",\"k_chunk\":" << a.k_chunk << ",\"passes\":" << p.passes << ",\"chain\":" << chain << ",\"vec_x\":" << (p.choice.vec_x ? "true" : "false")
+      << ",\"k_chunk\":" << a.k_chunk << ",\"k_seg\":" << a.k_seg << ",\"passes\":" << p.passes << ",\"chain\":" << chain << ",\"vec_x\":" << (p.choice.vec_x ? "true" : "false")
       << ",\"vec_y\":" << (p.choice.vec_y ? "true" : "false") << ",\"kvec_x\":" << (p.choice.kvec_x ? "true" : "false")
       << ",\"kvec_y\":" << (p.choice.kvec_y ? "true" : "false") << ",\"tma_x\":" << (p.choice.tma_x ? "true" : "false")
       << ",\"tma_y\":" << (p.choice.tma_y ? "true" : "false") << ",\"tma_xe\":" << (p.choice.tma_xe ? "true" : "false")

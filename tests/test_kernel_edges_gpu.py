@@ -103,6 +103,16 @@ def test_slices_combined_in_parts(pkg, orc, dtype, tol, split):
     assert err <= tol
 
 
+@pytest.mark.parametrize("expr", [
+    "C [a,510,b,316] += sum(c,64,d,64) * A [c,a,d] * B [d,b,c];",       # 14 slices of 19 steps, in segments of ten
+    "C [a,310,b,200] -= sum(c,9000) * A [c,a] * B [c,b];",              # a last segment that is shorter, a last step of eight
+    "C [a,270,b,66,c,21] = sum(k,4,l,352) * A [l,c,k] * B [a,k,l,b];",
+])
+def test_slices_added_up_in_segments(pkg, orc, expr):
+    d, err = _run(pkg, orc, expr)
+    assert d["kernel"] == "dmma_ws_128x64" and d["ksplit"] > 1 and 16 * d["k_seg"] < d["k_chunk"] and err <= 1e-12
+
+
 @pytest.mark.parametrize("expr,kw", [
     ("C [i,64,j,48,k,32] += sum(l,40) * A [l,k,i] * B [j,l];", {}),
     ("C [a,70,b,45] += sum(c,700) * A [c,a] * B [c,b];", {"split_k": 5}),

@@ -427,3 +427,16 @@ def test_contractions_that_blocks_would_pad_keep_the_plain_order(pkg, c, d):
     """More than a tenth of added products where X can be read by vector, more than a third where it cannot."""
     p = _plan(pkg, "t3 [a,2048,b,2048] += sum(c,%d,d,%d) * t2 [c,a,d] * v2 [d,b,c];" % (c, d)).describe()
     assert p["Kflat"] == c * d
+
+
+@pytest.mark.parametrize("tiles_m", [1, 3, 7, 11, 16, 37, 73])
+@pytest.mark.parametrize("k", [1100, 2048, 9000, 97344])
+def test_few_slices_do_not_lengthen_the_chains_of_additions(pkg, tiles_m, k):
+    """A slice is added up in segments no longer than four work items for each of the 148 multiprocessors, or sixteen
+    steps, would make slices."""
+    d = _plan(pkg, "C [a,%d,b,128] += sum(c,%d) * A [c,a] * B [b,c];" % (128 * tiles_m, k)).describe()
+    if d["kernel"] != "dmma_ws_128x64" or d["ksplit"] == 1:
+        return
+    tiles, steps = d["tiles"][0] * d["tiles"][1], (k + 15) // 16
+    most = max(1, min((4 * 148 + tiles - 1) // tiles, steps // 16))
+    assert 0 < d["k_seg"] <= (steps + most - 1) // most and 16 * d["k_seg"] <= d["k_chunk"]
