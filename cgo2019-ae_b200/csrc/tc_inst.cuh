@@ -20,7 +20,8 @@ typedef int (*tc_inst_fn)(int mode_x, int mode_y, const TcKernelArgs* args, void
 
 namespace tck {
 
-// Launch that may, where `chained`, overlap the end of the kernel before it in the stream (see chain_wait).
+// Launch that may, where `chained`, overlap the end of the kernel before it in the stream (see chain_wait).  A failure is
+// returned and not left in the runtime, where the next launch's check would take it for its own.
 template <class... P, class... A>
 cudaError_t launch_chained(bool chained, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchAttribute at{};
@@ -33,7 +34,9 @@ cudaError_t launch_chained(bool chained, void (*kern)(P...), dim3 grid, unsigned
   cfg.stream = stream;
   cfg.attrs = &at;
   cfg.numAttrs = chained ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  const cudaError_t st = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  if (st != cudaSuccess) (void)cudaGetLastError();
+  return st;
 }
 
 template <class CF>

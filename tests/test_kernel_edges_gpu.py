@@ -182,3 +182,45 @@ def test_split_groups_of_the_persistent_fp32_kernel(pkg, orc, k):
         assert plan.status() == 0
         assert np.abs(got.cpu().numpy() - want).max() / np.abs(want).max() <= 1e-5
     plan.close()
+
+
+REFUSED_LAUNCH = """
+import ctypes, sys
+sys.path.insert(0, {root!r})
+import __graft_entry__ as entry
+import torch
+pkg = entry.load_package()
+torch.cuda.set_device(0)
+small = pkg.Plan("C [i,64,j,48,k,32] += sum(l,40) * A [l,k,i] * B [j,l];").commit()        # one-tile kernel
+sliced = pkg.Plan("C [a,70,b,45] += sum(c,700) * A [c,a] * B [c,b];", split_k=5).commit()  # ... and a combine step
+large = pkg.Plan("C [a,48,b,48,c,48,d,48] += sum(e,48) * A [a,e,b,d] * B [e,c];").commit()  # persistent kernel
+bufs = [torch.zeros(n, dtype=torch.float64, device="cuda") for n in (48 ** 4, 48 ** 4, 48 ** 3)]
+for plan in (small, sliced, large):
+    plan.execute(*bufs)
+torch.cuda.synchronize()
+rt = ctypes.CDLL("libcudart.so.12")
+for refused in (small, sliced):
+    stream, graph = ctypes.c_void_p(), ctypes.c_void_p()
+    assert rt.cudaStreamCreate(ctypes.byref(stream)) == 0
+    assert rt.cudaStreamBeginCapture(stream, 0) == 0
+    try:
+        refused.execute(*bufs, stream=1)       # the legacy stream: the runtime refuses it while a blocking stream captures
+        raise SystemExit("accepted")
+    except pkg.TcError as e:
+        assert e.status == 5, e
+    assert rt.cudaStreamEndCapture(stream, ctypes.byref(graph)) != 0
+    rt.cudaGetLastError()
+    large.execute(*bufs)                       # not this call's failure
+    torch.cuda.synchronize()
+    assert large.status() == 0
+print("held")
+"""
+
+
+def test_a_refused_launch_is_not_reported_again():
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", REFUSED_LAUNCH.format(root=root)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "held", r.stdout + r.stderr
