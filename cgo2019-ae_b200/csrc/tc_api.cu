@@ -1,6 +1,5 @@
 // C ABI: plan / execute / free, the seeded input generator and small utilities.
 // Declarations and the reference interfaces they replace are in include/tc_b200.h.
-#include <cuda.h>  // types of the tensor-map encoder only; the entry point is looked up at run time
 #include <cuda_runtime.h>
 #include <stdlib.h>
 
@@ -12,6 +11,7 @@
 
 #include "tc_inst.cuh"
 #include "tc_internal.h"
+#include "tc_tensor_map.h"
 
 // ---------------------------------------------------------------- errors ----
 static thread_local char g_cuda_error[256] = "";
@@ -121,17 +121,7 @@ static int mode_of(bool ext_vec, bool k_vec) { return ext_vec ? 1 : k_vec ? 2 : 
 // index at `pitch` elements; box = rows x 16, no swizzle, zero fill outside the tensor.
 static bool encode_operand_map_ext(TcTensorMap* out, const void* base, uint64_t ext_extent, uint64_t k_extent,
                                    uint64_t pitch, uint32_t rows) {
-  typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static encode_fn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<encode_fn>(f);
-  }();
+  const tc_encode_fn fn = tc_tensor_map_encoder();
   if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || (pitch * 4) % 16 != 0 || rows > 256 || rows % 4 != 0) return false;
   const cuuint64_t dims[2] = {ext_extent, k_extent};
   const cuuint64_t strides[1] = {pitch * 4};
@@ -144,20 +134,10 @@ static bool encode_operand_map_ext(TcTensorMap* out, const void* base, uint64_t 
 
 // Tiled TMA descriptor of an operand seen as a 2-D matrix of `es`-byte elements: dimension 0 = contraction index
 // (stride 1), dimension 1 = flattened external index at `pitch` elements; box = 16 x rows, swizzled over the box
-// row (128 bytes for fp64, 64 for fp32), zero fill outside the tensor.  cuTensorMapEncodeTiled is resolved through the runtime (no link against libcuda).
+// row (128 bytes for fp64, 64 for fp32), zero fill outside the tensor.
 static bool encode_operand_map(TcTensorMap* out, const void* base, uint64_t k_extent, uint64_t ext_extent,
                                uint64_t pitch, uint32_t rows, int es = 8) {
-  typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static encode_fn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<encode_fn>(f);
-  }();
+  const tc_encode_fn fn = tc_tensor_map_encoder();
   if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || (pitch * es) % 16 != 0 || rows > 256) return false;
   const cuuint64_t dims[2] = {k_extent, ext_extent};
   const cuuint64_t strides[1] = {pitch * (uint64_t)es};
@@ -177,17 +157,7 @@ static bool encode_operand_map(TcTensorMap* out, const void* base, uint64_t k_ex
 // (bm, 2, bn / 2) for a whole tile.  No swizzle, no fill.
 static bool encode_output_map(TcTensorMap* out, const void* base, const TcOutMap& o, uint32_t bw, uint32_t bh,
                               uint32_t bq) {
-  typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static encode_fn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<encode_fn>(f);
-  }();
+  const tc_encode_fn fn = tc_tensor_map_encoder();
   if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || bw > 256 || bq > 256 || o.e0 == 0 || o.f0 < 2 || o.ne + o.me > 2) return false;
   cuuint64_t dims[5] = {o.e0, 2, o.f0 / 2, 1, 1};
   cuuint64_t strides[4] = {(cuuint64_t)o.stride_n * 8, (cuuint64_t)o.stride_n * 16, 0, 0};
@@ -205,17 +175,7 @@ static bool encode_output_map(TcTensorMap* out, const void* base, const TcOutMap
 
 // The same output as the boxes of the output-resident kernel's cut tiles (TcBoxMap).
 static bool encode_box_output_map(TcTensorMap* out, const void* base, const TcBoxMap& o) {
-  typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static encode_fn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<encode_fn>(f);
-  }();
+  const tc_encode_fn fn = tc_tensor_map_encoder();
   if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || o.rank < 1 || o.rank > 5) return false;
   cuuint64_t dims[5] = {1, 1, 1, 1, 1}, strides[4];
   cuuint32_t box[5] = {1, 1, 1, 1, 1};
@@ -292,9 +252,13 @@ int tc_launch_contraction(const tc_plan& p, const TcKernelArgs& args, void* C, c
   const uintptr_t cu = reinterpret_cast<uintptr_t>(C);
   if ((cu & 15) != 0) a.vec_c = 1;
   int vx = x16 ? mode_of(c.vec_x, c.kvec_x) : 0, vy = y16 ? mode_of(c.vec_y, c.kvec_y) : 0;
+  // The C-resident kernel moves whole output tiles as boxes of a view of C: the view must exist and the base must be
+  // 16-byte aligned.  Otherwise the same tiles run on the persistent kernel that reaches C through reduce-adds or plain
+  // read-modify-writes.
+  const bool resident = tc_kernel_is_c_resident(c) && c.box_c && encode_box_output_map(&a.tmap_ct, C, a.cbox);
   // Persistent kernels fetch operands that are plain 2-D matrices with one tiled TMA copy per stage.
   if (tc_kernel_is_persistent(c) && c.math == TC_MATH_DMMA && p.opt.tma != 1) {
-    const bool operands = p.opt.tma == 0 || p.opt.tma == 2 || p.opt.tma == 4, output = p.opt.tma == 0 || p.opt.tma == 3 || p.opt.tma == 4;
+    const bool operands = p.opt.tma == 0 || p.opt.tma == 2 || p.opt.tma == 4, output = !resident && (p.opt.tma == 0 || p.opt.tma == 3 || p.opt.tma == 4);
     if (operands && c.tma_x && encode_operand_map(&a.tmap_x, X, a.Kflat, a.Mflat, (uint64_t)a.M.s_in[0], (uint32_t)a.bm)) vx = 3;
     if (operands && c.tma_y && encode_operand_map(&a.tmap_y, Y, a.Kflat, a.Nflat, (uint64_t)a.N.s_in[0], (uint32_t)a.bn)) vy = 3;
     a.c_tensor = (output && c.tma_c && a.c_mode == 2 &&
@@ -305,18 +269,11 @@ int tc_launch_contraction(const tc_plan& p, const TcKernelArgs& args, void* C, c
   }
   tc_inst_fn fn = pick_inst(c);
   int passes = p.passes;
-  if (tc_kernel_is_c_resident(c)) {
-    // The C-resident kernel moves whole output tiles as boxes of the rank-5 view of C: the view must exist and the
-    // base must be 16-byte aligned.  Otherwise the same tiles run on the persistent kernel that reaches C through
-    // reduce-adds or plain read-modify-writes.
-    const bool ok = c.box_c && encode_box_output_map(&a.tmap_ct, C, a.cbox);
-    if (ok) a.c_tensor = 0;
-    if (!ok) {
-      a.vec_c = std::min(a.vec_c, a.standin_vec_c);
-      TcKernelChoice alt = c;
-      alt.variant = 2;
-      fn = pick_inst(alt);
-    }
+  if (tc_kernel_is_c_resident(c) && !resident) {
+    a.vec_c = std::min(a.vec_c, a.standin_vec_c);
+    TcKernelChoice alt = c;
+    alt.variant = 2;
+    fn = pick_inst(alt);
   }
   if (tc_kernel_is_tmem_persistent(c) && ((cu & 15) != 0 || p.opt.c_path == 2)) {
     // The persistent tcgen05 kernel moves its output tiles as bulk copies of 16-byte aligned chunks; an output

@@ -16,7 +16,6 @@
 // the term's own (row, col) -> box-offset tables.  After the last term the box is added to C once.
 // fp64 only.  Operator per term: += or -=.  Plans whose inputs can arrive as tiled boxes run on tc_fused_box_kernel
 // (tc_fused_box.cuh) instead: 3.94 against 9.78 ms on the nine doubles terms of CCSD(T), extents 24.
-#include <cuda.h>  // types of the tensor-map encoder only; the entry point is looked up at run time
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,6 +27,7 @@
 #include <vector>
 
 #include "tc_fused_box.cuh"
+#include "tc_tensor_map.h"
 #include "tc_kernels.cuh"
 
 namespace {
@@ -495,17 +495,7 @@ static void box_positions(const tc_fused_plan* p, int k, int part, int32_t* pos)
 // Rank-5 descriptor of one input: dimension 0 = contraction index, then the output indices it carries; box 16 x b_i.
 static bool encode_box_map(TcTensorMap* out, const void* base, const FusedArgs& a, uint32_t kflat,
                            const std::vector<tc_fused_plan::BoxDim>& dims_in) {
-  typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static encode_fn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<encode_fn>(f);
-  }();
+  const tc_encode_fn fn = tc_tensor_map_encoder();
   if (!fn || (reinterpret_cast<uintptr_t>(base) & 15)) return false;
   cuuint64_t dims[5] = {kflat, 1, 1, 1, 1}, strides[4];
   cuuint32_t box[5] = {16, 1, 1, 1, 1};
@@ -806,6 +796,7 @@ extern "C" int tc_execute_fused(tc_fused_plan* p, void* C, const void* const* A,
       TC_CUDA_OK(cudaGetLastError());
       return TC_OK;
     }
+    // (only where the driver cannot encode: the plan has seen to the strides, the checks above to the addresses)
   }
   tc_fused_kernel<<<(unsigned)p->args.total_boxes, kThreads, fused_smem_bytes(p->args.n_terms), static_cast<cudaStream_t>(stream)>>>(
       p->args, ptrs, static_cast<double*>(C));
