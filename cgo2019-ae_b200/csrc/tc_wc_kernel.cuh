@@ -4,11 +4,11 @@
 // Same tiling, address tables, operand images and DMMA fragment mapping as tc_ws_dmma_kernel
 // (tc_ws_kernel.cuh); what differs is the way the result meets C:
 //
-//   * a consumer group (eight warps of 32 x 32 on a 128 x 64 tile) owns TWO output-tile buffers in shared memory,
+//   * the consumers (eight warps of 32 x 32 on a 128 x 64 tile) own TWO output-tile buffers in shared memory,
 //     used alternately;
-//   * one thread per group (the "C thread", first lane of a warp of its own) moves whole output tiles with tiled TMA
+//   * one thread (the "C thread", first lane of a warp of its own) moves whole output tiles with tiled TMA
 //     copies of the rank-5 view of C: it LOADS the tile of C a whole tile ahead of its use
-//     (cp.async.bulk.tensor.5d into the group's free buffer, completion on an mbarrier), waits until the
+//     (cp.async.bulk.tensor.5d into the free buffer, completion on an mbarrier), waits until the
 //     consumers have added their products into the buffer, STORES it back (cp.async.bulk.tensor.5d, plain
 //     store) and, once the copy engine has read the buffer, issues the load of the tile after next;
 //   * the consumers never touch global memory and never wait for the copy engine in their epilogue: they wait
@@ -16,7 +16,7 @@
 //     (the two halves of a thread's 32 bytes are visited in opposite order by even and odd row groups, which
 //     makes the accesses bank-conflict free on the dense rows the copy engine wants), and go on to
 //     their next tile;
-//   * producer warps fill the group's operand ring exactly as in tc_ws_dmma_kernel.
+//   * producer warps fill the operand ring exactly as in tc_ws_dmma_kernel.
 //
 // Why: on B200 the reduce-add stream of the copy engine (cp.reduce.async.bulk.tensor ... add) tops out near
 // 5.2 TB/s of read+write traffic for this access pattern, while tiled loads plus tiled stores through the SM
@@ -47,14 +47,14 @@ struct WcCfg {
   using T = double;
   static constexpr int BM = BM_, BN = BN_, BK = 16, STAGES = STAGES_;
   static constexpr int MODEX = MODEX_, MODEY = MODEY_;
-  static constexpr int GROUPS = 1, WGM = WGM_, WGN = WGN_, CW = WGM * WGN;  // consumer warps per group
+  static constexpr int WGM = WGM_, WGN = WGN_, CW = WGM * WGN;  // consumer warps
   static constexpr int WM = BM / WGM, WN = BN / WGN;
   static constexpr int CONSUMER_THREADS = CW * 32;
-  // producer warps per group: two where every operand arrives 16 bytes (or a tiled copy) at a time, four where one is
+  // producer warps: two where every operand arrives 16 bytes (or a tiled copy) at a time, four where one is
   // gathered element by element
   static constexpr bool ELEM = MODEX == LM_ELEM || MODEY == LM_ELEM;
   static constexpr int PWARPS = ELEM ? 4 : 2;
-  static constexpr int THREADS = 32 * PWARPS;    // producer threads per group
+  static constexpr int THREADS = 32 * PWARPS;    // producer threads
   // last warpgroup(s): the producer warps, then a warp whose first lane is the C thread
   static constexpr int CTA_THREADS = CONSUMER_THREADS + (ELEM ? 256 : 128);
   static_assert(CW % 4 == 0, "warp roles");
@@ -69,11 +69,10 @@ struct WcCfg {
   static constexpr uint32_t TMA_BYTES = (MODEX == LM_TMA_K ? BM * BK * 8 : 0) + (MODEY == LM_TMA_K ? BN * BK * 8 : 0);
   static constexpr int FULL_ARRIVALS = THREADS + (ANY_TMA ? 1 : 0);
   static constexpr int TABLE_ELEMS = BM + BN;    // offx_m, offy_n (the output is addressed by the copy engine)
-  static constexpr int CBUFS = 2;                // output-tile buffers per group
+  static constexpr int CBUFS = 2;                // output-tile buffers
   static constexpr int CTILE_ELEMS = BM * BN;
-  static constexpr int NBARS = GROUPS * (2 * STAGES + 2 * CBUFS);
-  static constexpr int SMEM_BYTES = (GROUPS * STAGES * STAGE_ELEMS + GROUPS * CBUFS * CTILE_ELEMS + GROUPS * 2 * TABLE_ELEMS) * 8 +
-                                    NBARS * 8;
+  static constexpr int NBARS = 2 * STAGES + 2 * CBUFS;
+  static constexpr int SMEM_BYTES = (STAGES * STAGE_ELEMS + CBUFS * CTILE_ELEMS + 2 * TABLE_ELEMS) * 8 + NBARS * 8;
   static constexpr int PRODUCER_REGS = 56;
   static_assert(SMEM_BYTES <= 232448, "shared memory");
 };
@@ -108,23 +107,18 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
   constexpr int CW = CF::CW;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   double* stages = reinterpret_cast<double*>(smem_raw);  // first: TMA images need 1024-byte alignment
-  double* cbufs = stages + CF::GROUPS * STAGES * CF::STAGE_ELEMS;
-  int64_t* tables = reinterpret_cast<int64_t*>(cbufs + CF::GROUPS * CF::CBUFS * CF::CTILE_ELEMS);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(tables + CF::GROUPS * 2 * CF::TABLE_ELEMS);
+  double* cbufs = stages + STAGES * CF::STAGE_ELEMS;
+  int64_t* tables = reinterpret_cast<int64_t*>(cbufs + CF::CBUFS * CF::CTILE_ELEMS);  // two sets, alternating per tile
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
-  constexpr int CWARPS = CF::GROUPS * CW, PW = CF::PWARPS;
-  const bool is_producer = warp >= CWARPS && warp < CWARPS + CF::GROUPS * PW;
-  const bool is_cwg = warp >= CWARPS + CF::GROUPS * PW;  // C threads (first lanes of the first GROUPS warps here), idle warps
-  const int gi = warp < CWARPS ? warp / CW : is_producer ? (warp - CWARPS) / PW : (warp - CWARPS - CF::GROUPS * PW) % CF::GROUPS;
-  uint64_t* full = bars + gi * (2 * STAGES + 2 * CF::CBUFS);  // [STAGES] operands of a stage have landed
-  uint64_t* empty = full + STAGES;                            // [STAGES] the consumers are done with a stage
-  uint64_t* c_ready = empty + STAGES;                         // [CBUFS] the buffer holds the tile of C (or is free, for `=`)
-  uint64_t* c_staged = c_ready + CF::CBUFS;                   // [CBUFS] the consumers have added their products
-  int64_t* gtab = tables + gi * 2 * CF::TABLE_ELEMS;          // two table sets, alternating per tile
-  double* gstage = stages + gi * STAGES * CF::STAGE_ELEMS;
-  double* gcbuf = cbufs + gi * CF::CBUFS * CF::CTILE_ELEMS;
+  constexpr int PW = CF::PWARPS;
+  const bool is_producer = warp >= CW && warp < CW + PW;
+  const bool is_cwg = warp >= CW + PW;  // the C thread (first lane of the first warp here), idle warps
+  uint64_t* full = reinterpret_cast<uint64_t*>(tables + 2 * CF::TABLE_ELEMS);  // [STAGES] operands of a stage have landed
+  uint64_t* empty = full + STAGES;           // [STAGES] the consumers are done with a stage
+  uint64_t* c_ready = empty + STAGES;        // [CBUFS] the buffer holds the tile of C (or is free, for `=`)
+  uint64_t* c_staged = c_ready + CF::CBUFS;  // [CBUFS] the consumers have added their products
 
   if (tid == 32) {  // descriptors into the copy engine's cache before the first copy needs them
     if constexpr (CF::MODEX == LM_TMA_K) asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&p.tmap_x)) : "memory");
@@ -132,17 +126,14 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&p.tmap_ct)) : "memory");
   }
   if (tid == 0) {
-    for (int q = 0; q < CF::GROUPS; ++q) {
-      uint64_t* b = bars + q * (2 * STAGES + 2 * CF::CBUFS);
-      for (int s = 0; s < STAGES; ++s) { mbar_init(b + s, CF::FULL_ARRIVALS); mbar_init(b + STAGES + s, CW); }
-      for (int s = 0; s < CF::CBUFS; ++s) { mbar_init(b + 2 * STAGES + s, 1); mbar_init(b + 2 * STAGES + CF::CBUFS + s, CW); }
-    }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(full + s, CF::FULL_ARRIVALS); mbar_init(empty + s, CW); }
+    for (int s = 0; s < CF::CBUFS; ++s) { mbar_init(c_ready + s, 1); mbar_init(c_staged + s, CW); }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
 
   const uint32_t total = p.tiles_m * p.tiles_n;
-  const uint32_t first = (uint32_t)CF::GROUPS * blockIdx.x + gi, step = (uint32_t)CF::GROUPS * gridDim.x;
+  const uint32_t first = blockIdx.x, step = gridDim.x;
   const int nk = (int)((p.Kflat + BK - 1) / BK);
   const uint32_t kend = p.Kflat;
   const bool accumulate = p.beta != 0;
@@ -150,7 +141,7 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
   if (is_cwg) {
     // --------------------------------------------------------------- C thread ----
     reg_dec<CF::PRODUCER_REGS>();  // one value for the whole warpgroup
-    if ((tid & 31) != 0 || warp >= CWARPS + CF::GROUPS * (PW + 1)) return;
+    if ((tid & 31) != 0 || warp > CW + PW) return;
     const uint64_t tmap = reinterpret_cast<uint64_t>(&p.tmap_ct);
     const uint32_t ntiles = first < total ? (total - first + step - 1) / step : 0u;
     struct Corner { int c[5]; };
@@ -161,14 +152,14 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
       tile_box_coords(p, tm, tn, r.c);
       return r;
     };
-    auto fetch = [&](uint32_t j, const Corner& at) {  // tile j of this group into buffer j & 1 (or just: the buffer is free)
+    auto fetch = [&](uint32_t j, const Corner& at) {  // tile j of this CTA into buffer j & 1 (or just: the buffer is free)
       const uint32_t b = j & 1u;
       const int(&c)[5] = at.c;
       if (!accumulate) { mbar_arrive(&c_ready[b]); return; }
       mbar_arrive_expect_tx(&c_ready[b], p.mcut.b0 * p.mcut.b1 * p.ncut.b0 * p.ncut.b1 * 8u);
       asm volatile(
           "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];\n" ::"r"(
-              smem_u32(gcbuf + b * CF::CTILE_ELEMS)),
+              smem_u32(cbufs + b * CF::CTILE_ELEMS)),
           "l"(tmap), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(smem_u32(&c_ready[b]))
           : "memory");
     };
@@ -182,7 +173,7 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
       const int(&c)[5] = here.c;
       if (!mbar_wait(&c_staged[b], (j >> 1) & 1u, p.status, 6, p.spin_limit)) return;
       asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4, %5}], [%6];\n" ::"l"(tmap),
-                   "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(smem_u32(gcbuf + b * CF::CTILE_ELEMS))
+                   "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(smem_u32(cbufs + b * CF::CTILE_ELEMS))
                    : "memory");
       asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
       if (j + CF::CBUFS < ntiles) {
@@ -199,14 +190,14 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
   if (is_producer) {
     // ------------------------------------------------------------ producer ----
     reg_dec<CF::PRODUCER_REGS>();
-    const int ptid = tid - (CWARPS + gi * PW) * 32;
+    const int ptid = tid - CW * 32;
     // element copies: 0 = lanes walk the external index, else the step between the positions of the 4 lanes that walk k
     const int lgx = p.lanes_k_x == 1 ? 0 : p.kstep_x, lgy = p.lanes_k_y == 1 ? 0 : p.kstep_y;
     uint32_t it = 0, titer = 0;
     for (uint32_t tile = first; tile < total; tile += step, ++titer) {
-      // Two table sets used alternately: the barrier below is passed only when every producer of the group has
+      // Two table sets used alternately: the barrier below is passed only when every producer has
       // issued the previous tile's loads, so the set written now (last read two tiles ago) is free.
-      int64_t* offx_m = gtab + (titer & 1) * CF::TABLE_ELEMS;
+      int64_t* offx_m = tables + (titer & 1) * CF::TABLE_ELEMS;
       int64_t* offy_n = offx_m + BM;
       uint32_t tm, tn;
       tile_coords(p, tile, &tm, &tn);
@@ -217,14 +208,14 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
         if (i < BM) decode(p.M, cut_flat(p.mcut, mt, i), p.Mflat, &offx_m[i], &unused);
         else decode(p.N, cut_flat(p.ncut, nt, i - BM), p.Nflat, &offy_n[i - BM], &unused);
       }
-      group_bar_sync(1 + gi, CF::THREADS);
+      group_bar_sync(1, CF::THREADS);
       int64_t kx = ws_koff(p.koff_x, 0, kend, ptid), ky = ws_koff(p.koff_y, 0, kend, ptid);
       for (int ks = 0; ks < nk; ++ks, ++it) {
         const uint32_t s = it % STAGES;
         const int64_t nx = ws_koff(p.koff_x, (uint32_t)(ks + 1) * BK, kend, ptid), ny = ws_koff(p.koff_y, (uint32_t)(ks + 1) * BK, kend, ptid);
         // (one decision per warp: the loaders below shuffle)
         if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.status, 2, p.spin_limit))) return;
-        double* xs = gstage + s * CF::STAGE_ELEMS;
+        double* xs = stages + s * CF::STAGE_ELEMS;
         double* ys = xs + CF::XIMG;
         const uint32_t k0 = (uint32_t)ks * BK;
         if constexpr (CF::ANY_TMA) {
@@ -239,7 +230,7 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
         kx = nx;
         ky = ny;
         // tests only: one producer thread of CTA 0 never announces its copies of one stage
-        if (p.test_fault == 1 && blockIdx.x == 0 && gi == 0 && it == 1 && ptid == 7) continue;
+        if (p.test_fault == 1 && blockIdx.x == 0 && it == 1 && ptid == 7) continue;
         mbar_arrive_on_copies(&full[s]);
       }
     }
@@ -249,7 +240,7 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
   // -------------------------------------------------------------- consumer ----
   constexpr int WM = CF::WM, WN = CF::WN;
   constexpr int MB2 = WM / 16, NB2 = WN / 16;
-  const int lane = tid & 31, cw = warp % CW;
+  const int lane = tid & 31, cw = warp;
   const int g = lane >> 2, t = lane & 3;
   const int wm0 = (cw % CF::WGM) * WM, wn0 = (cw / CF::WGM) * WN;
   const double alpha = p.alpha;
@@ -279,7 +270,7 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
     for (int ks = 0; ks < nk; ++ks, ++it) {
       const uint32_t s = it % STAGES;
       if (!mbar_wait(&full[s], (it / STAGES) & 1, p.status, 3, p.spin_limit)) return;
-      const double* xs = gstage + s * CF::STAGE_ELEMS;
+      const double* xs = stages + s * CF::STAGE_ELEMS;
       const double* ys = xs + CF::XIMG;
       const int kleft = (int)kend - ks * BK;
       const int nks = kleft >= BK ? BK / 4 : (kleft + 3) / 4;
@@ -309,7 +300,7 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
     // ---- epilogue: buffer (+)= alpha * acc in shared memory; the C thread stores the buffer ----
     const uint32_t b = titer & 1u;
     if (!mbar_wait(&c_ready[b], (titer >> 1) & 1u, p.status, 4, p.spin_limit)) return;
-    double* tb = gcbuf + b * CF::CTILE_ELEMS;
+    double* tb = cbufs + b * CF::CTILE_ELEMS;
     // (tiles that are plain ranges keep addresses the compiler knows: the general form cost 2.5 % on the 40^6 slab)
     if (dense) {
 #pragma unroll

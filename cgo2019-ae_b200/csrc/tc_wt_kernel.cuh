@@ -73,7 +73,6 @@ struct WtCfg {
   static constexpr bool BOXES = (TMAX || TMAXE) && (TMAY || TMAYE);  // both operands: one thread is the whole loader role
   static constexpr int FULL_ARRIVALS = BOXES ? 1 : THREADS + (ANY_TMA ? 1 : 0);  // the loaders' copies, and the announcement of the boxes
   static constexpr int UMMA_ELEMS = 2 * BK * BM;         // hi and lo images of X for one K step (those of Y live in tensor memory)
-  static constexpr int GROUPS = 1;                       // tiles a CTA works on at a time (launch arithmetic)
   // Six warpgroups: epilogue, epilogue, split, split, loaders, {MMA, fetch, store, a warp without work}.
   static constexpr int CTA_THREADS = 24 * 32;
   static constexpr int SPLIT_WARPS = 8, SPLIT_THREADS = 256, EPI_WARPS = 8;
