@@ -780,7 +780,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     double best_fill = 0;
     for (int64_t rounds = 1; rounds <= 4 && best_fill < 0.95; ++rounds) {
       const int64_t ks = std::min<int64_t>(rounds * slots / tiles, ksteps / 16);
-      if (ks < 1) continue;
+      if (ks < 2) continue;  // (one slice goes into C by itself and has no partial tile to be added up in)
       const int64_t items = ks * tiles, used = (items + slots - 1) / slots;
       const double fill = (double)items / (double)(used * slots);
       if (fill > best_fill) { best_fill = fill; ksplit = ks; }
@@ -837,7 +837,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     ksplit = (steps + chunk_steps - 1) / chunk_steps;
     a.ksplit = (uint32_t)ksplit;
     a.k_chunk = (uint32_t)(chunk_steps * bk);
-    const int64_t segs = (chunk_steps + seg_steps - 1) / seg_steps;
+    const int64_t segs = ksplit > 1 ? (chunk_steps + seg_steps - 1) / seg_steps : 1;
     a.k_seg = (uint32_t)((chunk_steps + segs - 1) / segs);
     a.k_segs = (uint32_t)((chunk_steps + a.k_seg - 1) / a.k_seg);
   }

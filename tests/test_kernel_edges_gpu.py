@@ -107,6 +107,7 @@ def test_slices_combined_in_parts(pkg, orc, dtype, tol, split):
     "C [a,510,b,316] += sum(c,64,d,64) * A [c,a,d] * B [d,b,c];",       # 14 slices of 19 steps, in segments of ten
     "C [a,310,b,200] -= sum(c,9000) * A [c,a] * B [c,b];",              # a last segment that is shorter, a last step of eight
     "C [a,270,b,66,c,21] = sum(k,4,l,352) * A [l,c,k] * B [a,k,l,b];",
+    "C [a,34,b,24,c,28,d,35] = sum(k,35,l,33) * A [k,l,b] * B [l,k,a,d,c];",    # 261 tiles: more than a slice of each to a round
 ])
 def test_slices_added_up_in_segments(pkg, orc, expr):
     d, err = _run(pkg, orc, expr)

@@ -440,3 +440,15 @@ def test_few_slices_do_not_lengthen_the_chains_of_additions(pkg, tiles_m, k):
     tiles, steps = d["tiles"][0] * d["tiles"][1], (k + 15) // 16
     most = max(1, min((4 * 148 + tiles - 1) // tiles, steps // 16))
     assert 0 < d["k_seg"] <= (steps + most - 1) // most and 16 * d["k_seg"] <= d["k_chunk"]
+
+
+@pytest.mark.parametrize("expr", [
+    "C [a,34,b,24,c,28,d,35] = sum(k,35,l,33) * A [k,l,b] * B [l,k,a,d,c];",     # 261 tiles: a round holds one slice of each
+    "C [a,123,b,15,c,299,d,4,e,1] = sum(k,12,l,152) * A [k,a,l,d,e] * B [l,k,c,b];",
+    "C [a,32,b,215,c,84] += sum(k,39,l,30) * A [k,c,b,l] * B [l,a,k];",
+    "C [a,96,b,96,c,96,d,96] += sum(e,96) * A [a,e,b,d] * B [e,c];",             # not sliced at all
+])
+def test_only_slices_are_added_up_in_segments(pkg, expr):
+    """A sum that is not sliced goes into C in one piece."""
+    d = _plan(pkg, expr).describe()
+    assert d["ksplit"] > 1 or d["k_seg"] * 16 >= d["Kflat"]
