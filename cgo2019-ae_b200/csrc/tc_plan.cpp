@@ -410,12 +410,14 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   // the low parts put first -- (4 of X's, 4 of Y's, the rest): a K step of sixteen is then a 4 x 4 block of which both
   // inputs read whole sectors.  Extents that four does not divide are rounded up; positions beyond them have offset -1
   // in the tables, which the loaders of the persistent fp64 kernels (and only they) turn into zeros.
-  // What is rounded up costs products, so blocks are taken only where they add few.  Measured on one B200 (2048 x 2048 and
-  // 48 x 48 x 48 x 40 outputs, 312 x 296 outputs of long sums), time in plain order over time in blocks:
-  //   X's extent even (plain order reads X 16 bytes at a time): 1.05 to 2.3 where nothing or up to 7 % is added, 0.98 at
-  //   14 %, 0.92 to 0.96 at 19 to 24 %, 0.81 to 0.96 at 33 to 39 %, 0.56 to 0.61 at 100 %;
-  //   odd (both inputs go element by element): 1.11 to 1.22 up to 14 %, 1.03 to 1.19 at 18 to 25 %, 1.06 to 1.14 at 33 %,
-  //   0.95 at 38 %, 0.88 at 52 %, 0.69 to 0.93 at 60 %.
+  // What is rounded up costs products, so blocks are taken only where they add few.  In plain order a sector of Y is met
+  // again only after all positions of the contraction indices before Y's: while Y stays in L2 that costs little, beyond
+  // that memory is read up to four times.  Measured on one B200, 14 000 random sums, time in plain order over time in
+  // blocks, per product (10 % / half of them are above): Y over 32 MB 1.15 / 1.36 to 2.4 where X's extent is even (plain
+  // order reads X 16 bytes at a time), 1.14 / 1.39 to 2.2 where it is odd; up to 32 MB 1.02 / 1.08 to 1.16 even, and odd
+  // 1.18 / 1.39 with fewer than 8 positions before Y's index, 0.98 / 1.19 with fewer than 32, beyond 0.9 / 1.11 (Y over
+  // 16 MB) and 0.76 / 0.9.  With the limits below the choice is 1.4 % slower than the better of the two throughout;
+  // blocks always 5.8 %, never 24 %.
   int64_t kcut_x = 0, kcut_y = 0;  // extents of the two digits that were cut (0: none)
   if (p->dtype == TC_F64 && p->block_k && x_k_unit && y_k_unit && !dk.empty() && dk[0].s_in == 1 && dk[0].s_out != 1 &&
       dk.size() + 2 <= (size_t)TC_MAX_DIMS) {
@@ -424,7 +426,14 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       const Dim x = dk[0], y = dk[j];
       const double given = (double)x.extent * (double)y.extent;
       const double rounded = 16.0 * (double)((x.extent + 3) / 4) * (double)((y.extent + 3) / 4);
-      if (rounded > given * (x.extent % 2 == 0 ? 1.1 : 1.34)) break;
+      double before = 1.0;
+      for (size_t i = 0; i < j; ++i) before *= (double)dk[i].extent;
+      const bool even = x.extent % 2 == 0;
+      const double y_bytes = (double)(p->swapped ? p->count_a : p->count_b) * es;
+      const double limit = y_bytes > 32.0e6 ? (even ? 1.35 : 1.5)
+                           : even           ? 1.1
+                                            : before < 8.0 ? 1.34 : before < 32.0 ? 1.15 : y_bytes > 16.0e6 ? 1.1 : 0.0;
+      if (rounded > given * limit) break;
       kcut_x = x.extent;
       kcut_y = y.extent;
       std::vector<Dim> r = {{4, x.s_in, x.s_out}, {4, y.s_in, y.s_out}};

@@ -66,13 +66,14 @@ def test_output_resident_plans_kept_from_the_copy_engine(pkg, orc, expr, tma, c_
     assert "cbox" not in d and err <= 1e-12
 
 
-@pytest.mark.parametrize("c,d", [(61, 66), (64, 64), (4, 150), (7, 41), (63, 50), (5, 10), (3, 3)])
+@pytest.mark.parametrize("c,d,b", [(61, 66, 1100), (64, 64, 70), (4, 150, 70), (7, 41, 70), (63, 50, 1300), (9, 10, 5000),
+                                   (5, 10, 70), (3, 3, 70)])
 @pytest.mark.parametrize("split", [0, 3])
-def test_blocked_contractions_against_the_loop_nest(pkg, orc, c, d, split):
-    expr = "t3 [a,150,b,70] += sum(c,%d,d,%d) * t2 [c,a,d] * v2 [d,b,c];" % (c, d)
+def test_blocked_contractions_against_the_loop_nest(pkg, orc, c, d, b, split):
+    expr = "t3 [a,70,b,%d] += sum(c,%d,d,%d) * t2 [c,a,d] * v2 [d,b,c];" % (b, c, d)
     desc, err = _run(pkg, orc, expr, tile=(128, 64), variant=3, split_k=split)
     rounded = (c + 3) // 4 * 4 * ((d + 3) // 4 * 4)
-    assert desc["Kflat"] == (c * d if (c, d) in ((3, 3), (5, 10)) else rounded) and err <= 1e-12  # 78 and 92 % more: plain order
+    assert desc["Kflat"] == (c * d if c * d < 91 else rounded) and err <= 1e-12  # the last three add 60 to 90 %: plain order
 
 
 def test_contractions_that_were_rounded_up_run_without_scratch(pkg, orc):

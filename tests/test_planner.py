@@ -422,11 +422,18 @@ def test_rounding_a_contraction_up_makes_no_further_slices(pkg):
     assert d["ksplit"] == 1 and d["workspace_bytes"] == 0
 
 
-@pytest.mark.parametrize("c,d", [(30, 30), (22, 22), (2, 200), (200, 2), (100, 3), (6, 50), (5, 5), (17, 17), (63, 5), (5, 8000)])
+@pytest.mark.parametrize("c,d", [(30, 30), (22, 22), (2, 200), (200, 2), (100, 3), (6, 50), (5, 5), (17, 17), (63, 5), (5, 8000), (33, 16)])
 def test_contractions_that_blocks_would_pad_keep_the_plain_order(pkg, c, d):
-    """More than a tenth of added products where X can be read by vector, more than a third where it cannot."""
+    """More added products than the larger operand's traffic saves."""
     p = _plan(pkg, "t3 [a,2048,b,2048] += sum(c,%d,d,%d) * t2 [c,a,d] * v2 [d,b,c];" % (c, d)).describe()
     assert p["Kflat"] == c * d
+
+
+def test_blocks_may_add_more_where_the_operand_streams_from_memory(pkg):
+    """26 x 50 x 50 values, 12 % more in blocks: taken for 248 columns (129 MB), not for 24 (12 MB)."""
+    expr = "C [a,8,b,%d,c,1] -= sum(k,26,l,50,m,50) * A [k,m,a,l] * B [l,k,c,b,m];"
+    assert _plan(pkg, expr % 248).describe()["Kflat"] == 28 * 52 * 50
+    assert _plan(pkg, expr % 24).describe()["Kflat"] == 26 * 50 * 50
 
 
 @pytest.mark.parametrize("tiles_m", [1, 3, 7, 11, 16, 37, 73])
