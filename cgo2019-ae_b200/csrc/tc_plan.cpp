@@ -573,7 +573,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   //   * vector pipe: 128 x 128;
   //   * anything that would leave most SMs without a tile: 64 x 64, one CTA per tile.
   const int64_t sms = p->sm_count > 0 ? p->sm_count : TC_DEFAULT_SMS;
-  int bm = 128, bn = 128, variant = 0;
+  int bm = 128, bn = 128, variant = 0, fill_bm = 0, fill_bn = 0;
   bool slice_persistent = false;  // the persistent reduce-add kernel with K slices (few tiles, long contraction)
   if (p->box_order >= 0) {  // second pass: the tile is the first pass's
     bm = p->box_bm;
@@ -587,68 +587,94 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     if (c.math == TC_MATH_DMMA) {
       // fp64 on the tensor pipe: the persistent kernels, chosen by a small cost model (this takes the place of the
       // reference's ranking of mappings by estimated DRAM transactions, cogent/src/algs/bases/cost_models.py:191-574).
-      // Per candidate (tile, kernel) the time of one SM is  tiles per SM  x  max(products + idle, output bytes / rate):
+      // Per candidate (tile, kernel) the time of one SM is
+      //   tiles per SM  x  max(products + idle, output bytes / rate, least):
       //   products   2 bm bn K / (DMMA rate of one SM x the share of it the kernel's main loop reaches), K rounded up to 4;
+      //              the share depends on which operands are copied element by element (medians, K from 120 to 400);
       //   idle       cycles per tile during which the pipe waits (epilogue, hand-overs), measured per kernel;
       //   rate       what the kernel's way of reaching C sustains: reduce-adds of the copy engine 0.76 of the
       //              measured copy bandwidth, tiled loads + stores of a resident tile 0.92;
-      //   tiles per SM is rounded up (wave quantisation) and edge tiles count in full (waste).
-      // Constants come from the B200 measurements recorded beside the kernels; the device's SM count is the plan's.
-      struct Cand { int bm, bn, variant; double idle, rate, eff; };  // eff: share of the DMMA rate its main loop reaches
-      const Cand cands[] = {{128, 64, 2, 2100.0, 0.76, 0.90}, {64, 96, 2, 800.0, 0.76, 0.86}, {128, 32, 2, 1500.0, 0.76, 0.84},
-                            {128, 64, 3, 1450.0, 0.92, 0.92}, {128, 32, 3, 1200.0, 0.92, 0.84}};
+      //   least      cycles that a tile takes however little is in it: the chain of its copies and hand-overs (medians of
+      //              tiles of 32 to 1024 elements with up to 16 products each; a resident tile of 120 elements takes as
+      //              long as one of 1000, which made a 20 x 6 x 6 x 95 x 2 x 23 output 358 us instead of 60);
+      //   tiles per SM is rounded up (wave quantisation), edge tiles count in full.
+      // Constants come from the B200 measurements recorded beside the kernels; the device's SM count is the plan's.  On
+      // 8 212 random one-index contractions the choice is 5 % slower than the best of the five, and 0.4 % of them run
+      // 30 % slower than on the tiles of before cut tiles.  (One share per kernel, no `least` and 9000 cycles for any
+      // element epilogue: 9 and 4 %.)
+      struct Cand { int bm, bn, variant; double idle, rate, eff, least, share[4]; };  // share: neither, X, Y, both by element
+      const Cand cands[] = {{128, 64, 2, 2100.0, 0.76, 0.90, 4000.0, {0.88, 0.65, 0.80, 0.65}},
+                            {64, 96, 2, 800.0, 0.76, 0.86, 3500.0, {0.85, 0.78, 0.73, 0.72}},
+                            {128, 32, 2, 1500.0, 0.76, 0.84, 3600.0, {0.78, 0.45, 0.60, 0.40}},
+                            {128, 64, 3, 1450.0, 0.92, 0.92, 4400.0, {0.81, 0.67, 0.80, 0.66}},
+                            {128, 32, 3, 1200.0, 0.92, 0.84, 3800.0, {0.60, 0.55, 0.61, 0.54}}};
+      const bool boxes_in = p->opt.tma == 0 || p->opt.tma == 2 || p->opt.tma == 4;
+      const int by_element = (c.vec_x || c.kvec_x || (boxes_in && c.tma_x) ? 0 : 1) + (c.vec_y || c.kvec_y || (boxes_in && c.tma_y) ? 0 : 2);
       const double clk = 1.9e9, flop_per_clk = 37.0e12 / 148.0 / clk, byte_per_clk = 6.5e12 / 148.0 / clk;
       const double kpad = (double)((k_true + 3) / 4 * 4);
-      double best = 0;
       // Outputs whose rows are shorter than a consumer warp's leave the reduce-add kernels element by element (their
-      // epilogue reads and writes C through registers, a round trip per batch); the resident tile takes them as boxes.
+      // epilogue reads and writes C through registers, a round trip per batch): 1.25 cycles an element where C is read,
+      // 0.55 where it is overwritten (full tiles, K up to 16: 13 800 against 8 300 cycles of the bulk epilogue on
+      // 128 x 64, 9 700 against 6 100 on 64 x 96, 7 500 against 5 000 on 128 x 32; overwritten 7 300 / 5 700, 5 200 /
+      // 4 500, 4 950 / 4 300).  The resident tile takes them as boxes.
       int64_t run_c = 0;
       if (a.M.n > 0 && a.M.s_out[0] == 1) {
         run_c = a.M.extent[0];
         for (int d = 1; d < a.M.n && a.M.s_out[d] == run_c; ++d) run_c *= a.M.extent[d];
       }
-      // Where the caller names the variant and leaves the tile to the planner, the model knows no cut tiles: they would
-      // draw the choice to tiles that the named variant is not compiled for.
-      const bool named = p->opt.variant > 0;
-      const bool short_runs = !named && (a.vec_c < 4 || run_c < 64);
       p->why.clear();
-      for (const Cand& k : cands) {
-        if (!tc_kernel_exists(TC_F64, TC_MATH_DMMA, k.bm, k.bn, k.variant)) continue;
-        double tiles_c = (double)((mf + k.bm - 1) / k.bm) * (double)((nf + k.bn - 1) / k.bn);
-        if (named && k.variant == 3 && k.bn == 32) continue;
-        double out_elems = (double)k.bm * k.bn, idle = k.idle;
-        int order = -1;  // M's dimension that comes second
-        if (k.variant == 3) {  // needs tiles that are boxes of a rank-5 view of C, and nothing that pins the epilogue
-          if (p->opt.tma == 1 || p->opt.tma == 2 || p->opt.c_path != 0) continue;
-          // ... and pays only where the output traffic is the longer side: per output element the memory system moves
-          // 16 bytes while the pipe does 2 K flops, equal near K = 46.  On long contractions its single consumer group
-          // and two producer warps measured a third slower than the two-group kernel (21 against 31 TFLOP/s).
-          const double limit = short_runs ? 3.0 : 1.0;
-          if (limit * 2.0 * es / 6.5e12 < 0.85 * 2.0 * (double)k_true / 37.0e12) continue;
-          if (named) {
-            TcOutMap view;
-            bool per_warp = false, per_tile = false;
-            out_box_view(a, es, k.bm, k.bn, &view, &per_warp, &per_tile);
-            if (!per_tile) continue;
-          } else {
-            const BoxPlan bp = best_boxes(k.bm, k.bn, &order);
-            if (!bp.ok) continue;
-            tiles_c = bp.tiles;
-            out_elems = (double)mf * (double)nf / bp.tiles;
+      // The plain model (`eff` for the share, no `least`, no cut tiles) speaks first.  Its tile is final where the caller
+      // names the variant: the full model's could be one that the variant is not compiled for.  And its tile says, below,
+      // whether there are too few tiles to fill the GPU: which sums are sliced and need scratch does not move with the rest.
+      struct Pick { int bm, bn, variant; double t; };
+      auto choose = [&](bool plain) {
+        Pick best = {bm, bn, variant, 0};
+        const bool short_runs = !plain && (a.vec_c < 4 || run_c < 64);
+        for (const Cand& k : cands) {
+          if (!tc_kernel_exists(TC_F64, TC_MATH_DMMA, k.bm, k.bn, k.variant)) continue;
+          double tiles_c = (double)((mf + k.bm - 1) / k.bm) * (double)((nf + k.bn - 1) / k.bn);
+          if (plain && k.variant == 3 && k.bn == 32) continue;
+          double out_elems = plain ? (double)k.bm * k.bn : (double)mf * (double)nf / tiles_c, idle = k.idle;
+          int order = -1;  // M's dimension that comes second
+          if (k.variant == 3) {  // needs tiles that are boxes of a rank-5 view of C, and nothing that pins the epilogue
+            if (p->opt.tma == 1 || p->opt.tma == 2 || p->opt.c_path != 0) continue;
+            // ... and pays only where the output traffic is the longer side: per output element the memory system moves
+            // 16 bytes while the pipe does 2 K flops, equal near K = 46.  On long contractions its single consumer group
+            // and two producer warps measured a third slower than the two-group kernel (21 against 31 TFLOP/s).
+            const double limit = short_runs ? 3.0 : 1.0;
+            if (limit * 2.0 * es / 6.5e12 < 0.85 * 2.0 * (double)k_true / 37.0e12) continue;
+            if (plain) {
+              TcOutMap view;
+              bool per_warp = false, per_tile = false;
+              out_box_view(a, es, k.bm, k.bn, &view, &per_warp, &per_tile);
+              if (!per_tile) continue;
+            } else {
+              const BoxPlan bp = best_boxes(k.bm, k.bn, &order);
+              if (!bp.ok) continue;
+              tiles_c = bp.tiles;
+              out_elems = (double)mf * (double)nf / bp.tiles;
+            }
+          } else if (short_runs) {
+            idle += (e.op == 0 ? 0.55 : 1.25) * out_elems;
           }
-        } else if (short_runs) {
-          idle += 9000.0;
+          const double products = 2.0 * k.bm * k.bn * kpad / (flop_per_clk * (plain ? k.eff : k.share[by_element]));
+          const double out_bytes = (e.op == 0 ? 1.0 : 2.0) * out_elems * es;
+          const double per_tile = std::max(std::max(products + idle, out_bytes / (byte_per_clk * k.rate)), plain ? 0.0 : k.least);
+          const double t = std::ceil(tiles_c / (double)sms) * per_tile / clk;
+          // an earlier candidate stays unless a later one is estimated a twentieth faster (a tenth in the plain model): the
+          // models know tiles, waste and waves, not how well each loader shape feeds each tile
+          // (the output-resident kernel has its own gate above and the same tile: any estimated gain counts)
+          if (best.t == 0 || t < best.t * (k.variant == 3 ? 0.98 : plain ? 0.90 : 0.95)) best = {k.bm, k.bn, k.variant, t};
         }
-        const double products = 2.0 * k.bm * k.bn * kpad / (flop_per_clk * k.eff);
-        const double out_bytes = (e.op == 0 ? 1.0 : 2.0) * out_elems * es;
-        const double per_tile = std::max(products + idle, out_bytes / (byte_per_clk * k.rate));
-        const double t = std::ceil(tiles_c / (double)sms) * per_tile / clk;
-        // the first candidate (128 x 64, two groups) stays unless another is estimated a tenth faster: the model knows
-        // tiles, waste and waves, not how well each loader shape feeds each tile
-        // (the output-resident kernel has its own gate above and the same tile: any estimated gain counts)
-        if (best == 0 || t < best * (k.variant == 3 ? 0.98 : 0.90)) { best = t; bm = k.bm; bn = k.bn; variant = k.variant; }
-      }
-      p->estimate_s = best;
+        return best;
+      };
+      const Pick first = choose(true), pick = p->opt.variant > 0 ? first : choose(false);
+      bm = pick.bm;
+      bn = pick.bn;
+      variant = pick.variant;
+      fill_bm = first.bm;
+      fill_bn = first.bn;
+      p->estimate_s = pick.t;
     }
     if (c.math != TC_MATH_DMMA && c.dtype == TC_F32) {
       // fp32: 96 rows instead of 128 when that makes the tile a whole number of the output's contiguous
@@ -686,7 +712,8 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       const bool vector_loads = (c.vec_x || c.kvec_x) && (c.vec_y || c.kvec_y);
       if (vector_loads && wt_eligible(a, tbm, es) && tc_kernel_exists(TC_F32, TC_MATH_TF32TC, tbm, 128, 1)) { bm = tbm; bn = 128; variant = 1; }
     }
-    const int64_t ctas = ((mf + bm - 1) / bm) * ((nf + bn - 1) / bn);
+    if (fill_bm == 0) { fill_bm = bm; fill_bn = bn; }
+    const int64_t ctas = ((mf + fill_bm - 1) / fill_bm) * ((nf + fill_bn - 1) / fill_bn);
     if (ctas < 2 * sms) {
       // Too few tiles to fill the GPU.  fp64 with a long contraction stays on the persistent 128 x 64 kernel and
       // slices K over its CTAs instead (16-byte loads along k, tiled TMA operands and two consumer groups are worth

@@ -459,3 +459,32 @@ def test_only_slices_are_added_up_in_segments(pkg, expr):
     """A sum that is not sliced goes into C in one piece."""
     d = _plan(pkg, expr).describe()
     assert d["ksplit"] > 1 or d["k_seg"] * 16 >= d["Kflat"]
+
+
+@pytest.mark.parametrize("expr", [
+    "C [a,20,b,6,c,6,d,95,e,2,f,23] = sum(k,2) * A [k,e,d,c,a,f] * B [k,b];",      # boxes of 20 x 6
+    "C [a,26,b,4,c,6,d,36,e,8,f,4] = sum(k,6) * A [k,b] * B [k,f,a,e,d,c];",
+    "C [a,2,b,24,c,10,d,2,e,21,f,172] = sum(k,10) * A [k,a] * B [d,c,b,e,f,k];",   # runs of two
+    "C [a,32,b,8,c,9,d,2,e,216,f,3] += sum(k,3) * A [e,d,a,f,k,c] * B [k,b];",
+    "C [a,4,b,35,c,220,d,96] -= sum(k,34) * A [k,a] * B [k,c,b,d];",
+])
+def test_outputs_of_thin_boxes_stay_off_the_resident_tile(pkg, expr):
+    """A resident tile takes some 4000 cycles however little of the output is in its box."""
+    assert not _plan(pkg, expr).describe()["kernel"].startswith("dmma_wc")
+
+
+@pytest.mark.parametrize("expr", [
+    "C [a,24,b,16,c,16,d,24,e,16,f,16] -= sum(g,24) * A [d,e,g,a] * B [g,f,b,c];",
+    "C [a,40,b,40,c,40,d,40,e,40,f,5] += sum(g,40) * A [g,a,b,c] * B [d,e,f,g];",
+])
+def test_outputs_of_full_boxes_stay_on_the_resident_tile(pkg, expr):
+    assert _plan(pkg, expr).describe()["kernel"].startswith("dmma_wc")
+
+
+@pytest.mark.parametrize("expr", [
+    "C [a,96,b,8,c,31,d,40] += sum(k,282,l,15,m,8) * A [l,b,a,m,c,k] * B [l,k,m,d];",
+    "C [a,64,b,32,c,121,d,6] = sum(k,260,l,240) * A [k,c,l] * B [l,b,a,k,d];",
+])
+def test_the_choice_of_a_tile_brings_no_slices(pkg, expr):
+    """Whether there are too few tiles to fill the GPU is the plain model's question: these sums need no scratch."""
+    assert _plan(pkg, expr).describe()["workspace_bytes"] == 0
