@@ -166,7 +166,7 @@ def test_fused_boxes_against_the_loop_nest(pkg, orc, k, ext):
 
 @pytest.mark.parametrize("k", [160, 264, 520, 1032])
 def test_split_groups_of_the_persistent_fp32_kernel(pkg, orc, k):
-    """Odd and even numbers of K steps, a last step of eight, more than one tile per CTA: the two groups' turns."""
+    """Odd and even numbers of K steps, a last step of eight, more than one tile per CTA, three launches in a row."""
     expr = "C [a,3072,b,2048] += sum(c,%d) * A [c,a] * B [c,b];" % k
     import numpy as np
     import torch
