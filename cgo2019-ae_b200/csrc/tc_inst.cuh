@@ -7,6 +7,7 @@
 #include "tc_kernels.cuh"
 #include "tc_ws_kernel.cuh"
 #include "tc_wc_kernel.cuh"
+#include "tc_wp_kernel.cuh"
 #include "tc_wt_kernel.cuh"
 
 // TC_INST_CARVE (persistent tcgen05 kernel): *threads = operand stages that fit beside args->out_bufs output tile
@@ -109,6 +110,17 @@ int run_ws_variant(const TcKernelArgs* a, void* C, const void* X, const void* Y,
 template <class CF>
 int run_wc_variant(const TcKernelArgs* a, void* C, const void* X, const void* Y, cudaStream_t stream, int mode,
                    int* threads, int* smem_bytes) {
+  if constexpr (CF::BM == 128 && CF::BN == 64) {  // the form that keeps X's tile too (args.panel)
+    using WP = WpCfg<CF::MODEX, CF::MODEY>;
+    if (mode == TC_INST_PREPARE) {
+      const int st = run_persistent<WP>(tc_wp_dmma_kernel<WP>, a, C, X, Y, stream, mode, threads, smem_bytes);
+      if (st != TC_OK) return st;
+    } else if (mode == TC_INST_LAUNCH && a->panel) {
+      TcKernelArgs b = *a;
+      b.ring_stages = WP::stages_for((int)((a->Kflat + WP::BK - 1) / WP::BK));
+      return run_persistent<WP>(tc_wp_dmma_kernel<WP>, &b, C, X, Y, stream, mode, threads, smem_bytes);
+    }
+  }
   return run_persistent<CF>(tc_wc_dmma_kernel<CF>, a, C, X, Y, stream, mode, threads, smem_bytes);
 }
 template <class CF>

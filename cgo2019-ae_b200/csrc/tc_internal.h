@@ -105,6 +105,7 @@ struct TcKernelArgs {
   uint32_t mblock_w;  // persistent kernels walk the tiles in column blocks of this many M tiles (0: M fastest over all of M)
   TcCut mcut, ncut;    // persistent fp64 kernels: the index ranges of a tile
   TcBoxMap cbox;       // ... and, for the output-resident kernel, the tile as a box of C
+  int32_t panel;       // output-resident kernel: X's tile stays in shared memory over a whole row of tiles (tc_wp_kernel.cuh)
   int32_t rows_across_x, rows_across_y;  // element copies: lanes walk the second digit of the cut (where the operand's sectors lie)
   int32_t bm, bn;    // CTA tile of the chosen kernel
   int32_t c_mode;    // 0: read-modify-write epilogue, 1: accumulators start from C,
@@ -117,7 +118,7 @@ struct TcKernelArgs {
   uint32_t k_first;  // first flattened contraction index of this launch (plans that run K in sequential passes)
   uint32_t spin_limit;  // polls a bounded wait may take before it gives up
   int32_t test_fault;   // tests only: 1 = the persistent kernel's producers leave one stage unannounced
-  int32_t out_bufs, img_sets, ring_stages;  // persistent tcgen05 kernel: how its shared memory is carved (set at launch)
+  int32_t out_bufs, img_sets, ring_stages;  // how the shared memory of the persistent tcgen05 kernel and of panels is carved (set at launch)
   const int64_t* koff_x;  // [Kflat] offset of flattened contraction index k inside X (-1: no such value, persistent fp64 kernels)
   const int64_t* koff_y;  // [Kflat] the same inside Y
   int32_t lanes_k_x;  // element-wise loader: consecutive lanes that walk k (1 = lanes walk the external index)

@@ -781,6 +781,8 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       plain_n = plain(bp.n, nf, bn);
       a.tiles_m = (uint32_t)tm;
       a.tiles_n = (uint32_t)tn;
+      // Panels (tc_wp_kernel.cuh): X's tile is kept for a whole row of tiles where the contraction is at most three K steps.
+      a.panel = bm == 128 && bn == 64 && kf <= 3 * TC_BK && tn >= 2;
       // a tiled TMA box of an operand takes consecutive values of the flattened index
       if (bp.m.b1 > 1 && bp.m.b0 != bp.m.e0) c.tma_x = false;
       if (bp.n.b1 > 1 && bp.n.b0 != bp.n.e0) c.tma_y = false;
@@ -950,7 +952,7 @@ std::string tc_plan_to_json(const tc_plan& p) {
     if (p.choice.box_c) {
       const TcBoxMap& b = a.cbox;
       auto cut = [&](const TcCut& c) { o << "[" << c.b0 << "," << c.b1 << "," << c.e0 << "," << c.e1 << "," << c.t0 << "," << c.t1 << "]"; };
-      o << ",\"cbox\":{\"m\":";
+      o << ",\"panel\":" << (a.panel ? "true" : "false") << ",\"cbox\":{\"m\":";
       cut(a.mcut);
       o << ",\"n\":";
       cut(a.ncut);

@@ -226,3 +226,14 @@ def test_a_refused_launch_is_not_reported_again():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", REFUSED_LAUNCH.format(root=root)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "held", r.stdout + r.stderr
+
+
+# Panels: every loader of both operands, one to three K steps with remainders, fewer panels than CTAs and more (whole
+# panels first, then runs of the rest), rows of two and three tiles (a group without a tile of a panel), cut tiles.
+@pytest.mark.parametrize("k", [1, 16, 17, 24, 40, 48])
+@pytest.mark.parametrize("left,right", [("e,a,b", "e,c,d"), ("a,e,b", "c,d,e"), ("e,b,a", "e,d,c"), ("b,e,a", "d,e,c")])
+@pytest.mark.parametrize("a,b,c,d,op", [(38, 90, 33, 10, "+="), (130, 150, 14, 10, "-="), (128, 149, 13, 8, "=")])
+def test_panels_against_the_loop_nest(pkg, orc, a, b, c, d, op, left, right, k):
+    expr = "C [a,%d,b,%d,c,%d,d,%d] %s sum(e,%d) * A [%s] * B [%s];" % (a, b, c, d, op, k, left, right)
+    desc, err = _run(pkg, orc, expr, tile=(128, 64), variant=4)
+    assert desc["kernel"] == "dmma_wc_128x64" and desc["panel"] and err <= 1e-12, (desc["cbox"], err)
