@@ -781,8 +781,12 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       plain_n = plain(bp.n, nf, bn);
       a.tiles_m = (uint32_t)tm;
       a.tiles_n = (uint32_t)tn;
-      // Panels (tc_wp_kernel.cuh): X's tile is kept for a whole row of tiles where the contraction is at most three K steps.
-      a.panel = bm == 128 && bn == 64 && kf <= 3 * TC_BK && tn >= 2;
+      // Panels (tc_wp_kernel.cuh): X's tile is kept for a whole row of tiles.  That pays where fetching X again and again is
+      // what takes the time: X gathered across its sectors (K = 24 156 -> 129 us, K = 10 93 -> 71), or three K steps
+      // (K = 40 1 736 -> 1 633).  Shorter contractions whose X is read along its sectors are bound by C, which the ring
+      // kernel's order of tiles -- neighbours in M at the same time -- moves 2 to 16 % faster (K = 12 to 24, nine shapes);
+      // and a CTA has to have enough tiles to hide its first panel (three tiles 14.4 -> 17.2 us, six 26.6 either way).
+      a.panel = bm == 128 && bn == 64 && kf <= 3 * TC_BK && (kf > 2 * TC_BK || (a.lanes_k_x == 1 && !c.vec_x)) && tn >= 2 && tm * tn >= 8 * sms;
       // a tiled TMA box of an operand takes consecutive values of the flattened index
       if (bp.m.b1 > 1 && bp.m.b0 != bp.m.e0) c.tma_x = false;
       if (bp.n.b1 > 1 && bp.n.b0 != bp.n.e0) c.tma_y = false;

@@ -229,11 +229,16 @@ def test_a_refused_launch_is_not_reported_again():
 
 
 # Panels: every loader of both operands, one to three K steps with remainders, fewer panels than CTAs and more (whole
-# panels first, then runs of the rest), rows of two and three tiles (a group without a tile of a panel), cut tiles.
-@pytest.mark.parametrize("k", [1, 16, 17, 24, 40, 48])
-@pytest.mark.parametrize("left,right", [("e,a,b", "e,c,d"), ("a,e,b", "c,d,e"), ("e,b,a", "e,d,c"), ("b,e,a", "d,e,c")])
-@pytest.mark.parametrize("a,b,c,d,op", [(38, 90, 33, 10, "+="), (130, 150, 14, 10, "-="), (128, 149, 13, 8, "=")])
-def test_panels_against_the_loop_nest(pkg, orc, a, b, c, d, op, left, right, k):
-    expr = "C [a,%d,b,%d,c,%d,d,%d] %s sum(e,%d) * A [%s] * B [%s];" % (a, b, c, d, op, k, left, right)
+# panels first, then runs of the rest), an odd number of tiles in a row, cut tiles.  Up to two K steps are panels only where
+# X is gathered across its sectors.
+PANEL_SIZES = [(38, 90, 283, 10, "+="), (130, 150, 64, 8, "-="), (128, 149, 65, 8, "=")]
+PANELS = [(x, y, (33, 40, 48)[(i + j) % 3], PANEL_SIZES[(i + 2 * j) % 3]) for i, x in enumerate(("e,a,b", "a,e,b", "e,b,a", "b,e,a"))
+          for j, y in enumerate(("e,c,d", "c,d,e", "e,d,c", "d,e,c"))]
+PANELS += [("b,e,a", y, k, PANEL_SIZES[(i + k) % 3]) for i, k in enumerate((1, 16, 17, 24)) for y in ("e,c,d", "d,e,c")]
+
+
+@pytest.mark.parametrize("left,right,k,size", PANELS)
+def test_panels_against_the_loop_nest(pkg, orc, left, right, k, size):
+    expr = "C [a,%d,b,%d,c,%d,d,%d] %s sum(e,%d) * A [%s] * B [%s];" % (*size, k, left, right)
     desc, err = _run(pkg, orc, expr, tile=(128, 64), variant=4)
     assert desc["kernel"] == "dmma_wc_128x64" and desc["panel"] and err <= 1e-12, (desc["cbox"], err)
