@@ -118,14 +118,14 @@ static tc_inst_fn pick_inst(const TcKernelChoice& c) {
 static int mode_of(bool ext_vec, bool k_vec) { return ext_vec ? 1 : k_vec ? 2 : 0; }
 
 // The transposed operand matrix (fp32): dimension 0 = flattened external index (stride 1), dimension 1 = contraction
-// index at `pitch` elements; box = rows x 16, no swizzle, zero fill outside the tensor.
+// index at `pitch` elements; box = rows x kbox, no swizzle, zero fill outside the tensor.
 static bool encode_operand_map_ext(TcTensorMap* out, const void* base, uint64_t ext_extent, uint64_t k_extent,
-                                   uint64_t pitch, uint32_t rows) {
+                                   uint64_t pitch, uint32_t rows, uint32_t kbox = TC_BK) {
   const tc_encode_fn fn = tc_tensor_map_encoder();
   if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || (pitch * 4) % 16 != 0 || rows > 256 || rows % 4 != 0) return false;
   const cuuint64_t dims[2] = {ext_extent, k_extent};
   const cuuint64_t strides[1] = {pitch * 4};
-  const cuuint32_t box[2] = {rows, (cuuint32_t)TC_BK};
+  const cuuint32_t box[2] = {rows, kbox};
   const cuuint32_t estr[2] = {1, 1};
   return fn(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box,
             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -133,20 +133,20 @@ static bool encode_operand_map_ext(TcTensorMap* out, const void* base, uint64_t 
 }
 
 // Tiled TMA descriptor of an operand seen as a 2-D matrix of `es`-byte elements: dimension 0 = contraction index
-// (stride 1), dimension 1 = flattened external index at `pitch` elements; box = 16 x rows, swizzled over the box
-// row (128 bytes for fp64, 64 for fp32), zero fill outside the tensor.
+// (stride 1), dimension 1 = flattened external index at `pitch` elements; box = kbox x rows, swizzled over the box
+// row (128 bytes for fp64 and pairs of fp32 K steps, 64 for one fp32 K step), zero fill outside the tensor.
 static bool encode_operand_map(TcTensorMap* out, const void* base, uint64_t k_extent, uint64_t ext_extent,
-                               uint64_t pitch, uint32_t rows, int es = 8) {
+                               uint64_t pitch, uint32_t rows, int es = 8, uint32_t kbox = TC_BK) {
   const tc_encode_fn fn = tc_tensor_map_encoder();
   if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || (pitch * es) % 16 != 0 || rows > 256) return false;
   const cuuint64_t dims[2] = {k_extent, ext_extent};
   const cuuint64_t strides[1] = {pitch * (uint64_t)es};
-  const cuuint32_t box[2] = {16, rows};
+  const cuuint32_t box[2] = {kbox, rows};
   const cuuint32_t estr[2] = {1, 1};
   static_assert(sizeof(CUtensorMap) == sizeof(TcTensorMap), "tensor map storage");
   return fn(reinterpret_cast<CUtensorMap*>(out), es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
             const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            es == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            kbox * es == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -209,6 +209,11 @@ int tc_kernels_prepare(const TcKernelChoice& c) {
     alt.variant = 2;
     st = kernels_prepare_one(alt);
   }
+  if (st == TC_OK && c.pair) {  // compiled with the persistent kernel of single CTAs
+    TcKernelChoice alt = c;
+    alt.variant = 1;
+    st = kernels_prepare_one(alt);
+  }
   if (st == TC_OK && tc_kernel_is_tmem_persistent(c)) {  // its stand-in for outputs without 16-byte alignment
     TcKernelChoice alt = c;
     alt.variant = 0;
@@ -269,6 +274,29 @@ int tc_launch_contraction(const tc_plan& p, const TcKernelArgs& args, void* C, c
   }
   tc_inst_fn fn = pick_inst(c);
   int passes = p.passes;
+  auto operand_boxes = [&](uint32_t kbox) {  // fp32 operands that are plain matrices, in either orientation
+    if (c.tma_x && encode_operand_map(&a.tmap_x, X, a.Kflat, a.Mflat, (uint64_t)a.M.s_in[0], (uint32_t)a.bm, 4, kbox)) vx = 3;
+    if (c.tma_y && encode_operand_map(&a.tmap_y, Y, a.Kflat, a.Nflat, (uint64_t)a.N.s_in[0], (uint32_t)a.bn, 4, kbox)) vy = 3;
+    if (c.tma_xe && encode_operand_map_ext(&a.tmap_x, X, a.Mflat, a.Kflat, (uint64_t)p.kdims.s_in[0], (uint32_t)a.bm, kbox)) vx = 4;
+    if (c.tma_ye && encode_operand_map_ext(&a.tmap_y, Y, a.Nflat, a.Kflat, (uint64_t)p.kdims.s_out[0], (uint32_t)a.bn, kbox)) vy = 4;
+  };
+  if (c.pair && (cu & 15) == 0 && x16 && y16) {
+    const int mx = vx, my = vy;
+    operand_boxes(32);
+    a.pair = vx >= 3 && vy >= 3;
+    if (!a.pair) { vx = mx; vy = my; }
+  }
+  if (a.pair) {
+    TcKernelChoice alt = c;
+    alt.variant = 1;  // (the pairs' kernel is compiled with the single CTAs' one)
+    fn = pick_inst(alt);
+    passes = 1;
+    a.tiles_m = (a.Mflat + 255) / 256;
+    a.tiles_n = (a.Nflat + 255) / 256;
+    a.mblock_w = a.tiles_m > 32 && a.tiles_n > 1 ? 16 : 0;
+    if (!fn) return TC_ERR_UNSUPPORTED;
+    return fn(vx, vy, &a, C, X, Y, stream, TC_INST_LAUNCH, nullptr, nullptr);
+  }
   if (tc_kernel_is_c_resident(c) && !resident) {
     a.vec_c = std::min(a.vec_c, a.standin_vec_c);
     TcKernelChoice alt = c;
@@ -293,12 +321,7 @@ int tc_launch_contraction(const tc_plan& p, const TcKernelArgs& args, void* C, c
     // k: contraction lengths that would leave more than a fifth of the boxes' k outside the tensor keep the
     // per-thread copies (K = 24: boxes of either kind measured 2-3 % slower; long contractions a fifth faster).
     const bool boxes_pay = (uint64_t)a.Kflat * 5 >= (uint64_t)((a.Kflat + TC_BK - 1) / TC_BK * TC_BK) * 4;
-    if (p.opt.tma != 1 && p.opt.tma != 3 && boxes_pay) {
-      if (c.tma_x && encode_operand_map(&a.tmap_x, X, a.Kflat, a.Mflat, (uint64_t)a.M.s_in[0], (uint32_t)a.bm, 4)) vx = 3;
-      if (c.tma_y && encode_operand_map(&a.tmap_y, Y, a.Kflat, a.Nflat, (uint64_t)a.N.s_in[0], (uint32_t)a.bn, 4)) vy = 3;
-      if (c.tma_xe && encode_operand_map_ext(&a.tmap_x, X, a.Mflat, a.Kflat, (uint64_t)p.kdims.s_in[0], (uint32_t)a.bm)) vx = 4;
-      if (c.tma_ye && encode_operand_map_ext(&a.tmap_y, Y, a.Nflat, a.Kflat, (uint64_t)p.kdims.s_out[0], (uint32_t)a.bn)) vy = 4;
-    }
+    if (p.opt.tma != 1 && p.opt.tma != 3 && boxes_pay) operand_boxes(TC_BK);
     // How the kernel's shared memory is carved.  Short contractions are bound by the output stream: tile buffers,
     // so that enough of C is in flight.  Long ones are bound by the MMAs: one tile buffer, a second image set and
     // every operand stage that fits.  (Swept on B200 over both kernels and contractions of 24 to 2048: no other

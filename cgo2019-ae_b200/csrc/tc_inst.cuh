@@ -9,6 +9,7 @@
 #include "tc_wc_kernel.cuh"
 #include "tc_wp_kernel.cuh"
 #include "tc_wt_kernel.cuh"
+#include "tc_wd_kernel.cuh"
 
 // TC_INST_CARVE (persistent tcgen05 kernel): *threads = operand stages that fit beside args->out_bufs output tile
 // buffers and args->img_sets image sets.
@@ -130,6 +131,23 @@ int run_wt_variant(const TcKernelArgs* a, void* C, const void* X, const void* Y,
     if (!a || !threads || a->out_bufs < 1 || a->out_bufs > CF::MAX_CBUFS || a->img_sets < 1 || a->img_sets > CF::MAX_IMGS) return TC_ERR_INVALID_ARG;
     *threads = CF::stages_for(a->out_bufs, a->img_sets);
     return *threads >= 2 ? TC_OK : TC_ERR_UNSUPPORTED;
+  }
+  if constexpr (CF::BM == 128 && CF::MODEX >= 3 && CF::MODEY >= 3) {  // the form on pairs of CTAs (args.pair)
+    using WD = WdCfg<CF::MODEX, CF::MODEY>;
+    if (mode == TC_INST_PREPARE) {
+      const int st = run_persistent<WD>(tc_wd_tf32_kernel<WD>, a, C, X, Y, stream, mode, threads, smem_bytes);
+      if (st != TC_OK) return st;
+    } else if (mode == TC_INST_LAUNCH && a->pair) {
+      int dev = 0, sms = 0;
+      TC_CUDA_OK(cudaGetDevice(&dev));
+      TC_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      // (fewer tiles than half of the pairs: the kernel halves them)
+      const unsigned tiles = a->tiles_m * a->tiles_n, most = (unsigned)sms / 2, pairs = 2 * tiles <= most ? 2 * tiles : tiles < most ? tiles : most;
+      tc_wd_tf32_kernel<WD><<<2 * pairs, WD::CTA_THREADS, WD::SMEM_BYTES, stream>>>(*a, static_cast<float*>(C), static_cast<const float*>(X),
+                                                                                  static_cast<const float*>(Y));
+      TC_CUDA_OK(cudaGetLastError());
+      return TC_OK;
+    }
   }
   return run_persistent<CF>(tc_wt_tf32_kernel<CF>, a, C, X, Y, stream, mode, threads, smem_bytes);
 }

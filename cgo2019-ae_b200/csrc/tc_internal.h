@@ -105,7 +105,6 @@ struct TcKernelArgs {
   uint32_t mblock_w;  // persistent kernels walk the tiles in column blocks of this many M tiles (0: M fastest over all of M)
   TcCut mcut, ncut;    // persistent fp64 kernels: the index ranges of a tile
   TcBoxMap cbox;       // ... and, for the output-resident kernel, the tile as a box of C
-  int32_t panel;       // output-resident kernel: X's tile stays in shared memory over a whole row of tiles (tc_wp_kernel.cuh)
   int32_t rows_across_x, rows_across_y;  // element copies: lanes walk the second digit of the cut (where the operand's sectors lie)
   int32_t bm, bn;    // CTA tile of the chosen kernel
   int32_t c_mode;    // 0: read-modify-write epilogue, 1: accumulators start from C,
@@ -139,6 +138,8 @@ struct TcKernelArgs {
   TcTensorMap tmap_c;    // its rank-5 descriptor with box (warp rows, 1, 8, 1, 1)
   TcTensorMap tmap_ct;   // the same tensor with box (bm, 2, bn / 2, 1, 1); output-resident kernel: cbox
   int* status;       // device word: 0, or the code of a wait that ran out of polls (persistent kernels)
+  int32_t panel;     // output-resident kernel: X's tile stays in shared memory over a whole row of tiles (tc_wp_kernel.cuh)
+  int32_t pair;      // fp32: runs on 256 x 256 tiles on pairs of CTAs (tc_wd_kernel.cuh; set at launch)
 };
 
 enum TcMath { TC_MATH_DMMA = 0, TC_MATH_SIMT = 1, TC_MATH_TF32X3 = 2, TC_MATH_TF32TC = 3 };
@@ -155,6 +156,7 @@ struct TcKernelChoice {
   bool tma_c;           // a warp's 8-row output batch is a box of a rank-5 tensor over C
   bool tma_ct;          // ... and so is a whole bm x bn tile
   bool box_c;           // a cut tile is a box of C (args.cbox)
+  bool pair;            // fp32: 256 x 256 tiles on pairs of CTAs (tc_wd_kernel.cuh) wherever the tensors are 16-byte aligned
 };
 
 struct TcHostPipe;

@@ -574,6 +574,22 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   //   * anything that would leave most SMs without a tile: 64 x 64, one CTA per tile.
   const int64_t sms = p->sm_count > 0 ? p->sm_count : TC_DEFAULT_SMS;
   int bm = 128, bn = 128, variant = 0, fill_bm = 0, fill_bn = 0;
+  // fp32 on pairs of CTAs (tc_wd_kernel.cuh): both operands in tiled boxes that hold few k beyond the contraction, a
+  // contraction long enough for the products to be what takes the time, and an output of which 32 columns from a multiple
+  // of 32 on are neighbours.  Its time and that of the kernels it takes the place of, in us (measured on one B200, 720
+  // x 2064 to 4096 x 4096, K = 400 to 3664): a round of tiles takes 1.4 us per 32 k on the pairs (for four times the
+  // products) and 1.23 on 128 x 128 tiles; the mma.sync kernels, which take problems of fewer tiles, reach 25 to 33 TFLOP/s
+  // of products on whole tiles.
+  c.pair = false;
+  const bool boxes_pay = (uint64_t)kf * 5 >= (uint64_t)((kf + TC_BK - 1) / TC_BK * TC_BK) * 4;
+  const bool pair_shape = p->dtype == TC_F32 && p->opt.tma != 1 && p->opt.tma != 3 && p->opt.c_path == 0 && boxes_pay && kf >= 16 * TC_BK &&
+                          (c.tma_x || c.tma_xe) && (c.tma_y || c.tma_ye) && a.vec_c == 4 && (a.M.n == 1 || a.M.extent[0] % 32 == 0);
+  auto rounds_of = [](int64_t tiles, int64_t at_once) { return (double)((tiles + at_once - 1) / at_once); };
+  const int64_t pairs = std::max<int64_t>(1, sms / 2), pair_tiles = ((mf + 255) / 256) * ((nf + 255) / 256), pair_left = pair_tiles % pairs;
+  const double pair_rounds = (double)(pair_tiles / pairs) + (pair_left == 0 ? 0.0 : 2 * pair_left <= pairs ? 0.7 : 1.0);
+  const double pair_us = pair_rounds * (1.38 * (double)((kf + 31) / 32) + 4.0);
+  const double single_us = rounds_of(((mf + 127) / 128) * ((nf + 127) / 128), sms) * (0.0385 * (double)kf + 2.0);
+  const double sync_us = 2.0 * (double)((mf + 63) / 64 * 64) * (double)((nf + 63) / 64 * 64) * (double)kf / 32.0e6 + 5.0;
   bool slice_persistent = false;  // the persistent reduce-add kernel with K slices (few tiles, long contraction)
   if (p->box_order >= 0) {  // second pass: the tile is the first pass's
     bm = p->box_bm;
@@ -702,6 +718,12 @@ int tc_plan_build(tc_plan* p, std::string* why) {
         bn = 128;
       }
     }
+    if (c.math != TC_MATH_SIMT && pair_shape && path == TC_PATH_AUTO && p->opt.split_k == 0 &&
+        pair_us < 0.8 * (c.math == TC_MATH_TF32TC ? single_us : sync_us)) {
+      c.math = TC_MATH_TF32TC;
+      bm = bn = 128;
+      c.pair = true;
+    }
     if (c.math == TC_MATH_TF32TC && p->opt.split_k == 0 && p->opt.c_path != 2) {
       // ... as the persistent kernel (two accumulators in tensor memory, output tile staged in shared memory)
       // wherever its tile buffers can hold the output in runs that leave as bulk copies and both operands are
@@ -714,7 +736,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     }
     if (fill_bm == 0) { fill_bm = bm; fill_bn = bn; }
     const int64_t ctas = ((mf + fill_bm - 1) / fill_bm) * ((nf + fill_bn - 1) / fill_bn);
-    if (ctas < 2 * sms) {
+    if (ctas < 2 * sms && !c.pair) {
       // Too few tiles to fill the GPU.  fp64 with a long contraction stays on the persistent 128 x 64 kernel and
       // slices K over its CTAs instead (16-byte loads along k, tiled TMA operands and two consumer groups are worth
       // more than small tiles: measured 3-4 x on few-tile, long-K items of the reference's list); everything else
@@ -748,6 +770,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   c.bm = bm;
   c.bn = bn;
   c.variant = variant;
+  if (tc_kernel_is_tmem_persistent(c) && pair_shape && bm == 128 && p->opt.split_k == 0) c.pair = pair_us < single_us;
   if (tc_kernel_is_tmem_persistent(c) && !wt_eligible(a, bm, es)) {
     *why = "the persistent tcgen05 kernel needs an output whose tile rows are 16-byte aligned contiguous runs";
     return TC_ERR_UNSUPPORTED;
@@ -864,7 +887,8 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   if ((c.math == TC_MATH_TF32X3 || c.math == TC_MATH_TF32TC) && p->opt.split_k == 0 && !persistent) {
     const int64_t per_slice = tiles * bm * bn * (int64_t)es;
     const int64_t want = std::min<int64_t>((kf + TC_TF32_CHAIN - 1) / TC_TF32_CHAIN, ksteps);
-    if (want > 1 && want * per_slice > (int64_t(1) << 30) && ksplit == 1) p->passes = (int)std::min<int64_t>(want, 1 << 20);
+    if (c.pair) p->passes = (int)want;  // (what runs in its place where a tensor is not aligned; without scratch)
+    else if (want > 1 && want * per_slice > (int64_t(1) << 30) && ksplit == 1) p->passes = (int)std::min<int64_t>(want, 1 << 20);
     else ksplit = std::max<int64_t>(ksplit, want);
   }
   if (p->passes > 1) {
@@ -885,7 +909,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   }
   if (tiles * ksplit >= (int64_t(1) << 31)) { *why = "too many tiles"; return TC_ERR_UNSUPPORTED; }
   p->ws_bytes = ksplit > 1 ? (size_t)(ksplit * tiles * bm * bn) * es : 0;
-  p->launches = ksplit > 1 ? 2 : p->passes;
+  p->launches = ksplit > 1 ? 2 : c.pair ? 1 : p->passes;
 
   // Staged bulk epilogue of the vector-pipe kernels: the tile's rows split into runs of E0 elements
   // contiguous in the output; if the output's next index belongs to the other operand (its stride equals
@@ -929,7 +953,7 @@ std::string tc_plan_to_json(const tc_plan& p) {
     << "\",\"committed\":" << (p.committed ? "true" : "false");
   // longest tensor-core accumulation chain of the plan
   uint32_t chain = std::min<uint32_t>(a.k_chunk, a.Kflat);
-  if (tc_kernel_is_tmem_persistent(p.choice)) {
+  if (tc_kernel_is_tmem_persistent(p.choice) || p.choice.pair) {
     const uint32_t steps = (a.Kflat + TC_BK - 1) / TC_BK, segs = (steps + 31) / 32;
     chain = std::min<uint32_t>(a.Kflat, ((steps + segs - 1) / segs) * TC_BK);
   }
@@ -949,7 +973,8 @@ std::string tc_plan_to_json(const tc_plan& p) {
       << ",\"kvec_y\":" << (p.choice.kvec_y ? "true" : "false") << ",\"tma_x\":" << (p.choice.tma_x ? "true" : "false")
       << ",\"tma_y\":" << (p.choice.tma_y ? "true" : "false") << ",\"tma_xe\":" << (p.choice.tma_xe ? "true" : "false")
       << ",\"tma_ye\":" << (p.choice.tma_ye ? "true" : "false") << ",\"tma_c\":" << (p.choice.tma_c ? "true" : "false") << ",\"tma_ct\":" << (p.choice.tma_ct ? "true" : "false")
-      << ",\"lanes_k_x\":" << a.lanes_k_x
+
+      << ",\"pair\":" << (p.choice.pair ? "true" : "false") << ",\"lanes_k_x\":" << a.lanes_k_x
       << ",\"lanes_k_y\":" << a.lanes_k_y << ",\"vec_c\":" << a.vec_c << ",\"standin_vec_c\":" << a.standin_vec_c << ",\"epi_run\":" << a.epi_run << ",\"epi_n_span\":" << a.epi_n_span << ",\"beta\":" << a.beta
       << ",\"alpha\":" << a.alpha << ",\"workspace_bytes\":" << p.ws_bytes << ",\"launches\":" << p.launches
       << ",\"flops\":" << p.flops << ",\"bytes\":" << p.bytes;

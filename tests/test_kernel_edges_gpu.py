@@ -242,3 +242,42 @@ def test_panels_against_the_loop_nest(pkg, orc, left, right, k, size):
     expr = "C [a,%d,b,%d,c,%d,d,%d] %s sum(e,%d) * A [%s] * B [%s];" % (*size, k, left, right)
     desc, err = _run(pkg, orc, expr, tile=(128, 64), variant=4)
     assert desc["kernel"] == "dmma_wc_128x64" and desc["panel"] and err <= 1e-12, (desc["cbox"], err)
+
+
+# fp32 on pairs of CTAs: both orientations of either operand, rows and columns off the 256-wide tile, contractions whose
+# last unit of 32 has one to four groups of eight, chains of one and several segments, more tiles than pairs, rows in runs of
+# 32 and 64 of a three-index output; against 64 bits.
+PAIRS = [("C [a,%d,b,%d] += sum(c,%d) * A [c,a] * B [c,b];", (2048, 2048, 256)), ("C [a,%d,b,%d] -= sum(c,%d) * A [a,c] * B [c,b];", (1796, 1300, 260)),
+         ("C [a,%d,b,%d] = sum(c,%d) * A [c,a] * B [b,c];", (720, 2064, 1104)), ("C [a,%d,b,%d] += sum(c,%d) * A [a,c] * B [b,c];", (3328, 3332, 520)),
+         ("C [a,%d,b,%d] = sum(c,%d) * A [a,c] * B [c,b];", (2052, 1028, 2076)), ("C [a,32,b,%d,d,%d] += sum(c,%d) * A [c,a,d] * B [b,c];", (2400, 104, 548)),
+         ("C [a,64,b,%d,d,%d] -= sum(c,%d) * A [c,a,d] * B [c,b];", (2200, 54, 308))]
+
+
+@pytest.mark.parametrize("form,size", PAIRS)
+@pytest.mark.parametrize("shift", [0, 1])
+def test_pairs_of_ctas(pkg, form, size, shift):
+    import torch
+    torch.cuda.set_device(0)
+    expr = form % size
+    p = pkg.parse(expr)
+    ext = dict(zip(p["out_idx"] + p["sum_idx"], p["out_ext"] + p["sum_ext"]))
+    numel = lambda key: int(torch.tensor([ext[i] for i in p[key]]).prod())
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    # shift 1: no tensor is 16-byte aligned, and the plan runs on single CTAs
+    c, a, b = (torch.rand(numel(key) + 4, device="cuda", generator=gen)[shift:][:numel(key)] - 0.5 for key in ("out_idx", "left_idx", "right_idx"))
+    if shift:
+        c, a, b = (torch.cat([torch.zeros(1, device="cuda"), t])[1:] for t in (c, a, b))
+    view = lambda t, key: t.double().view([ext[i] for i in reversed(p[key])])
+    text = ["".join(reversed(p[key])) for key in ("out_idx", "left_idx", "right_idx")]
+    want = torch.einsum("%s,%s->%s" % (text[1], text[2], text[0]), view(a, "left_idx"), view(b, "right_idx")).reshape(-1)
+    want = want if p["op"] == "=" else c.double() - want if p["op"] == "-=" else c.double() + want
+    plan = pkg.Plan(expr, pkg.F32)
+    d = plan.describe()
+    assert d["pair"] and d["chain"] <= 512 and d["workspace_bytes"] == 0, d
+    for _ in range(2):
+        got = torch.cat([torch.zeros(4, device="cuda"), c])[4:] if not shift else torch.cat([torch.zeros(1, device="cuda"), c])[1:]
+        plan.execute(got, a, b)
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        assert float((got.double() - want).abs().max() / want.abs().max()) <= 1e-5
+    plan.close()
