@@ -751,6 +751,22 @@ int tc_plan_build(tc_plan* p, std::string* why) {
         slice_persistent = true;
       } else {
         bm = 64; bn = 64; variant = 0;
+        // fp64 again, where K is not sliced (too short, or enough tiles): the one-tile kernel waits for memory once per K
+        // step, 1.2 us a step where both operands load by vector and 2 to 5 where one is gathered, however little of the
+        // GPU its tiles fill; the persistent 128 x 32 kernels run ahead (two tiles per SM at 1.15 us a step, 1.35 where
+        // both have one and twice that where X is gathered across its sectors; the resident form, one per SM, 0.8).
+        // From five steps and 32 tiles on and up to one round of them: 35 sums, 1.1 to 2.4 times as fast (1088 x 688 x 436
+        // 62 -> 40 us; 19800 x 19 x 120, gathered, 42 -> 19); below that within 15 % either way, beyond 8 % slower (374).
+        const int64_t t32 = ((mf + 127) / 128) * ((nf + 31) / 32);
+        if (c.math == TC_MATH_DMMA && p->opt.split_k == 0 && p->opt.variant == 0 && p->opt.c_path == 0 && p->opt.tma == 0 && steps >= 5 && t32 >= 32 && t32 <= 2 * sms &&
+            !(t64 * 2 <= sms && steps >= 16)) {
+          bm = 128; bn = 32; variant = 2;
+          double ws_us = rounds_of(t32, 2 * sms) * (double)steps * (t32 > sms ? 1.35 : 1.15) + 6.0;
+          if (a.lanes_k_x == 1 && !c.vec_x) ws_us *= 2.0;
+          int order = -1;
+          const BoxPlan bp = best_boxes(128, 32, &order);
+          if (bp.ok && rounds_of((int64_t)bp.tiles, sms) * (double)steps * 0.8 + 5.0 < ws_us) variant = 3;
+        }
         if (c.math == TC_MATH_TF32TC) c.math = TC_MATH_TF32X3;  // no 64-wide tcgen05 tile: same arithmetic on mma.sync
       }
     }
