@@ -581,6 +581,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   // products) and 1.23 on 128 x 128 tiles; the mma.sync kernels, which take problems of fewer tiles, reach 25 to 33 TFLOP/s
   // of products on whole tiles.
   c.pair = false;
+  bool unaligned = false;  // fp32 without any alignment on the one-tile tcgen05 kernel
   const bool boxes_pay = (uint64_t)kf * 5 >= (uint64_t)((kf + TC_BK - 1) / TC_BK * TC_BK) * 4;
   const bool pair_shape = p->dtype == TC_F32 && p->opt.tma != 1 && p->opt.tma != 3 && p->opt.c_path == 0 && boxes_pay && kf >= 16 * TC_BK &&
                           (c.tma_x || c.tma_xe) && (c.tma_y || c.tma_ye) && a.vec_c == 4 && (a.M.n == 1 || a.M.extent[0] % 32 == 0);
@@ -718,6 +719,15 @@ int tc_plan_build(tc_plan* p, std::string* why) {
         bn = 128;
       }
     }
+    // Nothing aligned: both operands element by element and an output of odd extents.  The one-tile tcgen05 kernel is 1.2 to
+    // 2 times as fast as the mma.sync ones there (nineteen products of 39 to 180 565 rows, K = 10 to 3 795; one of K = 10
+    // 2 % slower); with 16-byte loads or stores somewhere they win as often as they lose.
+    if (c.math == TC_MATH_TF32X3 && path == TC_PATH_AUTO && p->opt.split_k == 0 && p->opt.c_path == 0 && a.vec_c == 1 && !c.vec_x && !c.kvec_x && !c.vec_y &&
+        !c.kvec_y && ((mf + 127) / 128) * ((nf + 127) / 128) >= 96) {
+      c.math = TC_MATH_TF32TC;
+      bm = bn = 128;
+      unaligned = true;
+    }
     if (c.math != TC_MATH_SIMT && pair_shape && path == TC_PATH_AUTO && p->opt.split_k == 0 &&
         pair_us < 0.8 * (c.math == TC_MATH_TF32TC ? single_us : sync_us)) {
       c.math = TC_MATH_TF32TC;
@@ -736,7 +746,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     }
     if (fill_bm == 0) { fill_bm = bm; fill_bn = bn; }
     const int64_t ctas = ((mf + fill_bm - 1) / fill_bm) * ((nf + fill_bn - 1) / fill_bn);
-    if (ctas < 2 * sms && !c.pair) {
+    if (ctas < 2 * sms && !c.pair && !unaligned) {
       // Too few tiles to fill the GPU.  fp64 with a long contraction stays on the persistent 128 x 64 kernel and
       // slices K over its CTAs instead (16-byte loads along k, tiled TMA operands and two consumer groups are worth
       // more than small tiles: measured 3-4 x on few-tile, long-K items of the reference's list); everything else
