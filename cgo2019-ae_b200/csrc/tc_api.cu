@@ -729,8 +729,11 @@ class CopyPool {
   size_t piece_ = 0, bytes_ = 0;
 };
 
-constexpr size_t kBounceBytes = size_t(8) << 20;
-constexpr int kBounceCount = 3;
+// Small buffers and all cores but a few: a copy over the link starts when its buffer is filled, so the first and the last
+// buffer are not overlapped with anything.  48^4 outputs and inputs (85 MB in, 42 MB out) on 16 cores: 9.0 ms with three
+// buffers of 8 MB and four helpers, 6.6 with twelve helpers, 4.9 with 2 MB and six, 4.0 with 2 MB and twelve.
+constexpr size_t kBounceBytes = size_t(2) << 20;
+constexpr int kBounceCount = 6;
 
 bool is_pageable(const void* ptr) {
   cudaPointerAttributes at;
@@ -896,7 +899,7 @@ static int host_pipe_enable_staging(TcHostPipe* h) {
   }
   TC_CUDA_OK(cudaStreamCreateWithFlags(&h->out_stream, cudaStreamNonBlocking));
   const unsigned hw = std::max(2u, std::thread::hardware_concurrency());
-  const int helpers = (int)std::min(6u, std::max(1u, hw / 4));
+  const int helpers = (int)std::min(12u, std::max(1u, hw - 2));
   h->pool_in = new CopyPool(helpers);
   h->pool_out = new CopyPool(helpers);
   return TC_OK;
@@ -935,7 +938,7 @@ struct Drain {
   void close() { { std::lock_guard<std::mutex> l(mu); closed = true; } cv.notify_one(); }
   int run_job(const DrainJob& j) {
     TC_CUDA_OK(cudaStreamWaitEvent(h->out_stream, j.after, 0));
-    // two-deep: the copy of chunk c + 1 is in flight while chunk c is emptied into the caller's memory
+    // the copies of the next chunks are in flight while chunk c is emptied into the caller's memory
     size_t issued = 0, drained = 0;
     int bi = 0, bd = 0;
     size_t len[kBounceCount] = {};
