@@ -724,9 +724,11 @@ int tc_plan_build(tc_plan* p, std::string* why) {
     // 2 % slower); with 16-byte loads or stores somewhere they win as often as they lose.
     if (c.math == TC_MATH_TF32X3 && path == TC_PATH_AUTO && p->opt.split_k == 0 && p->opt.c_path == 0 && a.vec_c == 1 && !c.vec_x && !c.kvec_x && !c.vec_y &&
         !c.kvec_y && ((mf + 127) / 128) * ((nf + 127) / 128) >= 96) {
-      c.math = TC_MATH_TF32TC;
-      bm = bn = 128;
-      unaligned = true;
+      // (up to 64 columns, of which it would compute 128, the small mma.sync tile: four sums, 1.2 to 1.3 times the 128-wide
+      // one, level with or up to 14 % ahead of tcgen05)
+      if (nf > 64) c.math = TC_MATH_TF32TC;
+      bm = bn = nf > 64 ? 128 : 64;
+      unaligned = nf > 64;
     }
     if (c.math != TC_MATH_SIMT && pair_shape && path == TC_PATH_AUTO && p->opt.split_k == 0 &&
         pair_us < 0.8 * (c.math == TC_MATH_TF32TC ? single_us : sync_us)) {
@@ -770,12 +772,12 @@ int tc_plan_build(tc_plan* p, std::string* why) {
         const int64_t t32 = ((mf + 127) / 128) * ((nf + 31) / 32);
         if (c.math == TC_MATH_DMMA && p->opt.split_k == 0 && p->opt.variant == 0 && p->opt.c_path == 0 && p->opt.tma == 0 && steps >= 5 && t32 >= 32 && t32 <= 2 * sms &&
             !(t64 * 2 <= sms && steps >= 16)) {
-          bm = 128; bn = 32; variant = 2;
-          double ws_us = rounds_of(t32, 2 * sms) * (double)steps * (t32 > sms ? 1.35 : 1.15) + 6.0;
-          if (a.lanes_k_x == 1 && !c.vec_x) ws_us *= 2.0;
+          const bool across = a.lanes_k_x == 1 && !c.vec_x;
+          const double ws_us = (rounds_of(t32, 2 * sms) * (double)steps * (t32 > sms ? 1.35 : 1.15) + 6.0) * (across ? 2.0 : 1.0);
           int order = -1;
           const BoxPlan bp = best_boxes(128, 32, &order);
-          if (bp.ok && rounds_of((int64_t)bp.tiles, sms) * (double)steps * 0.8 + 5.0 < ws_us) variant = 3;
+          if (bp.ok && rounds_of((int64_t)bp.tiles, sms) * (double)steps * 0.8 + 5.0 < ws_us) { bm = 128; bn = 32; variant = 3; }
+          else if (!across || nf <= 32) { bm = 128; bn = 32; variant = 2; }  // (more than once across its sectors: 61 -> 71 us)
         }
         if (c.math == TC_MATH_TF32TC) c.math = TC_MATH_TF32X3;  // no 64-wide tcgen05 tile: same arithmetic on mma.sync
       }
