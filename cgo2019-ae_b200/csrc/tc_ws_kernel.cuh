@@ -529,8 +529,8 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
     };
     uint32_t tm, tn;
     tile_coords(p, tile % tiles, &tm, &tn);
-    static_assert(NB2 <= 2, "groups of columns");
     const bool plain_n = p.ncut.b0 == BN && p.ncut.e0 == p.Nflat, plain_m = p.mcut.b0 == BM && p.mcut.e0 == p.Mflat;
+    static_assert(NB2 <= 2, "groups of columns");
     int cols = plain_n ? (int)p.Nflat - (int)(tn * BN) - wn0 : WN;  // of this warp's WN columns inside the tensor
     if (plain_m && tm * BM + wm0 >= p.Mflat) cols = 0;
     bool ok;
@@ -750,27 +750,35 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
           dst[1] = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
         }
         __syncwarp();
-        // four rows at a time: their old values are all on the way before the first sum is stored (a row at a time,
-        // which is what the compiler must do where rows could overlap, every row waits for memory by itself)
-        constexpr int MQ = (WM + 31) / 32;
+        // `+=` and `-=` are reductions in the memory system, as the bulk copies' are: nothing is read, no row waits for
+        // memory.  What a batch of rows needs is read before its first element is stored (the compiler may not move a read
+        // up past a store that could meet it).  One-index term 65 x 83 x 40 x 81, K = 32: 196 -> 123 us; triples terms of
+        // odd extents, K = 10 to 16: 74 -> 53, 45 -> 32, 262 -> 215; 61 x 31 x 47 x 67, K = 43: 72 -> 59.  (The whole tile
+        // through the staging area to the store warpgroup, so that the consumers go on: faster on two, 4 to 25 % slower on
+        // five others, overwritten outputs above all.)
+        constexpr int MQ = (WM + 31) / 32, RB = 4;
         int64_t co[MQ];
 #pragma unroll
         for (int q = 0; q < MQ; ++q) co[q] = lane + 32 * q < WM ? offc_m[wm0 + lane + 32 * q] : -1;
 #pragma unroll
-        for (int r0 = 0; r0 < 8; r0 += 4) {
-          int64_t cn[4];
-          double old[4][MQ];
+        for (int r0 = 0; r0 < 8; r0 += RB) {
+          int64_t cn[RB];
+          double v[RB][MQ];
 #pragma unroll
-          for (int r = 0; r < 4; ++r) {
+          for (int r = 0; r < RB; ++r) {
             cn[r] = offc_n[wn0 + 16 * (nb >> 1) + 2 * (r0 + r) + (nb & 1)];
 #pragma unroll
-            for (int q = 0; q < MQ; ++q) old[r][q] = accumulate && (cn[r] | co[q]) >= 0 ? C[cn[r] + co[q]] : 0.0;
+            for (int q = 0; q < MQ; ++q) v[r][q] = cst[(r0 + r) * CF::CPITCH + lane + 32 * q];
           }
 #pragma unroll
-          for (int r = 0; r < 4; ++r)
+          for (int r = 0; r < RB; ++r)
 #pragma unroll
-            for (int q = 0; q < MQ; ++q)
-              if ((cn[r] | co[q]) >= 0) C[cn[r] + co[q]] = cst[(r0 + r) * CF::CPITCH + lane + 32 * q] + old[r][q];
+            for (int q = 0; q < MQ; ++q) {
+              if ((cn[r] | co[q]) < 0) continue;
+              double* dst = C + cn[r] + co[q];
+              if (accumulate) asm volatile("red.global.add.f64 [%0], %1;\n" ::"l"(dst), "d"(v[r][q]) : "memory");
+              else *dst = v[r][q];
+            }
         }
         __syncwarp();
       }
