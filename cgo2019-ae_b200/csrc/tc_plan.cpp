@@ -772,7 +772,9 @@ int tc_plan_build(tc_plan* p, std::string* why) {
         const int64_t t32 = ((mf + 127) / 128) * ((nf + 31) / 32);
         if (c.math == TC_MATH_DMMA && p->opt.split_k == 0 && p->opt.variant == 0 && p->opt.c_path == 0 && p->opt.tma == 0 && steps >= 5 && t32 >= 32 && t32 <= 2 * sms &&
             !(t64 * 2 <= sms && steps >= 16)) {
-          const bool across = a.lanes_k_x == 1 && !c.vec_x;
+          // (lanes on M's first index read neighbours where that is X's fastest too, only an odd one: 979 x 1032 x 263
+          // 47 -> 40 us, 617 x 1840 x 281 49 -> 42)
+          const bool across = a.lanes_k_x == 1 && !c.vec_x && a.M.s_in[0] != 1;
           const double ws_us = (rounds_of(t32, 2 * sms) * (double)steps * (t32 > sms ? 1.35 : 1.15) + 6.0) * (across ? 2.0 : 1.0);
           int order = -1;
           const BoxPlan bp = best_boxes(128, 32, &order);
@@ -837,7 +839,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       // (K = 40 1 736 -> 1 633).  Shorter contractions whose X is read along its sectors are bound by C, which the ring
       // kernel's order of tiles -- neighbours in M at the same time -- moves 2 to 16 % faster (K = 12 to 24, nine shapes);
       // and a CTA has to have enough tiles to hide its first panel (three tiles 14.4 -> 17.2 us, six 26.6 either way).
-      a.panel = bm == 128 && bn == 64 && kf <= 3 * TC_BK && (kf > 2 * TC_BK || (a.lanes_k_x == 1 && !c.vec_x)) && tn >= 2 && tm * tn >= 8 * sms;
+      a.panel = bm == 128 && bn == 64 && kf <= 3 * TC_BK && (kf > 2 * TC_BK || (a.lanes_k_x == 1 && !c.vec_x && a.M.s_in[0] != 1)) && tn >= 2 && tm * tn >= 8 * sms;
       // a tiled TMA box of an operand takes consecutive values of the flattened index
       if (bp.m.b1 > 1 && bp.m.b0 != bp.m.e0) c.tma_x = false;
       if (bp.n.b1 > 1 && bp.n.b0 != bp.n.e0) c.tma_y = false;
