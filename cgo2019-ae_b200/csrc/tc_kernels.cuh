@@ -709,43 +709,52 @@ __global__ void __launch_bounds__(CF::THREADS, CF::MIN_CTAS) tc_contract_kernel(
     // consecutive lanes are on consecutive m, which are neighbours in C inside a run.  `+=` and `-=` are reductions in the
     // memory system: no element waits for its old value, and one access after another was what this epilogue took its time
     // for (39 x 50 x 28 sum 24 16.4 -> 5.4 us, 42 x 75 x 25 sum 14 10.8 -> 5.0, 31 x 39 x 53 x 25 sum 41 36.7 -> 18.5).
+    // The thread's index is read anew, out of the compiler's sight: with the places in the rows worked out from the values
+    // of the product loop it orders that loop differently where both operands load by vector (880 x 1864 sum 936 133 us, so
+    // 125).
     __syncthreads();
-    constexpr int CPITCH = WM + 2, MQ = (WM + 31) / 32, RB = 4;
-    static_assert(CF::WARPS * 8 * CPITCH <= STAGES * CF::STAGE_ELEMS, "rows in the stages");
-    double* cst = Xs + warp * 8 * CPITCH;
-    int64_t co[MQ];
+    int tx;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tx));
+    {
+      const int lane = tx & 31, warp = tx >> 5, g = lane >> 2, t = lane & 3;
+      const int wm0 = (warp % CF::WARPS_M) * WM, wn0 = (warp / CF::WARPS_M) * WN;
+      constexpr int CPITCH = WM + 2, MQ = (WM + 31) / 32, RB = 4;
+      static_assert(CF::WARPS * 8 * CPITCH <= STAGES * CF::STAGE_ELEMS, "rows in the stages");
+      double* cst = Xs + warp * 8 * CPITCH;
+      int64_t co[MQ];
 #pragma unroll
-    for (int q = 0; q < MQ; ++q) co[q] = lane + 32 * q < WM ? offc_m[wm0 + lane + 32 * q] : -1;
+      for (int q = 0; q < MQ; ++q) co[q] = lane + 32 * q < WM ? offc_m[wm0 + lane + 32 * q] : -1;
 #pragma unroll
-    for (int nb = 0; nb < 2 * NB2; ++nb) {
+      for (int nb = 0; nb < 2 * NB2; ++nb) {
 #pragma unroll
-      for (int i = 0; i < MB2; ++i) {
-        double2* dst = reinterpret_cast<double2*>(cst + g * CPITCH + 16 * i + 4 * t);
-        dst[0] = make_double2(alpha * acc[nb][2 * i][0], alpha * acc[nb][2 * i + 1][0]);
-        dst[1] = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int r0 = 0; r0 < 8; r0 += RB) {
-        int64_t cn[RB];
-        double v[RB][MQ];
-#pragma unroll
-        for (int r = 0; r < RB; ++r) {
-          cn[r] = offc_n[wn0 + 16 * (nb >> 1) + 2 * (r0 + r) + (nb & 1)];
-#pragma unroll
-          for (int q = 0; q < MQ; ++q) v[r][q] = lane + 32 * q < WM ? cst[(r0 + r) * CPITCH + lane + 32 * q] : 0.0;
+        for (int i = 0; i < MB2; ++i) {
+          double2* dst = reinterpret_cast<double2*>(cst + g * CPITCH + 16 * i + 4 * t);
+          dst[0] = make_double2(alpha * acc[nb][2 * i][0], alpha * acc[nb][2 * i + 1][0]);
+          dst[1] = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
         }
+        __syncwarp();
 #pragma unroll
-        for (int r = 0; r < RB; ++r)
+        for (int r0 = 0; r0 < 8; r0 += RB) {
+          int64_t cn[RB];
+          double v[RB][MQ];
 #pragma unroll
-          for (int q = 0; q < MQ; ++q) {
-            if ((cn[r] | co[q]) < 0) continue;
-            double* dst = C + cn[r] + co[q];
-            if (rmw) asm volatile("red.global.add.f64 [%0], %1;\n" ::"l"(dst), "d"(v[r][q]) : "memory");
-            else *dst = v[r][q];
+          for (int r = 0; r < RB; ++r) {
+            cn[r] = offc_n[wn0 + 16 * (nb >> 1) + 2 * (r0 + r) + (nb & 1)];
+#pragma unroll
+            for (int q = 0; q < MQ; ++q) v[r][q] = lane + 32 * q < WM ? cst[(r0 + r) * CPITCH + lane + 32 * q] : 0.0;
           }
+#pragma unroll
+          for (int r = 0; r < RB; ++r)
+#pragma unroll
+            for (int q = 0; q < MQ; ++q) {
+              if ((cn[r] | co[q]) < 0) continue;
+              double* dst = C + cn[r] + co[q];
+              if (rmw) asm volatile("red.global.add.f64 [%0], %1;\n" ::"l"(dst), "d"(v[r][q]) : "memory");
+              else *dst = v[r][q];
+            }
+        }
+        __syncwarp();
       }
-      __syncwarp();
     }
   } else if constexpr (CF::MATH == TC_MATH_TF32X3) {
     // ---------------- fp32 as three TF32 tensor-core products ----------------
@@ -883,46 +892,53 @@ __global__ void __launch_bounds__(CF::THREADS, CF::MIN_CTAS) tc_contract_kernel(
     // Any alignment: rows through shared memory, as the fp64 products leave (above), but added here -- reductions of fp32
     // would flush subnormal sums to zero.  A batch's old values are all on their way before its first sum is stored
     // (5 070 x 12 768 sum 25 267 -> 134 us, 27 x 47 x 31 x 47 sum 55 66 -> 27, 17 x 32 x 30 sum 18 16.2 -> 6.2).
+    // (The thread's index read anew, as there: 3 949 x 271 sum 1 715 196.8 -> 195.4 us, 1 122 x 1 712 sum 361 71.6 -> 70.4.)
     __syncthreads();
-    constexpr int CPITCH = WM + 4, MQ = (WM + 31) / 32, RB = 8 / MQ;
-    static_assert(CF::WARPS * 8 * CPITCH <= STAGES * CF::STAGE_ELEMS, "rows in the stages");
-    float* cst = Xs + warp * 8 * CPITCH;
-    int64_t co[MQ];
+    int tx;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tx));
+    {
+      const int lane = tx & 31, warp = tx >> 5, g = lane >> 2, t = lane & 3;
+      const int wm0 = (warp % CF::WARPS_M) * WM, wn0 = (warp / CF::WARPS_M) * WN;
+      constexpr int CPITCH = WM + 4, MQ = (WM + 31) / 32, RB = 8 / MQ;
+      static_assert(CF::WARPS * 8 * CPITCH <= STAGES * CF::STAGE_ELEMS, "rows in the stages");
+      float* cst = Xs + warp * 8 * CPITCH;
+      int64_t co[MQ];
 #pragma unroll
-    for (int q = 0; q < MQ; ++q) co[q] = lane + 32 * q < WM ? offc_m[wm0 + lane + 32 * q] : -1;
+      for (int q = 0; q < MQ; ++q) co[q] = lane + 32 * q < WM ? offc_m[wm0 + lane + 32 * q] : -1;
 #pragma unroll
-    for (int j = 0; j < NB; ++j)
+      for (int j = 0; j < NB; ++j)
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
+        for (int r = 0; r < 2; ++r) {
 #pragma unroll
-        for (int i = 0; i < MB2; ++i)
-          *reinterpret_cast<float4*>(cst + g * CPITCH + 16 * i + 4 * t) =
-              make_float4(alpha * acc[j][2 * i][2 * r], alpha * acc[j][2 * i + 1][2 * r], alpha * acc[j][2 * i][2 * r + 1],
-                          alpha * acc[j][2 * i + 1][2 * r + 1]);
-        __syncwarp();
+          for (int i = 0; i < MB2; ++i)
+            *reinterpret_cast<float4*>(cst + g * CPITCH + 16 * i + 4 * t) =
+                make_float4(alpha * acc[j][2 * i][2 * r], alpha * acc[j][2 * i + 1][2 * r], alpha * acc[j][2 * i][2 * r + 1],
+                            alpha * acc[j][2 * i + 1][2 * r + 1]);
+          __syncwarp();
 #pragma unroll
-        for (int r0 = 0; r0 < 8; r0 += RB) {
-          int64_t cn[RB];
-          float v[RB][MQ];
+          for (int r0 = 0; r0 < 8; r0 += RB) {
+            int64_t cn[RB];
+            float v[RB][MQ];
 #pragma unroll
-          for (int e = 0; e < RB; ++e) {
-            cn[e] = offc_n[wn0 + 16 * j + 8 * r + r0 + e];
+            for (int e = 0; e < RB; ++e) {
+              cn[e] = offc_n[wn0 + 16 * j + 8 * r + r0 + e];
 #pragma unroll
-            for (int q = 0; q < MQ; ++q) v[e][q] = rmw && (cn[e] | co[q]) >= 0 ? C[cn[e] + co[q]] : 0.f;
+              for (int q = 0; q < MQ; ++q) v[e][q] = rmw && (cn[e] | co[q]) >= 0 ? C[cn[e] + co[q]] : 0.f;
+            }
+#pragma unroll
+            for (int e = 0; e < RB; ++e)
+#pragma unroll
+              for (int q = 0; q < MQ; ++q)
+                if (lane + 32 * q < WM) v[e][q] += cst[(r0 + e) * CPITCH + lane + 32 * q];
+#pragma unroll
+            for (int e = 0; e < RB; ++e)
+#pragma unroll
+              for (int q = 0; q < MQ; ++q)
+                if ((cn[e] | co[q]) >= 0) C[cn[e] + co[q]] = v[e][q];
           }
-#pragma unroll
-          for (int e = 0; e < RB; ++e)
-#pragma unroll
-            for (int q = 0; q < MQ; ++q)
-              if (lane + 32 * q < WM) v[e][q] += cst[(r0 + e) * CPITCH + lane + 32 * q];
-#pragma unroll
-          for (int e = 0; e < RB; ++e)
-#pragma unroll
-            for (int q = 0; q < MQ; ++q)
-              if ((cn[e] | co[q]) >= 0) C[cn[e] + co[q]] = v[e][q];
+          __syncwarp();
         }
-        __syncwarp();
-      }
+    }
   } else if constexpr (CF::MATH == TC_MATH_TF32TC) {
     // ---------------- fp32 as three TF32 products on tcgen05, accumulators in tensor memory ----------------
     // D (tensor memory) has one lane per n (BN = 128) and one column per m (BM): D += Y * X^T.  Each K step the
