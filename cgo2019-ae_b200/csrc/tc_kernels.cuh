@@ -869,24 +869,32 @@ __global__ void __launch_bounds__(CF::THREADS, CF::MIN_CTAS) tc_contract_kernel(
         return;
       }
     }
+    // By 16 bytes: the old values of two rows are on their way before the first sum is stored (one after another a lane waited
+    // for each: 4 044 x 670 sum 94 36.4 -> 26.9 us, 700 x 1 100 sum 24 12.3 -> 8.2, 1 640 x 252 sum 30 7.3 -> 5.0).
     if (p.vec_c == 4) {
+      int64_t co[MB2];
 #pragma unroll
-      for (int j = 0; j < NB; ++j)
+      for (int i = 0; i < MB2; ++i) co[i] = offc_m[wm0 + 16 * i + 4 * t];
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        int64_t cn[2];
+        float4 c[2][MB2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const int64_t cn = offc_n[wn0 + 16 * j + g + 8 * r];
-          if (cn < 0) continue;
+          cn[r] = offc_n[wn0 + 16 * j + g + 8 * r];
+#pragma unroll
+          for (int i = 0; i < MB2; ++i) c[r][i] = rmw && (cn[r] | co[i]) >= 0 ? *reinterpret_cast<const float4*>(C + cn[r] + co[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
 #pragma unroll
           for (int i = 0; i < MB2; ++i) {
-            const int64_t co = offc_m[wm0 + 16 * i + 4 * t];
-            if (co < 0) continue;
-            float4* dst = reinterpret_cast<float4*>(C + cn + co);
-            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (rmw) c = *dst;
-            *dst = make_float4(fmaf(alpha, acc[j][2 * i][2 * r], c.x), fmaf(alpha, acc[j][2 * i + 1][2 * r], c.y),
-                               fmaf(alpha, acc[j][2 * i][2 * r + 1], c.z), fmaf(alpha, acc[j][2 * i + 1][2 * r + 1], c.w));
+            if ((cn[r] | co[i]) < 0) continue;
+            *reinterpret_cast<float4*>(C + cn[r] + co[i]) =
+                make_float4(fmaf(alpha, acc[j][2 * i][2 * r], c[r][i].x), fmaf(alpha, acc[j][2 * i + 1][2 * r], c[r][i].y),
+                            fmaf(alpha, acc[j][2 * i][2 * r + 1], c[r][i].z), fmaf(alpha, acc[j][2 * i + 1][2 * r + 1], c[r][i].w));
           }
-        }
+      }
       return;
     }
     // Any alignment: rows through shared memory, as the fp64 products leave (above), but added here -- reductions of fp32
