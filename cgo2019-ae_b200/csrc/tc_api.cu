@@ -732,7 +732,9 @@ class CopyPool {
 // Small buffers and all cores but a few: a copy over the link starts when its buffer is filled, so the first and the last
 // buffer are not overlapped with anything.  48^4 outputs and inputs (85 MB in, 42 MB out) on 16 cores: 9.0 ms with three
 // buffers of 8 MB and four helpers, 6.6 with twelve helpers, 4.9 with 2 MB and six, 4.0 with 2 MB and twelve.
-constexpr size_t kBounceBytes = size_t(2) << 20;
+// Calls that move more are bound by the host's memory and by the hand-over per piece, and take whole buffers (64^4, 268 MB
+// in: 10.5 ms in pieces of 2 MB, 9.5 in 4, 9.8 in 8; 96^4, 1.36 GB in: 51, 39, 47; with six or four helpers 42 to 52).
+constexpr size_t kBounceBytes = size_t(4) << 20, kShortPiece = size_t(2) << 20, kShortCall = size_t(192) << 20;
 constexpr int kBounceCount = 6;
 
 bool is_pageable(const void* ptr) {
@@ -759,6 +761,7 @@ struct TcHostPipe {
   // pageable staging
   void* bounce_in[kBounceCount] = {};
   void* bounce_out[kBounceCount] = {};
+  size_t piece = kBounceBytes;  // bytes of a buffer that the present call fills
   cudaEvent_t in_done[kBounceCount] = {};
   cudaEvent_t out_done[kBounceCount] = {};
   int in_next = 0;
@@ -911,8 +914,8 @@ static int copy_in(TcHostPipe* h, char* dst, const char* src, size_t bytes, bool
     TC_CUDA_OK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
     return TC_OK;
   }
-  for (size_t off = 0; off < bytes; off += kBounceBytes) {
-    const size_t n = std::min(kBounceBytes, bytes - off);
+  for (size_t off = 0; off < bytes; off += h->piece) {
+    const size_t n = std::min(h->piece, bytes - off);
     const int b = h->in_next;
     h->in_next = (b + 1) % kBounceCount;
     TC_CUDA_OK(cudaEventSynchronize(h->in_done[b]));  // the copy that last used this buffer has read it
@@ -944,7 +947,7 @@ struct Drain {
     size_t len[kBounceCount] = {};
     while (drained < j.bytes) {
       while (issued < j.bytes && bi - bd < kBounceCount - 1) {
-        const size_t n = std::min(kBounceBytes, j.bytes - issued);
+        const size_t n = std::min(h->piece, j.bytes - issued);
         const int b = bi % kBounceCount;
         TC_CUDA_OK(cudaMemcpyAsync(h->bounce_out[b], j.src + issued, n, cudaMemcpyDeviceToHost, h->out_stream));
         TC_CUDA_OK(cudaEventRecord(h->out_done[b], h->out_stream));
@@ -990,6 +993,7 @@ static int execute_host_locked(tc_plan* p, void* C, const void* A, const void* B
   if (page_c || page_a || page_b) {
     const int st = host_pipe_enable_staging(h);
     if (st != TC_OK) return st;
+    h->piece = (p->size_a + p->size_b + p->size_c) * es <= kShortCall ? kShortPiece : kBounceBytes;
   }
   const bool read_c = p->args.beta || p->size_c != p->count_c;
   cudaStream_t s0 = h->stream[0];
