@@ -726,9 +726,12 @@ int tc_plan_build(tc_plan* p, std::string* why) {
         !c.kvec_y && ((mf + 127) / 128) * ((nf + 127) / 128) >= 96) {
       // (up to 64 columns, of which it would compute 128, the small mma.sync tile: four sums, 1.2 to 1.3 times the 128-wide
       // one, level with or up to 14 % ahead of tcgen05)
-      if (nf > 64) c.math = TC_MATH_TF32TC;
-      bm = bn = nf > 64 ? 128 : 64;
-      unaligned = nf > 64;
+      // (up to 64 rows likewise, level with or up to 16 % ahead with 35 000 and 76 000 columns, five heights and three sums
+      // each; with 309 000 5 % ahead to 6 % behind: 57 x 35 061 sum 63 20.5 -> 18.5 us, 45 x 75 999 sum 33 37.0 -> 32.9)
+      const bool small = nf <= 64 || (mf <= 64 && nf <= 80000);
+      if (!small) c.math = TC_MATH_TF32TC;
+      bm = bn = small ? 64 : 128;
+      unaligned = !small;
     }
     if (c.math != TC_MATH_SIMT && pair_shape && path == TC_PATH_AUTO && p->opt.split_k == 0 &&
         pair_us < 0.8 * (c.math == TC_MATH_TF32TC ? single_us : sync_us)) {
