@@ -891,6 +891,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   }
   else if (persistent) ksplit = 1;
   else if (p->opt.split_k > 1) ksplit = std::min<int64_t>(p->opt.split_k, ksteps);
+  else if (c.pair) ksplit = 1;  // (the pairs cut their chains themselves, what stands in for them runs in passes: no scratch)
   else if (p->opt.split_k == 0 && tiles * 2 <= sms && ksteps >= 16)
   {
     ksplit = std::max<int64_t>(1, std::min<int64_t>((2 * sms) / tiles, ksteps / 8));

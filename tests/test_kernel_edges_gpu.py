@@ -281,3 +281,26 @@ def test_pairs_of_ctas(pkg, form, size, shift):
         assert plan.status() == 0
         assert float((got.double() - want).abs().max() / want.abs().max()) <= 1e-5
     plan.close()
+
+
+# The pairs run without scratch, whatever the number of tiles, and so does what stands in for them where one tensor is not
+# 16-byte aligned: the entry that allocates nothing takes both.
+@pytest.mark.parametrize("shift", [(0, 0, 0), (1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 1, 1)])
+@pytest.mark.parametrize("k", [512, 2000])
+def test_pairs_of_ctas_on_few_tiles_need_no_scratch(pkg, k, shift):
+    import torch
+    torch.cuda.set_device(0)
+    n = 900
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    c, a, b = (torch.rand(size + 4, device="cuda", generator=gen)[s:s + size] - 0.5 for size, s in zip((n * n, n * k, n * k), (0, 0, 0)))
+    place = lambda t, s: torch.cat([torch.zeros(s, device="cuda"), t])[s:]
+    c, a, b = (place(t, s) for t, s in zip((c, a, b), shift))
+    want = c.double() + (b.double().view(n, k) @ a.double().view(n, k).T).reshape(-1)
+    plan = pkg.Plan("C [a,%d,b,%d] += sum(c,%d) * A [c,a] * B [c,b];" % (n, n, k), pkg.F32).commit()
+    d = plan.describe()
+    assert d["pair"] and d["workspace_bytes"] == 0 and plan.workspace_bytes() == 0 and d["ksplit"] == 1, d
+    plan.execute_noalloc(c, a, b)
+    torch.cuda.synchronize()
+    assert plan.status() == 0
+    assert float((c.double() - want).abs().max() / want.abs().max()) <= 1e-5
+    plan.close()

@@ -488,3 +488,12 @@ def test_outputs_of_full_boxes_stay_on_the_resident_tile(pkg, expr):
 def test_the_choice_of_a_tile_brings_no_slices(pkg, expr):
     """Whether there are too few tiles to fill the GPU is the plain model's question: these sums need no scratch."""
     assert _plan(pkg, expr).describe()["workspace_bytes"] == 0
+
+
+def test_pairs_of_ctas_need_no_scratch(pkg):
+    # few tiles (64 of 128 x 128) and one or four chains: the pairs cut the chains themselves, what stands in for them where a
+    # tensor is not aligned runs in passes
+    for k, passes in ((512, 1), (2000, 4)):
+        d = _plan(pkg, "C [a,900,b,900] += sum(c,%d) * A [c,a] * B [c,b];" % k, "float32").describe()
+        assert d["pair"] and d["workspace_bytes"] == 0 and d["ksplit"] == 1 and d["launches"] == 1, d
+        assert d["passes"] == passes and d["chain"] <= 512, d
