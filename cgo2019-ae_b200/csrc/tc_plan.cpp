@@ -817,6 +817,7 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   a.ncut = {(uint32_t)bn, 1, (uint32_t)nf, 1, a.tiles_n, 1};
   a.rows_across_x = a.rows_across_y = 0;
   c.box_c = false;
+  a.panel = 0;
   bool plain_m = true, plain_n = true;  // tiles are plain ranges of the flattened index
   a.standin_vec_c = a.vec_c;
   if (tc_kernel_is_c_resident(c) && boxes_allowed) {
@@ -837,12 +838,29 @@ int tc_plan_build(tc_plan* p, std::string* why) {
       plain_n = plain(bp.n, nf, bn);
       a.tiles_m = (uint32_t)tm;
       a.tiles_n = (uint32_t)tn;
-      // Panels (tc_wp_kernel.cuh): X's tile is kept for a whole row of tiles.  That pays where fetching X again and again is
-      // what takes the time: X gathered across its sectors (K = 24 156 -> 129 us, K = 10 93 -> 71), or three K steps
-      // (K = 40 1 736 -> 1 633).  Shorter contractions whose X is read along its sectors are bound by C, which the ring
-      // kernel's order of tiles -- neighbours in M at the same time -- moves 2 to 16 % faster (K = 12 to 24, nine shapes);
-      // and a CTA has to have enough tiles to hide its first panel (three tiles 14.4 -> 17.2 us, six 26.6 either way).
-      a.panel = bm == 128 && bn == 64 && kf <= 3 * TC_BK && (kf > 2 * TC_BK || (a.lanes_k_x == 1 && !c.vec_x && a.M.s_in[0] != 1)) && tn >= 2 && tm * tn >= 8 * sms;
+      // Panels (tc_wp_kernel.cuh): X's tile is kept for a whole row of tiles, and a CTA has to have enough tiles to hide its
+      // first one (three tiles 14.4 -> 17.2 us, six 26.6 either way).  They save fetching X again and again and give up the
+      // ring kernel's order of tiles -- neighbours in M at the same time -- in which short runs of C share sectors and rows
+      // of memory.  Times as fast as the ring kernel, on 570 shapes of three to six indices, K = 8 to 48:
+      //   * tiles that cut M's first digit into short runs 0.50 to 1.3, 0.87 in the mean (22 x 16 x 19 x 16 x 24 x 16, K = 38,
+      //     199 -> 387 us);
+      //   * X gathered across its sectors, from K = 17 on 0.97 to 1.7, mean 1.24 (24 x 16 x 16 x 24 x 16 x 16, K = 24, 156 ->
+      //     129 us) but for the shortest runs (80 bytes 0.92 to 1.1); where C is only written 0.97 to 1.7 with any K; below
+      //     K = 16 C's traffic is the longer side, 0.80 to 1.08 where Y loads by vector (K = 12 54 -> 64 us), 0.99 to 1.2 else;
+      //   * else, three K steps: 0.91 to 0.99 where X comes in tiled boxes, which it is cheap to fetch again; 0.96 to 1.4, mean
+      //     1.12, otherwise, but for runs that are not whole sectors (0.77 to 1.25);
+      //   * runs of 64 and more, three K steps: 0.98 to 1.29 with a panel for every CTA (40^6 slab, K = 40, 1 736 -> 1 633 us),
+      //     where C's slower indices belong to M too, or X is gathered; else 0.81 to 1.02.
+      // A caller that names tile and variant gets panels wherever X takes three K steps or is gathered.
+      const bool across = a.lanes_k_x == 1 && !c.vec_x && a.M.s_in[0] != 1, whole = bp.m.b0 == bp.m.e0, sectors = bp.m.b0 % 4 == 0;
+      const bool three = kf > 2 * TC_BK;
+      bool pays = false;
+      if (p->opt.variant > 0 && p->opt.tile_m > 0) pays = three || across;
+      else if (bp.m.b0 >= 64 && (!whole || bp.m.b0 == (uint32_t)bm)) pays = three && tn >= 8 && (tm >= sms || (int64_t)bp.m.e0 < mf || !c.tma_x);
+      else if (whole && !across) pays = three && sectors && !c.tma_x;
+      else if (whole && (e.op == 0 || three)) pays = true;
+      else if (whole) pays = kf >= TC_BK ? bp.m.b0 >= 14 || (sectors && kf > TC_BK) : sectors && !c.vec_y && !c.kvec_y;
+      a.panel = bm == 128 && bn == 64 && kf <= 3 * TC_BK && pays && tn >= 2 && tm * tn >= 8 * sms;
       // a tiled TMA box of an operand takes consecutive values of the flattened index
       if (bp.m.b1 > 1 && bp.m.b0 != bp.m.e0) c.tma_x = false;
       if (bp.n.b1 > 1 && bp.n.b0 != bp.n.e0) c.tma_y = false;

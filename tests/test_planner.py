@@ -497,3 +497,24 @@ def test_pairs_of_ctas_need_no_scratch(pkg):
         d = _plan(pkg, "C [a,900,b,900] += sum(c,%d) * A [c,a] * B [c,b];" % k, "float32").describe()
         assert d["pair"] and d["workspace_bytes"] == 0 and d["ksplit"] == 1 and d["launches"] == 1, d
         assert d["passes"] == passes and d["chain"] <= 512, d
+
+
+# Panels: where they measured slower than the ring kernel it runs, and where faster, they do (K = 8 to 48).
+@pytest.mark.parametrize("extents,k,left,right,op,panel", [
+    ((22, 16, 19, 16, 24, 16), 38, "e,f,g,b", "g,d,a,c", "+=", False),   # the tiles cut M's first digit: 199 against 387 us
+    ((26, 20, 18, 22, 20, 16), 40, "d,e,g,a", "g,f,b,c", "=", False),    # ... X gathered, C only written: 264, 447
+    ((24, 16, 16, 24, 16, 16), 40, "d,f,g,b", "g,e,a,c", "+=", False),   # ... 187, 207
+    ((16, 17, 16, 24, 17, 15), 38, "e,f,g,b", "g,d,a,c", "=", True),     # whole digit, whole sectors: 114, 99
+    ((24, 16, 16, 24, 16, 16), 24, "d,e,g,a", "g,f,b,c", "-=", True),    # X gathered: 156, 129
+    ((16, 22, 11, 17, 24, 26), 10, "d,e,g,a", "g,f,b,c", "+=", False),   # ... short contraction: 110, 124
+    ((16, 16, 24, 24, 16, 11), 10, "d,e,g,a", "g,f,b,c", "=", True),     # ... C only written
+    ((10, 16, 20, 21, 14, 16), 20, "e,f,g,a", "g,d,b,c", "+=", False),   # ... runs of 80 bytes: 57, 59
+    ((24, 24, 10, 26, 16, 22), 38, "g,a,d,e", "b,c,g,f", "=", False),    # X in tiled boxes: 193, 201
+    ((25, 19, 30, 31, 32, 18), 36, "g,a,b,c", "d,e,f,g", "+=", False),   # fewer panels than CTAs: 759, 937
+    ((40, 40, 40, 40, 40, 5), 40, "g,a,b,c", "d,e,f,g", "+=", True),     # a slab of the 40^6 output: 1 736, 1 633
+])
+def test_panels_where_they_pay(pkg, extents, k, left, right, op, panel):
+    out = ",".join("%s,%d" % x for x in zip("abcdef", extents))
+    expr = "C [%s] %s sum(g,%d) * A [%s] * B [%s];" % (out, op, k, left, right)
+    d = _plan(pkg, expr).describe()
+    assert d["kernel"] == "dmma_wc_128x64" and d["panel"] == panel and d["tiles"][0] * d["tiles"][1] >= 8 * 148, d
