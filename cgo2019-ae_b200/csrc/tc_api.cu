@@ -295,9 +295,13 @@ int tc_launch_contraction(const tc_plan& p, const TcKernelArgs& args, void* C, c
     a.tiles_n = (a.Nflat + 255) / 256;
     a.mblock_w = a.tiles_m > 32 && a.tiles_n > 1 ? 16 : 0;
     if (!fn) return TC_ERR_UNSUPPORTED;
+    __atomic_store_n(&p.ran, (int)TC_ROUTE_PAIRS, __ATOMIC_RELAXED);
     return fn(vx, vy, &a, C, X, Y, stream, TC_INST_LAUNCH, nullptr, nullptr);
   }
+  // (a plan for the pairs that runs without them: on the single CTAs' kernel of its variant)
+  TcRoute route = c.pair ? TC_ROUTE_KERNEL : tc_plan_route(p);
   if (tc_kernel_is_c_resident(c) && !resident) {
+    route = TC_ROUTE_STANDIN;
     a.vec_c = std::min(a.vec_c, a.standin_vec_c);
     TcKernelChoice alt = c;
     alt.variant = 2;
@@ -306,6 +310,7 @@ int tc_launch_contraction(const tc_plan& p, const TcKernelArgs& args, void* C, c
   if (tc_kernel_is_tmem_persistent(c) && ((cu & 15) != 0 || p.opt.c_path == 2)) {
     // The persistent tcgen05 kernel moves its output tiles as bulk copies of 16-byte aligned chunks; an output
     // without that alignment (or accumulators that are to start from the output) runs the same tiles one CTA per tile.
+    route = TC_ROUTE_STANDIN;
     TcKernelChoice alt = c;
     alt.variant = 0;
     fn = pick_inst(alt);
@@ -335,6 +340,7 @@ int tc_launch_contraction(const tc_plan& p, const TcKernelArgs& args, void* C, c
     a.ring_stages = stages;
   }
   if (!fn) return TC_ERR_UNSUPPORTED;
+  __atomic_store_n(&p.ran, (int)route, __ATOMIC_RELAXED);
   // Plans whose contraction runs as sequential passes (fp32 tensor-core chains kept short on outputs too large
   // for slice scratch): one launch per range of k, the first with the expression's operator, the rest adding.
   for (int pass = 0; pass < passes; ++pass) {

@@ -159,6 +159,10 @@ struct TcKernelChoice {
   bool pair;            // fp32: 256 x 256 tiles on pairs of CTAs (tc_wd_kernel.cuh) wherever the tensors are 16-byte aligned
 };
 
+// What a launch of a plan runs: the plan's kernel, that kernel's form on pairs of CTAs or on panels, or what stands in for
+// it where a tensor is not aligned or the copy engine cannot address the output.
+enum TcRoute { TC_ROUTE_KERNEL = 0, TC_ROUTE_PAIRS = 1, TC_ROUTE_PANELS = 2, TC_ROUTE_STANDIN = 3 };
+
 struct TcHostPipe;
 
 // Host-side plan.
@@ -195,7 +199,8 @@ struct tc_plan {
   int64_t count_c = 0, count_a = 0, count_b = 0;  // logical element counts
   double flops = 0, bytes = 0;
   double estimate_s = 0;  // the planner's own estimate of one execute (persistent fp64 kernels; 0: none made)
-  int launches = 1;
+  int launches = 1;      // of one execute on 16-byte aligned tensors
+  mutable int ran = -1;  // which of the plan's kernels (TcRoute) the last launch took, -1: none yet; any thread's launch writes it
   std::string why;  // last planner message
 };
 
@@ -222,6 +227,12 @@ inline bool tc_kernel_is_persistent(const TcKernelChoice& c) {
 }
 // ... and keeps its output tile resident in shared memory (tc_wc_kernel.cuh)
 inline bool tc_kernel_is_c_resident(const TcKernelChoice& c) { return c.math == TC_MATH_DMMA && c.variant == 3; }
+// The route of a plan's launches on aligned tensors.
+inline TcRoute tc_plan_route(const tc_plan& p) {
+  if (p.choice.pair) return TC_ROUTE_PAIRS;
+  if (tc_kernel_is_c_resident(p.choice)) return !p.choice.box_c ? TC_ROUTE_STANDIN : p.args.panel ? TC_ROUTE_PANELS : TC_ROUTE_KERNEL;
+  return tc_kernel_is_tmem_persistent(p.choice) && p.opt.c_path == 2 ? TC_ROUTE_STANDIN : TC_ROUTE_KERNEL;
+}
 constexpr int TC_BK = 16;  // contraction step of every kernel
 
 #endif  // TC_INTERNAL_H_

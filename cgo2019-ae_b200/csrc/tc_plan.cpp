@@ -583,7 +583,9 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   c.pair = false;
   bool unaligned = false;  // fp32 without any alignment on the one-tile tcgen05 kernel
   const bool boxes_pay = (uint64_t)kf * 5 >= (uint64_t)((kf + TC_BK - 1) / TC_BK * TC_BK) * 4;
-  const bool pair_shape = p->dtype == TC_F32 && p->opt.tma != 1 && p->opt.tma != 3 && p->opt.c_path == 0 && boxes_pay && kf >= 16 * TC_BK &&
+  // (a caller that names a tile or a variant gets that kernel)
+  const bool named = p->opt.tile_m > 0 || p->opt.tile_n > 0 || p->opt.variant > 0;
+  const bool pair_shape = p->dtype == TC_F32 && !named && p->opt.tma != 1 && p->opt.tma != 3 && p->opt.c_path == 0 && boxes_pay && kf >= 16 * TC_BK &&
                           (c.tma_x || c.tma_xe) && (c.tma_y || c.tma_ye) && a.vec_c == 4 && (a.M.n == 1 || a.M.extent[0] % 32 == 0);
   auto rounds_of = [](int64_t tiles, int64_t at_once) { return (double)((tiles + at_once - 1) / at_once); };
   const int64_t pairs = std::max<int64_t>(1, sms / 2), pair_tiles = ((mf + 255) / 256) * ((nf + 255) / 256), pair_left = pair_tiles % pairs;
@@ -991,6 +993,15 @@ int tc_plan_build(tc_plan* p, std::string* why) {
   return TC_OK;
 }
 
+// "kernel" in the plan record is the kernel that the plan was made for; this is the one that a route takes.
+static std::string route_name(const tc_plan& p, int route) {
+  TcKernelChoice c = p.choice;
+  if (route == TC_ROUTE_PAIRS) return "tf32wd_256x256";
+  if (route == TC_ROUTE_PANELS) return "dmma_wp_128x64";
+  if (route == TC_ROUTE_STANDIN) c.variant = tc_kernel_is_c_resident(c) ? 2 : 0;
+  return tc_kernel_name(c);
+}
+
 std::string tc_plan_to_json(const tc_plan& p) {
   std::ostringstream o;
   o.precision(17);
@@ -1010,6 +1021,7 @@ std::string tc_plan_to_json(const tc_plan& p) {
     chain = std::min<uint32_t>(a.Kflat, ((steps + segs - 1) / segs) * TC_BK);
   }
   if (p.committed) {
+    const int ran = __atomic_load_n(&p.ran, __ATOMIC_RELAXED);
     o << ",\"swapped\":" << (p.swapped ? "true" : "false") << ",\"M\":";
     dims(a.M);
     o << ",\"N\":";
@@ -1019,13 +1031,13 @@ std::string tc_plan_to_json(const tc_plan& p) {
     o << ",\"Mflat\":" << a.Mflat << ",\"Nflat\":" << a.Nflat << ",\"Kflat\":" << a.Kflat
       << ",\"math\":\"" << (p.choice.math == TC_MATH_DMMA ? "dmma" : p.choice.math == TC_MATH_TF32X3 ? "tf32x3" : p.choice.math == TC_MATH_TF32TC ? "tf32x3_tcgen05" : (p.dtype == TC_F64 ? "dfma" : "ffma"))
       << "\",\"kernel\":\"" << tc_kernel_name(p.choice) << "\",\"tile\":[" << p.choice.bm << "," << p.choice.bn << "," << TC_BK
-      << "],\"variant\":" << p.choice.variant << ",\"tiles\":[" << a.tiles_m << "," << a.tiles_n << "],\"estimate_us\":" << p.estimate_s * 1e6 << ",\"mblock_w\":" << a.mblock_w << ",\"ksplit\":" << a.ksplit
+      << "],\"runs\":\"" << route_name(p, tc_plan_route(p)) << "\",\"runs_tile\":[" << (p.choice.pair ? 256 : p.choice.bm) << "," << (p.choice.pair ? 256 : p.choice.bn)
+      << "],\"ran\":" << (ran < 0 ? "null" : "\"" + route_name(p, ran) + "\"") << ",\"variant\":" << p.choice.variant << ",\"tiles\":[" << a.tiles_m << "," << a.tiles_n << "],\"estimate_us\":" << p.estimate_s * 1e6 << ",\"mblock_w\":" << a.mblock_w << ",\"ksplit\":" << a.ksplit
       << ",\"k_chunk\":" << a.k_chunk << ",\"k_seg\":" << a.k_seg << ",\"passes\":" << p.passes << ",\"chain\":" << chain << ",\"vec_x\":" << (p.choice.vec_x ? "true" : "false")
       << ",\"vec_y\":" << (p.choice.vec_y ? "true" : "false") << ",\"kvec_x\":" << (p.choice.kvec_x ? "true" : "false")
       << ",\"kvec_y\":" << (p.choice.kvec_y ? "true" : "false") << ",\"tma_x\":" << (p.choice.tma_x ? "true" : "false")
       << ",\"tma_y\":" << (p.choice.tma_y ? "true" : "false") << ",\"tma_xe\":" << (p.choice.tma_xe ? "true" : "false")
       << ",\"tma_ye\":" << (p.choice.tma_ye ? "true" : "false") << ",\"tma_c\":" << (p.choice.tma_c ? "true" : "false") << ",\"tma_ct\":" << (p.choice.tma_ct ? "true" : "false")
-
       << ",\"pair\":" << (p.choice.pair ? "true" : "false") << ",\"lanes_k_x\":" << a.lanes_k_x
       << ",\"lanes_k_y\":" << a.lanes_k_y << ",\"vec_c\":" << a.vec_c << ",\"standin_vec_c\":" << a.standin_vec_c << ",\"epi_run\":" << a.epi_run << ",\"epi_n_span\":" << a.epi_n_span << ",\"beta\":" << a.beta
       << ",\"alpha\":" << a.alpha << ",\"workspace_bytes\":" << p.ws_bytes << ",\"launches\":" << p.launches

@@ -116,7 +116,9 @@ int tc_plan_commit(tc_plan* plan);
 void tc_plan_destroy(tc_plan* plan);
 
 /* JSON: index classes, fused dimensions, tile shape, kernel variant, grid,
- * algorithmic flops and bytes. */
+ * algorithmic flops and bytes.  "kernel" and "tile" are what the plan was made
+ * for; "runs" and "runs_tile" name the form of it that a launch on aligned
+ * tensors takes (pairs of CTAs, panels), "ran" the kernel of the last launch. */
 int tc_plan_describe(const tc_plan* plan, char* buf, size_t cap);
 /* 2 * prod(all extents), and elemsize * (2|C| + |A| + |B|)  ('=' reads C zero times: |C|). */
 int tc_plan_cost(const tc_plan* plan, double* flops, double* bytes);

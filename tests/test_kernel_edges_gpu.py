@@ -304,3 +304,95 @@ def test_pairs_of_ctas_on_few_tiles_need_no_scratch(pkg, k, shift):
     assert plan.status() == 0
     assert float((c.double() - want).abs().max() / want.abs().max()) <= 1e-5
     plan.close()
+
+
+def _matrices(m, n, k, shift=(0, 0, 0), seed=11):
+    """C [b,a], A [a,c], B [b,c] as flat fp32 tensors, each `shift` elements past an aligned address, and C + A * B in 64 bits."""
+    import torch
+    torch.cuda.set_device(0)
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    place = lambda size, s: torch.cat([torch.zeros(s, device="cuda"), torch.rand(size, device="cuda", generator=gen) - 0.5])[s:]
+    c, a, b = (place(size, s) for size, s in zip((m * n, m * k, n * k), shift))
+    return c, a, b, c.double() + (b.double().view(n, k) @ a.double().view(m, k).T).reshape(-1)
+
+
+def _off(got, want):
+    return float((got.double() - want).abs().max() / want.abs().max())
+
+
+# Which kernel a plan for pairs takes where one tensor is not 16-byte aligned: without the output the one-tile kernel in
+# passes, without an operand the single CTAs' kernel with that operand fetched element by element.
+@pytest.mark.parametrize("shift,ran", [((0, 0, 0), "tf32wd_256x256"), ((1, 0, 0), "tf32tc_128x128"), ((0, 1, 0), "tf32wt_128x128"),
+                                       ((0, 0, 1), "tf32wt_128x128"), ((1, 1, 1), "tf32tc_128x128")])
+def test_pairs_of_ctas_and_what_stands_in_for_them(pkg, shift, ran):
+    import torch
+    c, a, b, want = _matrices(1024, 768, 1028, shift)
+    plan = pkg.Plan("C [a,1024,b,768] += sum(c,1028) * A [c,a] * B [c,b];", pkg.F32)
+    plan.execute(c, a, b)
+    torch.cuda.synchronize()
+    assert plan.status() == 0 and plan.describe()["ran"] == ran and _off(c, want) <= 1e-5, (plan.describe(), _off(c, want))
+    plan.close()
+
+
+# The single CTAs' kernel by name, at the lengths at which the planner now takes pairs.
+@pytest.mark.parametrize("k", [160, 264, 520, 1032])
+def test_split_groups_of_the_named_single_cta_kernel(pkg, k):
+    import torch
+    c, a, b, want = _matrices(3072, 2048, k)
+    plan = pkg.Plan("C [a,3072,b,2048] += sum(c,%d) * A [c,a] * B [c,b];" % k, pkg.F32, path=pkg.PATH_TCGEN05, tile=(128, 128), variant=2)
+    for _ in range(3):
+        got = c.clone()
+        plan.execute(got, a, b)
+        torch.cuda.synchronize()
+        assert plan.status() == 0 and plan.describe()["ran"] == "tf32wt_128x128" and _off(got, want) <= 1e-5
+    plan.close()
+
+
+# The pairs' kernel, repeatedly: several segments per tile, every stage and slot used again, each pass checked.
+@pytest.mark.parametrize("m,n,k", [(1024, 768, 1028), (1024, 768, 2112), (5120, 4096, 520)])
+def test_pairs_of_ctas_repeatedly(pkg, m, n, k):
+    import torch
+    c, a, b, want = _matrices(m, n, k)
+    plan = pkg.Plan("C [a,%d,b,%d] += sum(c,%d) * A [c,a] * B [c,b];" % (m, n, k), pkg.F32)
+    for _ in range(20):
+        got = c.clone()
+        plan.execute(got, a, b)
+        torch.cuda.synchronize()
+        assert plan.status() == 0 and _off(got, want) <= 1e-5
+    assert plan.describe()["ran"] == "tf32wd_256x256"
+    plan.close()
+
+
+def test_pairs_of_ctas_on_blocks_of_larger_matrices(pkg):
+    import torch
+    m, n, k = 1024, 768, 260
+    c, a, b, _ = _matrices(m, 896, 300, seed=12)             # B as [c,b]: b in [64, 832), c in [32, 292)
+    b = b.view(300, 896)
+    plan = pkg.Plan("C [a,%d,b,%d] += sum(c,%d) * A [c,a] * B [b,c];" % (m, n, k), pkg.F32)
+    plan.set_strides(pkg.TENSOR_LEFT, [1, 300]).set_strides(pkg.TENSOR_RIGHT, [1, 896])
+    want = c.double().view(896, m).clone()
+    want[64:832] += b.double()[32:292, 64:832].T @ a.double().view(m, 300)[:, 32:292].T
+    got = c.clone()
+    plan.execute(got[64 * m:], a[32:], b.reshape(-1)[32 * 896 + 64:])
+    torch.cuda.synchronize()
+    got = got.view(896, m)
+    assert plan.status() == 0 and plan.describe()["ran"] == "tf32wd_256x256" and _off(got, want) <= 1e-5
+    assert torch.equal(got[:64], c.view(896, m)[:64]) and torch.equal(got[832:], c.view(896, m)[832:])
+    plan.close()
+
+
+def test_a_wait_of_the_pairs_that_gives_up(pkg):
+    import torch
+    expr = "C [a,1024,b,768] += sum(c,300) * A [c,a] * B [c,b];"
+    c, a, b, want = _matrices(1024, 768, 300)
+    bad = pkg.Plan(expr, pkg.F32, test_fault=1)
+    bad.execute(c.clone(), a, b)
+    torch.cuda.synchronize()
+    assert bad.status() in range(10, 18) and bad.describe()["ran"] == "tf32wd_256x256"
+    bad.close()
+    for _ in range(2):  # tensor memory was released
+        good, got = pkg.Plan(expr, pkg.F32), c.clone()
+        good.execute(got, a, b)
+        torch.cuda.synchronize()
+        assert good.status() == 0 and _off(got, want) <= 1e-5
+        good.close()

@@ -518,3 +518,20 @@ def test_panels_where_they_pay(pkg, extents, k, left, right, op, panel):
     expr = "C [%s] %s sum(g,%d) * A [%s] * B [%s];" % (out, op, k, left, right)
     d = _plan(pkg, expr).describe()
     assert d["kernel"] == "dmma_wc_128x64" and d["panel"] == panel and d["tiles"][0] * d["tiles"][1] >= 8 * 148, d
+
+
+def test_a_named_kernel_is_the_one_that_runs(pkg):
+    expr = "C [a,384,b,256] = sum(c,1028) * A [c,a] * B [c,b];"
+    for kw in (dict(path=pkg.PATH_TCGEN05, tile=(128, 128), variant=2), dict(tile=(128, 128), variant=1), dict(path=pkg.PATH_TCGEN05, tile=(96, 128), variant=2)):
+        d = _plan(pkg, expr, "float32", **kw).describe()
+        assert not d["pair"] and d["runs"] == d["kernel"] and d["runs_tile"] == d["tile"][:2] == list(kw["tile"]) and d["ran"] is None, d
+    # left to the planner: what runs is named beside what the plan was made for
+    d = _plan(pkg, "C [a,1024,b,768] = sum(c,1028) * A [c,a] * B [c,b];", "float32").describe()
+    assert d["pair"] and d["kernel"] == "tf32wt_128x128" and d["runs"] == "tf32wd_256x256" and d["runs_tile"] == [256, 256], d
+    d = _plan(pkg, "C [a,4096,b,4096] = sum(c,1028) * A [c,a] * B [c,b];", "float32", variant=2).describe()
+    assert not d["pair"] and d["runs"] == d["kernel"], d
+    six = "C [a,24,b,16,c,16,d,24,e,16,f,16] -= sum(g,24) * A [d,e,g,a] * B [g,f,b,c];"
+    d = _plan(pkg, six).describe()
+    assert d["panel"] and d["runs"] == "dmma_wp_128x64", d
+    d = _plan(pkg, six, tile=(128, 64), variant=4, tma=1).describe()   # no boxes of the output: the reduce-add kernel
+    assert d["runs"] == "dmma_ws_128x64" and d["kernel"] == "dmma_wc_128x64", d
