@@ -98,60 +98,6 @@ __device__ __forceinline__ void tile_box_coords(const TcKernelArgs& p, uint32_t 
   }
 }
 
-// A consumer thread's products into the tile buffer `tb`: buffer (+)= alpha * acc.  `dense`: the tile is BM consecutive
-// rows by all of its columns; else its rows lie where `mo` says (see the kernel).
-template <int BM, int MB2, int NB2>
-__device__ __forceinline__ void resident_add(double* tb, const double (&acc)[2 * NB2][2 * MB2][2], double alpha, bool accumulate, bool dense, int wm0,
-                                             int wn0, int g, int t, int b0, int tile_n, const int (&mo)[MB2][2]) {
-  const int h0 = g & 1;  // which 16-byte half of its 32 bytes a thread visits first (see the header)
-  // (tiles that are plain ranges keep addresses the compiler knows: the general form cost 2.5 % on the 40^6 slab)
-  if (dense) {
-#pragma unroll
-    for (int nb = 0; nb < 2 * NB2; ++nb) {
-      double* row = tb + (wn0 + 16 * (nb >> 1) + 2 * g + (nb & 1)) * BM + wm0 + 4 * t;
-#pragma unroll
-      for (int i = 0; i < MB2; ++i) {
-        double2* q = reinterpret_cast<double2*>(row + 16 * i);
-        // the thread's four consecutive outputs: lo = (m, m+1), hi = (m+2, m+3)
-        const double2 lo = make_double2(alpha * acc[nb][2 * i][0], alpha * acc[nb][2 * i + 1][0]);
-        const double2 hi = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
-        double2 first_v = h0 ? hi : lo, second_v = h0 ? lo : hi;
-        if (accumulate) {
-          const double2 c0 = q[h0], c1 = q[h0 ^ 1];
-          first_v.x += c0.x; first_v.y += c0.y;
-          second_v.x += c1.x; second_v.y += c1.y;
-        }
-        q[h0] = first_v;
-        q[h0 ^ 1] = second_v;
-      }
-    }
-  } else {
-#pragma unroll
-    for (int nb = 0; nb < 2 * NB2; ++nb) {
-      const int n = wn0 + 16 * (nb >> 1) + 2 * g + (nb & 1);
-      if (n >= tile_n) continue;
-      double* row = tb + n * b0;
-#pragma unroll
-      for (int i = 0; i < MB2; ++i) {
-        // the thread's four outputs: lo = (m, m+1), hi = (m+2, m+3), each pair in one run
-        const double2 lo = make_double2(alpha * acc[nb][2 * i][0], alpha * acc[nb][2 * i + 1][0]);
-        const double2 hi = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
-        const int q0 = h0 ? mo[i][1] : mo[i][0], q1 = h0 ? mo[i][0] : mo[i][1];
-        double2 first_v = h0 ? hi : lo, second_v = h0 ? lo : hi;
-        double2* f = reinterpret_cast<double2*>(row + q0);
-        double2* l = reinterpret_cast<double2*>(row + q1);
-        if (accumulate) {
-          const double2 c0 = q0 >= 0 ? *f : make_double2(0.0, 0.0), c1 = q1 >= 0 ? *l : make_double2(0.0, 0.0);
-          first_v.x += c0.x; first_v.y += c0.y;
-          second_v.x += c1.x; second_v.y += c1.y;
-        }
-        if (q0 >= 0) *f = first_v;
-        if (q1 >= 0) *l = second_v;
-      }
-    }
-  }
-}
-
 template <class CF>
 __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __grid_constant__ TcKernelArgs p,
                                                                          double* __restrict__ C,
@@ -298,6 +244,7 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
   const int g = lane >> 2, t = lane & 3;
   const int wm0 = (cw % CF::WGM) * WM, wn0 = (cw / CF::WGM) * WN;
   const double alpha = p.alpha;
+  const int h0 = g & 1;  // which 16-byte half of its 32 bytes a thread visits first (see the header)
   // Where this thread's pairs of rows lie in a tile buffer, whose order is (first digit of M, the tile's n, second digit
   // of M): runs of b0 (even) outputs, n at a pitch of b0, the second digit at b0 * tile_n.  -1: beyond the tile.
   const int b0 = (int)p.mcut.b0, tile_n = (int)(p.ncut.b0 * p.ncut.b1), tile_m = (int)(p.mcut.b0 * p.mcut.b1);
@@ -353,7 +300,55 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
     // ---- epilogue: buffer (+)= alpha * acc in shared memory; the C thread stores the buffer ----
     const uint32_t b = titer & 1u;
     if (!mbar_wait(&c_ready[b], (titer >> 1) & 1u, p.status, 4, p.spin_limit)) return;
-    resident_add<BM, MB2, NB2>(cbufs + b * CF::CTILE_ELEMS, acc, alpha, accumulate, dense, wm0, wn0, g, t, b0, tile_n, mo);
+    double* tb = cbufs + b * CF::CTILE_ELEMS;
+    // (the text of resident_add in tc_wp_kernel.cuh, in place: as a function called here it spilled where X loads along k and
+    // Y by element, and those plans took 3 to 9 % longer: 14 x 19 x 16 x 19 x 21 x 16, K = 40, 129 -> 141 us)
+    // (tiles that are plain ranges keep addresses the compiler knows: the general form cost 2.5 % on the 40^6 slab)
+    if (dense) {
+#pragma unroll
+      for (int nb = 0; nb < 2 * NB2; ++nb) {
+        double* row = tb + (wn0 + 16 * (nb >> 1) + 2 * g + (nb & 1)) * BM + wm0 + 4 * t;
+#pragma unroll
+        for (int i = 0; i < MB2; ++i) {
+          double2* q = reinterpret_cast<double2*>(row + 16 * i);
+          // the thread's four consecutive outputs: lo = (m, m+1), hi = (m+2, m+3)
+          const double2 lo = make_double2(alpha * acc[nb][2 * i][0], alpha * acc[nb][2 * i + 1][0]);
+          const double2 hi = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
+          double2 first_v = h0 ? hi : lo, second_v = h0 ? lo : hi;
+          if (accumulate) {
+            const double2 c0 = q[h0], c1 = q[h0 ^ 1];
+            first_v.x += c0.x; first_v.y += c0.y;
+            second_v.x += c1.x; second_v.y += c1.y;
+          }
+          q[h0] = first_v;
+          q[h0 ^ 1] = second_v;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int nb = 0; nb < 2 * NB2; ++nb) {
+        const int n = wn0 + 16 * (nb >> 1) + 2 * g + (nb & 1);
+        if (n >= tile_n) continue;
+        double* row = tb + n * b0;
+#pragma unroll
+        for (int i = 0; i < MB2; ++i) {
+          // the thread's four outputs: lo = (m, m+1), hi = (m+2, m+3), each pair in one run
+          const double2 lo = make_double2(alpha * acc[nb][2 * i][0], alpha * acc[nb][2 * i + 1][0]);
+          const double2 hi = make_double2(alpha * acc[nb][2 * i][1], alpha * acc[nb][2 * i + 1][1]);
+          const int q0 = h0 ? mo[i][1] : mo[i][0], q1 = h0 ? mo[i][0] : mo[i][1];
+          double2 first_v = h0 ? hi : lo, second_v = h0 ? lo : hi;
+          double2* f = reinterpret_cast<double2*>(row + q0);
+          double2* l = reinterpret_cast<double2*>(row + q1);
+          if (accumulate) {
+            const double2 c0 = q0 >= 0 ? *f : make_double2(0.0, 0.0), c1 = q1 >= 0 ? *l : make_double2(0.0, 0.0);
+            first_v.x += c0.x; first_v.y += c0.y;
+            second_v.x += c1.x; second_v.y += c1.y;
+          }
+          if (q0 >= 0) *f = first_v;
+          if (q1 >= 0) *l = second_v;
+        }
+      }
+    }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncwarp();
     if (lane == 0) mbar_arrive(&c_staged[b]);  // release: this warp's part of the tile is in the buffer
