@@ -22,7 +22,8 @@
 // copy bandwidth); one GPU's eighth of the 40^6 output, K = 40: 1 799 -> 1 733 us under the board's
 // power cap, 1 736 -> 1 633 in bursts that stay below it (floor 1 255).
 //
-// Every mbarrier wait is bounded (args.spin_limit) and reports through args.status.
+// Every mbarrier wait is bounded (args.spin_limit) and reports through args.status; a role that gives up leaves when what it
+// has under way has landed.
 #pragma once
 #include "tc_wc_kernel.cuh"
 
@@ -235,7 +236,11 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wp_dmma_kernel(const __
         for (int ks = 0; ks < nk; ++ks, ++it) {
           const int64_t ny = ws_koff(p.koff_y, (uint32_t)(ks + 1) * BK, kend, lane);
           // (one decision per warp: the loaders below shuffle)
-          if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], (use & 1u) ^ 1u, p.status, 2, p.spin_limit))) return;
+          if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], (use & 1u) ^ 1u, p.status, 2, p.spin_limit))) {
+            copies_landed();
+            if (CF::MODEY == LM_TMA_K && ptid == 0) fills_landed(full, it, S, p.status, p.spin_limit);
+            return;
+          }
           double* ys = ring + s * CF::YIMG;
           // tests only: one thread of CTA 0 never announces its copies of one stage
           const bool skip = p.test_fault == 1 && blockIdx.x == 0 && gi == 0 && it == 1;
@@ -280,7 +285,10 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wp_dmma_kernel(const __
         int next[5] = {0, 0, 0, 0, 0};  // (its divisions are done while the consumers work)
         more = w.next();
         if (more) tile_box_coords(p, w.tm, w.tn, next);
-        if (!mbar_wait(c_staged, j & 1u, p.status, 6, p.spin_limit)) return;
+        if (!mbar_wait(c_staged, j & 1u, p.status, 6, p.spin_limit)) {  // the tile on its way into the buffer lands first
+          mbar_wait(c_ready, j & 1u, p.status, 6, p.spin_limit);
+          break;
+        }
         asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4, %5}], [%6];\n" ::"l"(tmap), "r"(c[0]),
                      "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(buf)
                      : "memory");
@@ -313,7 +321,11 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wp_dmma_kernel(const __
       int64_t kx = ws_koff(p.koff_x, 0, kend, lane);
       for (int ks = 0; ks < nk; ++ks) {
         const int64_t nx = ws_koff(p.koff_x, (uint32_t)(ks + 1) * BK, kend, lane);
-        if (!__all_sync(0xffffffffu, mbar_wait(&pempty[ks], (seg & 1u) ^ 1u, p.status, 1, p.spin_limit))) return;
+        if (!__all_sync(0xffffffffu, mbar_wait(&pempty[ks], (seg & 1u) ^ 1u, p.status, 1, p.spin_limit))) {
+          copies_landed();
+          if (CF::MODEX == LM_TMA_K && ptid == 0) fills_landed(pfull, seg * nk + ks, nk, p.status, p.spin_limit);
+          return;
+        }
         double* xs = panel + ks * CF::XIMG;
         if constexpr (CF::MODEX == LM_TMA_K) {
           if (ptid == 0) {

@@ -39,6 +39,12 @@ namespace tck {
 __device__ __forceinline__ void mbar_arrive_on_copies(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
+// What a role has under way when one of its waits gives up must not outlive the shared memory it goes to: this thread's copies ...
+__device__ __forceinline__ void copies_landed() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+// ... and (with a limit again) the boxes of a ring's last fills before fill `it`.
+__device__ __forceinline__ void fills_landed(uint64_t* full, uint32_t it, uint32_t depth, int* status, uint32_t limit) {
+  for (uint32_t q = it > depth ? it - depth : 0u; q < it; ++q) mbar_wait(full + q % depth, (q / depth) & 1u, status, 2, limit);
+}
 // One arrival that also announces `bytes` of asynchronous (TMA) traffic for the current phase.
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}\n" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");

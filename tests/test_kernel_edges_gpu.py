@@ -396,3 +396,28 @@ def test_a_wait_of_the_pairs_that_gives_up(pkg):
         torch.cuda.synchronize()
         assert good.status() == 0 and _off(got, want) <= 1e-5
         good.close()
+
+
+# Output-resident kernels, panels and ring, whose waits run out (one stage is left unannounced): Y by copies of the threads,
+# by boxes, X by boxes; they end by themselves with the tiles of C that were on their way landed, and the next plan is right.
+GIVE_UP = [("C [a,24,b,16,c,16,d,24,e,16,f,16] -= sum(g,24) * A [d,e,g,a] * B [g,f,b,c];", {}, "dmma_wp_128x64", (False, False)),
+           ("C [a,48,b,64,c,40,d,80] += sum(e,40) * A [a,b,e] * B [e,c,d];", dict(tile=(128, 64), variant=4), "dmma_wp_128x64", (False, True)),
+           ("C [a,48,b,64,c,40,d,80] = sum(e,40) * A [e,a,b] * B [c,d,e];", dict(tile=(128, 64), variant=4), "dmma_wp_128x64", (True, False)),
+           ("C [a,48,b,64,c,40,d,20] += sum(e,40) * A [e,a,b] * B [e,c,d];", dict(tile=(128, 64), variant=4), "dmma_wc_128x64", (True, True)),
+           ("C [a,48,b,64,c,40,d,20] += sum(e,40) * A [a,e,b] * B [c,e,d];", dict(tile=(128, 32), variant=4), "dmma_wc_128x32", (False, False))]
+
+
+@pytest.mark.parametrize("expr,kw,runs,boxes", GIVE_UP)
+def test_resident_tiles_and_waits_that_give_up(pkg, orc, expr, kw, runs, boxes):
+    import torch
+    torch.cuda.set_device(0)
+    c0, a, b = (torch.from_numpy(x).cuda() for x in orc.make_inputs(expr, 14, "float64"))
+    bad = pkg.Plan(expr, test_fault=1, **kw)
+    d = bad.describe()
+    assert d["runs"] == runs and (d["tma_x"], d["tma_y"]) == boxes, d
+    bad.execute(c0.clone(), a, b)
+    torch.cuda.synchronize()          # returns: every wait is bounded
+    assert bad.status() in (1, 2, 3, 4, 5, 6) and bad.describe()["ran"] == runs
+    bad.close()
+    d, err = _run(pkg, orc, expr, seed=14, **kw)
+    assert d["runs"] == runs and err <= 1e-12, err
