@@ -670,21 +670,38 @@ extern "C" int tc_execute_noalloc(tc_plan* p, void* C, const void* A, const void
 #include <condition_variable>
 #include <deque>
 #include <map>
+#include <memory>
 #include <thread>
+#include <sched.h>
 
 namespace {
 
-// memcpy shared by a few persistent helper threads (one caller at a time per pool).
+// memcpy shared by helper threads.  One set of them per process, made when a plan first sees pageable memory and joined when the
+// last such plan is destroyed: every plan's copies, in and out, from any thread, take their helpers from it, so that neither
+// several plans nor a driver that makes plan after plan has more threads than the cores call for.
 class CopyPool {
  public:
-  explicit CopyPool(int n) {
-    for (int i = 0; i < n; ++i) workers_.emplace_back([this, i] { loop(i); });
+  static std::shared_ptr<CopyPool> get() {
+    static std::mutex mu;
+    static std::weak_ptr<CopyPool> kept;
+    std::lock_guard<std::mutex> l(mu);
+    std::shared_ptr<CopyPool> p = kept.lock();
+    if (!p) kept = p = std::make_shared<CopyPool>();
+    return p;
+  }
+  CopyPool() {
+    cpu_set_t set;
+    const int cores = sched_getaffinity(0, sizeof(set), &set) == 0 ? CPU_COUNT(&set) : (int)std::thread::hardware_concurrency();
+    const int n = std::min(12, std::max(1, cores - 2));  // (beside the caller and the thread that empties the buffers)
+    try {
+      for (int i = 0; i < n; ++i) workers_.emplace_back([this] { loop(); });
+    } catch (const std::exception&) {  // no more threads to be had: with those there are, or the callers alone
+    }
   }
   ~CopyPool() {
     {
       std::lock_guard<std::mutex> l(mu_);
       stop_ = true;
-      ++epoch_;
     }
     cv_.notify_all();
     for (std::thread& t : workers_) t.join();
@@ -692,52 +709,57 @@ class CopyPool {
   void copy(void* dst, const void* src, size_t bytes) {
     const size_t n = workers_.size();
     if (bytes < (1u << 20) || n == 0) { std::memcpy(dst, src, bytes); return; }
+    Job j = {static_cast<char*>(dst), static_cast<const char*>(src), bytes, ((bytes + n) / (n + 1) + 4095) / 4096 * 4096, 0, bytes, nullptr, nullptr};
     std::unique_lock<std::mutex> l(mu_);
-    dst_ = static_cast<char*>(dst);
-    src_ = static_cast<const char*>(src);
-    piece_ = ((bytes + n) / (n + 1) + 4095) / 4096 * 4096;
-    bytes_ = bytes;
-    pending_ = (int)n;
-    ++epoch_;
+    j.prev = last_;
+    (last_ ? last_->next : first_) = &j;
+    last_ = &j;
     l.unlock();
     cv_.notify_all();
-    part(n);  // the caller takes the last piece
     l.lock();
-    done_.wait(l, [this] { return pending_ == 0; });
+    while (j.at < j.bytes) take(&j, l);  // the caller copies too
+    done_.wait(l, [&] { return j.left == 0; });
   }
 
  private:
-  void part(size_t i) {
-    const size_t lo = std::min(bytes_, i * piece_), hi = std::min(bytes_, lo + piece_);
-    if (hi > lo) std::memcpy(dst_ + lo, src_ + lo, hi - lo);
+  struct Job {  // lives on its caller's stack until nothing of it is left
+    char* dst;
+    const char* src;
+    size_t bytes, piece, at, left;  // at: first byte that nobody has taken; left: bytes not copied yet
+    Job *prev, *next;
+  };
+  void take(Job* j, std::unique_lock<std::mutex>& l) {
+    const size_t lo = j->at, hi = std::min(j->bytes, lo + j->piece);
+    j->at = hi;
+    if (hi == j->bytes) {  // all of it is taken: out of the queue
+      (j->prev ? j->prev->next : first_) = j->next;
+      (j->next ? j->next->prev : last_) = j->prev;
+    }
+    l.unlock();
+    std::memcpy(j->dst + lo, j->src + lo, hi - lo);
+    l.lock();
+    j->left -= hi - lo;
+    if (j->left == 0) done_.notify_all();
   }
-  void loop(int i) {
-    uint64_t seen = 0;
+  void loop() {
+    std::unique_lock<std::mutex> l(mu_);
     for (;;) {
-      std::unique_lock<std::mutex> l(mu_);
-      cv_.wait(l, [&] { return epoch_ != seen; });
-      seen = epoch_;
+      cv_.wait(l, [&] { return stop_ || first_; });
       if (stop_) return;
-      l.unlock();
-      part((size_t)i);
-      l.lock();
-      if (--pending_ == 0) done_.notify_all();
+      take(first_, l);
     }
   }
   std::vector<std::thread> workers_;
   std::mutex mu_;
   std::condition_variable cv_, done_;
-  uint64_t epoch_ = 0;
   bool stop_ = false;
-  int pending_ = 0;
-  char* dst_ = nullptr;
-  const char* src_ = nullptr;
-  size_t piece_ = 0, bytes_ = 0;
+  Job *first_ = nullptr, *last_ = nullptr;  // jobs with bytes that nobody has taken
 };
 
-// Small buffers and all cores but a few: a copy over the link starts when its buffer is filled, so the first and the last
-// buffer are not overlapped with anything.  48^4 outputs and inputs (85 MB in, 42 MB out) on 16 cores: 9.0 ms with three
-// buffers of 8 MB and four helpers, 6.6 with twelve helpers, 4.9 with 2 MB and six, 4.0 with 2 MB and twelve.
+// Small buffers and many helpers: a copy over the link starts when its buffer is filled, so the first and the last buffer are
+// not overlapped with anything.  48^4 outputs and inputs (85 MB in, 42 MB out) on 16 cores, each direction with helpers of its
+// own: 9.0 ms with three buffers of 8 MB and four helpers, 6.6 with twelve, 4.9 with 2 MB and six, 4.0 with 2 MB and twelve.
+// Twelve for both directions together (in turn, medians): 48^4 3.7 -> 3.6 ms, 56^4 7.1 -> 6.5, 64^4 7.7 -> 6.9, 80^4 17.2 -> 15.1.
 // Calls that move more are bound by the host's memory and by the hand-over per piece, and take whole buffers (64^4, 268 MB
 // in: 10.5 ms in pieces of 2 MB, 9.5 in 4, 9.8 in 8; 96^4, 1.36 GB in: 51, 39, 47; with six or four helpers 42 to 52).
 constexpr size_t kBounceBytes = size_t(4) << 20, kShortPiece = size_t(2) << 20, kShortCall = size_t(192) << 20;
@@ -771,8 +793,7 @@ struct TcHostPipe {
   cudaEvent_t in_done[kBounceCount] = {};
   cudaEvent_t out_done[kBounceCount] = {};
   int in_next = 0;
-  CopyPool* pool_in = nullptr;
-  CopyPool* pool_out = nullptr;
+  std::shared_ptr<CopyPool> pool;
   std::vector<cudaEvent_t> slab_done;  // kernel of slab i finished (recorded on its stream)
   std::vector<cudaEvent_t> slab_in;    // inputs of slab i have arrived (page-locked callers: copies on their own stream)
 };
@@ -797,8 +818,6 @@ static void host_pipe_destroy(TcHostPipe* h) {
   }
   for (cudaEvent_t e : h->slab_done) cudaEventDestroy(e);
   for (cudaEvent_t e : h->slab_in) cudaEventDestroy(e);
-  delete h->pool_in;
-  delete h->pool_out;
   delete h;
 }
 
@@ -899,7 +918,7 @@ static int host_pipe_create(tc_plan* p) {
 
 // Bounce buffers, helper threads and the drain stream: only plans that ever see pageable memory pay for them.
 static int host_pipe_enable_staging(TcHostPipe* h) {
-  if (h->pool_in) return TC_OK;
+  if (h->pool) return TC_OK;
   for (int i = 0; i < kBounceCount; ++i) {
     TC_CUDA_OK(cudaMallocHost(&h->bounce_in[i], kBounceBytes));
     TC_CUDA_OK(cudaMallocHost(&h->bounce_out[i], kBounceBytes));
@@ -907,10 +926,11 @@ static int host_pipe_enable_staging(TcHostPipe* h) {
     TC_CUDA_OK(cudaEventCreateWithFlags(&h->out_done[i], cudaEventDisableTiming));
   }
   TC_CUDA_OK(cudaStreamCreateWithFlags(&h->out_stream, cudaStreamNonBlocking));
-  const unsigned hw = std::max(2u, std::thread::hardware_concurrency());
-  const int helpers = (int)std::min(12u, std::max(1u, hw - 2));
-  h->pool_in = new CopyPool(helpers);
-  h->pool_out = new CopyPool(helpers);
+  try {
+    h->pool = CopyPool::get();
+  } catch (const std::exception&) {
+    return TC_ERR_INVALID_ARG;
+  }
   return TC_OK;
 }
 
@@ -925,7 +945,7 @@ static int copy_in(TcHostPipe* h, char* dst, const char* src, size_t bytes, bool
     const int b = h->in_next;
     h->in_next = (b + 1) % kBounceCount;
     TC_CUDA_OK(cudaEventSynchronize(h->in_done[b]));  // the copy that last used this buffer has read it
-    h->pool_in->copy(h->bounce_in[b], src + off, n);
+    h->pool->copy(h->bounce_in[b], src + off, n);
     TC_CUDA_OK(cudaMemcpyAsync(dst + off, h->bounce_in[b], n, cudaMemcpyHostToDevice, s));
     TC_CUDA_OK(cudaEventRecord(h->in_done[b], s));
   }
@@ -963,7 +983,7 @@ struct Drain {
       }
       const int b = bd % kBounceCount;
       TC_CUDA_OK(cudaEventSynchronize(h->out_done[b]));
-      h->pool_out->copy(j.dst + drained, h->bounce_out[b], len[b]);
+      h->pool->copy(j.dst + drained, h->bounce_out[b], len[b]);
       drained += len[b];
       ++bd;
     }

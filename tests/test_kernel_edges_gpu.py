@@ -421,3 +421,39 @@ def test_resident_tiles_and_waits_that_give_up(pkg, orc, expr, kw, runs, boxes):
     bad.close()
     d, err = _run(pkg, orc, expr, seed=14, **kw)
     assert d["runs"] == runs and err <= 1e-12, err
+
+
+def test_helper_threads_are_one_set_for_all_plans(pkg, orc):
+    """Pageable host arrays: the helpers that share the copies belong to the process, not to each plan, and go with the last
+    plan that used them.  Two plans at once, from two threads, each checked."""
+    import threading
+    import numpy as np
+    import torch
+    torch.cuda.set_device(0)
+    tasks = lambda: len(__import__("os").listdir("/proc/self/task"))
+    exprs = ["C [a,128,b,96,c,40,d,10] %s sum(e,6) * A [a,e,b,d] * B [e,c];" % op for op in ("+=", "-=")]  # 39 MB of output: slabs
+    data = [orc.make_inputs(e, 15 + n, "float64") for n, e in enumerate(exprs)]
+    refs = [orc.contract(e, c.copy(), a, b) for e, (c, a, b) in zip(exprs, data)]
+    with_threads = pkg.Plan(exprs[0])                      # whatever the driver starts for itself is there after this
+    with_threads.execute_host(data[0][0].copy(), *data[0][1:])
+    with_threads.close()
+    start = tasks()
+    plans = [pkg.Plan(e) for e in exprs]
+    got = [[c.copy() for _ in range(3)] for c, _, _ in data]
+
+    def work(n):
+        for c in got[n]:
+            plans[n].execute_host(c, *data[n][1:])
+
+    callers = [threading.Thread(target=work, args=(n,)) for n in range(2)]
+    for t in callers:
+        t.start()
+    for t in callers:
+        t.join()
+    assert tasks() - start <= 12, (start, tasks())
+    plans[0].close()
+    plans[1].close()
+    assert tasks() <= start, (start, tasks())
+    for ref, results in zip(refs, got):
+        for c in results:
+            assert np.abs(c - ref).max() <= 1e-12 * np.abs(ref).max()
