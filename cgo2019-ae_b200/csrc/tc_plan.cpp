@@ -772,11 +772,16 @@ int tc_plan_build(tc_plan* p, std::string* why) {
         // step, 1.2 us a step where both operands load by vector and 2 to 5 where one is gathered, however little of the
         // GPU its tiles fill; the persistent 128 x 32 kernels run ahead (two tiles per SM at 1.15 us a step, 1.35 where
         // both have one and twice that where X is gathered across its sectors; the resident form, one per SM, 0.8).
-        // From five steps and 32 tiles on and up to one round of them: 35 sums, 1.1 to 2.4 times as fast (1088 x 688 x 436
+        // From five steps and 32 tiles on and up to one round of them: 195 sums, 1.0 to 2.5 times as fast (1088 x 688 x 436
         // 62 -> 40 us; 19800 x 19 x 120, gathered, 42 -> 19); below that within 15 % either way, beyond 8 % slower (374).
+        // Up to a hundred tiles of five to seven steps the one-tile kernel has as little to wait for where both operands and C
+        // are read by 16 bytes (6400 x 22 x 68 8.0 against 10.2 us) or where an odd X is read along its fastest index and C only
+        // written (1121 x 219 x 68 12.7 against 16.4).
         const int64_t t32 = ((mf + 127) / 128) * ((nf + 31) / 32);
+        const bool short_waits = t32 * 3 < 2 * sms && ((steps < 7 && c.vec_x && c.vec_y && a.vec_c == 4) ||
+                                                       (steps < 8 && e.op == 0 && a.lanes_k_x == 1 && !c.vec_x && a.M.s_in[0] == 1));
         if (c.math == TC_MATH_DMMA && p->opt.split_k == 0 && p->opt.variant == 0 && p->opt.c_path == 0 && p->opt.tma == 0 && steps >= 5 && t32 >= 32 && t32 <= 2 * sms &&
-            !(t64 * 2 <= sms && steps >= 16)) {
+            !short_waits && !(t64 * 2 <= sms && steps >= 16)) {
           // (lanes on M's first index read neighbours where that is X's fastest too, only an odd one: 979 x 1032 x 263
           // 47 -> 40 us, 617 x 1840 x 281 49 -> 42)
           const bool across = a.lanes_k_x == 1 && !c.vec_x && a.M.s_in[0] != 1;

@@ -535,3 +535,33 @@ def test_a_named_kernel_is_the_one_that_runs(pkg):
     assert d["panel"] and d["runs"] == "dmma_wp_128x64", d
     d = _plan(pkg, six, tile=(128, 64), variant=4, tma=1).describe()   # no boxes of the output: the reduce-add kernel
     assert d["runs"] == "dmma_ws_128x64" and d["kernel"] == "dmma_wc_128x64", d
+
+
+# fp64 sums of few tiles that are not sliced: on the persistent 128 x 32 kernels, but for short waits (times in us on those and
+# on the one-tile kernel).
+@pytest.mark.parametrize("form,op,runs", [
+    (((1088, 688), 436, "a,c", "c,b"), "+=", "dmma_w"),                # 40, 62
+    (((786, 160), 67, "a,c", "c,b"), "+=", "dmma_w"),                  # 8.2, 13.7: C in pairs
+    (((529, 496), 70, "a,c", "c,b"), "+=", "dmma_w"),                  # 12.3, 23.2: odd, added to C
+    (((1121, 219), 68, "a,c", "b,c"), "=", "dmma_64x64"),              # 16.4, 12.7: odd, only written
+    (((115, 1008), 105, "a,c", "b,c"), "=", "dmma_64x64"),             # 16.4, 13.9
+    (((392, 240), 92, "a,c", "b,c"), "=", "dmma_64x64"),               # 10.3, 9.1: 16-byte loads and stores
+    (((392, 240), 120, "a,c", "b,c"), "=", "dmma_w"),                  # ... two steps more
+    (((1088, 688), 60, "a,c", "c,b"), "+=", "dmma_64x64"),             # four steps
+])
+def test_few_tiles_on_the_narrow_persistent_kernels(pkg, form, op, runs):
+    (m, n), k, left, right = form
+    d = _plan(pkg, "C [a,%d,b,%d] %s sum(c,%d) * A [%s] * B [%s];" % (m, n, op, k, left, right)).describe()
+    assert d["runs"].startswith(runs) and d["ksplit"] == 1 and d["workspace_bytes"] == 0, d
+    if runs == "dmma_w":
+        assert d["runs_tile"] == [128, 32], d
+
+
+# fp32 without any alignment: tcgen05, one tile per CTA, but for few columns or few rows.
+@pytest.mark.parametrize("extents,k,runs", [((55, 31, 39, 39), 61, "tf32tc_128x128"), ((1641, 11, 23, 9), 61, "tf32tc_128x128"),
+                                            ((57, 31, 39, 29), 63, "tf32_64x64"), ((333, 333, 7, 9), 41, "tf32_64x64")])
+def test_fp32_without_alignment(pkg, extents, k, runs):
+    out = ",".join("%s,%d" % x for x in zip("abcd", extents))
+    left, right = ("e,a", "e,b,c,d") if extents[0] < 64 and extents[0] != 55 else ("a,b,e", "e,c,d")
+    d = _plan(pkg, "C [%s] += sum(e,%d) * A [%s] * B [%s];" % (out, k, left, right), "float32").describe()
+    assert d["vec_c"] == 1 and not (d["vec_x"] or d["kvec_x"] or d["vec_y"] or d["kvec_y"]) and d["runs"] == runs, d
