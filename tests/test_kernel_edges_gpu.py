@@ -457,3 +457,15 @@ def test_helper_threads_are_one_set_for_all_plans(pkg, orc):
     for ref, results in zip(refs, got):
         for c in results:
             assert np.abs(c - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+# Epilogues of the one-tile kernels: few columns of a tile (groups of eight and sixteen outside the tensor), even rows whose
+# pairs leave by 16 bytes, odd ones that do not, on tiles that are full and ragged.
+@pytest.mark.parametrize("op", ["=", "+=", "-="])
+@pytest.mark.parametrize("dtype,tile,kernel", [("float64", (64, 64), "dmma_64x64_w4"), ("float64", (64, 96), "dmma_64x96_w4"), ("float32", (64, 64), "tf32_64x64")])
+@pytest.mark.parametrize("m,n", [(58, 8), (58, 9), (59, 16), (130, 17), (131, 49), (22, 73), (66, 111)])
+def test_one_tile_epilogues_on_few_columns(pkg, orc, op, dtype, tile, kernel, m, n):
+    expr = "C [a,%d,b,%d,c,3] %s sum(d,23) * A [d,a,c] * B [b,d];" % (m, n, op)
+    d, err = _run(pkg, orc, expr, seed=16, dtype=dtype, tile=tile, variant=1)
+    assert d["runs"] == kernel and d["vec_c"] == 2 - m % 2, d
+    assert err <= (1e-12 if dtype == "float64" else 1e-5), err
