@@ -19,10 +19,12 @@
 //   warp 17     MMA       (first CTA of the pair) waits until both CTAs' images are written, issues, commits to both.
 //   warps 18-19 no work.
 //
-// Measured (one B200, against the kernels these problems ran on before): 4096 x 4096 x 2048 554 -> 314 us (219 TFLOP/s; the
-// MMAs alone take 207 in four rounds of 74 tiles, 181 with the last one halved), x 512 148 -> 118 with the first form; 720 x
-// 2064 x 3664 365 -> 133, 1496 x 1120 x 400 42 -> 25.  With the copies, the conversion or two of the three MMAs taken out in
-// turn 4096 x 4096 x 2048 took 279, 320 and 357 of the 361 us it stood at: what is left is all three meeting in 227 KB.
+// Measured (one B200, against the kernels these problems ran on before): 4096 x 4096 x 2048 554 -> 314 us in short runs (219
+// TFLOP/s; the MMAs alone take 207 in four rounds of 74 tiles, 181 with the last one halved) and 555 -> 352 in long ones, under
+// the board's power cap; 720 x 2064 x 3664 365 -> 133, 1496 x 1120 x 400 42 -> 25; 80 matrices of 200 to 4096 rows and
+// columns, K = 256 to 4096, 0.99 to 6.6 times as fast, 2.4 in the mean.  With the copies, the conversion or two of the three
+// MMAs taken out in turn 4096 x 4096 x 2048 took 279, 320 and 357 of the 361 us it stood at: what is left is all three meeting
+// in 227 KB.  Bulk reduce-adds keep subnormal sums; adding to C in registers was 1 to 19 % slower.
 //
 // Barriers that both CTAs arrive on live in the first CTA (arrivals of the second go there through the cluster's shared
 // memory); commits arrive on both CTAs' barriers.  Neither CTA leaves before the other has finished (cluster barrier), and
