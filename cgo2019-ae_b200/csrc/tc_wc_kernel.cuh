@@ -167,15 +167,12 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
     Corner here = corner(0), after = corner(1);
     if (ntiles > 0) fetch(0, here);
     if (ntiles > 1) fetch(1, after);
-    for (uint32_t j = 0; j < ntiles; ++j) {
+    uint32_t j = 0;
+    for (; j < ntiles; ++j) {
       const uint32_t b = j & 1u;
       const Corner next = corner(j + CF::CBUFS);
       const int(&c)[5] = here.c;
-      if (!mbar_wait(&c_staged[b], (j >> 1) & 1u, p.status, 6, p.spin_limit)) {  // the tiles on their way into both buffers land first
-        for (uint32_t q = j; q < ntiles && q < j + CF::CBUFS; ++q) mbar_wait(&c_ready[q & 1u], (q >> 1) & 1u, p.status, 6, p.spin_limit);
-        asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
-        return;
-      }
+      if (!mbar_wait(&c_staged[b], (j >> 1) & 1u, p.status, 6, p.spin_limit)) break;
       asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4, %5}], [%6];\n" ::"l"(tmap),
                    "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(smem_u32(cbufs + b * CF::CTILE_ELEMS))
                    : "memory");
@@ -187,6 +184,9 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
       here = after;
       after = next;
     }
+    // After a wait that gave up the tiles on their way into both buffers land first.  (The fetching warps have waited long enough for
+    // their copies when their own wait gives up; code for it in their loops cost kernels of 20 us 3 to 6 %.)
+    for (uint32_t q = j; q < ntiles && q < j + CF::CBUFS; ++q) mbar_wait(&c_ready[q & 1u], (q >> 1) & 1u, p.status, 6, p.spin_limit);
     asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
     return;
   }
@@ -218,12 +218,7 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_wc_dmma_kernel(const __
         const uint32_t s = it % STAGES;
         const int64_t nx = ws_koff(p.koff_x, (uint32_t)(ks + 1) * BK, kend, ptid), ny = ws_koff(p.koff_y, (uint32_t)(ks + 1) * BK, kend, ptid);
         // (one decision per warp: the loaders below shuffle)
-        if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.status, 2, p.spin_limit))) {
-          copies_landed();
-          if (CF::ANY_TMA && ptid == 0) fills_landed(full, it, STAGES, p.status, p.spin_limit);
-          for (uint32_t t = tile + step; t < total; t += step) group_bar_sync(1, CF::THREADS);  // the others may not have given up
-          return;
-        }
+        if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.status, 2, p.spin_limit))) return;
         double* xs = stages + s * CF::STAGE_ELEMS;
         double* ys = xs + CF::XIMG;
         const uint32_t k0 = (uint32_t)ks * BK;
