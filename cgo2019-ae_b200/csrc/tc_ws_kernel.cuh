@@ -441,11 +441,12 @@ __global__ void __launch_bounds__(CF::CTA_THREADS, 1) tc_ws_dmma_kernel(const __
   constexpr int MB2 = WM / 16, NB2 = WN / 16;
   // The second group's warps take the tile's blocks in the opposite order: at a ragged edge, where some blocks have less to
   // do, every scheduler then has one warp of each kind (one-index terms with 45 of 64 columns 61.5 -> 53.3 and 64.0 -> 58.2
-  // us, 96^4 545 -> 540; K slices, whose groups are on different tiles, 1 % slower).  Where Y comes in boxes, by the warp's
-  // number alone: told apart by slices too, the places that follow from it stayed in registers through the product loop,
-  // which spilled (59 of 64 columns, X by vector, 123 -> 128 us; the other instances run 1 to 3 % slower this way).
+  // us, 96^4 545 -> 540; K slices, whose groups are on different tiles, 1 % slower).  In three instances by the warp's number
+  // alone: told apart by slices too, the places that follow from it stayed in registers through the product loop, which
+  // spilled there (128 x 64, X by vector, Y in boxes, 59 of 64 columns 123 -> 128 us; the others run 1 to 3 % slower this way).
+  constexpr bool BY_WARP = CF::MODEY == LM_TMA_K && (BN == 64 ? CF::MODEX != LM_K_VEC : BM == 64 && CF::MODEX == LM_K_VEC);
   const int lane = tid & 31;
-  const int cw = CF::MODEY == LM_TMA_K ? (warp < CW ? warp : 2 * CW - 1 - warp) : gi == 1 && !sliced ? CW - 1 - warp % CW : warp % CW;
+  const int cw = BY_WARP ? (warp < CW ? warp : 2 * CW - 1 - warp) : gi == 1 && !sliced ? CW - 1 - warp % CW : warp % CW;
   const int g = lane >> 2, t = lane & 3;
   const int wm0 = (cw % CF::WGM) * WM, wn0 = (cw / CF::WGM) * WN;
   const double alpha = p.alpha;
