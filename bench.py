@@ -70,6 +70,7 @@ NCU_TRAFFIC_BYTES = {
     ("dmma_ws_64x96", "cfg2"): 1984793088, ("dmma_ws_128x64", "cfg3"): 1341919744, ("tf32tc_96x128", "cfg4"): 1472193280, ("tf32wt_96x128", "cfg4"): 1475021824,
     ("dmma_ws_128x64", "cfg5_shard8"): 8369612032, ("dmma_ws_128x64", "cfg5"): 8 * 8369612032,
     ("dmma_wc_128x64", "cfg5_shard8"): 8197418496, ("dmma_wc_128x64", "cfg5"): 8 * 8197418496,
+    ("dmma_wp_128x64", "cfg5_shard8"): 8168777216, ("dmma_wp_128x64", "cfg5"): 8 * 8168777216,
 }
 
 
@@ -306,7 +307,7 @@ def quick_config(pkg, orc, torch, name, steps=5, path="auto", cogent=False, labe
     del dc, da, db
     torch.cuda.empty_cache()
     row = {"workload": name, "dtype": dtype, "path": label or path, "gflops": flops * steps / sec * 1e-9, "ms": sec / steps * 1e3,
-           "algorithmic_gbs": nbytes * steps / sec * 1e-9, "kernel": d["kernel"], "device_status": status}
+           "algorithmic_gbs": nbytes * steps / sec * 1e-9, "kernel": d["runs"], "device_status": status}
     if cogent:
         extra = cogent_kernel_gflops(name, orc, flops)
         if extra:
@@ -502,7 +503,7 @@ def run_tccg(args):
         st = plan.status()
         pipe = peaks["dmma_m8n8k4"] if dtype == "f64" else peaks["ffma"]
         t_roof = max(d["bytes"] / (hbm_peak * 1e9), d["flops"] / (pipe * 1e12))
-        row = {"tag": it["tag"], "dtype": dtype, "kernel": d["kernel"], "ms": sec * 1e3, "gflops": d["flops"] / sec * 1e-9,
+        row = {"tag": it["tag"], "dtype": dtype, "kernel": d["runs"], "ms": sec * 1e3, "gflops": d["flops"] / sec * 1e-9,
                "algorithmic_gbs": d["bytes"] / sec * 1e-9, "of_roofline": t_roof / sec, "device_status": st,
                "tma": [d.get("tma_x"), d.get("tma_y"), d.get("tma_c"), d.get("tma_ct")]}
         for k in ("cogent_v100_gflops", "cogent_p100_gflops", "nwchem_v100_gflops"):
@@ -573,7 +574,7 @@ def run_fused(args):
                       "n_gpus": 1, "dtype": "f64", "fused": {"gflops": d["flops"] / t_f * 1e-9, "ms": t_f * 1e3, "launches": 1,
                                                                "algorithmic_bytes": d["bytes"], "kernel": d["kernel"], "box": d["box"]},
                       "term_by_term": {"gflops": d["flops"] / t_s * 1e-9, "ms": t_s * 1e3, "launches": 9,
-                                       "algorithmic_bytes": d["bytes_term_by_term"], "kernel": plans[0].describe()["kernel"]},
+                                       "algorithmic_bytes": d["bytes_term_by_term"], "kernel": plans[0].describe()["runs"]},
                       "parity": {"max_rel_err": worst, "tolerance": 1e-12, "ok": bool(worst <= 1e-12),
                                  "how": "two slabs of the fused result against the nine loop nests applied in order"}}))
 
@@ -723,9 +724,9 @@ def run_ours(args):
     roof["frac"] = roof["achieved"] / roof["peak"]
     # per launch, from one ncu capture of THIS kernel on this workload (null when the plan picked another kernel,
     # another arithmetic path, or the shard is not a captured size)
-    key = (desc["kernel"], name if world == 1 else ("cfg5_shard8" if (name, world) == ("cfg5", 8) else None))
+    key = (desc["runs"], name if world == 1 else ("cfg5_shard8" if (name, world) == ("cfg5", 8) else None))
     roof["traffic"] = NCU_TRAFFIC_BYTES.get(key) if args.path == "auto" else None
-    roof["kernel"] = desc["kernel"]
+    roof["kernel"] = desc["runs"]
     roof["algorithmic_bytes_per_launch"] = shard_bytes
     roof["algorithmic_flops_per_launch"] = shard_flops
     roof["hbm"] = {"achieved": shard_bytes / launch_s * 1e-9, "peak": hbm_peak, "unit": "GB/s",
@@ -738,7 +739,7 @@ def run_ours(args):
         "warmup": max(args.warmup, 3), "ms_per_step": sec / args.steps * 1e3, "higher_is_better": True,
         "scaling": "strong", "vs_baseline": None, "dtype": dtype, "data": "synthetic",
         "config": config_of(name, expr, seed, g.index, world, shard_bytes),
-        "plan": {k: desc[k] for k in ("kernel", "math", "tile", "tiles", "ksplit", "vec_c")},
+        "plan": {k: desc[k] for k in ("kernel", "runs", "math", "tile", "tiles", "ksplit", "vec_c")},
         "roofline": roof,
         "parity": parity,
         "e2e": {"value": e2e_value, "unit": "GFLOP/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": slab_bytes,
